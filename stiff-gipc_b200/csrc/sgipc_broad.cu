@@ -8,14 +8,24 @@
 // four-vertex pairs); _GroundCollisionDetect (GIPC.cu:6433) lists the surface points near the
 // ground.  The reference appends with atomics, so its order changes from run to run.
 //
-// Here a uniform grid replaces the trees.  The cell is wider than any triangle or edge box
-// grown by the contact gap sqrt(d-hat), so each grown box covers at most 2 x 2 x 2 cells; the
-// (cell, primitive) keys are radix-sorted once per call and a query binary-searches its cells.
-// A point visits its own cell; an edge visits the cells of its grown box and reports a pair
-// only in the cell holding the low corner of the two boxes' overlap, so every pair is found
-// once.  Two passes (count, exclusive scan, write) give a deterministic order: point-triangle
-// pairs by surface point, then by triangle; edge-edge pairs by (edge, other edge), sorted after
-// the write.  MatIndex is the rank in that order.  The pair tests restate the reference's
+// Here two packed trees of fan-out 32 replace them.  The triangles, the edges and the surface
+// points are sorted together by the Morton code of their box centres (one radix sort); 32
+// consecutive primitives form a leaf group, 32 groups a node, and a box is stored for every
+// primitive, group and node: there is no tree to build, only the boxes to reduce.  A warp takes
+// 32 neighbouring queries (points against triangles, edges against the edges behind them in
+// the sorted order) and walks the nodes and groups whose box meets the union of its queries'
+// boxes, one child per lane; the pairs of groups are then shared out evenly, one per warp: the
+// primitives that meet a query's own box are queued, and every 32 queued candidates are tested
+// exactly, one per lane.  Boxes are FP32, rounded outwards, so
+// that they only ever let more candidates through; every decision is made in FP64.  (The
+// search was a uniform grid before, its cell as wide as the scene's largest primitive, with
+// one thread per query and two passes: with small primitives beside large ones a cell held
+// hundreds of candidates, and the exact test ran in whichever lane had found one.)
+//
+// The records found are 64-bit keys (kind, query, primitive) and sorted once, which gives a
+// deterministic order: point-triangle pairs by surface point, then by triangle; edge-edge pairs
+// by (edge, other edge); then the ground points.  The pairs are encoded from the sorted keys,
+// and MatIndex is the rank in that order.  The pair tests restate the reference's
 // closest-feature classification and squared distances term for term; this file is compiled
 // without contracting multiply-adds (-fmad=false), so a pair at the edge of d-hat, or of a
 // feature region, is decided as the reference's own arithmetic decides it.
@@ -33,29 +43,22 @@ namespace sgipc {
 
 // per-context buffers of the pair search (grown when a call needs more)
 struct BroadWork {
-    int cap_tri = 0, cap_edge = 0, cap_q = 0, cap_rec = 0, cap_sv = 0;
-    unsigned long long* tkey = nullptr;    // [8 * faces] cell keys of the grown triangle boxes
-    unsigned long long* tkey_s = nullptr;
-    int* tval = nullptr;
-    int* tval_s = nullptr;
-    unsigned long long* ekey = nullptr;    // [8 * edges]
-    unsigned long long* ekey_s = nullptr;
-    int* eval = nullptr;
-    int* eval_s = nullptr;
-    unsigned long long* bounds = nullptr;  // [8] ordered min xyz, max xyz, largest box extent
-    double* grid = nullptr;                // [6] origin xyz, cell size, contact gap, error flag
-    int* counts = nullptr;                 // [queries + 1]
-    int* offs = nullptr;                   // [queries + 1]
-    int* gflag = nullptr;                  // [surface points + 1]
+    int cap_prim = 0, cap_leaf = 0, cap_item = 0, cap_rec = 0, cap_q = 0;
+    unsigned* key = nullptr;               // [primitives] kind and Morton code
+    unsigned* key_s = nullptr;
+    int* val = nullptr;                    // [primitives] index within its kind
+    int* val_s = nullptr;
+    float4* leaf = nullptr;                // [2 * leaves] boxes in sorted order: (lo, index), (hi, -)
+    float4* group = nullptr;               // [2 * leaves / 32]
+    float4* node = nullptr;                // [2 * leaves / 1024]
+    int2* item = nullptr;                  // [2 * items] query group and leaf group that meet
+    unsigned long long* bounds = nullptr;  // [8] ordered min xyz, max xyz, largest box extent, bad index
+    int* gflag = nullptr;                  // [pairs + 1] friction set-up: takes part, and its place
     int* goff = nullptr;
-    unsigned long long* reckey = nullptr;  // [records] (edge << 32 | other edge) of edge-edge records
+    unsigned long long* reckey = nullptr;  // [records] kind, query, primitive
     unsigned long long* reckey_s = nullptr;
-    int* recidx = nullptr;
-    int* recidx_s = nullptr;
-    int4* rec_pair = nullptr;              // unsorted edge-edge records
-    int4* rec_ccd = nullptr;
     unsigned long long* gscan = nullptr;   // [records] packed ranks per Hessian size
-    unsigned int* d_counts = nullptr;      // [4] pairs, point-triangle pairs, ground pairs, grid error
+    unsigned int* d_counts = nullptr;      // [16] see Count
     unsigned int* h_counts = nullptr;      // pinned copy
     void* cub = nullptr;
     size_t cub_bytes = 0;
@@ -68,9 +71,13 @@ using namespace sgipc;
 namespace {
 
 constexpr int kCellBits = 21;
-constexpr unsigned long long kNoKey = ~0ull;
 constexpr int kGroupBits = 21;  // packed rank fields: three 21-bit counters in one 64-bit word
-constexpr int kQueryThreads = 128;
+constexpr int kQueryWarps = 4;
+constexpr int kQueryCtas = 4;  // per SM (128 registers a thread)
+constexpr int kNodeLeaves = 1024;  // primitives below a node: 32 groups of 32
+// d_counts: records, ground points, scene error, pairs per Hessian size, edge and point items
+enum Count { kCntRec = 0, kCntGround = 2, kCntBad = 3, kCntSize = 4, kCntItem = 8, kCntNum = 16 };
+constexpr int kItemsPerGroup = 64;  // items of one kind the lists hold per query group, on average
 
 // order-preserving map of doubles to unsigned integers (min / max by integer atomics)
 __device__ __forceinline__ unsigned long long ord(double v) {
@@ -82,6 +89,8 @@ __device__ __forceinline__ double unord(unsigned long long u) {
 }
 
 __device__ __forceinline__ d3 ldp(const double* x, unsigned v) { return {x[3 * v], x[3 * v + 1], x[3 * v + 2]}; }
+
+constexpr int kBoundsWarps = 8;
 
 // scene bounds of the surface points and the largest extent of a triangle or edge box;
 // bounds[7] != 0 when an index names no vertex (nothing is loaded from such an index)
@@ -113,45 +122,37 @@ __global__ void k_bounds(const double* __restrict__ x, int nv, const unsigned* _
             ext = fmax(ext, fmax(fmax(a.z, b.z), c.z) - fmin(fmin(a.z, b.z), c.z));
         }
     }
+    // one atomic per value and CTA
+    __shared__ double s_red[kBoundsWarps][7];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double v[7] = {lo[0], lo[1], lo[2], -hi[0], -hi[1], -hi[2], -ext};  // all minima
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int q = 0; q < 7; q++) {
 #pragma unroll
-        for (int q = 0; q < 3; q++) {
-            lo[q] = fmin(lo[q], __shfl_xor_sync(0xffffffffu, lo[q], o));
-            hi[q] = fmax(hi[q], __shfl_xor_sync(0xffffffffu, hi[q], o));
-        }
-        ext = fmax(ext, __shfl_xor_sync(0xffffffffu, ext, o));
+        for (int o = 16; o > 0; o >>= 1) v[q] = fmin(v[q], __shfl_xor_sync(0xffffffffu, v[q], o));
+        if (lane == 0) s_red[w][q] = v[q];
     }
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            atomicMin(bounds + q, ord(lo[q]));
-            atomicMax(bounds + 3 + q, ord(hi[q]));
-        }
-        atomicMax(bounds + 6, ord(ext));
+    __syncthreads();
+    if (threadIdx.x < 7) {
+        double m = s_red[0][threadIdx.x];
+        for (int k = 1; k < kBoundsWarps; k++) m = fmin(m, s_red[k][threadIdx.x]);
+        if (threadIdx.x < 3) atomicMin(bounds + threadIdx.x, ord(m));
+        else atomicMax(bounds + threadIdx.x, ord(-m));
     }
 }
 
-// cell size and origin; grid[5] = 1 when the scene needs more than 2^21 cells along an axis,
-// 2 when an index names no vertex (every later kernel then returns at once)
-__global__ void k_grid(const unsigned long long* bounds, double gap, double* grid) {
+// 1 when the scene spans more than 2^21 times its largest primitive along an axis (or is not
+// finite), 2 when an index names no vertex (every later kernel then returns at once)
+__device__ int scene_error(const unsigned long long* bounds, double gap) {
     const double ext = unord(bounds[6]);
     const double h = (ext + 2.0 * gap) * 1.001 + 1e-12;
     int bad = 0;
 #pragma unroll
     for (int q = 0; q < 3; q++) {
         const double lo = unord(bounds[q]), hi = unord(bounds[3 + q]);
-        grid[q] = lo - gap - h;
-        if (!(hi >= lo) || (hi - grid[q]) / h + 2.0 >= (double)(1 << kCellBits)) bad = 1;
+        if (!(hi >= lo) || (hi - (lo - gap - h)) / h + 2.0 >= (double)(1 << kCellBits)) bad = 1;
     }
-    grid[3] = h;
-    grid[4] = gap;
-    grid[5] = bounds[7] ? 2 : bad;
-}
-
-__device__ __forceinline__ int cell_of(double v, double o, double h) { return (int)floor((v - o) / h); }
-__device__ __forceinline__ unsigned long long cell_key(int i, int j, int k) {
-    return (unsigned long long)i | ((unsigned long long)j << kCellBits) | ((unsigned long long)k << (2 * kCellBits));
+    return bounds[7] ? 2 : bad;
 }
 
 // grown box of a triangle (grow = gap) or an edge (grow = gap / 2)
@@ -168,32 +169,117 @@ __device__ __forceinline__ Box grown_box(const double* x, const unsigned* v, int
     return {{lo.x - grow, lo.y - grow, lo.z - grow}, {hi.x + grow, hi.y + grow, hi.z + grow}};
 }
 
-// keys of the (at most 8) cells a grown box covers; unused slots get kNoKey
-__global__ void k_insert(const double* __restrict__ x, const unsigned* __restrict__ prim, int n, int nvert,
-                         const double* __restrict__ grid, unsigned long long* key, int* val) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n || grid[5] != 0.0) return;
-    const double h = grid[3], gap = grid[4];
-    const Box b = grown_box(x, prim + (size_t)nvert * p, nvert, nvert == 3 ? gap : 0.5 * gap);
-    const int i0 = cell_of(b.lo.x, grid[0], h), j0 = cell_of(b.lo.y, grid[1], h), k0 = cell_of(b.lo.z, grid[2], h);
-    const int i1 = cell_of(b.hi.x, grid[0], h), j1 = cell_of(b.hi.y, grid[1], h), k1 = cell_of(b.hi.z, grid[2], h);
-#pragma unroll
-    for (int s = 0; s < 8; s++) {
-        const int i = i0 + (s & 1), j = j0 + ((s >> 1) & 1), k = k0 + (s >> 2);
-        key[8 * (size_t)p + s] = (i <= i1 && j <= j1 && k <= k1) ? cell_key(i, j, k) : kNoKey;
-        val[8 * (size_t)p + s] = p;
-    }
+// ten bits, spread to every third
+__device__ __forceinline__ unsigned spread3(unsigned v) {
+    v = (v | (v << 16)) & 0x030000ffu;
+    v = (v | (v << 8)) & 0x0300f00fu;
+    v = (v | (v << 4)) & 0x030c30c3u;
+    return (v | (v << 2)) & 0x09249249u;
 }
 
-// first index in sorted keys [0, n) not below k
-__device__ __forceinline__ int lower_bound(const unsigned long long* __restrict__ keys, int n, unsigned long long k) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(keys + mid) < k) lo = mid + 1;
-        else hi = mid;
+// Sort keys: kind (0 triangle, 1 edge, 2 surface point) above the 30-bit Morton code of the
+// box centre in the scene's bounds.  Ten bits an axis: finer codes sort no better (primitives of
+// one code stay in mesh order, which is local) and cost a radix pass each.
+__global__ void k_keys(const double* __restrict__ x, const unsigned* __restrict__ faces, int nf,
+                       const unsigned* __restrict__ edges, int ne, const unsigned* __restrict__ sv, int nsv,
+                       const unsigned long long* __restrict__ bounds, double gap, unsigned* __restrict__ key,
+                       int* __restrict__ val, unsigned* __restrict__ counts) {
+    __shared__ int s_bad;
+    __shared__ double s_lo[3], s_scale[3];
+    if (threadIdx.x == 0) {
+        s_bad = scene_error(bounds, gap);
+        if (blockIdx.x == 0) counts[kCntBad] = (unsigned)s_bad;
     }
-    return lo;
+    if (threadIdx.x < 3) {
+        const double lo = unord(bounds[threadIdx.x]), hi = unord(bounds[3 + threadIdx.x]);
+        s_lo[threadIdx.x] = lo;
+        s_scale[threadIdx.x] = hi > lo ? 1024.0 / (hi - lo) : 0.0;
+    }
+    __syncthreads();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nf + ne + nsv || s_bad) return;
+    const int kind = i < nf ? 0 : (i < nf + ne ? 1 : 2);
+    const int p = i - (kind > 0 ? nf : 0) - (kind > 1 ? ne : 0);
+    const unsigned* v = kind == 0 ? faces + 3 * (size_t)p : (kind == 1 ? edges + 2 * (size_t)p : sv + p);
+    const Box b = grown_box(x, v, 3 - kind, 0.0);
+    const double c[3] = {0.5 * (b.lo.x + b.hi.x), 0.5 * (b.lo.y + b.hi.y), 0.5 * (b.lo.z + b.hi.z)};
+    unsigned m = 0;
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+        m |= spread3((unsigned)fmin(fmax((c[q] - s_lo[q]) * s_scale[q], 0.0), 1023.0)) << q;
+    key[i] = ((unsigned)kind << 30) | m;
+    val[i] = p;
+}
+
+// FP32 boxes that enclose FP64 ones
+struct BoxF {
+    float lx, ly, lz, hx, hy, hz;
+};
+__device__ __forceinline__ BoxF outward(const Box& b) {
+    return {__double2float_rd(b.lo.x), __double2float_rd(b.lo.y), __double2float_rd(b.lo.z),
+            __double2float_ru(b.hi.x), __double2float_ru(b.hi.y), __double2float_ru(b.hi.z)};
+}
+__device__ __forceinline__ BoxF empty_box() { return {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY}; }
+__device__ __forceinline__ bool meet(const BoxF& a, const BoxF& b) {
+    return !(a.lx > b.hx || b.lx > a.hx || a.ly > b.hy || b.ly > a.hy || a.lz > b.hz || b.lz > a.hz);
+}
+__device__ __forceinline__ BoxF warp_union(BoxF b) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        b.lx = fminf(b.lx, __shfl_xor_sync(0xffffffffu, b.lx, o));
+        b.ly = fminf(b.ly, __shfl_xor_sync(0xffffffffu, b.ly, o));
+        b.lz = fminf(b.lz, __shfl_xor_sync(0xffffffffu, b.lz, o));
+        b.hx = fmaxf(b.hx, __shfl_xor_sync(0xffffffffu, b.hx, o));
+        b.hy = fmaxf(b.hy, __shfl_xor_sync(0xffffffffu, b.hy, o));
+        b.hz = fmaxf(b.hz, __shfl_xor_sync(0xffffffffu, b.hz, o));
+    }
+    return b;
+}
+__device__ __forceinline__ BoxF shfl_box(const BoxF& b, int j) {
+    return {__shfl_sync(0xffffffffu, b.lx, j), __shfl_sync(0xffffffffu, b.ly, j), __shfl_sync(0xffffffffu, b.lz, j),
+            __shfl_sync(0xffffffffu, b.hx, j), __shfl_sync(0xffffffffu, b.hy, j), __shfl_sync(0xffffffffu, b.hz, j)};
+}
+__device__ __forceinline__ void store_box(float4* at, int i, const BoxF& b, int id) {
+    at[2 * (size_t)i] = make_float4(b.lx, b.ly, b.lz, __int_as_float(id));
+    at[2 * (size_t)i + 1] = make_float4(b.hx, b.hy, b.hz, 0.f);
+}
+__device__ __forceinline__ BoxF load_box(const float4* at, int i, int& id) {
+    const float4 l = __ldg(at + 2 * (size_t)i), h = __ldg(at + 2 * (size_t)i + 1);
+    id = __float_as_int(l.w);
+    return {l.x, l.y, l.z, h.x, h.y, h.z};
+}
+
+// Boxes of the sorted triangles (grown by the gap) and edges (by half of it), of their groups of
+// 32 and of their nodes of 1024, one node per CTA; the first tri_nodes CTAs take the triangles.
+// Places beyond the last primitive get empty boxes and index -1.
+__global__ void __launch_bounds__(kNodeLeaves) k_boxes(const double* __restrict__ x,
+                                                       const unsigned* __restrict__ faces, int nf,
+                                                       const unsigned* __restrict__ edges, int ne, int tri_nodes,
+                                                       const int* __restrict__ val, double gap,
+                                                       const unsigned* __restrict__ counts, float4* leaf,
+                                                       float4* group, float4* node) {
+    __shared__ BoxF s_group[32];
+    if (counts[kCntBad]) return;
+    const bool tri = (int)blockIdx.x < tri_nodes;
+    const int k = ((int)blockIdx.x - (tri ? 0 : tri_nodes)) * kNodeLeaves + threadIdx.x;
+    BoxF b = empty_box();
+    int p = -1;
+    if (k < (tri ? nf : ne)) {
+        p = val[tri ? k : nf + k];
+        b = tri ? outward(grown_box(x, faces + 3 * (size_t)p, 3, gap)) : outward(grown_box(x, edges + 2 * (size_t)p, 2, 0.5 * gap));
+    }
+    const int i = blockIdx.x * kNodeLeaves + threadIdx.x, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    store_box(leaf, i, b, p);
+    b = warp_union(b);
+    if (lane == 0) {
+        s_group[w] = b;
+        store_box(group, i >> 5, b, 0);
+    }
+    __syncthreads();
+    if (w == 0) {
+        b = warp_union(s_group[lane]);
+        if (lane == 0) store_box(node, blockIdx.x, b, 0);
+    }
 }
 
 struct PairOut {
@@ -280,110 +366,247 @@ struct QueryArgs {
     const int* body;
     const int* btype;
     int nsv, nf, ne;
-    double dhat;
-    const double* grid;
-    const unsigned long long* tkey;
-    const int* tval;
-    const unsigned long long* ekey;
-    const int* eval;
+    double dhat, gap, ground_offset;
+    const int* val;  // the sorted order: triangles, edges, surface points
+    const float4* leaf;
+    const float4* group;
+    const float4* node;
+    int tri_nodes, edge_nodes, edge_groups, point_groups;
+    int2* item;  // [item_cap] of the edges, then [item_cap] of the points
+    unsigned item_cap;
+    unsigned* counts;
+    unsigned long long* rec;
+    unsigned rec_cap;
+    int qshift, kshift;  // key = kind << kshift | query << qshift | primitive
 };
 
 __device__ __forceinline__ bool all_fixed(const int* bt, unsigned a, unsigned b, unsigned c, unsigned d) {
     return bt && bt[a] >= 2 && bt[b] >= 2 && bt[c] >= 2 && bt[d] >= 2;
 }
 
-// Query q < nsv: surface point sv[q] against the triangles of its cell; q >= nsv: edge q - nsv
-// against the edges of its grown box's cells.  kWrite = false counts into counts[q]; true
-// writes the records from offs[q] on (edge-edge ones to the unsorted record buffers).
-template <bool kWrite>
-__global__ void k_query(QueryArgs a, int* counts, const int* offs, int4* pairs, int4* ccd, int* group,
-                        int4* rec_pair, int4* rec_ccd, unsigned long long* reckey, int* recidx) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= a.nsv + a.ne || a.grid[5] != 0.0) return;
-    const double h = a.grid[3], gap = a.grid[4];
-    int found = 0;
-    const int base = kWrite ? offs[q] : 0;
-    PairOut o;
-    if (q < a.nsv) {
-        const unsigned p = a.sv[q];
-        const d3 xp = ldp(a.x, p);
-        const unsigned long long key = cell_key(cell_of(xp.x, a.grid[0], h), cell_of(xp.y, a.grid[1], h),
-                                                cell_of(xp.z, a.grid[2], h));
-        const int n8 = 8 * a.nf;
-        for (int k = lower_bound(a.tkey, n8, key); k < n8 && __ldg(a.tkey + k) == key; k++) {
-            const int f = __ldg(a.tval + k);
-            const unsigned t0 = a.faces[3 * f], t1 = a.faces[3 * f + 1], t2 = a.faces[3 * f + 2];
-            // _selfQuery_vf's filters (mlbvh.cu:1350-1362)
-            if (!(a.body[p] != a.body[t0] || a.body[p] == -1)) continue;
-            if (p == t0 || p == t1 || p == t2) continue;
-            if (all_fixed(a.btype, p, t0, t1, t2)) continue;
-            if (!check_pt(a.x, p, t0, t1, t2, a.dhat, o)) continue;
-            if (kWrite) {
-                pairs[base + found] = o.pair;
-                ccd[base + found] = o.ccd;
-                group[base + found] = o.group;
-            }
-            found++;
-        }
-    } else {
-        const int s = q - a.nsv;
-        const unsigned e0 = a.edges[2 * s], e1 = a.edges[2 * s + 1];
-        const Box bs = grown_box(a.x, a.edges + 2 * s, 2, 0.5 * gap);
-        const int i0 = cell_of(bs.lo.x, a.grid[0], h), j0 = cell_of(bs.lo.y, a.grid[1], h), k0 = cell_of(bs.lo.z, a.grid[2], h);
-        const int i1 = cell_of(bs.hi.x, a.grid[0], h), j1 = cell_of(bs.hi.y, a.grid[1], h), k1 = cell_of(bs.hi.z, a.grid[2], h);
-        const int n8 = 8 * a.ne;
-        for (int c = 0; c < 8; c++) {
-            const int ci = i0 + (c & 1), cj = j0 + ((c >> 1) & 1), ck = k0 + (c >> 2);
-            if (ci > i1 || cj > j1 || ck > k1) continue;
-            const unsigned long long key = cell_key(ci, cj, ck);
-            for (int k = lower_bound(a.ekey, n8, key); k < n8 && __ldg(a.ekey + k) == key; k++) {
-                const int other = __ldg(a.eval + k);
-                if (other <= s) continue;  // each pair once, as (edge, larger edge) (mlbvh.cu:1550-1560)
-                const Box bo = grown_box(a.x, a.edges + 2 * other, 2, 0.5 * gap);
-                if (bo.lo.x > bs.hi.x || bs.lo.x > bo.hi.x || bo.lo.y > bs.hi.y || bs.lo.y > bo.hi.y ||
-                    bo.lo.z > bs.hi.z || bs.lo.z > bo.hi.z)
-                    continue;
-                // the one cell that reports this pair: the one holding the overlap's low corner
-                if (cell_of(fmax(bs.lo.x, bo.lo.x), a.grid[0], h) != ci ||
-                    cell_of(fmax(bs.lo.y, bo.lo.y), a.grid[1], h) != cj ||
-                    cell_of(fmax(bs.lo.z, bo.lo.z), a.grid[2], h) != ck)
-                    continue;
-                const unsigned f0 = a.edges[2 * other], f1 = a.edges[2 * other + 1];
-                // _selfQuery_ee's filters (mlbvh.cu:1550-1566)
-                if (!(a.body[e0] != a.body[f0] || a.body[e0] == -1)) continue;
-                if (e0 == f0 || e0 == f1 || e1 == f0 || e1 == f1) continue;
-                if (all_fixed(a.btype, e0, e1, f0, f1)) continue;
-                if (!check_ee(a.x, a.rest, e0, e1, f0, f1, other, a.dhat, o)) continue;
-                if (kWrite) {
-                    const int r = base + found - offs[a.nsv];  // position among the edge-edge records
-                    rec_pair[r] = o.pair;
-                    rec_ccd[r] = o.ccd;
-                    reckey[r] = ((unsigned long long)s << 32) | (unsigned)other;
-                    recidx[r] = r;
-                }
-                found++;
-            }
-        }
+// surface point q against triangle f, with _selfQuery_vf's filters (mlbvh.cu:1350-1362)
+__device__ __forceinline__ bool test_pt(const QueryArgs& a, int q, int f, PairOut& o) {
+    const unsigned p = a.sv[q];
+    const unsigned t0 = a.faces[3 * (size_t)f], t1 = a.faces[3 * (size_t)f + 1], t2 = a.faces[3 * (size_t)f + 2];
+    if (!(a.body[p] != a.body[t0] || a.body[p] == -1)) return false;
+    if (p == t0 || p == t1 || p == t2) return false;
+    if (all_fixed(a.btype, p, t0, t1, t2)) return false;
+    return check_pt(a.x, p, t0, t1, t2, a.dhat, o);
+}
+
+// edge s against the edge `other` > s, with _selfQuery_ee's filters (mlbvh.cu:1550-1566); the two
+// boxes, each grown by half the gap, have to overlap
+__device__ __forceinline__ bool test_ee(const QueryArgs& a, int s, int other, PairOut& o) {
+    const unsigned e0 = a.edges[2 * (size_t)s], e1 = a.edges[2 * (size_t)s + 1];
+    const unsigned f0 = a.edges[2 * (size_t)other], f1 = a.edges[2 * (size_t)other + 1];
+    if (!(a.body[e0] != a.body[f0] || a.body[e0] == -1)) return false;
+    if (e0 == f0 || e0 == f1 || e1 == f0 || e1 == f1) return false;
+    if (all_fixed(a.btype, e0, e1, f0, f1)) return false;
+    const Box bs = grown_box(a.x, a.edges + 2 * (size_t)s, 2, 0.5 * a.gap);
+    const Box bo = grown_box(a.x, a.edges + 2 * (size_t)other, 2, 0.5 * a.gap);
+    if (bo.lo.x > bs.hi.x || bs.lo.x > bo.hi.x || bo.lo.y > bs.hi.y || bs.lo.y > bo.hi.y || bo.lo.z > bs.hi.z ||
+        bs.lo.z > bo.hi.z)
+        return false;
+    return check_ee(a.x, a.rest, e0, e1, f0, f1, other, a.dhat, o);
+}
+
+// appends the lanes' keys (one atomic per warp); a record past the capacity is counted only
+__device__ __forceinline__ void append(const QueryArgs& a, bool on, unsigned long long key) {
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (!m) return;
+    const int lane = threadIdx.x & 31;
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(a.counts + kCntRec, (unsigned)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
+    if (on && base < a.rec_cap) a.rec[base] = key;
+}
+
+// A warp's 32 queries of one kind (group g of the sorted edges or surface points) and their
+// candidates so far
+struct QueryGroup {
+    int q;     // the lane's query (-1: none)
+    BoxF box;  // and its box
+};
+template <bool kEdge>
+__device__ __forceinline__ QueryGroup query_group(const QueryArgs& a, int g) {
+    const int lane = threadIdx.x & 31;
+    QueryGroup r{-1, empty_box()};
+    if (kEdge) {
+        r.box = load_box(a.leaf, a.tri_nodes * kNodeLeaves + 32 * g + lane, r.q);
+    } else if (32 * g + lane < a.nsv) {
+        r.q = __ldg(a.val + a.nf + a.ne + 32 * g + lane);
+        r.box = outward(grown_box(a.x, a.sv + r.q, 1, 0.0));
     }
-    if (!kWrite) counts[q] = found;
+    return r;
 }
 
-// edge-edge records in (edge, other edge) order after the sort; their Hessian-size group
-__global__ void k_gather_ee(int n, int first, const int* __restrict__ idx, const int4* __restrict__ rp,
-                            const int4* __restrict__ rc, int4* pairs, int4* ccd, int* group) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const int r = idx[k];
-    const int4 p = rp[r];
-    pairs[first + k] = p;
-    ccd[first + k] = rc[r];
-    // point-point (z < 0, w at most -1), point-edge (w < 0), or edge-edge
-    group[first + k] = p.x >= 0 ? 2 : (p.z < 0 ? 0 : 1);
+// tests the last `count` (<= 32) queued candidates exactly, one per lane
+template <bool kEdge>
+__device__ __forceinline__ void drain(const QueryArgs& a, const int2* queue, int& queued, int count,
+                                      unsigned (&by_size)[3]) {
+    const int lane = threadIdx.x & 31;
+    bool found = false;
+    PairOut o;
+    unsigned long long key = 0;
+    if (lane < count) {
+        const int2 c = queue[queued - count + lane];
+        int s = c.x, t = c.y;
+        if (kEdge && t < s) s = c.y, t = c.x;  // each pair as (edge, larger edge) (mlbvh.cu:1550-1560)
+        found = kEdge ? test_ee(a, s, t, o) : test_pt(a, s, t, o);
+        key = ((kEdge ? 1ull : 0ull) << a.kshift) | ((unsigned long long)(unsigned)s << a.qshift) | (unsigned)t;
+    }
+    queued -= count;
+    __syncwarp();
+    if (found)
+#pragma unroll
+        for (int k = 0; k < 3; k++) by_size[k] += o.group == k;
+    append(a, found, key);
 }
 
-__global__ void k_group_flags(int n, const int* __restrict__ group, unsigned long long* flags) {
+// the queries of group g against the primitives of leaf group c: those that meet a query's box
+// are queued, and tested 32 at a time
+template <bool kEdge>
+__device__ __forceinline__ void query_leaves(const QueryArgs& a, int g, int c, const QueryGroup& qg, const BoxF& ub,
+                                             int2* queue, int& queued, unsigned (&by_size)[3]) {
+    const int lane = threadIdx.x & 31;
+    int prim;
+    const BoxF cb = load_box(a.leaf, (kEdge ? a.tri_nodes * kNodeLeaves : 0) + 32 * c + lane, prim);
+    for (unsigned m = __ballot_sync(0xffffffffu, prim >= 0 && meet(cb, ub)); m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        const BoxF jb = shfl_box(cb, j);
+        const int jp = __shfl_sync(0xffffffffu, prim, j);
+        // edges: only those behind the query in the sorted order (each unordered pair once)
+        const bool hit = qg.q >= 0 && meet(qg.box, jb) && (!kEdge || c > g || j > lane);
+        const unsigned h = __ballot_sync(0xffffffffu, hit);
+        if (!h) continue;
+        if (hit) queue[queued + __popc(h & ((1u << lane) - 1u))] = make_int2(qg.q, jp);
+        queued += __popc(h);
+        __syncwarp();
+        if (queued >= 32) drain<kEdge>(a, queue, queued, 32, by_size);
+    }
+}
+
+__device__ __forceinline__ void add_sizes(const QueryArgs& a, const unsigned (&by_size)[3]) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const unsigned t = __reduce_add_sync(0xffffffffu, by_size[k]);
+        if ((threadIdx.x & 31) == 0 && t) atomicAdd(a.counts + kCntSize + k, t);
+    }
+}
+
+// One warp per query group and 32 nodes: the leaf groups whose box meets the queries', as items
+// for k_query.  A group that the list has no room for is searched here and now.
+template <bool kEdge>
+__device__ __forceinline__ void group_items(const QueryArgs& a, int g, int n0, int2* queue) {
+    const int lane = threadIdx.x & 31;
+    const int node0 = kEdge ? a.tri_nodes : 0, nnode = kEdge ? a.edge_nodes : a.tri_nodes;
+    if (kEdge && n0 + 31 < (g >> 5)) return;  // edges: the leaf groups from the queries' own on
+    const QueryGroup qg = query_group<kEdge>(a, g);
+    const BoxF ub = warp_union(qg.box);
+    int2* list = a.item + (kEdge ? 0 : a.item_cap);
+    unsigned* count = a.counts + kCntItem + (kEdge ? 0 : 1);
+    unsigned by_size[3] = {0, 0, 0};
+    int queued = 0, id;
+    const bool on2 = n0 + lane < nnode && meet(load_box(a.node, node0 + n0 + lane, id), ub);
+    for (unsigned m2 = __ballot_sync(0xffffffffu, on2); m2; m2 &= m2 - 1) {
+        const int c = 32 * (n0 + __ffs(m2) - 1) + lane;  // the lane's leaf group
+        const bool on = (!kEdge || c >= g) && meet(load_box(a.group, 32 * node0 + c, id), ub);
+        const unsigned m1 = __ballot_sync(0xffffffffu, on);
+        if (!m1) continue;
+        unsigned base = 0;
+        if (lane == 0) base = atomicAdd(count, (unsigned)__popc(m1));
+        base = __shfl_sync(0xffffffffu, base, 0) + __popc(m1 & ((1u << lane) - 1u));
+        const bool room = base < a.item_cap;
+        if (on && room) list[base] = make_int2(g, c);
+        for (unsigned m = __ballot_sync(0xffffffffu, on && !room); m; m &= m - 1)
+            query_leaves<kEdge>(a, g, __shfl_sync(0xffffffffu, c, __ffs(m) - 1), qg, ub, queue, queued, by_size);
+    }
+    if (queued > 0) drain<kEdge>(a, queue, queued, queued, by_size);
+    add_sizes(a, by_size);
+}
+
+// Warps: edge groups x chunks of 32 edge nodes, then point groups x chunks of 32 triangle nodes;
+// the first chunk's also test the points against the ground plane (_GroundCollisionDetect,
+// GIPC.cu:6433-6450: (n.x - offset)^2 <= dHat with the normal +y).
+__global__ void __launch_bounds__(32 * kQueryWarps) k_items(QueryArgs a) {
+    __shared__ int2 s_queue[kQueryWarps][64];
+    if (a.counts[kCntBad]) return;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long i = (long long)blockIdx.x * kQueryWarps + w;  // warp-uniform, as all that follows
+    const long long edge_warps = (long long)a.edge_groups * ((a.edge_nodes + 31) / 32);
+    if (i < edge_warps) {
+        group_items<true>(a, (int)(i % a.edge_groups), (int)(i / a.edge_groups) * 32, s_queue[w]);
+        return;
+    }
+    const long long j = i - edge_warps;
+    const int chunk = a.point_groups > 0 ? (int)(j / a.point_groups) : 1, g = (int)(j - (long long)chunk * a.point_groups);
+    if (chunk > 0 && 32 * chunk >= a.tri_nodes) return;
+    if (chunk == 0) {
+        bool low = false;
+        int q = 0;
+        if (32 * g + lane < a.nsv) {
+            q = a.val[a.nf + a.ne + 32 * g + lane];
+            const double dist = a.x[3 * (size_t)a.sv[q] + 1] - a.ground_offset;
+            low = !(dist * dist > a.dhat);
+        }
+        append(a, low, (2ull << a.kshift) | ((unsigned long long)(unsigned)q << a.qshift));
+        const unsigned m = __ballot_sync(0xffffffffu, low);
+        if (lane == 0 && m) atomicAdd(a.counts + kCntGround, (unsigned)__popc(m));
+    }
+    if (32 * chunk < a.tri_nodes) group_items<false>(a, g, 32 * chunk, s_queue[w]);
+}
+
+template <bool kEdge>
+__device__ __forceinline__ void query_items(const QueryArgs& a, int w0, int nw, int2* queue) {
+    const int n = (int)min(a.counts[kCntItem + (kEdge ? 0 : 1)], a.item_cap);
+    const int2* list = a.item + (kEdge ? 0 : a.item_cap);
+    unsigned by_size[3] = {0, 0, 0};
+    int queued = 0;
+    for (int i = w0; i < n; i += nw) {  // warp-uniform
+        const int2 it = list[i];
+        const QueryGroup qg = query_group<kEdge>(a, it.x);
+        query_leaves<kEdge>(a, it.x, it.y, qg, warp_union(qg.box), queue, queued, by_size);
+    }
+    if (queued > 0) drain<kEdge>(a, queue, queued, queued, by_size);
+    add_sizes(a, by_size);
+}
+
+// The items, one per warp and turn; every warp takes its share of both kinds.  (With one warp
+// walking all of a query group's leaf groups, the few groups of large primitives beside small
+// ones ran for milliseconds after the others had ended: 5.8 ms for the 256^2 cloth over a sphere,
+// SMs busy 11 % of it.)
+__global__ void __launch_bounds__(32 * kQueryWarps) k_query(QueryArgs a) {
+    __shared__ int2 s_queue[kQueryWarps][64];
+    if (a.counts[kCntBad]) return;
+    const int nw = gridDim.x * kQueryWarps, w0 = blockIdx.x * kQueryWarps + (threadIdx.x >> 5);
+    int2* queue = s_queue[threadIdx.x >> 5];
+    query_items<true>(a, w0, nw, queue);
+    query_items<false>(a, nw - 1 - w0, nw, queue);
+}
+
+// The sorted records as pairs with their CCD candidates and Hessian sizes (flags of the rank
+// scan; mat_index holds the size codes until k_mat_index), then the ground points.
+__global__ void k_emit(QueryArgs a, int total, int ng, const unsigned long long* __restrict__ rec, int4* pairs,
+                       int4* ccd, int* mat_index, unsigned long long* flags, unsigned* ground, unsigned* gp_num) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) flags[k] = 1ull << (kGroupBits * group[k]);
+    if (k == 0) *gp_num = (unsigned)ng;
+    if (k >= total + ng) return;
+    const unsigned long long key = rec[k];
+    const int kind = (int)(key >> a.kshift);
+    const int q = (int)((key >> a.qshift) & ((1ull << (a.kshift - a.qshift)) - 1));
+    const int p = (int)(key & ((1ull << a.qshift) - 1));
+    if (kind == 2) {
+        ground[k - total] = a.sv[q];
+        return;
+    }
+    PairOut o;
+    o.group = 0;
+    if (kind == 0) test_pt(a, q, p, o);
+    else test_ee(a, q, p, o);
+    pairs[k] = o.pair;
+    ccd[k] = o.ccd;
+    mat_index[k] = o.group;
+    flags[k] = 1ull << (kGroupBits * o.group);
 }
 
 // MatIndex = rank among the pairs of the same group; cp_num = total, 0, per-group counts
@@ -399,30 +622,6 @@ __global__ void k_mat_index(int n, int* mat_index, const unsigned long long* __r
         cp_num[1] = 0;
         for (int g = 0; g < 3; g++) cp_num[2 + g] = (unsigned)((last >> (kGroupBits * g)) & m);
     }
-}
-
-// _GroundCollisionDetect (GIPC.cu:6433-6450): surface points with (n.x - offset)^2 <= dHat
-__global__ void k_ground_flags(const double* __restrict__ x, const unsigned* __restrict__ sv, int nsv, double offset,
-                               double dhat, const double* __restrict__ grid, int* flag) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nsv || grid[5] != 0.0) return;
-    const double dist = x[3 * sv[i] + 1] - offset;  // normal +y
-    flag[i] = dist * dist > dhat ? 0 : 1;
-}
-__global__ void k_ground_write(const unsigned* __restrict__ sv, int nsv, const int* __restrict__ flag,
-                               const int* __restrict__ off, unsigned* out, unsigned* gp_num) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nsv && flag[i]) out[off[i]] = sv[i];
-    if (i == nsv - 1) *gp_num = (unsigned)(off[i] + flag[i]);
-}
-
-__global__ void k_counts_out(const int* offs, int nsv, int nq, const int* goff, const int* gflag,
-                             const double* grid, unsigned* counts) {
-    unsigned* h_counts = counts;
-    h_counts[0] = (unsigned)offs[nq];
-    h_counts[1] = (unsigned)offs[nsv];
-    h_counts[2] = nsv > 0 ? (unsigned)(goff[nsv - 1] + gflag[nsv - 1]) : 0u;
-    h_counts[3] = (unsigned)grid[5];
 }
 
 // ------------------------------------------------------------------------------------------
@@ -503,12 +702,27 @@ __global__ void k_fric_setup(const double* __restrict__ x, const int4* __restric
                              const int* __restrict__ flag, const int* __restrict__ off, double dhat, double kappa,
                              int4* out_pairs, double* lambda, double* coord, double* basis, unsigned* cp_num_last) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n || !flag[k]) return;
-    const int4 p = pairs[k];
+    const bool on = k < n && flag[k];
+    const int4 p = on ? pairs[k] : make_int4(-1, 0, -1, -1);
+    // integer counts (the same totals in any order), one atomic per size and CTA: with one per
+    // pair the counters' address bounded the kernel (395 us for a million pairs)
+    __shared__ unsigned s_size[3];
+    if (threadIdx.x < 3) s_size[threadIdx.x] = 0;
+    __syncthreads();
+    const int size = p.x >= 0 ? 2 : (p.z < 0 ? 0 : (p.w < 0 ? 1 : 2));
+    for (int q = 0; q < 3; q++) {
+        const unsigned m = __ballot_sync(0xffffffffu, on && size == q);
+        if ((threadIdx.x & 31) == 0 && m) atomicAdd(s_size + q, (unsigned)__popc(m));
+    }
+    __syncthreads();
+    if (threadIdx.x < 3 && s_size[threadIdx.x]) {
+        atomicAdd(cp_num_last, s_size[threadIdx.x]);
+        atomicAdd(cp_num_last + 2 + threadIdx.x, s_size[threadIdx.x]);
+    }
+    if (!on) return;
     const int o = off[k];
     double dis, c0 = 0.0, c1 = 0.0;
     double* B = basis + 6 * (size_t)o;
-    int group;
     if (p.x >= 0) {  // edge-edge
         const d3 v0 = ldp(x, p.x), v1 = ldp(x, p.y), v2 = ldp(x, p.z), v3 = ldp(x, p.w);
         dis = ll_d2(v0, v1, v2, v3);
@@ -520,7 +734,6 @@ __global__ void k_fric_setup(const double* __restrict__ x, const int4* __restric
         c0 = R[0][0] * r0 + R[0][1] * r1;
         c1 = R[1][0] * r0 + R[1][1] * r1;
         store_basis(B, normalized(e01), normalized(cross(cross(e01, e23), e01)));
-        group = 2;
     } else {
         const unsigned v = (unsigned)(-p.x - 1);
         const d3 v0 = ldp(x, v), v1 = ldp(x, p.y);
@@ -530,14 +743,12 @@ __global__ void k_fric_setup(const double* __restrict__ x, const int4* __restric
             const d3 xc = {0.0, -v01.z, v01.y}, yc = {v01.z, 0.0, -v01.x};
             const d3 t0 = sq(xc) > sq(yc) ? xc : yc;
             store_basis(B, normalized(t0), normalized(cross(v01, t0)));
-            group = 0;
         } else if (p.w < 0) {  // point-edge
             const d3 v2 = ldp(x, p.z);
             dis = pe_d2(v0, v1, v2);
             const d3 e12 = v2 - v1;
             c0 = dot(v0 - v1, e12) / sq(e12);
             store_basis(B, normalized(e12), normalized(cross(e12, v0 - v1)));
-            group = 1;
         } else {  // point-triangle
             const d3 v2 = ldp(x, p.z), v3 = ldp(x, p.w);
             dis = pplane_d2(v0, v1, v2, v3);
@@ -551,7 +762,6 @@ __global__ void k_fric_setup(const double* __restrict__ x, const int4* __restric
             c0 = R[0][0] * b0 + R[0][1] * b1;
             c1 = R[1][0] * b0 + R[1][1] * b1;
             store_basis(B, normalized(v12), normalized(cross(cross(v12, v13), v12)));
-            group = 2;
         }
     }
     const double l = log(dis / dhat);
@@ -559,9 +769,6 @@ __global__ void k_fric_setup(const double* __restrict__ x, const int4* __restric
     coord[2 * (size_t)o] = c0;
     coord[2 * (size_t)o + 1] = c1;
     out_pairs[o] = p;
-    // integer counts: the same totals in any order
-    atomicAdd(cp_num_last, 1u);
-    atomicAdd(cp_num_last + 2 + group, 1u);
 }
 
 // _calFrictionLastH_gd (GIPC.cu:8362-8386): the ground pairs' normal forces (the RANK-1 form
@@ -585,99 +792,82 @@ __global__ void k_fric_ground(const double* __restrict__ x, int nv, const unsign
     out[k] = g;
 }
 
-// buffers for nsv points, nf triangles, ne edges and cap records
-SgipcStatus broad_reserve(SgipcCtx* c, int nsv, int nf, int ne, int cap) {
-    if (!c->broad) {
-        c->broad = new BroadWork();
-        BroadWork& w = *c->broad;
-        SG_CHECK(c, cudaMalloc((void**)&w.bounds, sizeof(unsigned long long) * 8));
-        SG_CHECK(c, cudaMalloc((void**)&w.grid, sizeof(double) * 8));
-        SG_CHECK(c, cudaMalloc((void**)&w.d_counts, sizeof(unsigned) * 4));
-        SG_CHECK(c, cudaMallocHost((void**)&w.h_counts, sizeof(unsigned) * 4));
-    }
+template <class T>
+SgipcStatus regrow(SgipcCtx* c, T** p, size_t n) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+    SG_CHECK(c, cudaMalloc((void**)p, sizeof(T) * (n > 0 ? n : 1)));
+    return SGIPC_OK;
+}
+
+// buffers for np primitives, nl leaf places (whole nodes), ni items of each kind, nrec records
+// and nfr friction pairs
+SgipcStatus broad_reserve(SgipcCtx* c, int np, int nl, int ni, int nrec, int nfr) {
+    if (!c->broad) c->broad = new BroadWork();
     BroadWork& w = *c->broad;
-    bool cub_again = false;
-    if (8 * nf > w.cap_tri) {
-        const int m = 8 * nf;
-        for (unsigned long long** p : {&w.tkey, &w.tkey_s}) {
-            if (*p) cudaFree(*p);
-            SG_CHECK(c, cudaMalloc((void**)p, sizeof(unsigned long long) * (size_t)(m > 0 ? m : 1)));
-        }
-        for (int** p : {&w.tval, &w.tval_s}) {
-            if (*p) cudaFree(*p);
-            SG_CHECK(c, cudaMalloc((void**)p, sizeof(int) * (size_t)(m > 0 ? m : 1)));
-        }
-        w.cap_tri = m;
+    if (!w.bounds) SG_CHECK(c, cudaMalloc((void**)&w.bounds, sizeof(unsigned long long) * 8));
+    if (!w.d_counts) SG_CHECK(c, cudaMalloc((void**)&w.d_counts, sizeof(unsigned) * kCntNum));
+    if (!w.h_counts) SG_CHECK(c, cudaMallocHost((void**)&w.h_counts, sizeof(unsigned) * kCntNum));
+    SgipcStatus st;
+    bool cub_again = !w.cub;
+    // a capacity is raised only after all of its buffers exist
+    if (np > w.cap_prim) {
+        w.cap_prim = 0;
+        if ((st = regrow(c, &w.key, np)) || (st = regrow(c, &w.key_s, np)) || (st = regrow(c, &w.val, np)) ||
+            (st = regrow(c, &w.val_s, np)))
+            return st;
+        w.cap_prim = np;
         cub_again = true;
     }
-    if (8 * ne > w.cap_edge) {
-        const int m = 8 * ne;
-        for (unsigned long long** p : {&w.ekey, &w.ekey_s}) {
-            if (*p) cudaFree(*p);
-            SG_CHECK(c, cudaMalloc((void**)p, sizeof(unsigned long long) * (size_t)(m > 0 ? m : 1)));
-        }
-        for (int** p : {&w.eval, &w.eval_s}) {
-            if (*p) cudaFree(*p);
-            SG_CHECK(c, cudaMalloc((void**)p, sizeof(int) * (size_t)(m > 0 ? m : 1)));
-        }
-        w.cap_edge = m;
+    if (nl > w.cap_leaf) {
+        w.cap_leaf = 0;
+        if ((st = regrow(c, &w.leaf, 2 * (size_t)nl)) || (st = regrow(c, &w.group, 2 * (size_t)nl / 32)) ||
+            (st = regrow(c, &w.node, 2 * (size_t)nl / kNodeLeaves)))
+            return st;
+        w.cap_leaf = nl;
+    }
+    if (ni > w.cap_item) {
+        w.cap_item = 0;
+        if ((st = regrow(c, &w.item, 2 * (size_t)ni))) return st;
+        w.cap_item = ni;
+    }
+    if (nrec > w.cap_rec) {
+        w.cap_rec = 0;
+        if ((st = regrow(c, &w.reckey, nrec)) || (st = regrow(c, &w.reckey_s, nrec)) || (st = regrow(c, &w.gscan, nrec)))
+            return st;
+        w.cap_rec = nrec;
         cub_again = true;
     }
-    if (nsv + ne + 1 > w.cap_q) {
-        const int m = nsv + ne + 1;
-        for (int** p : {&w.counts, &w.offs}) {
-            if (*p) cudaFree(*p);
-            SG_CHECK(c, cudaMalloc((void**)p, sizeof(int) * (size_t)m));
-        }
-        w.cap_q = m;
-        cub_again = true;
-    }
-    if (nsv + 1 > w.cap_sv) {
-        const int m = nsv + 1;
-        for (int** p : {&w.gflag, &w.goff}) {
-            if (*p) cudaFree(*p);
-            SG_CHECK(c, cudaMalloc((void**)p, sizeof(int) * (size_t)m));
-        }
-        w.cap_sv = m;
-        cub_again = true;
-    }
-    if (cap > w.cap_rec) {
-        const int m = cap > 1 ? cap : 1;
-        for (unsigned long long** p : {&w.reckey, &w.reckey_s, &w.gscan}) {
-            if (*p) cudaFree(*p);
-            SG_CHECK(c, cudaMalloc((void**)p, sizeof(unsigned long long) * (size_t)m));
-        }
-        for (int** p : {&w.recidx, &w.recidx_s}) {
-            if (*p) cudaFree(*p);
-            SG_CHECK(c, cudaMalloc((void**)p, sizeof(int) * (size_t)m));
-        }
-        for (int4** p : {&w.rec_pair, &w.rec_ccd}) {
-            if (*p) cudaFree(*p);
-            SG_CHECK(c, cudaMalloc((void**)p, sizeof(int4) * (size_t)m));
-        }
-        w.cap_rec = m;
+    if (nfr + 1 > w.cap_q) {
+        w.cap_q = 0;
+        if ((st = regrow(c, &w.gflag, (size_t)nfr + 1)) || (st = regrow(c, &w.goff, (size_t)nfr + 1))) return st;
+        w.cap_q = nfr + 1;
         cub_again = true;
     }
     if (cub_again) {
         size_t b = 0, t = 0;
-        SG_CHECK(c, cub::DeviceRadixSort::SortPairs(nullptr, t, w.tkey, w.tkey_s, w.tval, w.tval_s, w.cap_tri));
+        SG_CHECK(c, cub::DeviceRadixSort::SortPairs(nullptr, t, w.key, w.key_s, w.val, w.val_s, w.cap_prim));
         b = t > b ? t : b;
-        SG_CHECK(c, cub::DeviceRadixSort::SortPairs(nullptr, t, w.ekey, w.ekey_s, w.eval, w.eval_s, w.cap_edge));
+        SG_CHECK(c, cub::DeviceRadixSort::SortKeys(nullptr, t, w.reckey, w.reckey_s, w.cap_rec));
         b = t > b ? t : b;
-        SG_CHECK(c, cub::DeviceRadixSort::SortPairs(nullptr, t, w.reckey, w.reckey_s, w.recidx, w.recidx_s,
-                                                    w.cap_rec));
+        SG_CHECK(c, cub::DeviceScan::ExclusiveSum(nullptr, t, w.gflag, w.goff, w.cap_q));
         b = t > b ? t : b;
-        SG_CHECK(c, cub::DeviceScan::ExclusiveSum(nullptr, t, w.counts, w.offs, w.cap_q));
+        SG_CHECK(c, cub::DeviceScan::ExclusiveSum(nullptr, t, w.gscan, w.reckey, w.cap_rec));
         b = t > b ? t : b;
-        SG_CHECK(c, cub::DeviceScan::ExclusiveSum(nullptr, t, w.gscan, w.gscan, w.cap_rec));
-        b = t > b ? t : b;
-        if (b > w.cub_bytes) {
-            if (w.cub) cudaFree(w.cub);
-            SG_CHECK(c, cudaMalloc(&w.cub, b));
+        if (b > w.cub_bytes || !w.cub) {
+            w.cub_bytes = 0;
+            if ((st = regrow(c, (char**)&w.cub, b))) return st;
             w.cub_bytes = b;
         }
     }
     return SGIPC_OK;
+}
+
+// bits that hold 0 .. n - 1
+int index_bits(int n) {
+    int b = 1;
+    while (b < 31 && (1LL << b) < (long long)n) b++;
+    return b;
 }
 
 }  // namespace
@@ -686,9 +876,8 @@ namespace sgipc {
 void broad_destroy(SgipcCtx* c) {
     if (!c->broad) return;
     BroadWork& w = *c->broad;
-    void* ps[] = {w.tkey, w.tkey_s, w.tval, w.tval_s, w.ekey, w.ekey_s, w.eval, w.eval_s, w.bounds, w.grid, w.d_counts,
-                  w.counts, w.offs, w.gflag, w.goff, w.reckey, w.reckey_s, w.recidx, w.recidx_s, w.rec_pair,
-                  w.rec_ccd, w.gscan, w.cub};
+    void* ps[] = {w.key, w.key_s, w.val, w.val_s, w.leaf, w.group, w.node, w.item, w.bounds, w.d_counts, w.gflag, w.goff,
+                  w.reckey, w.reckey_s, w.gscan, w.cub};
     for (void* p : ps)
         if (p) cudaFree(p);
     if (w.h_counts) cudaFreeHost(w.h_counts);
@@ -715,61 +904,55 @@ extern "C" SgipcStatus sgipc_build_cp(SgipcCtx* c, const double* x, const double
     }
     SG_DEVICE(c);
     cudaStream_t s = (cudaStream_t)stream;
-    SgipcStatus st = broad_reserve(c, nsv, nf, ne, cap);
+    const int tri_nodes = nblk(nf, kNodeLeaves), edge_nodes = nblk(ne, kNodeLeaves);
+    const int np = nf + ne + nsv;
+    const int edge_groups = nblk(ne, 32), point_groups = nblk(nsv, 32);
+    const int items = kItemsPerGroup * (edge_groups > point_groups ? edge_groups : point_groups) + 1024;
+    SgipcStatus st = broad_reserve(c, np, (tri_nodes + edge_nodes) * kNodeLeaves, items, cap + nsv, 0);
     if (st != SGIPC_OK) return st;
     BroadWork& w = *c->broad;
-    const int nq = nsv + ne;
     const double gap = sqrt(dHat);
     // bounds: min entries start at the largest key, max entries at 0
     SG_CHECK(c, cudaMemsetAsync(w.bounds, 0xff, sizeof(unsigned long long) * 3, s));
     SG_CHECK(c, cudaMemsetAsync(w.bounds + 3, 0, sizeof(unsigned long long) * 5, s));  // and the index flag
-    SG_COUNT(c, 1);
-    k_bounds<<<148, 256, 0, s>>>(x, c->nv, surf->surf_verts, nsv, surf->faces, nf, surf->edges, ne, w.bounds);
-    SG_COUNT(c, 1);
-    k_grid<<<1, 1, 0, s>>>(w.bounds, gap, w.grid);
-    if (nf > 0) {
-        SG_COUNT(c, 1);
-        k_insert<<<nblk(nf), SGIPC_BLOCK, 0, s>>>(x, surf->faces, nf, 3, w.grid, w.tkey, w.tval);
+    SG_CHECK(c, cudaMemsetAsync(w.d_counts, 0, sizeof(unsigned) * kCntNum, s));
+    SG_COUNT(c, 2);
+    k_bounds<<<148, 32 * kBoundsWarps, 0, s>>>(x, c->nv, surf->surf_verts, nsv, surf->faces, nf, surf->edges, ne,
+                                               w.bounds);
+    k_keys<<<nblk(np > 0 ? np : 1), SGIPC_BLOCK, 0, s>>>(x, surf->faces, nf, surf->edges, ne, surf->surf_verts, nsv,
+                                                         w.bounds, gap, w.key, w.val, w.d_counts);
+    QueryArgs qa{x, rest, surf->surf_verts, surf->faces, surf->edges, body_id, boundary_type, nsv, nf, ne, dHat, gap,
+                 ground_offset, w.val_s, w.leaf, w.group, w.node, tri_nodes, edge_nodes, edge_groups, point_groups,
+                 w.item, (unsigned)items, w.d_counts, w.reckey, (unsigned)(cap + nsv), 0, 0};
+    qa.qshift = index_bits(nf > ne ? nf : ne);
+    qa.kshift = qa.qshift + index_bits(nsv > ne ? nsv : ne);
+    if (np > 0) {
         size_t t = w.cub_bytes;
-        SG_CHECK(c, cub::DeviceRadixSort::SortPairs(w.cub, t, w.tkey, w.tkey_s, w.tval, w.tval_s, 8 * nf, 0, 64, s));
+        SG_CHECK(c, cub::DeviceRadixSort::SortPairs(w.cub, t, w.key, w.key_s, w.val, w.val_s, np, 0, 32, s));
+        if (tri_nodes + edge_nodes > 0) {
+            SG_COUNT(c, 1);
+            k_boxes<<<tri_nodes + edge_nodes, kNodeLeaves, 0, s>>>(x, surf->faces, nf, surf->edges, ne, tri_nodes,
+                                                                   w.val_s, gap, w.d_counts, w.leaf, w.group, w.node);
+        }
+        SG_COUNT(c, 2);
+        const int tri_chunks = nblk(tri_nodes, 32);
+        const long long warps = (long long)edge_groups * nblk(edge_nodes, 32) +
+                                (long long)point_groups * (tri_chunks > 1 ? tri_chunks : 1);
+        k_items<<<nblk(warps, kQueryWarps), 32 * kQueryWarps, 0, s>>>(qa);
+        k_query<<<148 * kQueryCtas, 32 * kQueryWarps, 0, s>>>(qa);
     }
-    if (ne > 0) {
-        SG_COUNT(c, 1);
-        k_insert<<<nblk(ne), SGIPC_BLOCK, 0, s>>>(x, surf->edges, ne, 2, w.grid, w.ekey, w.eval);
-        size_t t = w.cub_bytes;
-        SG_CHECK(c, cub::DeviceRadixSort::SortPairs(w.cub, t, w.ekey, w.ekey_s, w.eval, w.eval_s, 8 * ne, 0, 64, s));
-    }
-    QueryArgs qa{x, rest, surf->surf_verts, surf->faces, surf->edges, body_id, boundary_type, nsv, nf, ne, dHat,
-                 w.grid, w.tkey_s, w.tval_s, w.ekey_s, w.eval_s};
-    SG_CHECK(c, cudaMemsetAsync(w.counts, 0, sizeof(int) * (size_t)(nq + 1), s));
-    if (nq > 0) {
-        SG_COUNT(c, 1);
-        k_query<false><<<nblk(nq, kQueryThreads), kQueryThreads, 0, s>>>(qa, w.counts, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                                nullptr, nullptr);
-    }
-    size_t t = w.cub_bytes;
-    SG_CHECK(c, cub::DeviceScan::ExclusiveSum(w.cub, t, w.counts, w.offs, nq + 1, s));
-    SG_CHECK(c, cudaMemsetAsync(w.gflag, 0, sizeof(int) * (size_t)(nsv + 1), s));
-    if (nsv > 0) {
-        SG_COUNT(c, 1);
-        k_ground_flags<<<nblk(nsv), SGIPC_BLOCK, 0, s>>>(x, surf->surf_verts, nsv, ground_offset, dHat, w.grid,
-                                                         w.gflag);
-    }
-    t = w.cub_bytes;
-    SG_CHECK(c, cub::DeviceScan::ExclusiveSum(w.cub, t, w.gflag, w.goff, nsv + 1, s));
-    SG_COUNT(c, 1);
-    k_counts_out<<<1, 1, 0, s>>>(w.offs, nsv, nq, w.goff, w.gflag, w.grid, w.d_counts);
-    SG_CHECK(c, cudaMemcpyAsync(w.h_counts, w.d_counts, sizeof(unsigned) * 4, cudaMemcpyDeviceToHost, s));
+    SG_CHECK(c, cudaMemcpyAsync(w.h_counts, w.d_counts, sizeof(unsigned) * kCntNum, cudaMemcpyDeviceToHost, s));
     SG_CHECK(c, cudaStreamSynchronize(s));
-    const int total = (int)w.h_counts[0], npt = (int)w.h_counts[1], ng = (int)w.h_counts[2];
+    const unsigned* h = w.h_counts;
+    const int ng = (int)h[kCntGround], total = (int)(h[kCntRec] - h[kCntGround]);
     for (int k = 0; k < 5; k++) h_cp_num[k] = 0;
     h_cp_num[0] = (unsigned)total;
     *h_gp_num = (unsigned)ng;
-    if (w.h_counts[3] == 2) {
+    if (h[kCntBad] == 2) {
         snprintf(c->err, sizeof(c->err), "build_cp: a surface point, triangle or edge names a vertex outside the mesh");
         return SGIPC_BAD_INPUT;
     }
-    if (w.h_counts[3]) {
+    if (h[kCntBad]) {
         snprintf(c->err, sizeof(c->err), "build_cp: the scene spans more than 2^%d grid cells along an axis",
                  kCellBits);
         return SGIPC_BAD_INPUT;
@@ -779,42 +962,22 @@ extern "C" SgipcStatus sgipc_build_cp(SgipcCtx* c, const double* x, const double
                  total, cap, ng, ground_cap);
         return SGIPC_CAPACITY;
     }
-    int4* P = reinterpret_cast<int4*>(pairs);
-    int4* Q = reinterpret_cast<int4*>(ccd_pairs);
-    // group codes of the final order, kept in gscan (an int per record fits) until they move to
-    // mat_index; gscan then takes the packed flags
-    int* group = reinterpret_cast<int*>(w.gscan);
-    if (nq > 0) {
-        SG_COUNT(c, 1);
-        k_query<true><<<nblk(nq, kQueryThreads), kQueryThreads, 0, s>>>(qa, nullptr, w.offs, P, Q, group, w.rec_pair, w.rec_ccd, w.reckey,
-                                               w.recidx);
+    for (int k = 0; k < 3; k++) h_cp_num[2 + k] = h[kCntSize + k];
+    if (total + ng > 0) {
+        size_t t = w.cub_bytes;
+        SG_CHECK(c, cub::DeviceRadixSort::SortKeys(w.cub, t, w.reckey, w.reckey_s, total + ng, 0, qa.kshift + 2, s));
     }
-    const int nee = total - npt;
-    if (nee > 0) {
-        t = w.cub_bytes;
-        SG_CHECK(c, cub::DeviceRadixSort::SortPairs(w.cub, t, w.reckey, w.reckey_s, w.recidx, w.recidx_s, nee, 0, 64,
-                                                    s));
-        SG_COUNT(c, 1);
-        k_gather_ee<<<nblk(nee), SGIPC_BLOCK, 0, s>>>(nee, npt, w.recidx_s, w.rec_pair, w.rec_ccd, P, Q, group);
-    }
-    // ranks per Hessian size: the group codes move to mat_index first (gscan is rewritten)
+    SG_COUNT(c, 2);
+    k_emit<<<nblk(total + ng > 0 ? total + ng : 1, 128), 128, 0, s>>>(
+        qa, total, ng, w.reckey_s, reinterpret_cast<int4*>(pairs), reinterpret_cast<int4*>(ccd_pairs), mat_index,
+        w.gscan, ground_pairs, gp_num);
+    // ranks per Hessian size (the unsorted records are no longer needed: their buffer takes the scan)
     if (total > 0) {
-        SG_CHECK(c, cudaMemcpyAsync(mat_index, group, sizeof(int) * (size_t)total, cudaMemcpyDeviceToDevice, s));
-        SG_COUNT(c, 1);
-        k_group_flags<<<nblk(total), SGIPC_BLOCK, 0, s>>>(total, mat_index, w.gscan);
-        t = w.cub_bytes;
+        size_t t = w.cub_bytes;
         SG_CHECK(c, cub::DeviceScan::ExclusiveSum(w.cub, t, w.gscan, w.reckey, total, s));
     }
-    SG_COUNT(c, 1);
     k_mat_index<<<nblk(total > 0 ? total : 1), SGIPC_BLOCK, 0, s>>>(total, mat_index, w.gscan, w.reckey, cp_num);
-    if (nsv > 0) {
-        SG_COUNT(c, 1);
-        k_ground_write<<<nblk(nsv), SGIPC_BLOCK, 0, s>>>(surf->surf_verts, nsv, w.gflag, w.goff, ground_pairs, gp_num);
-    } else {
-        SG_CHECK(c, cudaMemsetAsync(gp_num, 0, sizeof(unsigned), s));
-    }
     SG_LAUNCH_CHECK(c, "build_cp");
-    SG_CHECK(c, cudaMemcpyAsync(h_cp_num, cp_num, sizeof(unsigned) * 5, cudaMemcpyDeviceToHost, s));
     SG_CHECK(c, cudaStreamSynchronize(s));
     return SGIPC_OK;
 }
@@ -831,7 +994,7 @@ extern "C" SgipcStatus sgipc_friction_setup(SgipcCtx* c, const double* x, const 
     if (ground_num > 0 && (!ground_pairs || !fric_gd_pairs || !fric_gd_lambda)) return SGIPC_BAD_INPUT;
     SG_DEVICE(c);
     cudaStream_t s = (cudaStream_t)stream;
-    SgipcStatus st = broad_reserve(c, pair_num, 0, 0, pair_num);  // flags / offsets over the pairs
+    SgipcStatus st = broad_reserve(c, 0, 0, 0, 0, pair_num);  // flags / offsets over the pairs
     if (st != SGIPC_OK) return st;
     BroadWork& w = *c->broad;
     SG_CHECK(c, cudaMemsetAsync(cp_num_last, 0, sizeof(unsigned) * 5, s));

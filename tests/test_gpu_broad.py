@@ -182,3 +182,46 @@ def test_capacity_is_reported():
         assert out["cp_num"][0] == len(sc.pairs)
     finally:
         g.close()
+
+
+def _soup_scene(kind, n, seed):
+    """Loose triangles (``n`` of them, each a body of its own): ``mixed`` scatters sizes over a
+    factor of 200, ``stack`` piles equal ones 0.3 d-hat apart, ``flat`` puts all in one plane."""
+    rng = np.random.default_rng(seed)
+    dhat = 1e-3
+    size = 10.0 ** rng.uniform(-3, -0.7, n) if kind == "mixed" else np.full(n, 5e-3)
+    centre = rng.uniform(0.0, 0.02, (n, 3))
+    if kind == "stack":
+        centre = np.stack([rng.uniform(0, 5e-3, n), 0.3 * dhat * np.arange(n), rng.uniform(0, 5e-3, n)], 1)
+    tri = centre[:, None] + size[:, None, None] * rng.uniform(-1.0, 1.0, (n, 3, 3))
+    if kind != "mixed":
+        tri[:, :, 1] = centre[:, None, 1] if kind == "stack" else 0.01
+    verts = tri.reshape(-1, 3) + np.array([0.0, scenes.GROUND_OFFSET, 0.0])
+    bodies = [dict(verts=v.reshape(3, 3), tris=np.array([[0, 1, 2]]), affine=True) for v in verts.reshape(n, 9)]
+    # (a soft tetrahedron far away: a scene has at least one element)
+    v, t = scenes.lattice_tets(2, 0.01, (0.5, scenes.GROUND_OFFSET + 0.5, 0.5))
+    return scenes.build_tet_scene("soup", [dict(verts=v, tets=t, E=1e5)] + bodies, dt=0.01, dhat_abs=dhat,
+                                  density=1000.0, nu=0.4, mu_friction=0.0, seed=seed, perturb=0.0)
+
+
+@pytest.mark.parametrize("kind,n", [("mixed", 1), ("mixed", 10), ("mixed", 32), ("mixed", 33), ("mixed", 341),
+                                    ("mixed", 400), ("stack", 64), ("stack", 350), ("flat", 40)])
+def test_pairs_of_loose_triangles(kind, n):
+    """Remainders of the 32-wide groups and 1024-wide nodes, primitives of very different size,
+    coincident Morton codes: the same pairs and order as the host generator finds."""
+    sc = _soup_scene(kind, n, seed=n)
+    pairs, ccd = contacts.find_pairs(sc.vertexes, sc.rest_vertexes, sc.surf_tris, sc.surf_edges, sc.surf_verts,
+                                     sc.params["dHat"], sc.body_of_vertex, with_ccd=True)
+    g = system.GIPC(sc, pair_capacity=len(pairs) + 1)
+    out = g.buildCP(update=False)
+    p, c = out["pairs"].cpu().numpy(), out["ccd_pairs"].cpu().numpy()
+    assert len(p) == len(pairs)
+    if len(p):
+        assert np.array_equal(_rows_sorted(p, c), _rows_sorted(pairs, ccd))
+    _check_mat_index(p, out["mat_index"].cpu().numpy(), out["cp_num"])
+    ground = contacts.ground_pairs(sc.vertexes, sc.surf_verts, sc.params["dHat"], sc.params["ground_offset"])
+    assert np.array_equal(out["ground_pairs"].cpu().numpy(), ground)
+    if len(p) > 1:  # one place short: the counts come back, nothing is written
+        with pytest.raises(Exception, match="capacity"):
+            g.buildCP(update=False, capacity=len(p) - 1)
+    g.close()
