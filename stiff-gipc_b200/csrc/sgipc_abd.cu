@@ -11,10 +11,13 @@
 //   contacts: point gradients g -> J^T g, point blocks H_ij -> J_i^T H_ij J_j between
 //   bodies and J_i^T H_ij between a body and a FEM vertex (setup...cu:349-610);
 //   preconditioner: the inverse of each body's 12x12 diagonal block (setup...cu:612-655).
-// The B200 version: one thread per body for the body terms (the 9x9 projection by cyclic
-// Jacobi in registers / local memory), one thread per point block for the mappings, a
-// deterministic per-body gather of point gradients (points are numbered body by body), a
-// keyed radix-sort merge of the body-space blocks, Gauss-Jordan inverses per body.
+// The B200 version: one warp per body for the body terms (the 9x9 projection by Jacobi, the four
+// disjoint rotations of a round side by side in shared memory), one thread per point block for
+// the mappings, a deterministic per-body gather of point gradients (points are numbered body
+// by body), a keyed radix-sort merge of the body-space blocks summed by one warp per block, and
+// Gauss-Jordan inverses by one warp per body.  A few hundred bodies fill a fraction of the chip
+// with one thread each, and such a thread's serial chain was the whole time: at 500 bodies the
+// body terms took 219 us, the inverses 87 us and the block sums 140 us.
 #include <cub/cub.cuh>
 #include <vector>
 
@@ -56,122 +59,178 @@ __device__ void dyadic_mv(const double* dm, const double* v, double* out) {
     }
 }
 
-// cyclic Jacobi eigen-decomposition of a symmetric n x n matrix (row-major, in place:
-// A -> diag(w)); V accumulates the eigenvectors as columns
-template <int N>
-__device__ void jacobi_eig(double (&A)[N][N], double (&V)[N][N]) {
-    for (int i = 0; i < N; i++)
-        for (int j = 0; j < N; j++) V[i][j] = i == j ? 1.0 : 0.0;
+constexpr int kBodyWarps = 2;  // bodies per CTA of the warp-per-body kernels
+
+// Jacobi eigen-decomposition of a symmetric 9 x 9 matrix by one warp (A -> diag(w), V its
+// eigenvectors as columns; shared memory).  A sweep is nine rounds of four disjoint rotations
+// (the round-robin order of ten players, the tenth a bye), which commute: every pair is met once.
+__device__ void jacobi_eig9(double (*A)[9], double (*V)[9], double (*rot)[2]) {
+    const int lane = threadIdx.x & 31;
+    for (int e = lane; e < 81; e += 32) V[e / 9][e % 9] = e / 9 == e % 9 ? 1.0 : 0.0;
+    __syncwarp();
     for (int sweep = 0; sweep < 20; sweep++) {
         double off = 0.0, diag = 0.0;
-        for (int i = 0; i < N; i++) {
-            diag += A[i][i] * A[i][i];
-            for (int j = i + 1; j < N; j++) off += A[i][j] * A[i][j];
+        for (int e = lane; e < 81; e += 32) {
+            const double v = A[e / 9][e % 9];
+            if (e / 9 == e % 9) diag += v * v;
+            else if (e / 9 < e % 9) off += v * v;
         }
-        if (off <= 1e-30 * diag || off == 0.0) break;
-        for (int p = 0; p < N - 1; p++)
-            for (int q = p + 1; q < N; q++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            off += __shfl_xor_sync(0xffffffffu, off, o);
+            diag += __shfl_xor_sync(0xffffffffu, diag, o);
+        }
+        if (off <= 1e-30 * diag || off == 0.0) break;  // warp-uniform
+        for (int round = 0; round < 9; round++) {
+            // pair k of the round: players round + k and round - k (mod 9), k = 1 .. 4
+            if (lane < 4) {
+                int p = (round + lane + 1) % 9, q = (round + 8 - lane) % 9;
+                if (p > q) {
+                    const int t = p;
+                    p = q;
+                    q = t;
+                }
                 const double apq = A[p][q];
-                if (apq == 0.0) continue;
-                const double th = (A[q][q] - A[p][p]) / (2.0 * apq);
-                const double t = (th >= 0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
-                const double cs = 1.0 / sqrt(t * t + 1.0), sn = t * cs;
-                for (int k = 0; k < N; k++) {  // A <- A R (columns p, q)
-                    const double akp = A[k][p], akq = A[k][q];
-                    A[k][p] = cs * akp - sn * akq;
-                    A[k][q] = sn * akp + cs * akq;
+                double cs = 1.0, sn = 0.0;
+                if (apq != 0.0) {
+                    const double th = (A[q][q] - A[p][p]) / (2.0 * apq);
+                    const double t = (th >= 0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
+                    cs = 1.0 / sqrt(t * t + 1.0);
+                    sn = t * cs;
                 }
-                for (int k = 0; k < N; k++) {  // A <- R^T A (rows p, q)
-                    const double apk = A[p][k], aqk = A[q][k];
-                    A[p][k] = cs * apk - sn * aqk;
-                    A[q][k] = sn * apk + cs * aqk;
-                }
-                for (int k = 0; k < N; k++) {
-                    const double vkp = V[k][p], vkq = V[k][q];
-                    V[k][p] = cs * vkp - sn * vkq;
-                    V[k][q] = sn * vkp + cs * vkq;
-                }
+                rot[lane][0] = cs;
+                rot[lane][1] = sn;
             }
+            __syncwarp();
+            // columns p, q of A (tasks 0 .. 35) and V (36 .. 71), then rows p, q of A
+            for (int e = lane; e < 72; e += 32) {
+                double (*M)[9] = e < 36 ? A : V;
+                const int f = e < 36 ? e : e - 36, k = f % 9, i = f / 9;
+                int p = (round + i + 1) % 9, q = (round + 8 - i) % 9;
+                if (p > q) {
+                    const int t = p;
+                    p = q;
+                    q = t;
+                }
+                const double cs = rot[i][0], sn = rot[i][1], mp = M[k][p], mq = M[k][q];
+                M[k][p] = cs * mp - sn * mq;
+                M[k][q] = sn * mp + cs * mq;
+            }
+            __syncwarp();
+            for (int e = lane; e < 36; e += 32) {
+                const int k = e % 9, i = e / 9;
+                int p = (round + i + 1) % 9, q = (round + 8 - i) % 9;
+                if (p > q) {
+                    const int t = p;
+                    p = q;
+                    q = t;
+                }
+                const double cs = rot[i][0], sn = rot[i][1], mp = A[p][k], mq = A[q][k];
+                A[p][k] = cs * mp - sn * mq;
+                A[q][k] = sn * mp + cs * mq;
+            }
+            __syncwarp();
+        }
     }
 }
 
-// body terms: gradient (12) and the 10 upper 3x3 blocks of the 12x12 body Hessian
-__global__ void k_abd_body(int B, const double* __restrict__ q, const double* __restrict__ qt,
-                           const double* __restrict__ dmass, const double* __restrict__ vol,
-                           const int* __restrict__ bt, double kappa, double dt, double* __restrict__ grad,
-                           unsigned long long* __restrict__ key, int* __restrict__ idx, double* __restrict__ val) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
+// body terms: gradient (12) and the 10 upper 3x3 blocks of the 12x12 body Hessian; one warp per
+// body
+__global__ void __launch_bounds__(32 * kBodyWarps) k_abd_body(int B, const double* __restrict__ q,
+                                                              const double* __restrict__ qt,
+                                                              const double* __restrict__ dmass,
+                                                              const double* __restrict__ vol,
+                                                              const int* __restrict__ bt, double kappa, double dt,
+                                                              double* __restrict__ grad,
+                                                              unsigned long long* __restrict__ key,
+                                                              int* __restrict__ idx, double* __restrict__ val) {
+    __shared__ double sH[kBodyWarps][12][12], sA[kBodyWarps][9][9], sV[kBodyWarps][9][9], sR[kBodyWarps][4][2];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b = blockIdx.x * kBodyWarps + w;
+    if (b >= B) return;  // warp-uniform; no CTA barrier below
+    double (*H)[12] = sH[w];
+    double (*A)[9] = sA[w];
+    double (*V)[9] = sV[w];
     const double* dm = dmass + 13 * (size_t)b;
     double qb[12], dq[12], G[12];
     for (int k = 0; k < 12; k++) {
         qb[k] = q[12 * (size_t)b + k];
         dq[k] = qb[k] - qt[12 * (size_t)b + k];
+        G[k] = 0.0;
     }
-    double H[12][12];
-    for (int i = 0; i < 12; i++)
-        for (int j = 0; j < 12; j++) H[i][j] = 0.0;
     // dyadic mass matrix
-    for (int r = 0; r < 3; r++) {
-        H[r][r] = dm[0];
-        for (int c = 0; c < 3; c++) {
-            H[r][3 + 3 * r + c] = dm[1 + c];
-            H[3 + 3 * r + c][r] = dm[1 + c];
-            for (int d = 0; d < 3; d++) H[3 + 3 * r + c][3 + 3 * r + d] = dm[4 + 3 * c + d];
-        }
+    for (int e = lane; e < 144; e += 32) {
+        const int i = e / 12, j = e % 12;
+        double h = 0.0;
+        if (i < 3 && j < 3) h = i == j ? dm[0] : 0.0;
+        else if (i < 3) h = (j - 3) / 3 == i ? dm[1 + (j - 3) % 3] : 0.0;
+        else if (j < 3) h = (i - 3) / 3 == j ? dm[1 + (i - 3) % 3] : 0.0;
+        else if ((i - 3) / 3 == (j - 3) / 3) h = dm[4 + 3 * ((i - 3) % 3) + (j - 3) % 3];
+        H[i][j] = h;
     }
-    const bool fixed = bt[b] != 0;
-    if (fixed) {
-        for (int k = 0; k < 12; k++) G[k] = 0.0;
-    } else {
+    if (bt[b] == 0) {
         dyadic_mv(dm, dq, G);
         const double kvt2 = kappa * vol[b] * dt * dt;
         const double* a[3] = {qb + 3, qb + 6, qb + 9};
-        double Hs[9][9], V[9][9];
-        for (int i = 0; i < 3; i++) {
-            const double aii = a[i][0] * a[i][0] + a[i][1] * a[i][1] + a[i][2] * a[i][2];
+        double aa[3][3];
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int j = 0; j < 3; j++) aa[i][j] = a[i][0] * a[j][0] + a[i][1] * a[j][1] + a[i][2] * a[j][2];
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
             for (int p = 0; p < 3; p++) {
-                double g = 4.0 * (aii - 1.0) * a[i][p];
-                for (int j = 0; j < 3; j++) {
-                    if (j == i) continue;
-                    const double aij = a[i][0] * a[j][0] + a[i][1] * a[j][1] + a[i][2] * a[j][2];
-                    g += 4.0 * aij * a[j][p];
-                }
+                double g = 4.0 * (aa[i][i] - 1.0) * a[i][p];
+#pragma unroll
+                for (int j = 0; j < 3; j++)
+                    if (j != i) g += 4.0 * aa[i][j] * a[j][p];
                 G[3 + 3 * i + p] += kvt2 * g;
             }
-            for (int j = 0; j < 3; j++) {
-                const double aij = a[i][0] * a[j][0] + a[i][1] * a[j][1] + a[i][2] * a[j][2];
+        // every lane forms the whole matrix in registers and stores the entries of its rows
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int j = 0; j < 3; j++)
+#pragma unroll
                 for (int p = 0; p < 3; p++)
+#pragma unroll
                     for (int r = 0; r < 3; r++) {
                         double h;
                         if (i == j) {
-                            h = 8.0 * a[i][p] * a[i][r] + (p == r ? 4.0 * (aii - 1.0) : 0.0);
+                            h = 8.0 * a[i][p] * a[i][r] + (p == r ? 4.0 * (aa[i][i] - 1.0) : 0.0);
+#pragma unroll
                             for (int k = 0; k < 3; k++)
                                 if (k != i) h += 4.0 * a[k][p] * a[k][r];
                         } else {
-                            h = 4.0 * a[j][p] * a[i][r] + (p == r ? 4.0 * aij : 0.0);
+                            h = 4.0 * a[j][p] * a[i][r] + (p == r ? 4.0 * aa[i][j] : 0.0);
                         }
-                        Hs[3 * i + p][3 * j + r] = kvt2 * h;
+                        if (lane == 3 * i + p) A[3 * i + p][3 * j + r] = kvt2 * h;
                     }
-            }
+        __syncwarp();
+        jacobi_eig9(A, V, sR[w]);
+        for (int e = lane; e < 81; e += 32) {
+            const int i = e / 9, j = e % 9;
+            double s = 0.0;
+            for (int k = 0; k < 9; k++)
+                if (A[k][k] > 0.0) s += V[i][k] * A[k][k] * V[j][k];
+            H[3 + i][3 + j] += s;
         }
-        jacobi_eig<9>(Hs, V);
-        for (int i = 0; i < 9; i++)
-            for (int j = 0; j < 9; j++) {
-                double s = 0.0;
-                for (int k = 0; k < 9; k++)
-                    if (Hs[k][k] > 0.0) s += V[i][k] * Hs[k][k] * V[j][k];
-                H[3 + i][3 + j] += s;
-            }
     }
-    for (int k = 0; k < 12; k++) grad[12 * (size_t)b + k] = G[k];
-    const int pa[10] = {0, 0, 0, 0, 1, 1, 1, 2, 2, 3}, pb[10] = {0, 1, 2, 3, 1, 2, 3, 2, 3, 3};
-    for (int s = 0; s < 10; s++) {
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 12; k++)
+        if (lane == k) grad[12 * (size_t)b + k] = G[k];
+    for (int e = lane; e < 90; e += 32) {
+        const int s = e / 9, p = (e % 9) / 3, r = e % 3;
+        // upper block pairs in row order: (0,0..3), (1,1..3), (2,2..3), (3,3)
+        const int pa = s < 4 ? 0 : (s < 7 ? 1 : (s < 9 ? 2 : 3)), pb = s < 4 ? s : (s < 7 ? s - 3 : (s < 9 ? s - 5 : 3));
         const size_t o = 10 * (size_t)b + s;
-        key[o] = bkey(4 * b + pa[s], 4 * b + pb[s]);
-        idx[o] = (int)o;
-        for (int p = 0; p < 3; p++)
-            for (int r = 0; r < 3; r++) val[9 * o + 3 * p + r] = H[3 * pa[s] + p][3 * pb[s] + r];
+        if (p == 0 && r == 0) {
+            key[o] = bkey(4 * b + pa, 4 * b + pb);
+            idx[o] = (int)o;
+        }
+        val[9 * o + 3 * p + r] = H[3 * pa + p][3 * pb + r];
     }
 }
 
@@ -310,21 +369,50 @@ __global__ void k_heads(int m, const unsigned long long* __restrict__ ks, int* _
     flag[i] = (k != kNoKey && (i == 0 || ks[i - 1] != k)) ? 1 : 0;
 }
 
-__global__ void k_reduce(int m, const unsigned long long* __restrict__ ks, const int* __restrict__ is,
-                         const int* __restrict__ uid, const double* __restrict__ val, int* __restrict__ ur,
-                         int* __restrict__ uc, double* __restrict__ uv, int* __restrict__ nu) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) nu[0] = uid[m];
-    if (i >= m) return;
-    const unsigned long long k = ks[i];
-    if (k == kNoKey || (i > 0 && ks[i - 1] == k)) return;
-    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int j = i; j < m && ks[j] == k; j++)
-        for (int q = 0; q < 9; q++) acc[q] += val[9 * (size_t)is[j] + q];
+// first sorted slot, row and column of each unique block; start[nu] = end of the last run
+__global__ void k_starts(int m, const unsigned long long* __restrict__ ks, const int* __restrict__ uid,
+                         int* __restrict__ start, int* __restrict__ ur, int* __restrict__ uc, int* __restrict__ nu) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > m) return;
+    const unsigned long long k = i < m ? ks[i] : kNoKey, prev = i > 0 ? ks[i - 1] : kNoKey;
+    if (k == kNoKey) {  // the unused slots sort last: the first of them, or m, ends the last run
+        if (i == 0 || prev != kNoKey) {
+            nu[0] = uid[m];
+            start[uid[m]] = i;
+        }
+        return;
+    }
+    if (i > 0 && prev == k) return;
     const int u = uid[i];
+    start[u] = i;
     ur[u] = (int)(k >> 32);
     uc[u] = (int)(k & 0xffffffffull);
-    for (int q = 0; q < 9; q++) uv[9 * (size_t)u + q] = acc[q];
+}
+
+// Unique blocks, one warp each: lane l adds the run's slots l, l + 32, ... in order, then a fixed
+// xor tree (a body's diagonal blocks collect hundreds of contact blocks)
+__global__ void __launch_bounds__(256) k_reduce(const int* __restrict__ nu, const int* __restrict__ start,
+                                                const int* __restrict__ is, const double* __restrict__ val,
+                                                double* __restrict__ uv) {
+    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5, n = nu[0];
+    for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += nw) {
+        const int j1 = start[u + 1];
+        double acc[9];
+#pragma unroll
+        for (int q = 0; q < 9; q++) acc[q] = 0.0;
+        for (int j = start[u] + lane; j < j1; j += 32) {
+            const double* v = val + 9 * (size_t)is[j];
+#pragma unroll
+            for (int q = 0; q < 9; q++) acc[q] += v[q];
+        }
+#pragma unroll
+        for (int q = 0; q < 9; q++)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+#pragma unroll
+        for (int q = 0; q < 9; q++)
+            if (lane == q) uv[9 * (size_t)u + q] = acc[q];
+    }
 }
 
 // body diagonal groups of the merged matrix into dense 12x12 blocks (both triangles)
@@ -344,40 +432,55 @@ __global__ void k_pfill(const int* __restrict__ nu, const int* __restrict__ ur, 
         }
 }
 
-// in-place Gauss-Jordan inverse with partial pivoting, one thread per body
-__global__ void k_pinv(int B, double* __restrict__ Pm) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    double A[12][24];
-    const double* M = Pm + 144 * (size_t)b;
-    for (int i = 0; i < 12; i++)
-        for (int j = 0; j < 12; j++) {
-            A[i][j] = M[12 * i + j];
-            A[i][12 + j] = i == j ? 1.0 : 0.0;
-        }
+// in-place Gauss-Jordan inverse with partial pivoting, one warp per body ([A | I] in shared
+// memory; the elementwise operations and the pivot rule of a serial elimination)
+__global__ void __launch_bounds__(32 * kBodyWarps) k_pinv(int B, double* __restrict__ Pm) {
+    __shared__ double sA[kBodyWarps][12][25];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b = blockIdx.x * kBodyWarps + w;
+    if (b >= B) return;  // warp-uniform; no CTA barrier below
+    double (*A)[25] = sA[w];
+    double* M = Pm + 144 * (size_t)b;
+    for (int e = lane; e < 288; e += 32) {
+        const int i = e / 24, j = e % 24;
+        A[i][j] = j < 12 ? M[12 * i + j] : (i == j - 12 ? 1.0 : 0.0);
+    }
+    __syncwarp();
     for (int c = 0; c < 12; c++) {
+        // the largest |A(i, c)|, i >= c; the lowest row of equal ones.  A NaN never wins against
+        // the row before it, nor loses to one behind it: the serial rule of `>`, row by row
         int piv = c;
-        for (int i = c + 1; i < 12; i++)
-            if (fabs(A[i][c]) > fabs(A[piv][c])) piv = i;
-        if (piv != c)
-            for (int j = 0; j < 24; j++) {
-                const double t = A[c][j];
-                A[c][j] = A[piv][j];
-                A[piv][j] = t;
+        {
+            double best = fabs(A[c][c]);
+            for (int i = c + 1; i < 12; i++) {
+                const double v = fabs(A[i][c]);
+                if (v > best) best = v, piv = i;
             }
+        }
+        __syncwarp();
+        if (piv != c && lane < 24) {
+            const double t = A[c][lane];
+            A[c][lane] = A[piv][lane];
+            A[piv][lane] = t;
+        }
+        __syncwarp();
         const double d = A[c][c];
         const double inv = d != 0.0 ? 1.0 / d : 0.0;
-        for (int j = 0; j < 24; j++) A[c][j] *= inv;
-        for (int i = 0; i < 12; i++) {
-            if (i == c) continue;
-            const double f = A[i][c];
-            if (f == 0.0) continue;
-            for (int j = 0; j < 24; j++) A[i][j] -= f * A[c][j];
+        __syncwarp();
+        if (lane < 24) A[c][lane] *= inv;
+        __syncwarp();
+        double f[9];
+#pragma unroll
+        for (int u = 0; u < 9; u++) f[u] = A[(lane + 32 * u) / 24][c];
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 9; u++) {
+            const int i = (lane + 32 * u) / 24, j = (lane + 32 * u) % 24;
+            if (i != c && f[u] != 0.0) A[i][j] -= f[u] * A[c][j];
         }
+        __syncwarp();
     }
-    double* O = Pm + 144 * (size_t)b;
-    for (int i = 0; i < 12; i++)
-        for (int j = 0; j < 12; j++) O[12 * i + j] = A[i][12 + j];
+    for (int e = lane; e < 144; e += 32) M[e] = A[e / 12][12 + e % 12];
 }
 
 __global__ void k_papply(int B, const double* __restrict__ Pm, const double* __restrict__ r, double* __restrict__ z) {
@@ -414,10 +517,12 @@ extern "C" SgipcStatus sgipc_abd_destroy(SgipcAbdCtx* c) {
     sgipc::DeviceScope dev_scope(c->device);
     void* ps[] = {c->point_body, c->body_ptr, c->bt, c->x_bar, c->dmass, c->vol, c->key, c->key_s, c->idx,
                   c->idx_s, c->val, c->flag, c->nu, c->u_row, c->u_col, c->u_val, c->pinv, c->cub_tmp,
-                  c->g_rptr, c->g_cptr, c->g_tkey, c->g_tkey_s, c->g_tidx, c->g_tidx_s, c->g_vec, c->g_dot,
+                  c->g_rptr, c->g_cptr, c->g_tkey, c->g_tkey_s, c->g_tidx, c->g_tidx_s, c->g_vec, c->g_part, c->g_dot,
                   c->g_cub};
     for (void* p : ps)
         if (p) cudaFree(p);
+    for (cudaEvent_t e : c->g_ev)
+        if (e) cudaEventDestroy(e);
     delete c;
     return SGIPC_OK;
 }
@@ -485,7 +590,7 @@ extern "C" SgipcStatus sgipc_abd_grad_hess(SgipcAbdCtx* c, const double* q, cons
     const int B = c->B;
     AB_CHECK(c, cudaMemsetAsync(c->flag + c->cap, 0, sizeof(int), s));  // input-error word
     int* eflag = c->flag + c->cap;
-    k_abd_body<<<nblk(B, 64), 64, 0, s>>>(B, q, qt, c->dmass, c->vol, c->bt, kappa, dt, body_grad, c->key, c->idx,
+    k_abd_body<<<nblk(B, kBodyWarps), 32 * kBodyWarps, 0, s>>>(B, q, qt, c->dmass, c->vol, c->bt, kappa, dt, body_grad, c->key, c->idx,
                                           c->val);
     if (point_grad && c->P)
         k_abd_point_grad<<<nblk(B, 128), 128, 0, s>>>(B, c->body_ptr, c->bt, c->x_bar, point_grad, body_grad);
@@ -501,7 +606,11 @@ extern "C" SgipcStatus sgipc_abd_grad_hess(SgipcAbdCtx* c, const double* q, cons
     const int m = base;
     c->m_last = m;
     size_t tb = c->cub_bytes;
-    AB_CHECK(c, cub::DeviceRadixSort::SortPairs(c->cub_tmp, tb, c->key, c->key_s, c->idx, c->idx_s, m, 0, 64, s));
+    // columns in the low 32 bits, then rows < 4B; the unused-slot key's row bits, all ones, sort last
+    int row_bits = 1;
+    while ((1LL << row_bits) <= 4LL * B) row_bits++;
+    AB_CHECK(c, cub::DeviceRadixSort::SortPairs(c->cub_tmp, tb, c->key, c->key_s, c->idx, c->idx_s, m, 0,
+                                                32 + row_bits, s));
     // the scan input/output must not overlap the error word: heads for m entries + 1
     int hflag = 0;
     AB_CHECK(c, cudaMemcpyAsync(&hflag, eflag, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -513,8 +622,11 @@ extern "C" SgipcStatus sgipc_abd_grad_hess(SgipcAbdCtx* c, const double* q, cons
     k_heads<<<nblk(m + 1), SGIPC_BLOCK, 0, s>>>(m, c->key_s, c->flag);
     tb = c->cub_bytes;
     AB_CHECK(c, cub::DeviceScan::ExclusiveSum(c->cub_tmp, tb, c->flag, c->flag, m + 1, s));
-    k_reduce<<<nblk(m), SGIPC_BLOCK, 0, s>>>(m, c->key_s, c->idx_s, c->flag, c->val, c->u_row, c->u_col, c->u_val,
-                                             c->nu);
+    // (the unsorted keys' buffer is free: it takes the run starts, m + 1 ints at most)
+    int* start = reinterpret_cast<int*>(c->key);
+    k_starts<<<nblk(m + 1), SGIPC_BLOCK, 0, s>>>(m, c->key_s, c->flag, start, c->u_row, c->u_col, c->nu);
+    k_reduce<<<nblk(32LL * m) < 8 * 148 ? nblk(32LL * m) : 8 * 148, SGIPC_BLOCK, 0, s>>>(c->nu, start, c->idx_s,
+                                                                                        c->val, c->u_val);
     AB_CHECK(c, cudaGetLastError());
     c->assembled = 1;
     c->pbuilt = 0;
@@ -548,7 +660,7 @@ extern "C" SgipcStatus sgipc_abd_precond_build(SgipcAbdCtx* c, void* stream) {
     AB_CHECK(c, cudaMemsetAsync(c->pinv, 0, sizeof(double) * 144 * c->B, s));
     k_pfill<<<nblk(c->m_last > 0 ? c->m_last : 1), SGIPC_BLOCK, 0, s>>>(c->nu, c->u_row, c->u_col, c->u_val, c->B,
                                                                        c->pinv);
-    k_pinv<<<nblk(c->B, 64), 64, 0, s>>>(c->B, c->pinv);
+    k_pinv<<<nblk(c->B, kBodyWarps), 32 * kBodyWarps, 0, s>>>(c->B, c->pinv);
     AB_CHECK(c, cudaGetLastError());
     c->pbuilt = 1;
     return SGIPC_OK;
@@ -562,8 +674,4 @@ extern "C" SgipcStatus sgipc_abd_precond_apply(SgipcAbdCtx* c, const double* r, 
     k_papply<<<nblk(12LL * c->B), SGIPC_BLOCK, 0, (cudaStream_t)stream>>>(c->B, c->pinv, r, z);
     AB_CHECK(c, cudaGetLastError());
     return SGIPC_OK;
-}
-
-void sgipc::abd_precond_apply_async(SgipcAbdCtx* c, const double* r, double* z, cudaStream_t s) {
-    k_papply<<<nblk(12LL * c->B), SGIPC_BLOCK, 0, s>>>(c->B, c->pinv, r, z);
 }

@@ -40,13 +40,11 @@ struct SgipcAbdCtx {
     unsigned long long* g_tkey_s;
     int* g_tidx;
     int* g_tidx_s;
-    double* g_vec;       // r, z, p, Ap of the global vector
-    double* g_dot;       // device scalars
+    double* g_vec;       // r, z, two p, Ap of the global vector
+    double* g_part;      // per-CTA partial sums of the dot products
+    double* g_dot;       // device scalars and the loop's state
+    cudaEvent_t g_ev[2];  // an iteration's state is on the host
     void* g_cub;
     size_t g_cub_bytes;
 };
 
-namespace sgipc {
-// z_b = P_b^-1 r_b for every body (the ABD block Jacobi of the last precond build), on s
-void abd_precond_apply_async(SgipcAbdCtx* c, const double* r, double* z, cudaStream_t s);
-}  // namespace sgipc

@@ -15,19 +15,21 @@
 // dx = J(x_bar) dq (ABDLinearSubsystem::retrieve_solution, abd_linear_subsystem.cu:33-56,
 // cal_x_from_q.cu:34-66 forms J q - J (q - dq), the same quantity).
 //
-// B200 layout: the FEM rows run the FEM context's SpMV and MAS unchanged; the body rows
-// (a few thousand block rows at the C4 size) are one thread per block row over the row-
-// sorted merged blocks and a column-sorted index of their transposes, so every output is
-// summed in a fixed order (no atomics).  The loop's scalars (alpha, beta, the stop tests) live on
-// the device: small kernels compute them from the dot products and the vector kernels read
-// them, so the host reads the state back once per iteration, after the update and its stop
-// tests (the reference reads two scalars back per iteration).  Enqueuing several iterations per
-// read-back (the kernels after a stop return at once) measured slower on the affine-body bed:
-// its solves take about six iterations, and the preconditioner and SpMV of the iterations past
-// the stop cost more than the read-backs saved.
+// B200 layout: one kernel multiplies: FEM rows as the FEM context's SpMV (four lanes a row,
+// contact lists included) with their transposed coupling blocks, body rows by one warp each over
+// the row-sorted merged blocks and a column-sorted index of their transposes, so every output is
+// summed in a fixed order (no atomics).  It forms p = z + beta p_old where it reads it and p.Ap
+// with it; the kernel that prolongs the MAS and applies the bodies' block Jacobi also takes r.z.
+// The last CTA of each adds the partial sums in order and writes the loop's scalars (alpha,
+// beta, the stop tests), which live on the device.  The host enqueues one iteration ahead and
+// then waits for the state of the one before: the kernels of an iteration after the stop return
+// at once, so that the read-back costs no idle time and the last iteration a few empty launches.
+// (Sixteen launches an iteration and a wait after each: 2.17 ms for 500 boxes over a bed; the
+// body rows with one thread each took 28 us, the coupling 13 us.)
 #include <cub/cub.cuh>
 
 #include "sgipc_abd_ctx.cuh"
+#include "sgipc_pcg_dev.cuh"
 
 using namespace sgipc;
 
@@ -59,138 +61,267 @@ __global__ void k_g_rowptr(int nrows, const int* __restrict__ nu, const int* __r
     if (r <= nrows) rptr[r] = lower_bound_i(u_row, nu[0], r);
 }
 
-// transposed index: the off-diagonal blocks keyed by (col, row); diagonal blocks and unused
-// slots sort past every column
-__global__ void k_g_tkeys(int cap, const int* __restrict__ nu, const int* __restrict__ u_row,
+// transposed index: the off-diagonal blocks keyed by (col, row), the row in `bits` bits; diagonal
+// blocks, unused slots and columns beyond the FEM rows sort past every column
+__global__ void k_g_tkeys(int m, int bits, int ncols, const int* __restrict__ nu, const int* __restrict__ u_row,
                           const int* __restrict__ u_col, unsigned long long* __restrict__ key, int* __restrict__ idx) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= cap) return;
-    const bool off = k < nu[0] && u_row[k] != u_col[k];
-    key[k] = off ? (((unsigned long long)(unsigned)u_col[k] << 32) | (unsigned)u_row[k]) : ~0ull;
+    if (k >= m) return;
+    const bool off = k < nu[0] && u_row[k] != u_col[k] && (unsigned)u_col[k] < (unsigned)ncols;
+    key[k] = off ? (((unsigned long long)(unsigned)u_col[k] << bits) | (unsigned)u_row[k]) : ~0ull;
     idx[k] = k;
 }
 
-__global__ void k_g_colptr(int ncols, int m, const unsigned long long* __restrict__ key_s, int* __restrict__ cptr) {
+__global__ void k_g_colptr(int ncols, int m, int bits, const unsigned long long* __restrict__ key_s,
+                           int* __restrict__ cptr) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c <= ncols) cptr[c] = lower_bound_k(key_s, m, (unsigned long long)(unsigned)c << 32);
+    if (c <= ncols) cptr[c] = lower_bound_k(key_s, m, (unsigned long long)(unsigned)c << bits);
 }
 
-__device__ __forceinline__ void block_mv(const double* V, const double* x, double (&y)[3]) {
+__device__ __forceinline__ void block_mv(const double* V, const double (&x)[3], double (&y)[3]) {
     y[0] += V[0] * x[0] + V[1] * x[1] + V[2] * x[2];
     y[1] += V[3] * x[0] + V[4] * x[1] + V[5] * x[2];
     y[2] += V[6] * x[0] + V[7] * x[1] + V[8] * x[2];
 }
 
-__device__ __forceinline__ void block_mtv(const double* V, const double* x, double (&y)[3]) {
+__device__ __forceinline__ void block_mtv(const double* V, const double (&x)[3], double (&y)[3]) {
     y[0] += V[0] * x[0] + V[3] * x[1] + V[6] * x[2];
     y[1] += V[1] * x[0] + V[4] * x[1] + V[7] * x[2];
     y[2] += V[2] * x[0] + V[5] * x[1] + V[8] * x[2];
 }
 
-// y[r] for the body rows: the row's blocks times x, then the transposed blocks whose column
-// is r (global block indices; x, y global vectors)
-__global__ void k_g_body_rows(int nrows, const int* __restrict__ rptr, const int* __restrict__ cptr,
-                              const int* __restrict__ tidx, const int* __restrict__ u_row,
-                              const int* __restrict__ u_col, const double* __restrict__ u_val,
-                              const double* __restrict__ x, double* __restrict__ y) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nrows) return;
-    double acc[3] = {0.0, 0.0, 0.0};
-    for (int k = rptr[r]; k < rptr[r + 1]; k++) block_mv(u_val + 9 * (size_t)k, x + 3 * (size_t)u_col[k], acc);
-    for (int j = cptr[r]; j < cptr[r + 1]; j++) {
-        const int k = tidx[j];
-        block_mtv(u_val + 9 * (size_t)k, x + 3 * (size_t)u_row[k], acc);
-    }
-    for (int q = 0; q < 3; q++) y[3 * (size_t)r + q] = acc[q];
-}
-
-// FEM rows: add the transposed coupling blocks (body row, FEM column) to the FEM SpMV's y
-__global__ void k_g_fem_coupling(int nfem, int off, const int* __restrict__ cptr, const int* __restrict__ tidx,
-                                 const int* __restrict__ u_row, const double* __restrict__ u_val,
-                                 const double* __restrict__ x, double* __restrict__ y) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= nfem) return;
-    const int c = off + v;
-    const int j0 = cptr[c], j1 = cptr[c + 1];
-    if (j0 == j1) return;
-    double acc[3] = {0.0, 0.0, 0.0};
-    for (int j = j0; j < j1; j++) {
-        const int k = tidx[j];
-        block_mtv(u_val + 9 * (size_t)k, x + 3 * (size_t)u_row[k], acc);
-    }
-    for (int q = 0; q < 3; q++) y[3 * (size_t)c + q] += acc[q];
-}
-
-// Device state of the loop (PCGSolver::pcg's scalars).  halt: 0 running, 1 stopped (converged
-// or broken down), 2 stopped at the iteration cap.
+// Device state of the loop (PCGSolver::pcg's scalars).  stop: 0 running, 1 converged or broken
+// down, 2 at the iteration cap; an iteration that finds it set does nothing.
 struct GState {
-    double rz0, rz, bn2, alpha, beta;
-    int iters, halt, status, stop;
+    double rz0, rz, bn2, alpha, beta, res2;
+    int iters, halt, status, stop;  // halt: alpha is not usable, the update of this iteration is skipped
 };
-// dot-product slots: d[0] p.Ap, d[1] r.r, d[2] r.z (new), d[3] r0.z0, d[4] b.b, d[5] residual^2;
-// the state from d + kStateOff
-constexpr int kStateOff = 16;
+constexpr int kGThreads = 256;
+constexpr int kGBodyRows = kGThreads / 32;        // body rows per CTA of the SpMV
+constexpr int kGFemRows = kGThreads / kSpG;       // FEM rows per CTA
 
-__global__ void k_g_start(GState* st, const double* __restrict__ d) {
-    const double rz0 = d[3];
-    const bool run = rz0 > 0.0 && isfinite(rz0);
-    st->rz0 = st->rz = rz0;
-    st->bn2 = d[4];
-    st->alpha = st->beta = 0.0;
-    st->iters = 0;
-    st->stop = 0;
-    st->halt = run ? 0 : 1;
-    st->status = (!run && (!isfinite(rz0) || rz0 < 0.0)) ? SGIPC_BREAKDOWN : SGIPC_OK;
+// Adds v over the grid: per-CTA partials, and the last CTA to arrive adds them (each thread its
+// strided share in order, then fixed trees).  True in the last CTA's thread 0, with the total.
+__device__ bool grid_total(double v, double* part, unsigned int* ticket, double& total) {
+    __shared__ double smem[32];
+    __shared__ bool s_last;
+    double a[1] = {v};
+    block_sum<1>(a, smem);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = a[0];
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return false;
+    __threadfence();
+    a[0] = 0.0;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) a[0] += __ldcg(part + k);
+    block_sum<1>(a, smem);
+    if (threadIdx.x != 0) return false;
+    *ticket = 0u;
+    total = a[0];
+    return true;
 }
 
-// alpha = r.z / p.Ap of iteration k; the r.z test of the current iterate (the reference stops
-// after this iteration's update)
-__global__ void k_g_alpha(GState* st, const double* __restrict__ d, int k, int crit, double tol) {
-    if (st->halt) return;
-    const double pAp = d[0];
+struct GMat {
+    Topo tp;
+    MatView<double> A;
+    int nb, nfem;  // body block rows, FEM block rows
+    const int* rptr;
+    const int* cptr;
+    const int* tidx;
+    const int* u_row;
+    const int* u_col;
+    const double* u_val;
+};
+
+// kResidual = false: p = z + beta p_old (p = z in the first iteration), y = A p, alpha = r.z / p.Ap and
+// the stop tests of iteration k.  kResidual = true: y = b - A z, y.y into st->res2.
+template <bool kResidual>
+__global__ void __launch_bounds__(kGThreads) k_g_spmv(GMat g, GState* st, const double* __restrict__ z,
+                                                      const double* __restrict__ p_old, double* __restrict__ p,
+                                                      double* __restrict__ y, const double* __restrict__ b, int k,
+                                                      int crit, double tol, int max_iter, double* part,
+                                                      unsigned int* ticket) {
+    if (!kResidual && (st->stop || st->halt)) return;
+    const int lane = threadIdx.x & 31;
+    const int body_ctas = (g.nb + kGBodyRows - 1) / kGBodyRows;
+    Operand<double, 1> op;
+    op.a = z;
+    op.b = p_old;
+    op.beta[0] = kResidual ? 0.0 : st->beta;
+    double dot = 0.0;
+    int row = -1;            // the global block row this thread finishes
+    double acc[1][3] = {{0.0, 0.0, 0.0}};
+    if ((int)blockIdx.x < body_ctas) {
+        const int r = blockIdx.x * kGBodyRows + (int)(threadIdx.x >> 5);
+        if (r < g.nb) {
+            const int k0 = g.rptr[r], n0 = g.rptr[r + 1] - k0, j0 = g.cptr[r], n = n0 + g.cptr[r + 1] - j0;
+            for (int e = lane; e < n; e += 32) {
+                const bool up = e < n0;
+                const int u = up ? k0 + e : g.tidx[j0 + e - n0];
+                double xj[1][3];
+                op.load(up ? g.u_col[u] : g.u_row[u], xj);
+                if (up) block_mv(g.u_val + 9 * (size_t)u, xj[0], acc[0]);
+                else block_mtv(g.u_val + 9 * (size_t)u, xj[0], acc[0]);
+            }
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) acc[0][q] += __shfl_xor_sync(0xffffffffu, acc[0][q], o);
+            if (lane == 0) row = r;
+        }
+    } else {
+        const int t = (blockIdx.x - body_ctas) * kGThreads + threadIdx.x;
+        const int i = t / kSpG, l = t % kSpG;
+        Operand<double, 1> fo = op;  // FEM columns are counted from the FEM vector's start
+        fo.a = z + 3 * (size_t)g.nb;
+        fo.b = p_old ? p_old + 3 * (size_t)g.nb : nullptr;
+        row_mv<double, 1>(g.tp, g.A, fo, i, l, acc);
+        int j0 = 0, j1 = 0;
+        if (i < g.nfem) j0 = g.cptr[g.nb + i], j1 = g.cptr[g.nb + i + 1];
+        if (__any_sync(0xffffffffu, j0 < j1)) {
+            double c3[3] = {0.0, 0.0, 0.0};
+            for (int j = j0 + l; j < j1; j += kSpG) {
+                const int u = g.tidx[j];
+                double xj[1][3];
+                op.load(g.u_row[u], xj);
+                block_mtv(g.u_val + 9 * (size_t)u, xj[0], c3);
+            }
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+#pragma unroll
+                for (int o = 1; o < kSpG; o <<= 1) c3[q] += __shfl_xor_sync(0xffffffffu, c3[q], o, kSpG);
+                acc[0][q] += c3[q];
+            }
+        }
+        if (i < g.nfem && l == 0) row = g.nb + i;
+    }
+    if (row >= 0) {
+        double x3[1][3];
+        if (!kResidual) op.load(row, x3);
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const size_t e = 3 * (size_t)row + q;
+            if (kResidual) {
+                const double r = b[e] - acc[0][q];
+                y[e] = r;
+                dot += r * r;
+            } else {
+                p[e] = x3[0][q];
+                y[e] = acc[0][q];
+                dot += x3[0][q] * acc[0][q];
+            }
+        }
+    }
+    double total;
+    if (!grid_total(dot, part, ticket, total)) return;
+    if (kResidual) {
+        st->res2 = total;
+        return;
+    }
+    // alpha = r.z / p.Ap; the r.z test is that of the current iterate (the reference stops after
+    // this iteration's update), then the iteration cap
     st->iters = k;
-    if (!(pAp > 0.0) || !isfinite(pAp)) {
+    if (!(total > 0.0) || !isfinite(total)) {
         st->status = SGIPC_BREAKDOWN;
         st->halt = 1;
         return;
     }
-    st->alpha = st->rz / pAp;
-    st->stop = crit == SGIPC_CRIT_RZ && fabs(st->rz) <= tol * st->rz0;
+    st->alpha = st->rz / total;
+    if (crit == SGIPC_CRIT_RZ && fabs(st->rz) <= tol * st->rz0) st->stop = 1;
+    else if (crit == SGIPC_CRIT_RZ && k + 1 >= max_iter) st->stop = 2;
 }
 
-// after the update: the true-residual test, or the r.z one decided before it; the cap
-__global__ void k_g_after(GState* st, const double* __restrict__ d, int k, int crit, double tol, int max_iter) {
-    if (st->halt) return;
-    const bool stop = crit == SGIPC_CRIT_TRUE ? d[1] <= tol * tol * st->bn2 : st->stop != 0;
-    if (stop) st->halt = 1;
-    else if (k + 1 >= max_iter) st->halt = 2;
+// x += alpha p, r -= alpha Ap of iteration k; with the true-residual test also r.r and the stop.
+// (The stop that the SpMV of this iteration set does not skip its update: st->iters tells.)
+__global__ void __launch_bounds__(kGThreads) k_g_update(long long n, GState* st, const double* __restrict__ p,
+                                                        const double* __restrict__ Ap, double* __restrict__ x,
+                                                        double* __restrict__ r, int k, int crit, double tol,
+                                                        int max_iter, double* part, unsigned int* ticket) {
+    if (st->halt || st->iters != k) return;
+    const long long i = (long long)blockIdx.x * kGThreads + threadIdx.x;
+    double dot = 0.0;
+    if (i < n) {
+        const double alpha = st->alpha;
+        x[i] += alpha * p[i];
+        const double v = r[i] - alpha * Ap[i];
+        r[i] = v;
+        dot = v * v;
+    }
+    if (crit != SGIPC_CRIT_TRUE) return;
+    double total;
+    if (!grid_total(dot, part, ticket, total)) return;
+    if (total <= tol * tol * st->bn2) st->stop = 1;
+    else if (k + 1 >= max_iter) st->stop = 2;
 }
 
-__global__ void k_g_beta(GState* st, const double* __restrict__ d) {
-    if (st->halt) return;
-    const double rz_new = d[2];
-    st->beta = rz_new / st->rz;
-    st->rz = rz_new;
+// x = 0, r = b, b.b
+__global__ void __launch_bounds__(kGThreads) k_g_init(long long n, GState* st, const double* __restrict__ b,
+                                                      double* __restrict__ x, double* __restrict__ r, double* part,
+                                                      unsigned int* ticket) {
+    const long long i = (long long)blockIdx.x * kGThreads + threadIdx.x;
+    double v = 0.0;
+    if (i < n) {
+        v = b[i];
+        x[i] = 0.0;
+        r[i] = v;
+    }
+    double total;
+    if (!grid_total(v * v, part, ticket, total)) return;
+    *st = GState{};
+    st->bn2 = total;
 }
 
-__global__ void k_g_update(long long n, const GState* __restrict__ st, const double* __restrict__ p,
-                           const double* __restrict__ Ap, double* __restrict__ x, double* __restrict__ r) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || st->halt) return;
-    const double alpha = st->alpha;
-    x[i] += alpha * p[i];
-    r[i] -= alpha * Ap[i];
-}
-
-__global__ void k_g_direction(long long n, const GState* __restrict__ st, const double* __restrict__ z,
-                              double* __restrict__ p) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && !st->halt) p[i] = z[i] + st->beta * p[i];
-}
-
-__global__ void k_g_residual(long long n, const double* __restrict__ b, double* __restrict__ y) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = b[i] - y[i];
+// z = M^-1 r: the bodies' block Jacobi (12 x 12 inverses), the sum of the MAS levels on the FEM rows;
+// r.z, and from it beta (or, at the start, r0.z0).  One thread per block row.
+template <class M>
+__global__ void __launch_bounds__(kGThreads) k_g_precond(int nb, int nfem, GState* st, const double* __restrict__ pinv,
+                                                         const int* __restrict__ table, int L,
+                                                         const M* __restrict__ Z, const double* __restrict__ r,
+                                                         double* __restrict__ z, int start, double* part,
+                                                         unsigned int* ticket) {
+    if (!start && (st->stop || st->halt)) return;
+    const int t = blockIdx.x * kGThreads + threadIdx.x;
+    double zz[3] = {0.0, 0.0, 0.0}, dot = 0.0;
+    if (t < nb) {
+        const double* P = pinv + 144 * (size_t)(t / 4) + 36 * (t % 4);
+        const double* rb = r + 12 * (size_t)(t / 4);
+#pragma unroll
+        for (int j = 0; j < 12; j++) {
+            const double v = rb[j];
+#pragma unroll
+            for (int q = 0; q < 3; q++) zz[q] += P[12 * q + j] * v;
+        }
+    } else if (t < nb + nfem) {
+        const int* tv = table + (size_t)(t - nb) * L;
+        M s[3] = {0, 0, 0};
+        for (int l = 0; l < L; l++) {
+            const int c = tv[l];
+#pragma unroll
+            for (int q = 0; q < 3; q++) s[q] += Z[3 * (size_t)c + q];
+        }
+#pragma unroll
+        for (int q = 0; q < 3; q++) zz[q] = (double)s[q];
+    }
+    if (t < nb + nfem)
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            z[3 * (size_t)t + q] = zz[q];
+            dot += r[3 * (size_t)t + q] * zz[q];
+        }
+    double total;
+    if (!grid_total(dot, part, ticket, total)) return;
+    if (start) {
+        const bool run = total > 0.0 && isfinite(total);
+        st->rz0 = st->rz = total;
+        st->halt = run ? 0 : 1;
+        st->status = (!run && (!isfinite(total) || total < 0.0)) ? SGIPC_BREAKDOWN : SGIPC_OK;
+    } else {
+        st->beta = total / st->rz;
+        st->rz = total;
+    }
 }
 
 // dx of every ABD point: J(x_bar) dq of its body (translation + x_bar . da_r per row)
@@ -220,33 +351,29 @@ struct Global {
     long long N;
     cudaStream_t s;
     int fp32_mas;
+    GMat mat;
+    GState* st;
+    double* part;
+    unsigned int* ticket;
 };
 
-// y = A x over the global vector
-SgipcStatus g_spmv(const Global& g, const double* x, double* y) {
-    SgipcAbdCtx* a = g.a;
-    SgipcStatus st = spmv_t<double>(g.f, x + 3 * (size_t)g.nb, y + 3 * (size_t)g.nb, g.s);
+int g_spmv_grid(int nb, int nfem) { return nblk(nb, kGBodyRows) + nblk(nfem, kGFemRows); }
+
+// z = M^-1 r and the scalars that follow from r.z
+SgipcStatus g_precond(const Global& g, const double* r, double* z, bool start) {
+    const MasWork& m = g.f->mas;
+    SgipcStatus st = mas_domains(g.f, r + 3 * (size_t)g.nb, g.fp32_mas, start ? nullptr : &g.st->stop, g.s);
     if (st != SGIPC_OK) return st;
-    SG_COUNT(g.f, 2);
-    k_g_body_rows<<<nblk(g.nb, 128), 128, 0, g.s>>>(g.nb, a->g_rptr, a->g_cptr, a->g_tidx_s, a->u_row, a->u_col,
-                                                     a->u_val, x, y);
-    k_g_fem_coupling<<<nblk(g.nfem), SGIPC_BLOCK, 0, g.s>>>(g.nfem, g.nb, a->g_cptr, a->g_tidx_s, a->u_row,
-                                                             a->u_val, x, y);
-    SG_LAUNCH_CHECK(g.f, "global spmv");
-    return SGIPC_OK;
-}
-
-// z = M^-1 r: ABD block Jacobi on the body rows, MAS on the FEM rows
-SgipcStatus g_precond(const Global& g, const double* r, double* z) {
     SG_COUNT(g.f, 1);
-    abd_precond_apply_async(g.a, r, z, g.s);
-    SG_LAUNCH_CHECK(g.f, "abd block jacobi");
-    return mas_apply_t<double>(g.f, r + 3 * (size_t)g.nb, z + 3 * (size_t)g.nb, g.fp32_mas, g.s);
-}
-
-// u . v into the device slot d[slot] (no read-back)
-SgipcStatus g_dot(const Global& g, const double* u, const double* v, int slot) {
-    return dot64(g.f, u, v, (int)g.N, g.a->g_dot + slot, g.s);
+    const int grid = nblk((long long)g.nb + g.nfem, kGThreads);
+    if (g.fp32_mas)
+        k_g_precond<float><<<grid, kGThreads, 0, g.s>>>(g.nb, g.nfem, g.st, g.a->pinv, m.table, m.levelnum, m.Z32, r, z,
+                                                        start, g.part, g.ticket);
+    else
+        k_g_precond<double><<<grid, kGThreads, 0, g.s>>>(g.nb, g.nfem, g.st, g.a->pinv, m.table, m.levelnum, m.Z64, r,
+                                                         z, start, g.part, g.ticket);
+    SG_LAUNCH_CHECK(g.f, "global preconditioner");
+    return SGIPC_OK;
 }
 
 }  // namespace
@@ -265,16 +392,14 @@ extern "C" SgipcStatus sgipc_global_pcg_solve(SgipcCtx* f, SgipcAbdCtx* a, Sgipc
         return SGIPC_NOT_READY;
     }
     SG_DEVICE(f);
-    Global g{f, a, 4 * a->B, f->n, 3LL * (4LL * a->B + f->n), (cudaStream_t)stream, f->mas.built == SGIPC_FP64 + 1 ? 0 : 1};
+    Global g{f, a, 4 * a->B, f->n, 3LL * (4LL * a->B + f->n), (cudaStream_t)stream,
+             f->mas.built == SGIPC_FP64 + 1 ? 0 : 1, {}, nullptr, nullptr, nullptr};
     if (g.N > 0x7fffffffLL) return SGIPC_CAPACITY;
     if (max_iter <= 0) max_iter = (int)(0.3 * (double)g.N);
     if (max_iter < 2) max_iter = 2;
     // ---- buffers (grown on demand) and the merged blocks' row / column index
-    int nu = 0;
-    SG_CHECK(f, cudaMemcpyAsync(&nu, a->nu, sizeof(int), cudaMemcpyDeviceToHost, g.s));
-    SG_CHECK(f, cudaStreamSynchronize(g.s));
     SgipcStatus st;
-    const int ncols = g.nb + g.nfem;
+    const int ncols = g.nb + g.nfem, m = a->m_last;  // m: emitted slots, at least the unique blocks
     if (a->g_cap_blk < a->cap) {
         if ((st = grow(f, &a->g_tkey, a->cap)) || (st = grow(f, &a->g_tkey_s, a->cap)) ||
             (st = grow(f, &a->g_tidx, a->cap)) || (st = grow(f, &a->g_tidx_s, a->cap)))
@@ -290,73 +415,83 @@ extern "C" SgipcStatus sgipc_global_pcg_solve(SgipcCtx* f, SgipcAbdCtx* a, Sgipc
         a->g_cap_ptr = ncols + 1;
     }
     if (a->g_cap_vec < (size_t)g.N) {
-        if ((st = grow(f, &a->g_vec, 4 * (size_t)g.N)) || (st = grow(f, &a->g_dot, 32))) return st;
+        const int parts = std::max(g_spmv_grid(g.nb, g.nfem), nblk(g.N, kGThreads));
+        a->g_cap_vec = 0;
+        if ((st = grow(f, &a->g_vec, 5 * (size_t)g.N)) || (st = grow(f, &a->g_part, parts)) ||
+            (st = grow(f, &a->g_dot, 32)))
+            return st;
+        SG_CHECK(f, cudaMemset(a->g_dot, 0, sizeof(double) * 32));  // the ticket
         a->g_cap_vec = (size_t)g.N;
     }
+    for (cudaEvent_t& e : a->g_ev)
+        if (!e) SG_CHECK(f, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    int row_bits = 1, col_bits = 1;
+    while ((1LL << row_bits) < g.nb) row_bits++;
+    while ((1LL << col_bits) <= ncols) col_bits++;  // all ones stays above every column
     SG_COUNT(f, 3);
     k_g_rowptr<<<nblk(g.nb + 1), SGIPC_BLOCK, 0, g.s>>>(g.nb, a->nu, a->u_row, a->g_rptr);
-    k_g_tkeys<<<nblk(a->cap), SGIPC_BLOCK, 0, g.s>>>(a->cap, a->nu, a->u_row, a->u_col, a->g_tkey, a->g_tidx);
+    k_g_tkeys<<<nblk(m), SGIPC_BLOCK, 0, g.s>>>(m, row_bits, ncols, a->nu, a->u_row, a->u_col, a->g_tkey, a->g_tidx);
     size_t tb = a->g_cub_bytes;
-    SG_CHECK(f, cub::DeviceRadixSort::SortPairs(a->g_cub, tb, a->g_tkey, a->g_tkey_s, a->g_tidx, a->g_tidx_s,
-                                                nu > 0 ? nu : 1, 0, 64, g.s));
-    k_g_colptr<<<nblk(ncols + 1), SGIPC_BLOCK, 0, g.s>>>(ncols, nu, a->g_tkey_s, a->g_cptr);
+    SG_CHECK(f, cub::DeviceRadixSort::SortPairs(a->g_cub, tb, a->g_tkey, a->g_tkey_s, a->g_tidx, a->g_tidx_s, m, 0,
+                                                row_bits + col_bits, g.s));
+    k_g_colptr<<<nblk(ncols + 1), SGIPC_BLOCK, 0, g.s>>>(ncols, m, row_bits, a->g_tkey_s, a->g_cptr);
     SG_LAUNCH_CHECK(f, "global index");
 
     // ---- PCG (PCGSolver::pcg semantics, as the persistent FEM solve)
     double* r = a->g_vec;
     double* z = r + g.N;
-    double* p = z + g.N;
-    double* Ap = p + g.N;
-    const int gb = nblk(g.N);
-    double* d = a->g_dot;
-    GState* gst = reinterpret_cast<GState*>(d + kStateOff);
-    SG_CHECK(f, cudaMemsetAsync(x, 0, sizeof(double) * g.N, g.s));
-    SG_CHECK(f, cudaMemcpyAsync(r, b, sizeof(double) * g.N, cudaMemcpyDeviceToDevice, g.s));
-    if ((st = g_precond(g, r, z))) return st;
-    if ((st = g_dot(g, r, z, 3)) || (st = g_dot(g, b, b, 4))) return st;
-    SG_CHECK(f, cudaMemcpyAsync(p, z, sizeof(double) * g.N, cudaMemcpyDeviceToDevice, g.s));
+    double* p[2] = {z + g.N, z + 2 * g.N};
+    double* Ap = z + 3 * g.N;
+    const int gb = nblk(g.N, kGThreads), gs = g_spmv_grid(g.nb, g.nfem);
+    g.st = reinterpret_cast<GState*>(a->g_dot);
+    g.ticket = reinterpret_cast<unsigned int*>(a->g_dot + 24);
+    g.part = a->g_part;
+    g.mat = GMat{topo_of(f), mat_view<double>(f), g.nb, g.nfem, a->g_rptr, a->g_cptr, a->g_tidx_s, a->u_row, a->u_col,
+                 a->u_val};
+    GState* hs = reinterpret_cast<GState*>(f->h_pinned + 40);  // [2], pinned
+    static_assert(2 * sizeof(GState) <= 24 * sizeof(double) && sizeof(GState) <= 24 * sizeof(double), "state slots");
     SG_COUNT(f, 1);
-    k_g_start<<<1, 1, 0, g.s>>>(gst, d);
-    GState hs{};
-    SG_CHECK(f, cudaMemcpyAsync(&hs, gst, sizeof(hs), cudaMemcpyDeviceToHost, g.s));
-    SG_CHECK(f, cudaStreamSynchronize(g.s));
-    for (int k = 1; !hs.halt && k < max_iter; k++) {
-        if ((st = g_spmv(g, p, Ap)) || (st = g_dot(g, p, Ap, 0))) return st;
+    k_g_init<<<gb, kGThreads, 0, g.s>>>(g.N, g.st, b, x, r, g.part, g.ticket);
+    if ((st = g_precond(g, r, z, true))) return st;
+    auto iterate = [&](int k) -> SgipcStatus {
+        double* pn = p[k & 1];
+        const double* po = k == 1 ? nullptr : p[(k + 1) & 1];
         SG_COUNT(f, 2);
-        k_g_alpha<<<1, 1, 0, g.s>>>(gst, d, k, (int)crit, tol);
-        k_g_update<<<gb, SGIPC_BLOCK, 0, g.s>>>(g.N, gst, p, Ap, x, r);
-        if (crit == SGIPC_CRIT_TRUE && (st = g_dot(g, r, r, 1))) return st;
-        SG_COUNT(f, 1);
-        k_g_after<<<1, 1, 0, g.s>>>(gst, d, k, (int)crit, tol, max_iter);
+        k_g_spmv<false><<<gs, kGThreads, 0, g.s>>>(g.mat, g.st, z, po, pn, Ap, nullptr, k, (int)crit, tol, max_iter,
+                                                   g.part, g.ticket);
+        k_g_update<<<gb, kGThreads, 0, g.s>>>(g.N, g.st, pn, Ap, x, r, k, (int)crit, tol, max_iter, g.part, g.ticket);
         SG_LAUNCH_CHECK(f, "global pcg");
-        // the one read-back of the iteration: stopped (converged, broken down, at the cap)?
-        SG_CHECK(f, cudaMemcpyAsync(&hs, gst, sizeof(hs), cudaMemcpyDeviceToHost, g.s));
-        SG_CHECK(f, cudaStreamSynchronize(g.s));
-        if (hs.halt) break;
-        if ((st = g_precond(g, r, z)) || (st = g_dot(g, r, z, 2))) return st;
-        SG_COUNT(f, 2);
-        k_g_beta<<<1, 1, 0, g.s>>>(gst, d);
-        k_g_direction<<<gb, SGIPC_BLOCK, 0, g.s>>>(g.N, gst, z, p);
+        SG_CHECK(f, cudaMemcpyAsync(hs + (k & 1), g.st, sizeof(GState), cudaMemcpyDeviceToHost, g.s));
+        SG_CHECK(f, cudaEventRecord(a->g_ev[k & 1], g.s));
+        return g_precond(g, r, z, false);
+    };
+    // iteration k + 1 is enqueued before iteration k's state is awaited
+    int k = 1;
+    if ((st = iterate(1))) return st;
+    for (;; k++) {
+        const bool more = k + 1 < max_iter;
+        if (more && (st = iterate(k + 1))) return st;
+        SG_CHECK(f, cudaEventSynchronize(a->g_ev[k & 1]));
+        if (hs[k & 1].halt || hs[k & 1].stop || !more) break;
     }
-    int status = hs.status;
+    const GState fin = hs[k & 1];
+    int status = fin.status;
     // still running at the cap: not converged
-    if (status == SGIPC_OK && hs.halt != 1) status = SGIPC_NOT_CONVERGED;
+    if (status == SGIPC_OK && !fin.halt && fin.stop != 1) status = SGIPC_NOT_CONVERGED;
     // ---- true residual, distribute_solution
-    if ((st = g_spmv(g, x, Ap))) return st;
     SG_COUNT(f, 1);
-    k_g_residual<<<gb, SGIPC_BLOCK, 0, g.s>>>(g.N, b, Ap);
-    if ((st = g_dot(g, Ap, Ap, 5))) return st;
-    SG_CHECK(f, cudaMemcpyAsync(f->h_pinned, d + 5, sizeof(double), cudaMemcpyDeviceToHost, g.s));
-    SG_CHECK(f, cudaStreamSynchronize(g.s));
-    const double res2 = f->h_pinned[0], bn2 = hs.bn2;
-    const double rel = bn2 > 0 ? std::sqrt(res2 / bn2) : std::sqrt(res2);
-    const double rz0 = hs.rz0, rz = hs.rz;
-    const int iters = hs.iters;
+    k_g_spmv<true><<<gs, kGThreads, 0, g.s>>>(g.mat, g.st, x, nullptr, nullptr, Ap, b, 0, 0, 0.0, 0, g.part, g.ticket);
+    SG_CHECK(f, cudaMemcpyAsync(hs, g.st, sizeof(GState), cudaMemcpyDeviceToHost, g.s));
     if (abd_point_dx && a->P > 0) {
         SG_COUNT(f, 1);
         k_g_point_dx<<<nblk(a->P), SGIPC_BLOCK, 0, g.s>>>(a->P, a->point_body, a->x_bar, x, abd_point_dx);
-        SG_LAUNCH_CHECK(f, "abd point dx");
     }
+    SG_LAUNCH_CHECK(f, "global residual, abd point dx");
+    SG_CHECK(f, cudaStreamSynchronize(g.s));
+    const double res2 = hs->res2, bn2 = fin.bn2;
+    const double rel = bn2 > 0 ? std::sqrt(res2 / bn2) : std::sqrt(res2);
+    const double rz0 = fin.rz0, rz = fin.rz;
+    const int iters = fin.iters;
     if (stats) {
         *stats = SgipcSolveStats{};
         stats->iterations = iters;

@@ -376,6 +376,10 @@ SgipcStatus mas_prescatter(SgipcCtx* c, cudaStream_t s);
 // out_dot[0] when out_dot != nullptr, using r . z with r in T precision).
 template <class T>
 SgipcStatus mas_apply_t(SgipcCtx* c, const T* r, T* z, int fp32_inv, cudaStream_t s);
+// The first part of it: r restricted to every level and the domains solved, the result in
+// mas.Z32 / Z64 (z is its sum over a vertex's clusters).  stop (device, or nullptr): the kernels
+// return at once when it is not zero.
+SgipcStatus mas_domains(SgipcCtx* c, const double* r, int fp32_inv, const int* stop, cudaStream_t s);
 SgipcStatus pcg_create(SgipcCtx* c);
 void pcg_destroy(SgipcCtx* c);
 template <class T>

@@ -171,12 +171,13 @@ __global__ void k_assign(int nv, int L, int level, const int* __restrict__ bank_
 // (blocks with the same (cluster(r), cluster(c)) at level l share it at level l + 1), so
 // each level adds only the previous level's group sums, carried by their leaders: a few
 // per warp at the coarse levels, where nearly every block of the warp lands on one entry.
-// Levels l >= l_top (at most kTopLevels of them, each one domain of <= 16 nodes) go to the
-// CTA's shared copies s_top[l - l_top] of their domains instead (flushed by flush_top).
+// At the top kTopLevels levels the CTA's own ("hot") domain goes to the CTA's shared copy
+// s_top[l - l_top] instead (flushed by flush_top): slots are in row order, so nearly all of a
+// CTA's blocks land there.
 constexpr int kTopLevels = 2;
 __device__ __forceinline__ void scatter_block_warp(double* dom, const int* __restrict__ table, int L, int r, int c,
                                                    const double (&B)[9], bool valid, int l_first, int l_top,
-                                                   double (*s_top)[2304]) {
+                                                   const int* s_hot, double (*s_top)[2304]) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     double V[9];
@@ -216,7 +217,7 @@ __device__ __forceinline__ void scatter_block_warp(double* dom, const int* __res
             for (int q = 0; q < 9; q++) S[q] += __shfl_sync(grp, V[q], j);
         }
         if (valid && lead && (ga >> 4) == (gb >> 4)) {
-            double* D = l >= l_top ? s_top[l - l_top] : dom + (size_t)(ga >> 4) * 2304;
+            double* D = l >= l_top && (ga >> 4) == s_hot[l - l_top] ? s_top[l - l_top] : dom + (size_t)(ga >> 4) * 2304;
             int ra = 3 * (ga & 15), cb = 3 * (gb & 15);
 #pragma unroll
             for (int i = 0; i < 3; i++)
@@ -236,26 +237,26 @@ __device__ __forceinline__ void scatter_block_warp(double* dom, const int* __res
 
 // The top levels' domain copies of the CTA: zeroed, filled by scatter_block_warp, then added
 // to the global domains (one atomic per non-zero entry and CTA instead of one per warp
-// group: every block of the grid lands on the few entries of these levels).
-// levels l >= l_top accumulated per CTA: the top levels (at most kTopLevels) whose nodes
-// form one domain starting on a domain boundary (info[l] = first node, info[8 + l] = count)
-__device__ __forceinline__ int top_levels_dev(const int* __restrict__ info, int L) {
-    int l = L;
-    while (l > 1 && L - (l - 1) <= kTopLevels && info[8 + l - 1] <= 16 && (info[l - 1] & 15) == 0) l--;
-    return l;
-}
+// group).  The domain kept of each level is that of the CTA's first block, whose row is given:
+// with a single domain it is the level's only one; a level of several (bodies without contact
+// between them never join) still has most of a CTA's blocks in one, and sending those to global
+// atomics made the scatter of the 500 affine boxes' scene four times slower.
+__device__ __forceinline__ int top_levels(int L) { return L - kTopLevels > 1 ? L - kTopLevels : 1; }
 
-__device__ __forceinline__ void zero_top(int ntop, double (*s_top)[2304]) {
+__device__ __forceinline__ void zero_top(const int* __restrict__ table, int L, int row, int l_top, int* s_hot,
+                                         double (*s_top)[2304]) {
+    const int ntop = L - l_top;
+    if ((int)threadIdx.x < ntop) s_hot[threadIdx.x] = table[(size_t)row * L + l_top + threadIdx.x] >> 4;
     for (int k = threadIdx.x; k < ntop * 2304; k += blockDim.x) s_top[k / 2304][k % 2304] = 0.0;
     __syncthreads();
 }
 
-__device__ __forceinline__ void flush_top(const int* __restrict__ info, int l_top, int ntop, double (*s_top)[2304],
+__device__ __forceinline__ void flush_top(int ntop, const int* s_hot, double (*s_top)[2304],
                                           double* __restrict__ dom) {
     __syncthreads();
     for (int k = threadIdx.x; k < ntop * 2304; k += blockDim.x) {
         const double v = s_top[k / 2304][k % 2304];
-        if (v != 0.0) atomicAdd(dom + (size_t)(info[l_top + k / 2304] >> 4) * 2304 + k % 2304, v);
+        if (v != 0.0) atomicAdd(dom + (size_t)s_hot[k / 2304] * 2304 + k % 2304, v);
     }
 }
 
@@ -263,16 +264,18 @@ __global__ void k_scatter_static(int nnz, const int* __restrict__ slot_row, cons
                                  const double* __restrict__ val, const int* __restrict__ table, int L,
                                  const int* __restrict__ info, double* __restrict__ dom) {
     __shared__ double s_top[kTopLevels][2304];
+    __shared__ int s_hot[kTopLevels];
     if (info[21]) return;  // aborted hierarchy build: the host rejects its tables
-    const int l_top = top_levels_dev(info, L), ntop = L - l_top;
-    zero_top(ntop, s_top);
+    const int l_top = top_levels(L);
     int s = blockIdx.x * blockDim.x + threadIdx.x;
+    zero_top(table, L, slot_row[blockIdx.x * blockDim.x], l_top, s_hot, s_top);
     bool valid = s < nnz;
     double B[9];
 #pragma unroll
     for (int q = 0; q < 9; q++) B[q] = valid ? val[9 * (size_t)s + q] : 0.0;
-    scatter_block_warp(dom, table, L, valid ? slot_row[s] : 0, valid ? col[s] : 0, B, valid, 1, l_top, s_top);
-    flush_top(info, l_top, ntop, s_top, dom);
+    scatter_block_warp(dom, table, L, valid ? slot_row[s] : 0, valid ? col[s] : 0, B, valid, 1, l_top, s_hot,
+                       s_top);
+    flush_top(L - l_top, s_hot, s_top, dom);
 }
 
 // Level 0 of the static blocks, without atomics: the level-0 domains are the banks of the
@@ -318,17 +321,17 @@ __global__ void k_scatter_contact(int cap, const int* __restrict__ nuc, const in
                                   const int* __restrict__ table, int L, const int* __restrict__ info,
                                   double* __restrict__ dom) {
     __shared__ double s_top[kTopLevels][2304];
-    const int l_top = top_levels_dev(info, L);
+    __shared__ int s_hot[kTopLevels];
+    const int l_top = top_levels(L);
     int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (blockIdx.x * blockDim.x >= nuc[0]) return;  // whole block beyond the unique blocks
-    const int ntop = L - l_top;
-    zero_top(ntop, s_top);
+    zero_top(table, L, ur[blockIdx.x * blockDim.x], l_top, s_hot, s_top);
     bool valid = u < cap && u < nuc[0];
     double B[9];
 #pragma unroll
     for (int q = 0; q < 9; q++) B[q] = valid ? val[9 * (size_t)u + q] : 0.0;
-    scatter_block_warp(dom, table, L, valid ? ur[u] : 0, valid ? uc[u] : 0, B, valid, 0, l_top, s_top);
-    flush_top(info, l_top, ntop, s_top, dom);
+    scatter_block_warp(dom, table, L, valid ? ur[u] : 0, valid ? uc[u] : 0, B, valid, 0, l_top, s_hot, s_top);
+    flush_top(L - l_top, s_hot, s_top, dom);
 }
 
 // Gauss-Jordan inversion without pivoting, in place, one 48x48 domain per 64-thread CTA.
@@ -421,7 +424,8 @@ namespace sgipc {
 // level 0 and level 1 of the restriction: one thread per position
 template <class T, class M>
 __global__ void k_restrict01(int npos, const T* __restrict__ r, const int* __restrict__ part_map,
-                             const int* __restrict__ up, M* __restrict__ R) {
+                             const int* __restrict__ up, M* __restrict__ R, const int* __restrict__ stop = nullptr) {
+    if (stop && *stop) return;
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     int v = p < npos ? part_map[p] : -1;
     M val[3] = {0, 0, 0};
@@ -440,15 +444,33 @@ __global__ void k_restrict01(int npos, const T* __restrict__ r, const int* __res
 
 template <class M>
 __global__ void __launch_bounds__(1024) k_restrict_coarse(const int* __restrict__ info, const int* __restrict__ up,
-                                                          int L, M* __restrict__ R) {
+                                                          int L, M* __restrict__ R,
+                                                          const int* __restrict__ stop = nullptr) {
+    if (stop && *stop) return;
     restrict_coarse_cta<M, 1>(info, up, L, R);
+}
+
+// one level of it over many CTAs
+template <class M>
+__global__ void k_restrict_level(const int* __restrict__ info, const int* __restrict__ up, int l, M* __restrict__ R,
+                                 const int* __restrict__ stop) {
+    if (stop && *stop) return;
+    const int a = blockIdx.x * blockDim.x + threadIdx.x, g = info[l] + a;
+    const bool on = a < info[8 + l];
+    M v[3] = {0, 0, 0};
+    if (on)
+#pragma unroll
+        for (int q = 0; q < 3; q++) v[q] = R[3 * (size_t)g + q];
+    bank_reduce_store<M, 1>(on ? up[g] : -1, v, R);
 }
 
 // Z_d = A_d^-1 R_d, four domains per 192-thread CTA
 template <class M>
 __global__ void __launch_bounds__(192) k_domain_mv(const int* __restrict__ info, const M* __restrict__ inv,
-                                                   const M* __restrict__ R, M* __restrict__ Z) {
+                                                   const M* __restrict__ R, M* __restrict__ Z,
+                                                   const int* __restrict__ stop = nullptr) {
     __shared__ M sR[4][48];
+    if (stop && *stop) return;
     const int ndom = info[16] >> 4;
     const int ld = threadIdx.x / 48, i = threadIdx.x % 48;
     const int d = blockIdx.x * 4 + ld;
@@ -479,22 +501,47 @@ __global__ void k_prolong(int nv, const int* __restrict__ table, int L, const M*
     z[3 * v + 2] = (T)w;
 }
 
+template <class T, class M>
+static void restrict_and_solve(SgipcCtx* c, const T* r, const M* inv, M* R, M* Z, const int* stop, cudaStream_t s) {
+    MasWork& m = c->mas;
+    const int L = m.levelnum, ndom = m.h_info[16] / 16;
+    k_restrict01<T, M><<<nblk(m.npos), SGIPC_BLOCK, 0, s>>>(m.npos, r, m.part_map, m.up, R, stop);
+    // One CTA takes 1024 nodes of a level per turn, about 1.5 us each (24 us for the 16 turns of
+    // 500 boxes over a bed, 4000 of whose points no contact joins); a launch of its own costs a
+    // level about 2.5 us, so it pays from two turns a level on.
+    int turns = 0;
+    for (int l = 1; l + 1 < L; l++) turns += nblk(m.h_info[8 + l], 1024);
+    if (turns > 2 * (L - 2)) {
+        SG_COUNT(c, L);
+        for (int l = 1; l + 1 < L; l++)
+            k_restrict_level<M><<<nblk(m.h_info[8 + l]), SGIPC_BLOCK, 0, s>>>(m.info, m.up, l, R, stop);
+    } else {
+        SG_COUNT(c, 3);
+        k_restrict_coarse<M><<<1, 1024, 0, s>>>(m.info, m.up, L, R, stop);
+    }
+    k_domain_mv<M><<<(ndom + 3) / 4, 192, 0, s>>>(m.info, inv, R, Z, stop);
+}
+
+SgipcStatus mas_domains(SgipcCtx* c, const double* r, int fp32_inv, const int* stop, cudaStream_t s) {
+    MasWork& m = c->mas;
+    if (!m.built) return SGIPC_NOT_READY;
+    if (fp32_inv) restrict_and_solve<double, float>(c, r, m.dom32, m.R32, m.Z32, stop, s);
+    else restrict_and_solve<double, double>(c, r, m.dom64, m.R64, m.Z64, stop, s);
+    SG_LAUNCH_CHECK(c, "mas domains");
+    return SGIPC_OK;
+}
+
 template <class T>
 SgipcStatus mas_apply_t(SgipcCtx* c, const T* r, T* z, int fp32_inv, cudaStream_t s) {
     MasWork& m = c->mas;
     if (!m.built) return SGIPC_NOT_READY;
     const int L = m.levelnum;
-    const int ndom = m.h_info[16] / 16;
-    SG_COUNT(c, 4);
+    SG_COUNT(c, 1);
     if (fp32_inv) {
-        k_restrict01<T, float><<<nblk(m.npos), SGIPC_BLOCK, 0, s>>>(m.npos, r, m.part_map, m.up, m.R32);
-        k_restrict_coarse<float><<<1, 1024, 0, s>>>(m.info, m.up, L, m.R32);
-        k_domain_mv<float><<<(ndom + 3) / 4, 192, 0, s>>>(m.info, m.dom32, m.R32, m.Z32);
+        restrict_and_solve<T, float>(c, r, m.dom32, m.R32, m.Z32, nullptr, s);
         k_prolong<T, float><<<nblk(c->nv), SGIPC_BLOCK, 0, s>>>(c->nv, m.table, L, m.Z32, z);
     } else {
-        k_restrict01<T, double><<<nblk(m.npos), SGIPC_BLOCK, 0, s>>>(m.npos, r, m.part_map, m.up, m.R64);
-        k_restrict_coarse<double><<<1, 1024, 0, s>>>(m.info, m.up, L, m.R64);
-        k_domain_mv<double><<<(ndom + 3) / 4, 192, 0, s>>>(m.info, m.dom64, m.R64, m.Z64);
+        restrict_and_solve<T, double>(c, r, m.dom64, m.R64, m.Z64, nullptr, s);
         k_prolong<T, double><<<nblk(c->nv), SGIPC_BLOCK, 0, s>>>(c->nv, m.table, L, m.Z64, z);
     }
     SG_LAUNCH_CHECK(c, "mas apply");
@@ -504,8 +551,7 @@ SgipcStatus mas_apply_t(SgipcCtx* c, const T* r, T* z, int fp32_inv, cudaStream_
 template SgipcStatus mas_apply_t<double>(SgipcCtx*, const double*, double*, int, cudaStream_t);
 template SgipcStatus mas_apply_t<float>(SgipcCtx*, const float*, float*, int, cudaStream_t);
 
-// First of the coarsest levels (at most kTopLevels, each with <= 16 nodes, i.e. one domain
-// starting at a multiple of 16) that the scatter accumulates per CTA; L when none.
+// computeNumLevels (MASPreconditioner.cu:1724-1743)
 static int num_levels(int nodes) {
     int nLevel = 1;
     int levelSz = (nodes + 15) / 16 * 16;

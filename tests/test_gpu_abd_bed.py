@@ -179,3 +179,29 @@ def test_fullsize_coupled_solve_meets_its_criterion(full):
             sysm.close()
     d = (xs["ref"] - xs["fp64"]).norm() / xs["fp64"].norm()
     assert float(d) < 1e-3
+
+
+@pytest.mark.parametrize("boxes,cells", [(12, (6, 2, 6)), (300, (24, 3, 24))])
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-11), ("ref", 2e-5)])
+def test_mas_apply_of_unjoined_points(boxes, cells, prec, tol):
+    """z = sum_l P_l D_l P_l^T r from the exported tables and domain inverses.  A box's points no
+    contact joins stay nodes of their own on every level: 300 boxes give levels of over 2048
+    nodes, restricted level by level over many CTAs instead of by one."""
+    sc, _ = scenes.scene_abd_on_bed(boxes, cells, seed=2, contacts=False)
+    g = system.GIPC(sc, pair_capacity=60_000)
+    g.buildCP(body=_dev(sc.body_of_vertex, torch.int32))
+    g.computeGradientAndHessian()
+    mas = system.MASPreconditioner(g)
+    mas.setPreconditioner(prec)
+    L, counts, total = mas.info()
+    assert (counts[1] > 2048) == (boxes == 300)
+    r = torch.randn(3 * sc.nv, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    z = mas.preconditioning(r).cpu().numpy().reshape(-1, 3)
+    tab, dom = mas.tables(), mas.domains()
+    R = np.zeros((total, 3))
+    for l in range(L):
+        np.add.at(R, tab[:, l], r.cpu().numpy().reshape(-1, 3))
+    Z = np.einsum("dij,dj->di", dom, R.reshape(-1, 48)).reshape(-1, 3)
+    ref = sum(Z[tab[:, l]] for l in range(L))
+    assert np.abs(z - ref).max() <= tol * np.abs(ref).max()
+    g.close()
