@@ -167,27 +167,38 @@ static SgipcStatus build_static(SgipcCtx* c, const SgipcTopology* t) {
         SG_CHECK(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
         constexpr int rpc = 128;
         if (nsm > 0 && (long long)nsm * rpc >= n) {
-            std::vector<int> cptr2(nsm + 1, 0), ccols, lcol(std::max(c->nnz_full, 1), 0), dslot(std::max(n, 1), 0);
-            int cap = 0;
-            for (int b = 0; b < nsm; b++) {
-                const int r0 = std::min(n, b * rpc), r1 = std::min(n, r0 + rpc);
-                std::vector<int> set(fcol.begin() + frow[r0], fcol.begin() + frow[r1]);
-                std::sort(set.begin(), set.end());
-                set.erase(std::unique(set.begin(), set.end()), set.end());
-                cap = std::max(cap, (int)set.size());
-                for (int e = frow[r0]; e < frow[r1]; e++)
-                    lcol[e] = (int)(std::lower_bound(set.begin(), set.end(), fcol[e]) - set.begin());
-                for (int i = r0; i < r1; i++) dslot[i] = (int)(std::lower_bound(set.begin(), set.end(), i) - set.begin());
-                ccols.insert(ccols.end(), set.begin(), set.end());
-                cptr2[b + 1] = (int)ccols.size();
+            auto build = [&](int rows, int groups, SgipcCtx::ColumnSets& cs) -> SgipcStatus {
+                std::vector<int> cptr2(groups + 1, 0), ccols, lcol(std::max(c->nnz_full, 1), 0), dslot(std::max(n, 1), 0);
+                int cap = 0;
+                for (int b = 0; b < groups; b++) {
+                    const int r0 = std::min(n, b * rows), r1 = std::min(n, r0 + rows);
+                    std::vector<int> set(fcol.begin() + frow[r0], fcol.begin() + frow[r1]);
+                    std::sort(set.begin(), set.end());
+                    set.erase(std::unique(set.begin(), set.end()), set.end());
+                    cap = std::max(cap, (int)set.size());
+                    for (int e = frow[r0]; e < frow[r1]; e++)
+                        lcol[e] = (int)(std::lower_bound(set.begin(), set.end(), fcol[e]) - set.begin());
+                    for (int i = r0; i < r1; i++)
+                        dslot[i] = (int)(std::lower_bound(set.begin(), set.end(), i) - set.begin());
+                    ccols.insert(ccols.end(), set.begin(), set.end());
+                    cptr2[b + 1] = (int)ccols.size();
+                }
+                if (ccols.empty()) ccols.push_back(0);
+                SG_TRY(upload(c, &cs.ptr, cptr2));
+                SG_TRY(upload(c, &cs.cols, ccols));
+                SG_TRY(upload(c, &cs.lcol, lcol));
+                SG_TRY(upload(c, &cs.dslot, dslot));
+                cs.rows = rows;
+                cs.groups = groups;
+                cs.cap = cap;
+                return SGIPC_OK;
+            };
+            SG_TRY(build(rpc, nsm, c->cs));
+            if (n <= kClusterCtas * rpc) {  // small systems: spread over the CTAs of one cluster
+                int rows = kClusterMinRows;
+                while (rows * kClusterCtas < n) rows *= 2;
+                SG_TRY(build(rows, kClusterCtas, c->cs_small));
             }
-            if (ccols.empty()) ccols.push_back(0);
-            SG_TRY(upload(c, &c->cs_ptr, cptr2));
-            SG_TRY(upload(c, &c->cs_cols, ccols));
-            SG_TRY(upload(c, &c->cs_lcol, lcol));
-            SG_TRY(upload(c, &c->cs_dslot, dslot));
-            c->cs_grid = nsm;
-            c->cs_cap = cap;
         }
     }
     SG_TRY(dalloc(c, &c->fval64, (size_t)c->nnz_full * 9));
@@ -374,7 +385,8 @@ extern "C" SgipcStatus sgipc_destroy(SgipcCtx* c) {
                     c->cidx, c->cidx_s, c->cval, c->cflag, c->nuc, c->uc_row, c->uc_col, c->uc64, c->uc32,
                     c->cu_ptr, c->cl_ptr, c->cl_idx, c->lcount, c->lpos, c->cub_tmp, c->dflag,
                     c->frow_ptr, c->fcol, c->fup, c->flo, c->fval64, c->fval32, c->cl_col, c->cl64, c->cl32, c->run_start, c->en_part, c->en_terms, c->ccd_part, c->ccd_out, c->ccd_bad, c->en_ticket, c->ccd_ticket,
-                    c->cs_ptr, c->cs_cols, c->cs_lcol, c->cs_dslot, c->close_gid, c->close_gval, c->close_pid,
+                    c->cs.ptr, c->cs.cols, c->cs.lcol, c->cs.dslot, c->cs_small.ptr, c->cs_small.cols, c->cs_small.lcol,
+                    c->cs_small.dslot, c->close_gid, c->close_gval, c->close_pid,
                     c->close_pval, c->close_cnt};
     for (void* p : ptrs)
         if (p) cudaFree(p);

@@ -226,11 +226,18 @@ struct SgipcCtx {
     struct CoopCfg {
         int valid, usable, grid, ecap, kcap, dcap, ccap, zextra;
         size_t dyn;
-    } coop_cfg[6], fused_cfg[6];
-    // column sets of the fused persistent solve, built with the static pattern for a grid of
-    // cs_grid CTAs of 128 rows: per CTA the sorted distinct columns of its rows
-    // (cs_cols[cs_ptr[c] .. cs_ptr[c+1])), each full-pattern entry's slot among them
-    // (cs_lcol) and each row's own slot (cs_dslot); cs_cap = the largest set
+    } coop_cfg[6], fused_cfg[6], small_cfg[6];
+    // column sets of the fused persistent solve, built with the static pattern for `groups` CTAs
+    // of `rows` rows: per CTA the sorted distinct columns of its rows (cols[ptr[c] .. ptr[c+1])),
+    // each full-pattern entry's slot among them (lcol) and each row's own slot (dslot); cap =
+    // the largest set.  cs: one CTA per SM; cs_small: the CTAs of one cluster (small systems)
+    struct ColumnSets {
+        int* ptr;
+        int* cols;
+        int* lcol;
+        int* dslot;
+        int rows, groups, cap;
+    } cs, cs_small;
     // close constraints of the barrier-stiffness update (sgipc_close_record / _check): the
     // ground vertices and the pairs closer than dTol at the last record, with their values;
     // close_cnt [4] device counters (ground, pairs, the check's flag), close_num their host copy
@@ -240,12 +247,6 @@ struct SgipcCtx {
     double* close_pval;
     unsigned int* close_cnt;
     int close_num[2];
-    int* cs_ptr;
-    int* cs_cols;
-    int* cs_lcol;
-    int* cs_dslot;
-    int cs_grid;
-    int cs_cap;
 
     // ---- MAS and PCG ------------------------------------------------------------------
     sgipc::MasWork mas;
@@ -347,6 +348,11 @@ __device__ __forceinline__ void stn(T* p, const T (&v)[NR]) {
         for (int r = 0; r < NR; r++) p[r] = v[r];
     }
 }
+
+// the fused persistent solve of small systems: the CTAs of one thread-block cluster, with at least
+// kClusterMinRows rows each
+constexpr int kClusterCtas = 16;
+constexpr int kClusterMinRows = 16;
 
 inline int nblk(long long n, int b = SGIPC_BLOCK) { return (int)((n + b - 1) / b); }
 

@@ -174,6 +174,7 @@ struct CoopArgs {
     const int* cs_lcol;
     const int* cs_dslot;
     int ccap;
+    int rpc;     // rows per CTA (the cluster form's; 128 otherwise)
     int zextra;  // further z slots for the columns of resident contact entries outside the set
 };
 
@@ -267,6 +268,50 @@ __device__ bool grid_reduce(const GridBarrier& br, unsigned int epoch, int tag, 
     for (int r = 0; r < NR; r++) out[r] = s_tot[r];
     __syncthreads();  // s_tot is reused by the next call
     return ok;
+}
+
+// ---- the cluster form: all CTAs of the solve are one thread-block cluster --------------------
+// The hardware cluster barrier (release / acquire, so global memory written before it is seen
+// after it) takes the place of the arrival counter, and a dot product's partials go straight
+// into every CTA's shared memory, so that a reduction reads nothing from L2.  The barrier needs
+// no wait limit: the CTAs of a cluster run together or not at all, and all take the same steps.
+__device__ __forceinline__ void cluster_barrier(const GridBarrier& br, unsigned int epoch, int tag) {
+    if (threadIdx.x == 0) {
+        stamp(br, epoch, 0);
+        tag_phase(br, epoch, tag);
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (threadIdx.x == 0) stamp(br, epoch, 1);
+}
+
+// v summed over the cluster, in every thread; part[parity][value][CTA] in each CTA's shared memory
+// (the slots of one parity are rewritten two barriers later at the earliest)
+template <int NR, int S, int P>
+__device__ __forceinline__ void cluster_reduce(const GridBarrier& br, unsigned int epoch, int tag, double (&v)[NR],
+                                               double (&part)[2][P][kClusterCtas], double (&smem)[S],
+                                               double (&out)[NR]) {
+    static_assert(P >= NR && S >= NR * 32, "one slot row and 32 doubles of scratch per value");
+    block_sum<NR>(v, smem);
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < kClusterCtas) {  // lane r of warp 0 stores this CTA's sums in CTA r
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            const unsigned own = (unsigned)__cvta_generic_to_shared(&part[epoch & 1][r][blockIdx.x]);
+            unsigned there;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(own), "r"(lane));
+            asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(there), "d"(v[r]) : "memory");
+        }
+    }
+    cluster_barrier(br, epoch, tag);
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+        double s = part[epoch & 1][r][lane % kClusterCtas];
+#pragma unroll
+        for (int o = kClusterCtas / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        out[r] = s;
+    }
 }
 
 // ---- phases ---------------------------------------------------------------------------------
@@ -856,14 +901,15 @@ __device__ __forceinline__ void prolong_at(const MasView& mv, const M* Z, int j,
 
 // phase A.  dots[r] += r.z, dots[NR + r] += z.w, dots[2 NR + r] += z.Ap_old (not on the first
 // iteration); z and w of the CTA's rows go to a.z and a.w.
-template <class T, class M, int NR>
+template <class T, class M, int NR, bool kCl>
 __device__ void phase_fused_spmv(const CoopArgs<T, M, NR>& a, const RowCache<T>& rc, const FusedCache<T, NR>& fc,
                                  const T* rcur, const T* ap_old, bool first, const bool (&run)[NR],
                                  double (&dots)[3 * NR]) {
     const MasView& mv = a.mv;
-    constexpr int gpw = 32 / kSpG;
-    const int lane = threadIdx.x & 31, g = lane % kSpG;
-    const int i = rc.r0 + (int)(threadIdx.x >> 5) * gpw + lane / kSpG;
+    // lanes per row: with fewer rows in a CTA (the cluster form) each row takes more of them
+    const int gl = kCl ? kCoopThreads / a.rpc : kSpG;
+    const int lane = threadIdx.x & 31, g = lane % gl;
+    const int i = rc.r0 + (int)threadIdx.x / gl;
     // r and Ap_old of the row, issued before the z gathers (they do not depend on them)
     T rpre[3][NR], apre[3][NR];
     if (i < rc.r1 && g == 0) {
@@ -910,7 +956,7 @@ __device__ void phase_fused_spmv(const CoopArgs<T, M, NR>& a, const RowCache<T>&
     if (i < rc.r1) {
         const int li = i - rc.r0;
         const int s0 = rc.rp[li], s1 = rc.rp[li + 1];
-        for (int e = s0 + g; e < s1; e += kSpG) {
+        for (int e = s0 + g; e < s1; e += gl) {
             const T* bv = rc.val + 9 * e;
             const T* zp = fc.zs + (size_t)rc.col[e] * 3 * NR;
             T x3[3][NR];
@@ -933,7 +979,7 @@ __device__ void phase_fused_spmv(const CoopArgs<T, M, NR>& a, const RowCache<T>&
             u0 = a.tp.cu_ptr[i], nu = a.tp.cu_ptr[i + 1] - u0, l0 = a.tp.cl_ptr[i], nl = a.tp.cl_ptr[i + 1] - l0;
             kc = nullptr, kv = nullptr;
         }
-        for (int e = g; e < nu + nl; e += kSpG) {
+        for (int e = g; e < nu + nl; e += gl) {
             const bool up = e < nu;
             int cj;
             const T* src;
@@ -969,12 +1015,20 @@ __device__ void phase_fused_spmv(const CoopArgs<T, M, NR>& a, const RowCache<T>&
             }
         }
     }
+    if (kCl) {
+        for (int o = 1; o < gl; o <<= 1)
 #pragma unroll
-    for (int r = 0; r < NR; r++)
+            for (int r = 0; r < NR; r++)
 #pragma unroll
-        for (int q = 0; q < 3; q++)
+                for (int q = 0; q < 3; q++) acc[r][q] += __shfl_xor_sync(0xffffffffu, acc[r][q], o);
+    } else {
 #pragma unroll
-            for (int o = 1; o < kSpG; o <<= 1) acc[r][q] += __shfl_xor_sync(0xffffffffu, acc[r][q], o, kSpG);
+        for (int r = 0; r < NR; r++)
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+#pragma unroll
+                for (int o = 1; o < kSpG; o <<= 1) acc[r][q] += __shfl_xor_sync(0xffffffffu, acc[r][q], o, kSpG);
+    }
     if (i < rc.r1 && g == 0) {
         const T* zp = fc.zs + (size_t)fc.dsl[i - rc.r0] * 3 * NR;
 #pragma unroll
@@ -1547,7 +1601,11 @@ struct FusedState {
 template <int NR>
 constexpr int kFusedStride = 3 * NR;
 
-template <class T, class M, int NR>
+// kCl: the cluster form (one cluster of kClusterCtas CTAs, a.rpc rows each), for systems of up to
+// 2048 rows.  There the one-CTA-per-SM form has most CTAs idle in a phase and waits out 148
+// arrivals and an L2 round trip of partials at each of its three barriers (17 us per iteration
+// even for 250 rows).
+template <class T, class M, int NR, bool kCl>
 __global__ void __launch_bounds__(kCoopThreads) k_pcg_fused(CoopArgs<T, M, NR> a) {
     __shared__ double smem[kFusedStride<NR> * 32];  // block_sum of up to three values per right-hand side
     __shared__ __align__(16) M sR[kDomPerCta][48 * NR];
@@ -1555,7 +1613,27 @@ __global__ void __launch_bounds__(kCoopThreads) k_pcg_fused(CoopArgs<T, M, NR> a
     extern __shared__ __align__(16) unsigned char dsm[];
     unsigned int epoch = 0;
     if (threadIdx.x == 0) stamp(a.br, 0, 0);
-    constexpr int rpc = kCoopThreads / kSpG;
+    const int rpc = kCl ? a.rpc : kCoopThreads / kSpG;
+    __shared__ double s_part[kCl ? 2 : 1][kCl ? kFusedStride<NR> : 1][kClusterCtas];
+    // barriers and reductions of the two forms
+    auto barrier = [&](int tag) -> bool {
+        epoch++;
+        if constexpr (kCl) {
+            cluster_barrier(a.br, epoch, tag);
+            return true;
+        } else {
+            return grid_barrier(a.br, epoch, tag);
+        }
+    };
+    auto reduce = [&](int tag, auto& val, auto& tot) -> bool {
+        epoch++;
+        if constexpr (kCl) {
+            cluster_reduce(a.br, epoch, tag, val, s_part, smem, tot);
+            return true;
+        } else {
+            return grid_reduce(a.br, epoch, tag, val, a.partial, smem, tot, kFusedStride<NR>);
+        }
+    };
     __shared__ RowCache<T> rcs;
     __shared__ FusedCache<T, NR> fcs;
     __shared__ int s_pv[kPosBanks * 16], s_ppar[kPosBanks * 16], s_pup1[16];
@@ -1740,20 +1818,21 @@ __global__ void __launch_bounds__(kCoopThreads) k_pcg_fused(CoopArgs<T, M, NR> a
     T* acur = a.Ap;
     T* aalt = a.Ap2;
     phase_positions_l2<T, M, NR, 1>(a, S.alpha, nullptr, nullptr, rcur, S.run, v, s_l1);
-    bool ok = grid_reduce<NR>(a.br, ++epoch, kPhInit, v, a.partial, smem, t, kFusedStride<NR>);
+    if constexpr (kCl) cluster_barrier(a.br, ~0u, 0);  // every CTA runs before any writes to another's shared memory
+    bool ok = reduce(kPhInit, v, t);
     if (threadIdx.x == 0)
 #pragma unroll
         for (int r = 0; r < NR; r++) S.bn2[r] = S.rr[r] = t[r];
     if (ok) phase_fused_mas<T, M, NR>(a, sR, dcache, ndc, s_chain_up);
-    ok = ok && grid_barrier(a.br, ++epoch, kPhMas);
+    ok = ok && barrier(kPhMas);
     for (int k = 1; ok; k++) {
         // ---- A: z, w = A z, r.z, z.w, z.Ap_old
         double d3[3 * NR], t3[3 * NR];
 #pragma unroll
         for (int q = 0; q < 3 * NR; q++) d3[q] = 0.0;
         __syncthreads();  // S read below is settled
-        phase_fused_spmv<T, M, NR>(a, rcs, fcs, rcur, acur, k == 1, S.run, d3);
-        if (!(ok = grid_reduce<3 * NR>(a.br, ++epoch, kPhFusedA, d3, a.partial, smem, t3, kFusedStride<NR>))) break;
+        phase_fused_spmv<T, M, NR, kCl>(a, rcs, fcs, rcur, acur, k == 1, S.run, d3);
+        if (!(ok = reduce(kPhFusedA, d3, t3))) break;
         if (threadIdx.x == 0)
 #pragma unroll
             for (int r = 0; r < NR; r++) {
@@ -1805,7 +1884,7 @@ __global__ void __launch_bounds__(kCoopThreads) k_pcg_fused(CoopArgs<T, M, NR> a
         tmp = acur;
         acur = aalt;
         aalt = tmp;
-        if (!(ok = grid_reduce<2 * NR>(a.br, ++epoch, kPhFusedB, d2, a.partial, smem, t2, kFusedStride<NR>))) break;
+        if (!(ok = reduce(kPhFusedB, d2, t2))) break;
         if (threadIdx.x == 0)
 #pragma unroll
             for (int r = 0; r < NR; r++) {
@@ -1821,7 +1900,7 @@ __global__ void __launch_bounds__(kCoopThreads) k_pcg_fused(CoopArgs<T, M, NR> a
         if (!any || k + 1 >= a.max_iter) break;  // converged, or the iteration cap
         // ---- C: the MAS domain solves
         phase_fused_mas<T, M, NR>(a, sR, dcache, ndc, s_chain_up);
-        if (!(ok = grid_barrier(a.br, ++epoch, kPhMas))) break;
+        if (!(ok = barrier(kPhMas))) break;
     }
     double rz_ref = 0.0, rr_ref = 0.0;
     if constexpr (sizeof(T) == 4 && NR == 1) {
@@ -1830,17 +1909,17 @@ __global__ void __launch_bounds__(kCoopThreads) k_pcg_fused(CoopArgs<T, M, NR> a
             // M r64 (FP32 MAS); r64 . M r64
             v[0] = 0.0;
             phase_residual64(a, v[0]);
-            ok = grid_reduce<NR>(a.br, ++epoch, kPhRes64, v, a.partial, smem, t, kFusedStride<NR>);
+            ok = reduce(kPhRes64, v, t);
             rr_ref = t[0];
             if (ok) phase_accumulate64(a);
             v[0] = 0.0;
             if (ok) phase_positions_l2<T, M, NR, 2>(a, S.alpha, nullptr, nullptr, nullptr, S.run, v, s_l1);
-            ok = ok && grid_barrier(a.br, ++epoch, kPhRestr64);
+            ok = ok && barrier(kPhRestr64);
             if (ok) phase_fused_mas<T, M, NR>(a, sR, dcache, ndc, s_chain_up);
-            ok = ok && grid_barrier(a.br, ++epoch, kPhMas);
+            ok = ok && barrier(kPhMas);
             v[0] = 0.0;
             if (ok) phase_prolong_ref(a, v[0]);
-            ok = ok && grid_reduce<NR>(a.br, ++epoch, kPhProlong64, v, a.partial, smem, t, kFusedStride<NR>);
+            ok = ok && reduce(kPhProlong64, v, t);
             rz_ref = t[0];
         }
     }
@@ -1928,11 +2007,25 @@ SgipcStatus coop_configure(SgipcCtx* c, SgipcCtx::CoopCfg& cfg) {
     return SGIPC_OK;
 }
 
+// launch configuration of one cluster of `grid` CTAs
+inline void cluster_launch(cudaLaunchConfig_t& lc, cudaLaunchAttribute (&at)[1], int grid, size_t dyn, cudaStream_t s) {
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(kCoopThreads);
+    lc.dynamicSmemBytes = dyn;
+    lc.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = grid;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+}
+
 // The fused solve's configuration: one CTA per SM, every row resident (static and, when they
 // fit, contact entries), the column sets of the context (built for this grid), then as many of
 // the CTA's first round of MAS domain inverses as still fit.  usable = 0 sends the solve to
-// k_pcg_coop.
-template <class T, class M, int NR>
+// k_pcg_coop.  kCl: the cluster form, where the context has its column sets and the device holds
+// a cluster of that size.
+template <class T, class M, int NR, bool kCl>
 SgipcStatus fused_configure(SgipcCtx* c, SgipcCtx::CoopCfg& cfg) {
     cfg = SgipcCtx::CoopCfg{};
     cfg.valid = 1;
@@ -1940,11 +2033,12 @@ SgipcStatus fused_configure(SgipcCtx* c, SgipcCtx::CoopCfg& cfg) {
     SG_CHECK(c, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
     SG_CHECK(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     SG_CHECK(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-    constexpr int rpc = kCoopThreads / kSpG;
-    if (!coop || !c->cs_ptr || c->cs_grid != nsm || c->cs_cap > kFusedMaxCols || !c->h_frow_ptr ||
-        (long long)nsm * rpc < c->n || nsm > c->pcg64.coop_cap || nsm > c->pcg32.coop_cap)
+    const SgipcCtx::ColumnSets& cs = kCl ? c->cs_small : c->cs;
+    const int grid = kCl ? kClusterCtas : nsm, rpc = cs.rows;
+    if (!coop || !cs.ptr || cs.groups != grid || cs.cap > kFusedMaxCols || !c->h_frow_ptr ||
+        (long long)grid * rpc < c->n || grid > c->pcg64.coop_cap || grid > c->pcg32.coop_cap)
         return SGIPC_OK;
-    const void* fn = (const void*)k_pcg_fused<T, M, NR>;
+    const void* fn = (const void*)k_pcg_fused<T, M, NR, kCl>;
     cudaFuncAttributes fa;
     SG_CHECK(c, cudaFuncGetAttributes(&fa, fn));
     const long long budget = (long long)optin - (long long)fa.sharedSizeBytes - 1024;
@@ -1954,7 +2048,7 @@ SgipcStatus fused_configure(SgipcCtx* c, SgipcCtx::CoopCfg& cfg) {
         const int e = c->h_frow_ptr[r1] - c->h_frow_ptr[r0];
         if (e > ecap) ecap = e;
     }
-    const int ccap = c->cs_cap;
+    const int ccap = cs.cap;
     const size_t fixed = coop_rows_bytes(rpc, ecap, sizeof(T)) + fused_cols_bytes(ccap, sizeof(T), NR) +
                          (size_t)coop_pad4(rpc) * 4;
     if ((long long)fixed > budget) return SGIPC_OK;
@@ -1975,10 +2069,22 @@ SgipcStatus fused_configure(SgipcCtx* c, SgipcCtx::CoopCfg& cfg) {
     if (dcap > kDomPerCta) dcap = kDomPerCta;
     const size_t dyn = base + (size_t)dcap * 2304 * sizeof(M);
     SG_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    SG_CHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pcg_fused<T, M, NR>, kCoopThreads, dyn));
+    if constexpr (kCl) {
+        // 16 CTAs are above the portable cluster size
+        SG_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchConfig_t lc = {};
+        cudaLaunchAttribute at[1];
+        cluster_launch(lc, at, grid, dyn, nullptr);
+        if (cudaOccupancyMaxActiveClusters(&per, fn, &lc) != cudaSuccess) {
+            (void)cudaGetLastError();
+            per = 0;
+        }
+    } else {
+        SG_CHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kCoopThreads, dyn));
+    }
     if (per < 1) return SGIPC_OK;
     cfg.usable = 1;
-    cfg.grid = nsm;
+    cfg.grid = grid;
     cfg.ecap = ecap;
     cfg.kcap = kcap;
     cfg.dcap = dcap;
@@ -2012,17 +2118,30 @@ SgipcStatus run_pcg_coop(SgipcCtx* c, PcgWork& w, int fp32_mas, const double* b,
     SgipcCtx::CoopCfg& fcfg = c->fused_cfg[inst];
     bool fused = false;
     // (FP64 vectors with four right-hand sides measured slower fused: kept four-phase)
-    if (L >= 3 && !(fz && fz[0] == '0') && !(sizeof(T) == 8 && sizeof(M) == 8 && NR == 4)) {
+    // (a caller's wait limit needs barriers that can run out: not the cluster form's)
+    SgipcCtx::CoopCfg& scfg = c->small_cfg[inst];
+    bool cluster = false;
+    if (L >= 3 && !(fz && fz[0] == '0')) {
+        if (!scfg.valid) {
+            SgipcStatus st = fused_configure<T, M, NR, true>(c, scfg);
+            if (st != SGIPC_OK) return st;
+        }
+        cluster = scfg.usable && c->wait_limit == 0;
+        fused = cluster;
+    }
+    if (!cluster && L >= 3 && !(fz && fz[0] == '0') && !(sizeof(T) == 8 && sizeof(M) == 8 && NR == 4)) {
         if (!fcfg.valid) {
-            SgipcStatus st = fused_configure<T, M, NR>(c, fcfg);
+            SgipcStatus st = fused_configure<T, M, NR, false>(c, fcfg);
             if (st != SGIPC_OK) return st;
         }
         fused = fcfg.usable != 0;
     }
-    const SgipcCtx::CoopCfg& use = fused ? fcfg : cfg;
+    const SgipcCtx::CoopCfg& use = cluster ? scfg : (fused ? fcfg : cfg);
+    const SgipcCtx::ColumnSets& cs = cluster ? c->cs_small : c->cs;
     const int grid = use.grid, ecap = use.ecap, kcap = use.kcap, dcap = use.dcap;
     const size_t dyn = use.dyn;
-    const void* fn = fused ? (const void*)k_pcg_fused<T, M, NR> : (const void*)k_pcg_coop<T, M, NR>;
+    const void* fn = cluster ? (const void*)k_pcg_fused<T, M, NR, true>
+                             : (fused ? (const void*)k_pcg_fused<T, M, NR, false> : (const void*)k_pcg_coop<T, M, NR>);
     CoopArgs<T, M, NR> a;
     a.tp = topo_of(c);
     a.A = mat_view<T>(c);
@@ -2064,10 +2183,11 @@ SgipcStatus run_pcg_coop(SgipcCtx* c, PcgWork& w, int fp32_mas, const double* b,
     a.tol = tol;
     a.w = (T*)w.w;
     a.Ap2 = (T*)w.Ap2;
-    a.cs_ptr = c->cs_ptr;
-    a.cs_cols = c->cs_cols;
-    a.cs_lcol = c->cs_lcol;
-    a.cs_dslot = c->cs_dslot;
+    a.cs_ptr = cs.ptr;
+    a.cs_cols = cs.cols;
+    a.cs_lcol = cs.lcol;
+    a.cs_dslot = cs.dslot;
+    a.rpc = cluster ? cs.rows : kCoopThreads / kSpG;
     a.ccap = fused ? use.ccap : 0;
     a.zextra = fused ? use.zextra : 0;
     SG_CHECK(c, cudaMemsetAsync(w.ticket + 4, 0, 2 * sizeof(unsigned int), s));
@@ -2076,7 +2196,14 @@ SgipcStatus run_pcg_coop(SgipcCtx* c, PcgWork& w, int fp32_mas, const double* b,
     if (a.l2mode) SG_CHECK(c, cudaMemsetAsync(a.R, 0, sizeof(M) * 3 * (size_t)m.npos * NR, s));
     void* args[] = {&a};
     SG_COUNT(c, 1);
-    SG_CHECK(c, cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kCoopThreads), args, dyn, s));
+    if (cluster) {
+        cudaLaunchConfig_t lc = {};
+        cudaLaunchAttribute at[1];
+        cluster_launch(lc, at, grid, dyn, s);
+        SG_CHECK(c, cudaLaunchKernelExC(&lc, fn, args));
+    } else {
+        SG_CHECK(c, cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kCoopThreads), args, dyn, s));
+    }
     *used = true;
     return SGIPC_OK;
 }
