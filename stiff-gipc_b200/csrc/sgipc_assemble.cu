@@ -13,9 +13,15 @@
 //   * static part: element kernels write oriented 3x3 blocks into per-element slots
 //     (eblk) and per-vertex gradient rows (egrad); gather kernels sum them into the BSR
 //     values and shape_grads through CSR lists built at context creation;
-//   * dynamic part: every contact pair writes its upper blocks under a (row,col) key; one
-//     radix sort plus a segmented sum gives the unique contact blocks, kept row-sorted
-//     together with a transposed index list so that SpMV needs no atomics.
+//   * dynamic part: a contact pair's blocks are products of a few vectors, so each pair stores
+//     those (its factors, 128 B) instead of ten 3x3 blocks (840 B with their keys), and its
+//     vertices are sorted once, one 32-bit key each.  A warp (or a CTA, for long lists) then
+//     walks the pairs of one vertex in order, forms the blocks of that row and adds them up in
+//     shared memory: the unique blocks row-sorted, the transposed lists that the SpMV reads
+//     without atomics, and the contact gradient, all in a fixed order.  (Sorting the blocks
+//     themselves under 64-bit keys and summing the runs moved 4 GB for the million pairs of a
+//     256^2 rolled cloth: 3.3 ms of kernels.)
+#include <algorithm>
 #include <cmath>
 
 #include <cub/cub.cuh>
@@ -25,8 +31,6 @@
 using namespace sgipc;
 
 namespace {
-
-constexpr unsigned long long kBadKey = ~0ull;
 
 // ------------------------------------------------------------------------------------------
 // kinetic gradient, reset of the contact gradient
@@ -431,72 +435,86 @@ __global__ void k_rhs(int nv, const double* __restrict__ fb, const double* __res
 // ------------------------------------------------------------------------------------------
 // contact blocks
 // ------------------------------------------------------------------------------------------
-struct BlockSink {
-    unsigned long long* key;
-    int* idx;
-    double* val;
-    const int32_t* btype;  // Dirichlet flags (blocks touching a flagged vertex are zeroed); null: none
-    int bits;
+// A pair's factors, kFac doubles (one 128-byte line):
+//   barrier   [0] lam, [1..12] g (four vertices), [13] s:   block (a, b) = lam g_a g_b^T, gradient s g_a
+//   friction  [0..8] W, [9..12] c, [13..15] t:              block (a, b) = c_a c_b W,     gradient c_a t
+//   mollified [0] M11, [1..12] gf, [13] df, [14] M01, and a second line [0] M00, [1..12] gc, [13] dc:
+//             block (a, b) = M00 gc_a gc_b^T + M01 (gc_a gf_b^T + gf_a gc_b^T) + M11 gf_a gf_b^T,
+//             gradient dc gc_a + df gf_a
+// (a before b in the pair's order; the block of a vertex pair in the other order is its
+// transpose).  Ground contacts and soft constraints ("singles") store their 3x3 block.
+constexpr int kFac = 16;
+constexpr int kMollBit = 1 << 30;  // in vertex 0 of a mollified pair's ids
+struct ContactStore {
+    int4* ids;         // [pairs] vertices, -1 where a pair has fewer (all -1: no blocks)
+    double* fac;       // [kFac * pairs]
+    double* fac2;      // [kFac * barrier pairs] second line of the mollified ones
+    int* sid;          // [singles] vertex, -1: none
+    double* sval;      // [9 * singles]
+    uint32_t* key;     // [4 * pairs + singles] vertex of each incidence 4 pair + a, or 4 pairs + single; n: none
+    uint32_t* val;     // the incidence itself
+    int pairs, barrier_pairs, n;
     int nv;
-    int* flag;  // set to 1 when a pair names a vertex outside [0, nv)
+    int* flag;         // set to 1 when a pair names a vertex outside [0, nv)
 };
 
-__device__ __forceinline__ bool ids_ok(const BlockSink& bs, const int* v, int n) {
+__device__ __forceinline__ bool ids_ok(const ContactStore& cs, const int* v, int n) {
     for (int a = 0; a < n; a++)
-        if (v[a] < 0 || v[a] >= bs.nv) {
-            atomicOr(bs.flag, 1);
+        if (v[a] < 0 || v[a] >= cs.nv) {
+            atomicOr(cs.flag, 1);
             return false;
         }
     return true;
 }
 
-// store up to 10 upper blocks of an nv-vertex pair: H_ab = sum_t coef_t u_t,a w_t,b^T
-// expressed through a callback producing the 3x3 block for local (a,b)
-template <class BlockFn>
-__device__ __forceinline__ void emit_pair_blocks(const BlockSink& bs, int base, int nvp, const int* vid, BlockFn fn) {
-    // unrolled: the per-vertex arrays of the pair's lambdas are then indexed at compile time
-    // (rolled, they lived in local memory; friction terms 7 % faster)
-    int k = 0;
+// vertices and incidence keys of pair `item` (nvp of them in use; 0: no blocks)
+__device__ __forceinline__ void store_ids(const ContactStore& cs, int item, int nvp, const int* v, bool moll) {
+    int id[4];
+    uint32_t k[4];
 #pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = a; b < 4; b++, k++) {
-            int slot = base + k;
-            bs.idx[slot] = slot;
-            if (a >= nvp || b >= nvp) {
-                bs.key[slot] = kBadKey;
-                continue;
-            }
-            int r = vid[a], c = vid[b];
-            bool tr = r > c;
-            int rr = tr ? c : r, cc = tr ? r : c;
-            bs.key[slot] = ((unsigned long long)rr << bs.bits) | (unsigned long long)cc;
-            double H[3][3];
-            fn(a, b, H);
-            bool dir = bs.btype && (bs.btype[r] != 0 || bs.btype[c] != 0);
-            double* o = bs.val + 9 * (size_t)slot;
-#pragma unroll
-            for (int p = 0; p < 3; p++)
-#pragma unroll
-                for (int q = 0; q < 3; q++) o[3 * p + q] = dir ? 0.0 : (tr ? H[q][p] : H[p][q]);
-        }
+    for (int a = 0; a < 4; a++) {
+        id[a] = a < nvp ? v[a] : -1;
+        k[a] = a < nvp ? (uint32_t)v[a] : (uint32_t)cs.n;
+    }
+    if (moll && nvp > 0) id[0] |= kMollBit;
+    cs.ids[item] = make_int4(id[0], id[1], id[2], id[3]);
+    reinterpret_cast<uint4*>(cs.key)[item] = make_uint4(k[0], k[1], k[2], k[3]);
+    const uint32_t o = 4u * (uint32_t)item;
+    reinterpret_cast<uint4*>(cs.val)[item] = make_uint4(o, o + 1, o + 2, o + 3);
 }
 
-__device__ __forceinline__ void emit_diag_block(const BlockSink& bs, int slot, int v, const double H[3][3]) {
-    bs.idx[slot] = slot;
-    bs.key[slot] = ((unsigned long long)v << bs.bits) | (unsigned long long)v;
-    bool dir = bs.btype && bs.btype[v] != 0;
-    double* o = bs.val + 9 * (size_t)slot;
+__device__ __forceinline__ void store_single(const ContactStore& cs, int j, int v, const double (&H)[3][3]) {
+    const int o = 4 * cs.pairs + j;
+    cs.sid[j] = v;
+    cs.key[o] = v >= 0 ? (uint32_t)v : (uint32_t)cs.n;
+    cs.val[o] = (uint32_t)o;
 #pragma unroll
     for (int p = 0; p < 3; p++)
 #pragma unroll
-        for (int q = 0; q < 3; q++) o[3 * p + q] = dir ? 0.0 : H[p][q];
+        for (int q = 0; q < 3; q++) cs.sval[9 * (size_t)j + 3 * p + q] = H[p][q];
 }
 
-__device__ __forceinline__ void add_grad(double* fb, int v, d3 g) {
-    atomicAdd(fb + 3 * v, g.x);
-    atomicAdd(fb + 3 * v + 1, g.y);
-    atomicAdd(fb + 3 * v + 2, g.z);
+// Entry (p, q) of a pair's block at (row vertex a, column vertex b): the product is formed with
+// the pair's earlier vertex first, so that the blocks (a, b) and (b, a) are exact transposes.
+// f: the pair's factors, f2: the second line (mollified pairs).
+enum PairType { kPairBarrier = 0, kPairFriction = 1, kPairMollified = 2, kPairSingle = 3 };
+__device__ __forceinline__ double pair_entry(int type, const double* f, const double* f2, int a, int b, int p, int q) {
+    if (a > b) {
+        const int t = a, u = p;
+        a = b, b = t;
+        p = q, q = u;
+    }
+    if (type == kPairBarrier) return f[0] * (f[1 + 3 * a + p] * f[1 + 3 * b + q]);
+    if (type == kPairFriction) return f[9 + a] * f[9 + b] * f[3 * p + q];
+    const double *gf = f + 1, *gc = f2 + 1;
+    return f2[0] * gc[3 * a + p] * gc[3 * b + q] +
+           f[14] * (gc[3 * a + p] * gf[3 * b + q] + gf[3 * a + p] * gc[3 * b + q]) +
+           f[0] * gf[3 * a + p] * gf[3 * b + q];
+}
+__device__ __forceinline__ double pair_grad(int type, const double* f, const double* f2, int a, int q) {
+    if (type == kPairBarrier) return f[13] * f[1 + 3 * a + q];
+    if (type == kPairFriction) return f[9 + a] * f[13 + q];
+    return f2[13] * f2[1 + 3 * a + q] + f[13] * f[1 + 3 * a + q];
 }
 
 // Decoded barrier pair: kind 0 PP, 1 PE, 2 PT, 3 EE, 4 mollified EE, 5 mollified PE,
@@ -576,15 +594,17 @@ __device__ __forceinline__ void barrier_s(double I, double c, double& B, double&
     d2B = c * (2.0 * L * L + 8.0 * t * L / I + 2.0 * t * t * (1.0 - L) / (I * I));
 }
 
-__device__ __forceinline__ void barrier_one(int p, int np, const int4* __restrict__ pairs,
-                                            const double* __restrict__ x, const double* __restrict__ rest,
-                                            double dhat, double kappa, double* __restrict__ fb, BlockSink bs,
-                                            int base) {
+__device__ __forceinline__ void set3(double* f, d3 v) { f[0] = v.x, f[1] = v.y, f[2] = v.z; }
+
+// item p's factors into f (the CTA's staging line); false: it has no blocks
+__device__ __forceinline__ bool barrier_one(int p, const int4* __restrict__ pairs, const double* __restrict__ x,
+                                            const double* __restrict__ rest, double dhat, double kappa,
+                                            const ContactStore& cs, int item, double* f) {
     int v[4], nvp;
     int kind = decode_pair(pairs[p], v, nvp);
-    if (!ids_ok(bs, v, nvp)) {
-        emit_pair_blocks(bs, base + 10 * p, 0, v, [&](int, int, double H[3][3]) {});
-        return;
+    if (!ids_ok(cs, v, nvp)) {
+        store_ids(cs, item, 0, v, false);
+        return false;
     }
     d3 X[4];
 #pragma unroll
@@ -592,26 +612,25 @@ __device__ __forceinline__ void barrier_one(int p, int np, const int4* __restric
     d3 gd2[4];
     double d2 = dist2_grad(kind, X, gd2);
     const double sdh = sqrt(dhat), dist = sqrt(d2);
-    const double I = d2 / dhat, f = sqrt(I);
+    const double I = d2 / dhat, fr = sqrt(I);
     d3 gf[4];
 #pragma unroll
     for (int a = 0; a < 4; a++) gf[a] = (1.0 / (2.0 * dist * sdh)) * gd2[a];
     if (kind <= 3) {
         double B, dB, d2B;
         barrier_s(I, kappa * dhat * dhat, B, dB, d2B);
-        double dBdf = 2.0 * f * dB;
+        double dBdf = 2.0 * fr * dB;
         double Ic = d2 < 1e-6 * dhat ? 1e-6 : I;  // gassThreshold clamp (GIPC.cu:3258-3272)
         double Bc, dBc, d2Bc;
         barrier_s(Ic, kappa * dhat * dhat, Bc, dBc, d2Bc);
         double lam0 = 4.0 * Ic * d2Bc + 2.0 * dBc;
-        for (int a = 0; a < 4; a++) if (a < nvp) add_grad(fb, v[a], dBdf * gf[a]);
-        emit_pair_blocks(bs, base + 10 * p, nvp, v, [&](int a, int b, double H[3][3]) {
+        store_ids(cs, item, nvp, v, false);
+        f[0] = lam0;
 #pragma unroll
-            for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int j = 0; j < 3; j++) H[i][j] = lam0 * comp(gf[a], i) * comp(gf[b], j);
-        });
-        return;
+        for (int a = 0; a < 4; a++) set3(f + 1 + 3 * a, gf[a]);
+        f[13] = dBdf;
+        f[14] = f[15] = 0.0;
+        return true;
     }
     // mollified pairs: b = kappa e(c^2) Bt(I), c = |edge0 x edge1|
     int ea0, ea1, eb0, eb1;
@@ -622,8 +641,8 @@ __device__ __forceinline__ void barrier_one(int p, int np, const int4* __restric
     d3 n = cross(u, w);
     double I1 = sq(n);
     if (I1 == 0.0) {
-        emit_pair_blocks(bs, base + 10 * p, 0, v, [&](int, int, double H[3][3]) {});
-        return;
+        store_ids(cs, item, 0, v, false);
+        return false;
     }
     double c = sqrt(I1);
     d3 gc[4];
@@ -641,37 +660,32 @@ __device__ __forceinline__ void barrier_one(int p, int np, const int4* __restric
     double dem = -2.0 * I1 / (ex * ex) + 2.0 / ex;
     double B, dB, d2B;
     barrier_s(I, dhat * dhat, B, dB, d2B);
-    double dbdc = kappa * dem * 2.0 * c * B, dbdf = kappa * em * dB * 2.0 * f;
-    for (int a = 0; a < 4; a++) add_grad(fb, v[a], dbdc * gc[a] + dbdf * gf[a]);
+    double dbdc = kappa * dem * 2.0 * c * B, dbdf = kappa * em * dB * 2.0 * fr;
     double M00 = kappa * B * (-4.0 * (3.0 * I1 - ex) / (ex * ex));
     double M11 = kappa * em * (4.0 * I * d2B + 2.0 * dB);
-    double M01 = kappa * dem * 2.0 * c * dB * 2.0 * f;
+    double M01 = kappa * dem * 2.0 * c * dB * 2.0 * fr;
     make_pd2(M00, M01, M11);
-    emit_pair_blocks(bs, base + 10 * p, 4, v, [&](int a, int b, double H[3][3]) {
+    store_ids(cs, item, 4, v, true);
+    f[0] = M11;
+    f[13] = dbdf;
+    f[14] = M01;
+    f[15] = 0.0;
+    double* f2 = cs.fac2 + kFac * (size_t)item;  // rare: straight to memory
+    f2[0] = M00;
+    f2[13] = dbdc;
 #pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++)
-                H[i][j] = M00 * comp(gc[a], i) * comp(gc[b], j) +
-                          M01 * (comp(gc[a], i) * comp(gf[b], j) + comp(gf[a], i) * comp(gc[b], j)) +
-                          M11 * comp(gf[a], i) * comp(gf[b], j);
-    });
-}
-
-__global__ void __launch_bounds__(128) k_barrier(int np, const int4* __restrict__ pairs, const double* __restrict__ x,
-                                                 const double* __restrict__ rest, double dhat, double kappa,
-                                                 double* __restrict__ fb, BlockSink bs, int base) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= np) return;
-    barrier_one(p, np, pairs, x, rest, dhat, kappa, fb, bs, base);
+    for (int a = 0; a < 4; a++) {
+        set3(f + 1 + 3 * a, gf[a]);
+        set3(f2 + 1 + 3 * a, gc[a]);
+    }
+    return true;
 }
 
 // friction pairs (FrictionUtils.cuh, GIPC.cu:1439-1800 and 5087-5270), C1 static clamping
-__device__ __forceinline__ void friction_one(int p, int np, const int4* __restrict__ pairs,
-                                             const double* __restrict__ x, const double* __restrict__ x0,
-                                             const double* __restrict__ lam, const double* __restrict__ coord,
-                                             const double* __restrict__ basis, double mu, double eps2,
-                                             double* __restrict__ fb, BlockSink bs, int base) {
+__device__ __forceinline__ bool friction_one(int p, const int4* __restrict__ pairs, const double* __restrict__ x,
+                                             const double* __restrict__ x0, const double* __restrict__ lam,
+                                             const double* __restrict__ coord, const double* __restrict__ basis,
+                                             double mu, double eps2, const ContactStore& cs, int item, double* f) {
     int4 e = pairs[p];
     int v[4] = {0, 0, 0, 0}, nvp = 0;
     double cf[4] = {0, 0, 0, 0};
@@ -687,9 +701,9 @@ __device__ __forceinline__ void friction_one(int p, int np, const int4* __restri
         else if (e.w < 0) { v[1] = e.y; v[2] = e.z; nvp = 3; cf[0] = 1.0; cf[1] = g1 - 1.0; cf[2] = -g1; }
         else { v[1] = e.y; v[2] = e.z; v[3] = e.w; nvp = 4; cf[0] = 1.0; cf[1] = -1.0 + g1 + g2; cf[2] = -g1; cf[3] = -g2; }
     }
-    if (nvp == 0 || !ids_ok(bs, v, nvp)) {
-        emit_pair_blocks(bs, base + 10 * p, 0, v, [&](int, int, double H[3][3]) {});
-        return;
+    if (nvp == 0 || !ids_ok(cs, v, nvp)) {
+        store_ids(cs, item, 0, v, false);
+        return false;
     }
     const double* Tb = basis + 6 * (size_t)p;  // 3x2 row-major
     d3 t0 = mk(Tb[0], Tb[2], Tb[4]), t1 = mk(Tb[1], Tb[3], Tb[5]);
@@ -715,68 +729,54 @@ __device__ __forceinline__ void friction_one(int p, int np, const int4* __restri
     make_pd2(M00, M01, M11);
     const double s = mu * lam[p];
     d3 gt = (s * f1d) * (u0 * t0 + u1 * t1);
-    for (int a = 0; a < 4; a++) if (a < nvp) add_grad(fb, v[a], cf[a] * gt);
+    store_ids(cs, item, nvp, v, false);
     // W = basis M basis^T
-    double W[3][3];
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
         for (int j = 0; j < 3; j++) {
+            if (j < i) continue;
             double ti0 = comp(t0, i), ti1 = comp(t1, i), tj0 = comp(t0, j), tj1 = comp(t1, j);
-            W[i][j] = s * (ti0 * (M00 * tj0 + M01 * tj1) + ti1 * (M01 * tj0 + M11 * tj1));
+            f[3 * i + j] = f[3 * j + i] = s * (ti0 * (M00 * tj0 + M01 * tj1) + ti1 * (M01 * tj0 + M11 * tj1));
         }
-    emit_pair_blocks(bs, base + 10 * p, nvp, v, [&](int a, int b, double H[3][3]) {
-        double k = cf[a] * cf[b];
 #pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) H[i][j] = k * W[i][j];
-    });
-}
-
-__global__ void __launch_bounds__(128) k_friction(int np, const int4* __restrict__ pairs, const double* __restrict__ x,
-                                                  const double* __restrict__ x0, const double* __restrict__ lam,
-                                                  const double* __restrict__ coord, const double* __restrict__ basis,
-                                                  double mu, double eps2, double* __restrict__ fb, BlockSink bs,
-                                                  int base) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= np) return;
-    friction_one(p, np, pairs, x, x0, lam, coord, basis, mu, eps2, fb, bs, base);
+    for (int a = 0; a < 4; a++) f[9 + a] = cf[a];
+    set3(f + 13, gt);
+    return true;
 }
 
 // ground barrier (GIPC.cu:6463-6514), plane y = offset
-__device__ __forceinline__ void ground_one(int p, int ng, const uint32_t* __restrict__ gp,
-                                           const double* __restrict__ x, double offset, double dhat, double kappa,
-                                           double* __restrict__ fb, BlockSink bs, int base) {
+__device__ __forceinline__ void ground_one(int p, const uint32_t* __restrict__ gp, const double* __restrict__ x,
+                                           double offset, double dhat, double kappa, double* __restrict__ fb,
+                                           const ContactStore& cs, int single) {
     int v = gp[p];
-    if (!ids_ok(bs, &v, 1)) {
-        bs.idx[base + p] = base + p;
-        bs.key[base + p] = kBadKey;
+    double H[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    if (!ids_ok(cs, &v, 1)) {
+        store_single(cs, single, -1, H);
         return;
     }
     double dist = x[3 * v + 1] - offset, d2 = dist * dist, t = d2 - dhat;
     double gb = t * log(d2 / dhat) * -2.0 - (t * t) / d2;
     double hb = (log(d2 / dhat) * -2.0 - t * 4.0 / d2) + 1.0 / (d2 * d2) * (t * t);
     atomicAdd(fb + 3 * v + 1, kappa * gb * 2.0 * dist);
-    double H[3][3] = {{0, 0, 0}, {0, kappa * (4.0 * hb * d2 + 2.0 * gb), 0}, {0, 0, 0}};
-    emit_diag_block(bs, base + p, v, H);
+    H[1][1] = kappa * (4.0 * hb * d2 + 2.0 * gb);
+    store_single(cs, single, v, H);
 }
 
 
 // ground friction (GIPC.cu:1357-1437, 5047-5085), normal +y
-__device__ __forceinline__ void fric_ground_one(int p, int ng, const uint32_t* __restrict__ gp,
-                                                const double* __restrict__ x, const double* __restrict__ x0,
-                                                const double* __restrict__ lam, double mu, double eps2,
-                                                double* __restrict__ fb, BlockSink bs, int base) {
+__device__ __forceinline__ void fric_ground_one(int p, const uint32_t* __restrict__ gp, const double* __restrict__ x,
+                                                const double* __restrict__ x0, const double* __restrict__ lam,
+                                                double mu, double eps2, double* __restrict__ fb,
+                                                const ContactStore& cs, int single) {
     int v = gp[p];
-    if (!ids_ok(bs, &v, 1)) {
-        bs.idx[base + p] = base + p;
-        bs.key[base + p] = kBadKey;
+    double H[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    if (!ids_ok(cs, &v, 1)) {
+        store_single(cs, single, -1, H);
         return;
     }
     double vx = x[3 * v] - x0[3 * v], vz = x[3 * v + 2] - x0[3 * v + 2];
     double m2 = vx * vx + vz * vz, s = mu * lam[p], eps = sqrt(eps2);
-    double H[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
     if (m2 > eps2) {
         double m = sqrt(m2), k = s / (m2 * m);
         atomicAdd(fb + 3 * v, s * vx / m);
@@ -790,13 +790,15 @@ __device__ __forceinline__ void fric_ground_one(int p, int ng, const uint32_t* _
         H[0][0] = s / eps;
         H[2][2] = s / eps;
     }
-    emit_diag_block(bs, base + p, v, H);
+    store_single(cs, single, v, H);
 }
 
 
 // All contact terms of a call in one launch: the CTAs take the barrier pairs, then the
 // friction pairs, then the ground and the ground-friction vertices (128 threads each), so the
-// four kinds run side by side instead of one after another.
+// four kinds run side by side instead of one after another.  The factors of a CTA's pairs are
+// staged in shared memory and leave it as whole lines.  kGrad: the pairs' gradients are added
+// into fb here, by atomics (callers that do not build the matrix); else k_row_sums adds them.
 struct ContactLaunch {
     int np, nf, ng, ngf;           // items of each kind (0: none)
     int cb, cf, cg;                // first CTA of friction, ground, ground friction
@@ -812,191 +814,499 @@ struct ContactLaunch {
     const double* fbasis;
     const double* gflam;
     double dhat, kappa, mu, gmu, eps2, offset;
-    int base_b, base_f, base_g, base_gf;
 };
 
-__global__ void __launch_bounds__(128) k_contacts(ContactLaunch L, double* __restrict__ fb, BlockSink bs) {
-    const int b = blockIdx.x;
-    if (b < L.cb) {
-        const int p = b * 128 + threadIdx.x;
-        if (p < L.np) barrier_one(p, L.np, L.pairs, L.x, L.rest, L.dhat, L.kappa, fb, bs, L.base_b);
-    } else if (b < L.cf) {
-        const int p = (b - L.cb) * 128 + threadIdx.x;
-        if (p < L.nf)
-            friction_one(p, L.nf, L.fpairs, L.x, L.x0, L.flam, L.fcoord, L.fbasis, L.mu, L.eps2, fb, bs, L.base_f);
-    } else if (b < L.cg) {
-        const int p = (b - L.cf) * 128 + threadIdx.x;
-        if (p < L.ng) ground_one(p, L.ng, L.gpairs, L.x, L.offset, L.dhat, L.kappa, fb, bs, L.base_g);
-    } else {
-        const int p = (b - L.cg) * 128 + threadIdx.x;
-        if (p < L.ngf) fric_ground_one(p, L.ngf, L.gfpairs, L.x, L.x0, L.gflam, L.gmu, L.eps2, fb, bs, L.base_gf);
+constexpr int kConThreads = 128;
+template <bool kGrad>
+__global__ void __launch_bounds__(kConThreads) k_contacts(ContactLaunch L, double* __restrict__ fb, ContactStore cs) {
+    __shared__ double stage[kConThreads][kFac + 1];
+    const int b = blockIdx.x, t = threadIdx.x;
+    if (b >= L.cf) {  // CTA-uniform
+        if (b < L.cg) {
+            const int p = (b - L.cf) * kConThreads + t;
+            if (p < L.ng) ground_one(p, L.gpairs, L.x, L.offset, L.dhat, L.kappa, fb, cs, p);
+        } else {
+            const int p = (b - L.cg) * kConThreads + t;
+            if (p < L.ngf) fric_ground_one(p, L.gfpairs, L.x, L.x0, L.gflam, L.gmu, L.eps2, fb, cs, L.ng + p);
+        }
+        return;
     }
+    const bool fric = b >= L.cb;
+    const int p0 = (fric ? b - L.cb : b) * kConThreads, p = p0 + t, n = fric ? L.nf : L.np;
+    const int item0 = (fric ? L.np : 0) + p0;
+    bool on = false;
+    if (p < n)
+        on = fric ? friction_one(p, L.fpairs, L.x, L.x0, L.flam, L.fcoord, L.fbasis, L.mu, L.eps2, cs, item0 + t, stage[t])
+                  : barrier_one(p, L.pairs, L.x, L.rest, L.dhat, L.kappa, cs, item0 + t, stage[t]);
+    if (kGrad && on) {
+        const int4 id = cs.ids[item0 + t];
+        const int v[4] = {id.x & ~kMollBit, id.y, id.z, id.w};
+        const int type = fric ? kPairFriction : ((id.x & kMollBit) ? kPairMollified : kPairBarrier);
+        const double* f2 = type == kPairMollified ? cs.fac2 + kFac * (size_t)(item0 + t) : nullptr;
+        for (int a = 0; a < 4; a++)
+            if (v[a] >= 0)
+                for (int q = 0; q < 3; q++) atomicAdd(fb + 3 * (size_t)v[a] + q, pair_grad(type, stage[t], f2, a, q));
+    }
+    if (!on)
+#pragma unroll
+        for (int k = 0; k < kFac; k++) stage[t][k] = 0.0;
+    __syncthreads();
+    const int words = kFac * min(kConThreads, n - p0);
+    double* out = cs.fac + kFac * (size_t)item0;
+    for (int k = t; k < words; k += kConThreads) out[k] = stage[k / kFac][k % kFac];
 }
 
 // soft constraints (GIPC.cu:6363-6407)
 __global__ void k_soft(int ns, const uint32_t* __restrict__ idx, const double* __restrict__ x,
-                       const double* __restrict__ target, double k, double* __restrict__ sg, BlockSink bs, int base) {
+                       const double* __restrict__ target, double k, double* __restrict__ sg, ContactStore cs, int first) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= ns) return;
     int v = idx[p];
     for (int q = 0; q < 3; q++) atomicAdd(sg + 3 * v + q, k * (x[3 * v + q] - target[3 * p + q]));
     double H[3][3] = {{k, 0, 0}, {0, k, 0}, {0, 0, k}};
-    emit_diag_block(bs, base + p, v, H);
+    store_single(cs, first + p, v, H);
 }
 
-// ---- contact block merge ------------------------------------------------------------------
-// run heads of the sorted keys (the unused-slot key forms no run); flag[m] = 0
-__global__ void k_run_heads(int m, const unsigned long long* __restrict__ ks, int* __restrict__ flag) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > m) return;
-    if (i == m) {
-        flag[m] = 0;
-        return;
-    }
-    const unsigned long long k = ks[i];
-    flag[i] = (k != kBadKey && (i == 0 || ks[i - 1] != k)) ? 1 : 0;
-}
+// ---- contact rows ---------------------------------------------------------------------------
+// After the incidences are sorted by vertex (stable: each vertex's list is in pair order), row v
+// of the contact matrix is made from v's list alone: every pair in it gives the blocks (v, w) of
+// its vertices w.  One warp takes a row of up to kRowLong incidences, a CTA a longer one.  The
+// distinct columns go into a small hash table in shared memory and are ranked; the blocks are
+// added up in shared memory, pair by pair in the list's order (half-warps take consecutive parts
+// of the list and their sums are added in order): the same result on every run.  A row of more columns than the
+// table holds is made in windows of columns.
+constexpr int kRowWarps = 4;
+constexpr int kRowLong = 128;  // incidences above which a CTA takes the row
+constexpr int kRowHash = 256;
+constexpr int kRowCols = 80;   // columns of a window (each of 32 * kRowWarps lanes may add one more)
+constexpr int kRowBatch = 16;  // pairs staged at a time
+static_assert(kRowCols + 32 * kRowWarps < kRowHash, "the hash table never fills up");
 
-// after the exclusive scan flag[i] = run id of head i; start[u] = first sorted index of run
-// u, start[nuc] = end of the last run; row / column of every unique block
-__global__ void k_run_starts(int m, const unsigned long long* __restrict__ ks, const int* __restrict__ rid, int bits,
-                             int* __restrict__ start, int* __restrict__ uc_row, int* __restrict__ uc_col,
-                             int* __restrict__ nuc, int* __restrict__ lcount) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > m) return;
-    // end of the last run: the first unused-slot key (sorted last), or m; written by the
-    // thread at that boundary (a binary search by one thread took ~19 round trips)
-    {
-        const bool here = i == m ? (m == 0 || ks[m - 1] != kBadKey) : (ks[i] == kBadKey && (i == 0 || ks[i - 1] != kBadKey));
-        if (here) {
-            const int nu = rid[m];
-            nuc[0] = nu;
-            start[nu] = i;
-        }
-    }
-    if (i == m) return;
-    const unsigned long long k = ks[i];
-    if (k == kBadKey || (i > 0 && ks[i - 1] == k)) return;
-    const int u = rid[i];
-    start[u] = i;
-    const unsigned long long mask = (1ull << bits) - 1ull;
-    const int row = (int)(k >> bits), col = (int)(k & mask);
-    uc_row[u] = row;
-    uc_col[u] = col;
-    // off-diagonal blocks also appear transposed, in the list of row `col`
-    if (row != col) atomicAdd(lcount + col, 1);
-}
-
-// ... and entry q of the transposed copy at slot lpos[u] gets entry q of the block, at its
-// transposed place 3 (q % 3) + q / 3
-// One warp per unique block (grid-stride over the blocks): lane l adds the run's slots l,
-// l + 32, ... in order, then a fixed xor tree adds the lanes, so the sum is the same run to
-// run; lanes 0..8 store the nine entries (upper and, transposed, lower copies).
-__global__ void __launch_bounds__(256) k_run_sums(const int* __restrict__ nuc, const int* __restrict__ start,
-                                                  const int* __restrict__ is, const double* __restrict__ cval,
-                                                  const int* __restrict__ lpos, double* __restrict__ u64,
-                                                  float* __restrict__ u32, double* __restrict__ l64,
-                                                  float* __restrict__ l32) {
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    const int nu = nuc[0];
-    for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < nu; u += nw) {
-        const int j0 = start[u], j1 = start[u + 1];
-        double acc[9];
-#pragma unroll
-        for (int q = 0; q < 9; q++) acc[q] = 0.0;
-        for (int j = j0 + lane; j < j1; j += 32) {
-            const double* v = cval + 9 * (size_t)is[j];
-#pragma unroll
-            for (int q = 0; q < 9; q++) acc[q] += v[q];
-        }
-#pragma unroll
-        for (int q = 0; q < 9; q++)
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-        if (lane < 9) {
-            double a = acc[0];
-#pragma unroll
-            for (int q = 1; q < 9; q++)
-                if (lane == q) a = acc[q];
-            u64[9 * (size_t)u + lane] = a;
-            u32[9 * (size_t)u + lane] = (float)a;
-            const int k = lpos[u];
-            if (k >= 0) {
-                const int qt = 3 * (lane % 3) + lane / 3;
-                l64[9 * (size_t)k + qt] = a;
-                l32[9 * (size_t)k + qt] = (float)a;
-            }
-        }
-    }
-}
-
-// upper row pointers (thread i <= n: first unique block whose row >= i, by binary search over
-// the row-sorted blocks) and placement of each off-diagonal block u in the transposed list of
-// row uc_col[u], in the order the atomics hand out the slots
-__global__ void k_lower_place(int m, int n, const int* __restrict__ nuc, const int* __restrict__ uc_row,
-                              const int* __restrict__ uc_col, const int* __restrict__ cl_ptr, int* __restrict__ fill,
-                              int* __restrict__ cu_ptr, int* __restrict__ cl_idx) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nu = nuc[0];
-    if (t <= n) {
-        // first block with row >= t: an 8-way search, seven probes in flight per step (five
-        // round trips for 30 000 blocks instead of fifteen)
-        int lo = 0, hi = nu;
-        while (hi - lo > 8) {
+// row pointers of the sorted incidences, the lists of rows to make, zeroed block counts
+__global__ void k_inc_rows(int n, int m, const uint32_t* __restrict__ ks, int* __restrict__ ptr,
+                           int* __restrict__ list, int* __restrict__ cnt, unsigned long long* __restrict__ ucnt) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    auto first = [&](int v) {  // first incidence with key >= v: an 8-way search, seven probes in flight
+        int lo = 0, hi = m;
+        while (lo < hi) {
             const int step = (hi - lo + 7) >> 3;
-            int below = 0;  // probes lo + step .. lo + 7 step with row < t
+            int below = 0;
 #pragma unroll
             for (int j = 1; j < 8; j++) {
-                const int p = lo + j * step;
-                below += (p < hi && uc_row[p] < t) ? 1 : 0;
+                const int p = lo + j * step - 1;
+                below += (p < hi && (int)__ldg(ks + p) < v) ? 1 : 0;
             }
-            // the answer lies in (lo + below * step, lo + (below + 1) * step]
-            const int nlo = lo + below * step, nhi = min(hi, lo + (below + 1) * step);
-            lo = below > 0 ? nlo + 1 : lo;
-            hi = nhi;
-            if (below > 0 && lo > hi) lo = hi;
+            // the answer lies in [lo + below * step, lo + (below + 1) * step - 1], or up to hi
+            if (below < 7) hi = min(hi, lo + (below + 1) * step - 1);
+            lo += below * step;
         }
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (uc_row[mid] < t) lo = mid + 1; else hi = mid;
-        }
-        cu_ptr[t] = lo;
+        return lo;
+    };
+    const int p0 = t <= n ? first(t) : 0;
+    if (t <= n) {
+        ptr[t] = p0;
+        ucnt[t] = 0ull;
     }
-    if (t < nu) {
-        const int col = uc_col[t];
-        if (uc_row[t] != col) cl_idx[cl_ptr[col] + atomicAdd(fill + col, 1)] = t;
+    int p1 = __shfl_down_sync(0xffffffffu, p0, 1);
+    if (lane == 31 && t < n) p1 = first(t + 1);
+    const int len = t < n ? p1 - p0 : 0;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {  // short lists, long lists
+        const bool on = c == 0 ? len > 0 && len <= kRowLong : len > kRowLong;
+        const unsigned b = __ballot_sync(0xffffffffu, on);
+        if (!b) continue;
+        int base = 0;
+        if (lane == 0) base = atomicAdd(cnt + c, __popc(b));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (on) list[(size_t)c * n + base + __popc(b & ((1u << lane) - 1u))] = t;
     }
 }
 
-// final slot of each off-diagonal block in its transposed list: its rank by row among the
-// blocks of the same column, so that every transposed list is sorted by column whatever order
-// the placement atomics took; lpos[u] = -1 for diagonal blocks
-__global__ void k_lower_rank(const int* __restrict__ nuc, const int* __restrict__ uc_row,
-                             const int* __restrict__ uc_col, const int* __restrict__ cl_ptr,
-                             const int* __restrict__ cl_idx, int* __restrict__ lpos, int* __restrict__ cl_col) {
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= nuc[0]) return;
-    const int row = uc_row[u], col = uc_col[u];
-    if (row == col) {
-        lpos[u] = -1;
-        return;
+struct RowArgs {
+    ContactStore cs;
+    const uint32_t* inc;   // sorted incidences
+    const int* ptr;
+    const int* list;
+    const int* cnt;
+    int n;
+};
+
+// the vertices of incidence i's pair (a single's vertex alone); returns its type
+__device__ __forceinline__ int inc_pair(const RowArgs& a, uint32_t i, int (&v)[4], int& item, int& local) {
+    if (i >= 4u * (uint32_t)a.cs.pairs) {
+        item = (int)(i - 4u * (uint32_t)a.cs.pairs);
+        local = 0;
+        v[0] = a.cs.sid[item];
+        v[1] = v[2] = v[3] = -1;
+        return kPairSingle;
     }
-    const int k0 = cl_ptr[col], k1 = cl_ptr[col + 1];
-    int rank = 0;
-    int k = k0;
-    for (; k + 4 <= k1; k += 4) {  // four list entries in flight
-        int ix[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) ix[u] = __ldg(cl_idx + k + u);
-#pragma unroll
-        for (int u = 0; u < 4; u++) rank += __ldg(uc_row + ix[u]) < row;
-    }
-    for (; k < k1; k++) rank += __ldg(uc_row + __ldg(cl_idx + k)) < row;
-    lpos[u] = k0 + rank;
-    cl_col[k0 + rank] = row;
+    item = (int)(i >> 2);
+    local = (int)(i & 3u);
+    const int4 id = __ldg(a.cs.ids + item);
+    v[0] = id.x & ~kMollBit, v[1] = id.y, v[2] = id.z, v[3] = id.w;
+    return item >= a.cs.barrier_pairs ? kPairFriction : ((id.x & kMollBit) ? kPairMollified : kPairBarrier);
 }
 
+// shared state of one row: a warp's, or (long rows) the CTA's, kept in the first warp's
+struct RowTable {
+    int hash[kRowHash];             // column, -1: free
+    unsigned char rank[kRowHash];   // its place among the window's sorted columns
+    unsigned short slot[kRowCols + 32 * kRowWarps];  // table slots in use, in order of arrival
+    int col[kRowCols];              // sorted columns
+    int used, over;
+};
+
+template <bool kCta>
+__device__ __forceinline__ void row_sync() {
+    if (kCta) __syncthreads();
+    else __syncwarp();
+}
+
+// The distinct columns of the row in [lo, hi) into the table; false: more than kRowCols of them.
+// t: this thread's index among the nt of its row.
+template <bool kCta>
+__device__ __forceinline__ bool row_columns(const RowArgs& a, RowTable& T, int i0, int i1, int lo, int hi, int t, int nt) {
+    for (int k = t; k < kRowHash; k += nt) T.hash[k] = -1;
+    if (t == 0) T.used = T.over = 0;
+    row_sync<kCta>();
+    for (int i = i0 + t; i < i1; i += nt) {
+        int v[4], item, local;
+        inc_pair(a, __ldg(a.inc + i), v, item, local);
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            const int c = v[b];
+            if (c < lo || c >= hi) continue;  // (-1 is below every window)
+            unsigned h = ((unsigned)c * 2654435761u) >> 24;
+            for (;;) {
+                const int seen = *(volatile int*)&T.hash[h];
+                if (seen == c) break;
+                if (seen < 0) {
+                    if (*(volatile int*)&T.used > kRowCols) {  // full: the caller takes a smaller window
+                        T.over = 1;
+                        break;
+                    }
+                    const int old = atomicCAS(&T.hash[h], -1, c);
+                    if (old == c) break;
+                    if (old < 0) {
+                        T.slot[atomicAdd(&T.used, 1)] = (unsigned short)h;
+                        break;
+                    }
+                }
+                h = (h + 1) & (kRowHash - 1);
+            }
+        }
+    }
+    row_sync<kCta>();
+    const bool ok = !T.over && T.used <= kRowCols;
+    row_sync<kCta>();
+    return ok;
+}
+
+// ranks the table's columns; U of them
+template <bool kCta>
+__device__ __forceinline__ void row_ranks(RowTable& T, int t, int nt) {
+    const int U = T.used;
+    for (int k = t; k < U; k += nt) {
+        const int h = T.slot[k], c = T.hash[h];
+        int r = 0;
+        for (int j = 0; j < U; j++) r += T.hash[T.slot[j]] < c;
+        T.rank[h] = (unsigned char)r;
+        T.col[r] = c;
+    }
+    row_sync<kCta>();
+}
+
+// calls fn() with each window's columns in the table, windows in column order
+template <bool kCta, class Fn>
+__device__ __forceinline__ void row_windows(const RowArgs& a, RowTable& T, int i0, int i1, int t, int nt, Fn fn) {
+    int lo = 0, hi = a.n;
+    while (lo < a.n) {  // uniform over the row's threads
+        if (!row_columns<kCta>(a, T, i0, i1, lo, hi, t, nt)) {
+            hi = lo + (hi - lo + 1) / 2;  // a window of one column always fits
+            continue;
+        }
+        fn();
+        row_sync<kCta>();
+        lo = hi;
+        hi = a.n;
+    }
+}
+
+// rows of the grid's share: long ones by CTA, short ones by warp; fn(v, t, nt, table, cta flag)
+template <class Long, class Short>
+__device__ __forceinline__ void for_rows(const RowArgs& a, Long f_long, Short f_short) {
+    const int n_short = a.cnt[0], n_long = a.cnt[1];
+    for (int k = blockIdx.x; k < n_long; k += gridDim.x) f_long(a.list[(size_t)a.n + k]);
+    __syncthreads();
+    const int nw = gridDim.x * kRowWarps;
+    // (counted from the last CTA: the first ones may have taken a long row more)
+    for (int k = (gridDim.x - 1 - blockIdx.x) * kRowWarps + (threadIdx.x >> 5); k < n_short; k += nw)
+        f_short(a.list[k]);
+}
+
+// unique blocks of every row: upper ones (column >= row) and transposed ones (<< 32)
+__global__ void __launch_bounds__(32 * kRowWarps) k_row_counts(RowArgs a, unsigned long long* __restrict__ ucnt) {
+    __shared__ RowTable tables[kRowWarps];
+    auto count = [&](auto cta, int v, RowTable& T, int t, int nt) {
+        unsigned up = 0, low = 0;  // of this thread's share of the columns
+        row_windows<decltype(cta)::value>(a, T, a.ptr[v], a.ptr[v + 1], t, nt, [&]() {
+            for (int k = t; k < T.used; k += nt) {
+                if (T.hash[T.slot[k]] >= v) up++;
+                else low++;
+            }
+        });
+        up = __reduce_add_sync(0xffffffffu, up);
+        low = __reduce_add_sync(0xffffffffu, low);
+        if ((threadIdx.x & 31) == 0 && (up | low)) atomicAdd(ucnt + v, (unsigned long long)up | ((unsigned long long)low << 32));
+    };
+    for_rows(
+        a, [&](int v) { count(std::true_type{}, v, tables[0], threadIdx.x, 32 * kRowWarps); },
+        [&](int v) { count(std::false_type{}, v, tables[threadIdx.x >> 5], threadIdx.x & 31, 32); });
+}
+
+struct RowOut {
+    const unsigned long long* uoff;
+    const int32_t* btype;
+    int* nuc;
+    int* cu_ptr;
+    int* cl_ptr;
+    int* uc_row;
+    int* uc_col;
+    double* u64;
+    float* u32;
+    int* cl_col;
+    double* l64;
+    float* l32;
+    double* grad;
+};
+
+// A half-warp adds up its part of a row's list: lanes 0..11 take column q of the block of vertex b
+// (three entries each), lanes 12..14 the gradient's component q.  (With one lane per entry a pair
+// took 36 lanes, twice the instructions of a warp for each: 1557 us for the rolled cloth's eight
+// million incidences.)
+struct RowWarp {
+    double acc[2][kRowCols * 9];
+    double fac[kRowBatch][kFac];
+    int meta[kRowBatch];                 // type | local vertex << 8 (-1: none)
+    int item[kRowBatch];
+    signed char col[kRowBatch][4];       // window column of each of the pair's vertices, -1: none
+};
+constexpr size_t kRowShared = sizeof(RowTable) * kRowWarps + sizeof(RowWarp) * kRowWarps;
+
+// [j0, j1): this half-warp's part of the list, into its acc (zeroed) and, in the first window, g
+__device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable& T, RowWarp& W, int v, int U, int j0,
+                                               int j1, int lo, int hi, bool first, double& g) {
+    constexpr int kHalf = kRowBatch / 2;
+    const int lane = threadIdx.x & 31, h = lane >> 4, hl = lane & 15;
+    const bool grad = hl >= 12;
+    const int b = grad ? 0 : hl / 3, q = hl % 3;
+    double* acc = W.acc[h];
+    for (int k = lane; k < 9 * U; k += 32) W.acc[0][k] = W.acc[1][k] = 0.0;
+    int turns = (j1 - j0 + kHalf - 1) / kHalf;
+    turns = max(turns, __shfl_xor_sync(0xffffffffu, turns, 16));
+    for (int t = 0; t < turns; t++) {
+        // two lanes per pair: ids, then half of its line each and the window columns of two vertices
+        const int j = lane >> 1, half = lane & 1, i = j0 + t * kHalf + (j & (kHalf - 1));
+        __syncwarp();
+        int meta = -1;
+        if (i < j1) {
+            int w[4], item, local;
+            const int type = inc_pair(a, __ldg(a.inc + i), w, item, local);
+            meta = type | (local << 8);
+            if (type == kPairSingle) {
+                if (half == 0)
+#pragma unroll
+                    for (int k = 0; k < 9; k++) W.fac[j][k] = a.cs.sval[9 * (size_t)item + k];
+            } else {
+                const double2* src = reinterpret_cast<const double2*>(a.cs.fac + kFac * (size_t)item) + 4 * half;
+                double2 f[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) f[k] = __ldg(src + k);
+#pragma unroll
+                for (int k = 0; k < 4; k++) reinterpret_cast<double2*>(W.fac[j])[4 * half + k] = f[k];
+            }
+            if (half == 0) W.item[j] = item;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if ((k >> 1) != half) continue;
+                const int c = w[k];
+                int u = -1;
+                // (a vertex named twice by a pair: its block is counted in the pair's order only)
+                if (c >= lo && c < hi && !(c == v && k < local)) {
+                    unsigned x = ((unsigned)c * 2654435761u) >> 24;
+                    while (T.hash[x] != c) x = (x + 1) & (kRowHash - 1);
+                    u = T.rank[x];
+                }
+                W.col[j][k] = (signed char)u;
+            }
+        }
+        if (half == 0) W.meta[j] = meta;
+        __syncwarp();
+        // four pairs at a time: their products first, then the sums one pair after another
+#pragma unroll
+        for (int k0 = 0; k0 < kHalf; k0 += 4) {
+            double x[4][3];
+            int u[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int j2 = h * kHalf + k0 + k, m = W.meta[j2], type = m & 0xff, la = (m >> 8) & 3;
+                const double* f = W.fac[j2];
+                u[k] = m < 0 || hl == 15 ? -1 : (grad ? (first ? 0 : -1) : W.col[j2][b]);
+                if (type == kPairBarrier && m >= 0) {
+                    // lam (g_a g_b): the same product for the transposed block
+                    const double s = f[grad ? 13 : 1 + 3 * b + q], lam = grad ? 1.0 : f[0];
+                    const double* r = f + 1 + 3 * la + (grad ? q : 0);
+                    x[k][0] = lam * (r[0] * s);
+                    x[k][1] = lam * (r[grad ? 0 : 1] * s);
+                    x[k][2] = lam * (r[grad ? 0 : 2] * s);
+                } else if (type == kPairFriction && m >= 0) {
+                    const double s = f[9 + la] * (grad ? 1.0 : f[9 + b]);
+                    const double* r = f + (grad ? 13 + q : q);
+                    x[k][0] = s * r[0];
+                    x[k][1] = s * r[grad ? 0 : 3];
+                    x[k][2] = s * r[grad ? 0 : 6];
+                } else {
+                    x[k][0] = x[k][1] = x[k][2] = 0.0;
+                    if (m >= 0 && type == kPairSingle) {
+                        if (grad) u[k] = -1;  // the singles' gradient is added where they are made
+                        else
+#pragma unroll
+                            for (int p = 0; p < 3; p++) x[k][p] = f[3 * p + q];
+                    } else if (m >= 0) {
+                        const double* f2 = a.cs.fac2 + kFac * (size_t)W.item[j2];
+                        if (grad) x[k][0] = pair_grad(type, f, f2, la, q);
+                        else
+#pragma unroll
+                            for (int p = 0; p < 3; p++) x[k][p] = pair_entry(type, f, f2, la, b, p, q);
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (u[k] >= 0) {
+                    if (grad) {
+                        g += x[k][0];
+                    } else {
+                        double* d = acc + 9 * u[k] + q;
+                        const double d0 = d[0], d1 = d[3], d2 = d[6];
+                        d[0] = d0 + x[k][0];
+                        d[3] = d1 + x[k][1];
+                        d[6] = d2 + x[k][2];
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// stores the window's blocks (threads t of nt), acc summed over the row's warps in order
+template <bool kCta>
+__device__ __forceinline__ void row_store(const RowArgs& a, const RowOut& o, const RowTable& T, const RowWarp* W, int v,
+                                          int U, int t, int nt, unsigned& up, unsigned& low) {
+    int nlow = 0;
+    for (int k = 0; k < U; k++) nlow += T.col[k] < v;
+    const bool fixed_row = o.btype && o.btype[v] != 0;
+    for (int e = t; e < 9 * U; e += nt) {
+        const int u = e / 9, q = e % 9, c = T.col[u];
+        double s = W[0].acc[0][e] + W[0].acc[1][e];
+        if (kCta)
+#pragma unroll
+            for (int w = 1; w < kRowWarps; w++) s = s + W[w].acc[0][e] + W[w].acc[1][e];
+        if (fixed_row || (o.btype && o.btype[c] != 0)) s = 0.0;
+        if (c < v) {
+            const size_t k = low + u;
+            o.l64[9 * k + q] = s;
+            o.l32[9 * k + q] = (float)s;
+            if (q == 0) o.cl_col[k] = c;
+        } else {
+            const size_t k = up + (u - nlow);
+            o.u64[9 * k + q] = s;
+            o.u32[9 * k + q] = (float)s;
+            if (q == 0) {
+                o.uc_row[k] = v;
+                o.uc_col[k] = c;
+            }
+        }
+    }
+    up += U - nlow;
+    low += nlow;
+}
+
+__global__ void __launch_bounds__(32 * kRowWarps) k_row_sums(RowArgs a, RowOut o) {
+    extern __shared__ __align__(16) unsigned char row_smem[];
+    __shared__ double s_grad[2 * kRowWarps][3];
+    RowWarp* warps = reinterpret_cast<RowWarp*>(row_smem);
+    RowTable* tables = reinterpret_cast<RowTable*>(row_smem + sizeof(RowWarp) * kRowWarps);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, hw = threadIdx.x >> 4, hl = threadIdx.x & 15;
+    // row pointers of the two block lists
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= a.n; i += gridDim.x * blockDim.x) {
+        const unsigned long long f = o.uoff[i];
+        o.cu_ptr[i] = (int)(f & 0xffffffffull);
+        o.cl_ptr[i] = (int)(f >> 32);
+        if (i == a.n) o.nuc[0] = (int)(f & 0xffffffffull);
+    }
+    for_rows(
+        a,
+        [&](int v) {
+            RowTable& T = tables[0];
+            const int i0 = a.ptr[v], i1 = a.ptr[v + 1];
+            const int part = (i1 - i0 + 2 * kRowWarps - 1) / (2 * kRowWarps);
+            unsigned up = (unsigned)(o.uoff[v] & 0xffffffffull), low = (unsigned)(o.uoff[v] >> 32);
+            double g = 0.0;
+            bool first = true;
+            int lo = 0, hi = a.n;
+            while (lo < a.n) {
+                if (!row_columns<true>(a, T, i0, i1, lo, hi, threadIdx.x, 32 * kRowWarps)) {
+                    hi = lo + (hi - lo + 1) / 2;
+                    continue;
+                }
+                row_ranks<true>(T, threadIdx.x, 32 * kRowWarps);
+                row_accumulate(a, T, warps[w], v, T.used, min(i1, i0 + hw * part), min(i1, i0 + (hw + 1) * part), lo, hi,
+                               first, g);
+                __syncthreads();
+                row_store<true>(a, o, T, warps, v, T.used, threadIdx.x, 32 * kRowWarps, up, low);
+                __syncthreads();
+                first = false;
+                lo = hi;
+                hi = a.n;
+            }
+            if (hl >= 12 && hl < 15) s_grad[hw][hl - 12] = g;
+            __syncthreads();
+            if (threadIdx.x < 3) {
+                double s = s_grad[0][lane];
+#pragma unroll
+                for (int k = 1; k < 2 * kRowWarps; k++) s += s_grad[k][lane];
+                o.grad[3 * (size_t)v + lane] += s;
+            }
+            __syncthreads();
+        },
+        [&](int v) {
+            RowTable& T = tables[w];
+            const int i0 = a.ptr[v], i1 = a.ptr[v + 1];
+            unsigned up = (unsigned)(o.uoff[v] & 0xffffffffull), low = (unsigned)(o.uoff[v] >> 32);
+            double g = 0.0;
+            bool first = true;
+            int lo = 0, hi = a.n;
+            while (lo < a.n) {
+                if (!row_columns<false>(a, T, i0, i1, lo, hi, lane, 32)) {
+                    hi = lo + (hi - lo + 1) / 2;
+                    continue;
+                }
+                row_ranks<false>(T, lane, 32);
+                const int mid = i0 + (i1 - i0 + 1) / 2;
+                row_accumulate(a, T, warps[w], v, T.used, lane < 16 ? i0 : mid, lane < 16 ? mid : i1, lo, hi, first, g);
+                row_store<false>(a, o, T, warps + w, v, T.used, lane, 32, up, low);
+                __syncwarp();
+                first = false;
+                lo = hi;
+                hi = a.n;
+            }
+            g += __shfl_down_sync(0xffffffffu, g, 16);  // the halves in list order
+            if (lane >= 12 && lane < 15) o.grad[3 * (size_t)v + lane - 12] += g;
+        });
+}
 
 // ------------------------------------------------------------------------------------------
 // line-search energy (GIPC::computeEnergy, GIPC.cu:10520-10580; per-term reductions
@@ -1324,44 +1634,43 @@ static SgipcStatus check_inputs(SgipcCtx* c, const SgipcFemData* f, const SgipcC
     return SGIPC_OK;
 }
 
-static BlockSink sink(SgipcCtx* c, const SgipcFemData* f) {
-    BlockSink bs;
-    bs.key = c->ckey;
-    bs.idx = c->cidx;
-    bs.val = c->cval;
-    bs.btype = f->BoundaryType;
-    bs.bits = c->key_bits;
-    bs.nv = c->nv;
-    bs.flag = c->dflag;
-    return bs;
+// contact items of a call: barrier and friction pairs, ground and ground-friction vertices
+struct ContactCounts {
+    int np = 0, nf = 0, ng = 0, ngf = 0;
+    int pairs() const { return np + nf; }
+    int singles() const { return ng + ngf; }
+};
+static ContactCounts contact_counts(const SgipcContacts* k, const SgipcParams* p) {
+    ContactCounts c;
+    if (!k) return c;
+    c.np = k->pair_num > 0 ? k->pair_num : 0;
+    c.nf = k->fric_num > 0 && p->frictionRate > 0.0 ? k->fric_num : 0;
+    c.ng = k->ground_num > 0 ? k->ground_num : 0;
+    c.ngf = k->fric_gd_num > 0 && p->gd_frictionRate > 0.0 ? k->fric_gd_num : 0;
+    return c;
 }
 
-// contact block slots launch_contacts will use (soft constraints follow them)
-static int contact_slots(const SgipcContacts* k, const SgipcParams* p) {
-    if (!k) return 0;
-    int m = 0;
-    if (k->pair_num > 0) m += 10 * k->pair_num;
-    if (k->fric_num > 0 && p->frictionRate > 0.0) m += 10 * k->fric_num;
-    if (k->ground_num > 0) m += k->ground_num;
-    if (k->fric_gd_num > 0 && p->gd_frictionRate > 0.0) m += k->fric_gd_num;
-    return m;
+static ContactStore contact_store(SgipcCtx* c, const ContactCounts& cc) {
+    return {c->con_ids, c->con_fac, c->con_fac2, c->con_sid, c->con_sval, c->con_key, c->con_val,
+            cc.pairs(), cc.np, c->n, c->nv, c->dflag};
 }
 
-// launch the contact kernels; returns the number of contact block slots used
-static int launch_contacts(SgipcCtx* c, const SgipcFemData* f, const SgipcContacts* k, const SgipcParams* p,
-                           double* grad, cudaStream_t s, bool keep_dirichlet = false) {
-    BlockSink bs = sink(c, f);
-    if (keep_dirichlet) bs.btype = nullptr;
-    if (!k) return 0;
+// launch the contact kernel: factors, incidences and, into grad, the singles' gradient (kGrad:
+// the pairs' too)
+template <bool kGrad>
+static void launch_contacts(SgipcCtx* c, const SgipcFemData* f, const SgipcContacts* k, const SgipcParams* p,
+                            double* grad, cudaStream_t s) {
+    const ContactCounts cc = contact_counts(k, p);
+    if (cc.pairs() + cc.singles() == 0) return;
     ContactLaunch L{};
-    L.np = k->pair_num > 0 ? k->pair_num : 0;
-    L.nf = k->fric_num > 0 && p->frictionRate > 0.0 ? k->fric_num : 0;
-    L.ng = k->ground_num > 0 ? k->ground_num : 0;
-    L.ngf = k->fric_gd_num > 0 && p->gd_frictionRate > 0.0 ? k->fric_gd_num : 0;
-    L.cb = nblk(L.np, 128);
-    L.cf = L.cb + nblk(L.nf, 128);
-    L.cg = L.cf + nblk(L.ng, 128);
-    const int grid = L.cg + nblk(L.ngf, 128);
+    L.np = cc.np;
+    L.nf = cc.nf;
+    L.ng = cc.ng;
+    L.ngf = cc.ngf;
+    L.cb = nblk(L.np, kConThreads);
+    L.cf = L.cb + nblk(L.nf, kConThreads);
+    L.cg = L.cf + nblk(L.ng, kConThreads);
+    const int grid = L.cg + nblk(L.ngf, kConThreads);
     L.pairs = (const int4*)k->pairs;
     L.fpairs = (const int4*)k->fric_pairs;
     L.gpairs = k->ground_pairs;
@@ -1379,49 +1688,38 @@ static int launch_contacts(SgipcCtx* c, const SgipcFemData* f, const SgipcContac
     L.gmu = p->gd_frictionRate;
     L.eps2 = p->fDhat * p->dt * p->dt;
     L.offset = p->ground_offset;
-    L.base_b = 0;
-    L.base_f = 10 * L.np;
-    L.base_g = L.base_f + 10 * L.nf;
-    L.base_gf = L.base_g + L.ng;
-    if (grid > 0) {
-        SG_COUNT(c, 1);
-        k_contacts<<<grid, 128, 0, s>>>(L, grad, bs);
-    }
-    return L.base_gf + L.ngf;
+    SG_COUNT(c, 1);
+    k_contacts<kGrad><<<grid, kConThreads, 0, s>>>(L, grad, contact_store(c, cc));
 }
 
-static SgipcStatus merge_contacts(SgipcCtx* c, int m, cudaStream_t s) {
+// The contact rows (unique upper blocks, transposed lists, the pairs' gradient added into grad)
+// from the stored factors of cc's pairs and `singles` singles.
+static SgipcStatus merge_contacts(SgipcCtx* c, const ContactCounts& cc, int singles, const int32_t* btype,
+                                  double* grad, cudaStream_t s) {
+    const int m = 4 * cc.pairs() + singles, n = c->n;
     if (m == 0) {
         SG_CHECK(c, cudaMemsetAsync(c->nuc, 0, sizeof(int), s));
-        SG_CHECK(c, cudaMemsetAsync(c->cu_ptr, 0, sizeof(int) * (c->n + 1), s));
-        SG_CHECK(c, cudaMemsetAsync(c->cl_ptr, 0, sizeof(int) * (c->n + 1), s));
+        SG_CHECK(c, cudaMemsetAsync(c->cu_ptr, 0, sizeof(int) * (n + 1), s));
+        SG_CHECK(c, cudaMemsetAsync(c->cl_ptr, 0, sizeof(int) * (n + 1), s));
         return SGIPC_OK;
     }
-    const int endbit = 2 * c->key_bits, n = c->n;
-    SG_COUNT(c, 5);
-    // keys sorted with their slot ids; runs of equal keys numbered by a scan of run heads;
-    // each unique block summed by 9 threads (one per entry) over its run in sorted order
-    // (deterministic), with every load of a run independent of the previous one.  The
-    // transposed lists need no second sort: the run heads count the blocks of each column,
-    // a scan of the counts gives the row pointers, and each block's rank by row within its
-    // column gives its slot.
-    SG_CHECK(c, cudaMemsetAsync(c->lcount, 0, sizeof(int) * (2 * (size_t)n + 1), s));
+    SG_COUNT(c, 3);
+    SG_CHECK(c, cudaMemsetAsync(c->row_cnt, 0, 2 * sizeof(int), s));
     size_t tb = c->cub_tmp_bytes;
-    SG_CHECK(c, cub::DeviceRadixSort::SortPairs(c->cub_tmp, tb, c->ckey, c->ckey_s, c->cidx, c->cidx_s, m, 0, endbit, s));
-    k_run_heads<<<nblk(m + 1), SGIPC_BLOCK, 0, s>>>(m, c->ckey_s, c->cflag);
+    SG_CHECK(c, cub::DeviceRadixSort::SortPairs(c->cub_tmp, tb, c->con_key, c->con_key_s, c->con_val, c->con_val_s, m,
+                                                0, c->key_bits, s));
+    k_inc_rows<<<nblk(n + 1), SGIPC_BLOCK, 0, s>>>(n, m, c->con_key_s, c->inc_ptr, c->row_list, c->row_cnt, c->ucnt);
+    const RowArgs a{contact_store(c, cc), c->con_val_s, c->inc_ptr, c->row_list, c->row_cnt, n};
+    // (the grids cover the chip once; a CTA of k_row_sums holds 62 KB)
+    const int most = nblk(m, 8);  // no more CTAs than a small call has work for
+    k_row_counts<<<std::min(most, 148 * 8), 32 * kRowWarps, 0, s>>>(a, c->ucnt);
     tb = c->cub_tmp_bytes;
-    SG_CHECK(c, cub::DeviceScan::ExclusiveSum(c->cub_tmp, tb, c->cflag, c->cflag, m + 1, s));
-    k_run_starts<<<nblk(m + 1), SGIPC_BLOCK, 0, s>>>(m, c->ckey_s, c->cflag, c->key_bits, c->run_start, c->uc_row,
-                                                     c->uc_col, c->nuc, c->lcount);
-    tb = c->cub_tmp_bytes;
-    SG_CHECK(c, cub::DeviceScan::ExclusiveSum(c->cub_tmp, tb, c->lcount, c->cl_ptr, n + 1, s));
-    k_lower_place<<<nblk(std::max(m, n + 1)), SGIPC_BLOCK, 0, s>>>(m, n, c->nuc, c->uc_row, c->uc_col, c->cl_ptr,
-                                                                   c->lcount + n + 1, c->cu_ptr, c->cl_idx);
-    k_lower_rank<<<nblk(m), SGIPC_BLOCK, 0, s>>>(c->nuc, c->uc_row, c->uc_col, c->cl_ptr, c->cl_idx, c->lpos,
-                                                 c->cl_col);
-    k_run_sums<<<std::min(nblk(32LL * m), 8 * 148), SGIPC_BLOCK, 0, s>>>(c->nuc, c->run_start, c->cidx_s, c->cval,
-                                                                         c->lpos, c->uc64, c->uc32, c->cl64, c->cl32);
-    SG_LAUNCH_CHECK(c, "contact merge");
+    SG_CHECK(c, cub::DeviceScan::ExclusiveSum(c->cub_tmp, tb, c->ucnt, c->uoff, n + 1, s));
+    const RowOut o{c->uoff, btype, c->nuc, c->cu_ptr, c->cl_ptr, c->uc_row, c->uc_col, c->uc64, c->uc32, c->cl_col,
+                   c->cl64, c->cl32, grad};
+    SG_CHECK(c, cudaFuncSetAttribute(k_row_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowShared));
+    k_row_sums<<<std::min(std::max(most, 148), 148 * 3), 32 * kRowWarps, kRowShared, s>>>(a, o);
+    SG_LAUNCH_CHECK(c, "contact rows");
     return SGIPC_OK;
 }
 
@@ -1485,19 +1783,16 @@ extern "C" SgipcStatus sgipc_assemble(SgipcCtx* c, const SgipcFemData* f, const 
     // (the soft constraints go first on s: the merge needs their block slots, and they add
     // to shape_grads before the element gradients do)
     cudaStream_t sc = c->asm_stream;
-    const int m_con = contact_slots(k, p);
-    if (c->nsoft > 0) {
-        BlockSink bs = sink(c, f);
+    const ContactCounts cc = contact_counts(k, p);
+    if (c->nsoft > 0)
         k_soft<<<nblk(c->nsoft), SGIPC_BLOCK, 0, s>>>(c->nsoft, c->soft_idx, f->vertexes, f->targetVert,
-                                                      p->motionRate * p->softRate * p->softRate, c->shape_grads, bs,
-                                                      m_con);
-    }
+                                                      p->motionRate * p->softRate * p->softRate, c->shape_grads,
+                                                      contact_store(c, cc), cc.singles());
     SG_CHECK(c, cudaEventRecord(c->ev_asm[0], s));
     SG_CHECK(c, cudaStreamWaitEvent(sc, c->ev_asm[0], 0));
-    int m = launch_contacts(c, f, k, p, c->fb, sc);
+    launch_contacts<false>(c, f, k, p, c->fb, sc);
     SG_LAUNCH_CHECK(c, "contact kernels");
-    m += c->nsoft;
-    if ((st = merge_contacts(c, m, sc)) != SGIPC_OK) return st;
+    if ((st = merge_contacts(c, cc, cc.singles() + c->nsoft, f->BoundaryType, c->fb, sc)) != SGIPC_OK) return st;
     if ((st = launch_fem(c, f, p, s)) != SGIPC_OK) return st;
     if ((st = gather_static(c, f, s)) != SGIPC_OK) return st;
     // the static blocks into the prebuilt hierarchy's domains, on the MAS stream beside the merge
@@ -1522,9 +1817,10 @@ extern "C" SgipcStatus sgipc_barrier_grad_hess(SgipcCtx* c, const SgipcFemData* 
     only.fric_num = 0;
     only.ground_num = 0;
     only.fric_gd_num = 0;
-    int m = launch_contacts(c, f, &only, p, grad, s);
+    launch_contacts<false>(c, f, &only, p, grad, s);
     SG_LAUNCH_CHECK(c, "barrier");
-    return merge_contacts(c, m, s);
+    const ContactCounts cc = contact_counts(&only, p);
+    return merge_contacts(c, cc, cc.singles(), f->BoundaryType, grad, s);
 }
 
 extern "C" SgipcStatus sgipc_friction_grad_hess(SgipcCtx* c, const SgipcFemData* f, const SgipcContacts* k,
@@ -1537,9 +1833,10 @@ extern "C" SgipcStatus sgipc_friction_grad_hess(SgipcCtx* c, const SgipcFemData*
     SgipcContacts only = *k;
     only.pair_num = 0;
     only.ground_num = 0;
-    int m = launch_contacts(c, f, &only, p, grad, s);
+    launch_contacts<false>(c, f, &only, p, grad, s);
     SG_LAUNCH_CHECK(c, "friction");
-    return merge_contacts(c, m, s);
+    const ContactCounts cc = contact_counts(&only, p);
+    return merge_contacts(c, cc, cc.singles(), f->BoundaryType, grad, s);
 }
 
 extern "C" SgipcStatus sgipc_fem_grad_hess(SgipcCtx* c, const SgipcFemData* f, const SgipcParams* p, double* grad,
@@ -1563,52 +1860,76 @@ extern "C" SgipcStatus sgipc_fem_grad_hess(SgipcCtx* c, const SgipcFemData* f, c
 // ------------------------------------------------------------------------------------------
 namespace sgipc {
 // ---- class partition of the contact terms (affine-body points) ------------------------------
+// Upper block `slot` of the contact terms: 10 per pair ((a, b) with a <= b in the pair's order),
+// then one per single.  False: unused.  (r, c): its row and column, r <= c; a, b the local vertices
+// with a at r.
+__device__ __forceinline__ bool part_slot(const ContactStore& cs, int singles, int slot, int& r, int& c, int& item,
+                                          int& a, int& b) {
+    if (slot >= 10 * cs.pairs) {
+        item = slot - 10 * cs.pairs;
+        r = c = item < singles ? cs.sid[item] : -1;
+        a = b = 0;
+        return r >= 0;
+    }
+    item = slot / 10;
+    const int k = slot % 10;
+    a = k < 4 ? 0 : (k < 7 ? 1 : (k < 9 ? 2 : 3));
+    b = k < 4 ? k : (k < 7 ? k - 3 : (k < 9 ? k - 5 : 3));
+    const int4 id = cs.ids[item];
+    const int v[4] = {id.x < 0 ? -1 : id.x & ~kMollBit, id.y, id.z, id.w};
+    r = v[a], c = v[b];
+    if (r < 0 || c < 0) return false;
+    if (r > c) {
+        const int t = r, u = a;
+        r = c, c = t;
+        a = b, b = u;
+    }
+    return true;
+}
+// its entry (p, q)
+__device__ __forceinline__ double part_entry(const ContactStore& cs, int slot, int item, int a, int b, int p, int q) {
+    if (slot >= 10 * cs.pairs) return cs.sval[9 * (size_t)item + 3 * p + q];
+    const int type = item >= cs.barrier_pairs ? kPairFriction
+                                              : ((cs.ids[item].x & kMollBit) ? kPairMollified : kPairBarrier);
+    return pair_entry(type, cs.fac + kFac * (size_t)item, cs.fac2 + kFac * (size_t)item, a, b, p, q);
+}
+
 // slot s of the contact blocks: fa[s] = 1 for an ABD-ABD block, ff[s] = 1 for an ABD-FEM block
-// (upper keys: r <= c, so an ABD-FEM block has r < af <= c)
-__global__ void k_part_flags(int m, const unsigned long long* __restrict__ key, int bits, int af, int* __restrict__ fa,
-                             int* __restrict__ ff) {
+// (upper blocks: r <= c, so an ABD-FEM block has r < af <= c)
+__global__ void k_part_flags(int m, int singles, ContactStore cs, int af, int* __restrict__ fa, int* __restrict__ ff) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s > m) return;
-    int a = 0, f = 0;
-    if (s < m) {
-        const unsigned long long k = key[s];
-        if (k != kBadKey) {
-            const int r = (int)(k >> bits), c = (int)(k & ((1ull << bits) - 1));
-            a = r >= af;
-            f = r < af && c >= af;
-        }
-    }
-    fa[s] = a;
-    ff[s] = f;
+    int r, c, item, a, b;
+    const bool on = s < m && part_slot(cs, singles, s, r, c, item, a, b);
+    fa[s] = on && r >= af;
+    ff[s] = on && r < af && c >= af;
 }
 
 // emit the flagged blocks at their scanned positions (slot order): ABD-ABD as (point, point)
 // with point ids counted from af, ABD-FEM as (point, FEM vertex) with the block transposed to
 // that orientation
-__global__ void k_part_emit(int m, const unsigned long long* __restrict__ key, const double* __restrict__ val, int bits,
-                            int af, const int* __restrict__ oa, const int* __restrict__ of, int cap,
-                            int32_t* __restrict__ arow, int32_t* __restrict__ acol, double* __restrict__ aval,
-                            int32_t* __restrict__ frow, int32_t* __restrict__ fcol, double* __restrict__ fval) {
+__global__ void k_part_emit(int m, int singles, ContactStore cs, int af, const int* __restrict__ oa,
+                            const int* __restrict__ of, int cap, int32_t* __restrict__ arow,
+                            int32_t* __restrict__ acol, double* __restrict__ aval, int32_t* __restrict__ frow,
+                            int32_t* __restrict__ fcol, double* __restrict__ fval) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= m) return;
-    const unsigned long long k = key[s];
-    if (k == kBadKey) return;
-    const int r = (int)(k >> bits), c = (int)(k & ((1ull << bits) - 1));
-    const double* v = val + 9 * (size_t)s;
+    int r, c, item, a, b;
+    if (s >= m || !part_slot(cs, singles, s, r, c, item, a, b) || c < af) return;
+    const int i = r >= af ? oa[s] : of[s];
+    if (i >= cap) return;
     if (r >= af) {
-        const int i = oa[s];
-        if (i >= cap) return;
         arow[i] = r - af;
         acol[i] = c - af;
-        for (int q = 0; q < 9; q++) aval[9 * (size_t)i + q] = v[q];
-    } else if (c >= af) {
-        const int i = of[s];
-        if (i >= cap) return;
+    } else {
         frow[i] = c - af;
         fcol[i] = r;
-        for (int p = 0; p < 3; p++)
-            for (int q = 0; q < 3; q++) fval[9 * (size_t)i + 3 * p + q] = v[3 * q + p];
     }
+    for (int p = 0; p < 3; p++)
+        for (int q = 0; q < 3; q++) {
+            const double v = part_entry(cs, s, item, a, b, p, q);
+            if (r >= af) aval[9 * (size_t)i + 3 * p + q] = v;
+            else fval[9 * (size_t)i + 3 * q + p] = v;
+        }
 }
 
 __global__ void k_part_grad(int npt, int af, const double* __restrict__ g, double* __restrict__ pg) {
@@ -1634,19 +1955,22 @@ extern "C" SgipcStatus sgipc_contact_partition(SgipcCtx* c, const SgipcFemData* 
     SG_DEVICE(c);
     const int npt = c->nv - abd_first;
     SG_CHECK(c, cudaMemsetAsync(c->tmp64, 0, sizeof(double) * 3 * (size_t)c->nv, s));
-    const int m = launch_contacts(c, f, k, p, c->tmp64, s, true);
+    launch_contacts<true>(c, f, k, p, c->tmp64, s);
     SG_LAUNCH_CHECK(c, "contact kernels (partition)");
-    int* fa = c->cflag;
-    int* ff = c->run_start;
+    const ContactCounts cc = contact_counts(k, p);
+    const ContactStore cs = contact_store(c, cc);
+    const int m = 10 * cc.pairs() + cc.singles();
+    int* fa = c->part_a;
+    int* ff = c->part_f;
     SG_COUNT(c, 2 + (npt > 0 && point_grad ? 1 : 0));
-    k_part_flags<<<nblk(m + 1), SGIPC_BLOCK, 0, s>>>(m, c->ckey, c->key_bits, abd_first, fa, ff);
+    k_part_flags<<<nblk(m + 1), SGIPC_BLOCK, 0, s>>>(m, cc.singles(), cs, abd_first, fa, ff);
     size_t tb = c->cub_tmp_bytes;
     SG_CHECK(c, cub::DeviceScan::ExclusiveSum(c->cub_tmp, tb, fa, fa, m + 1, s));
     tb = c->cub_tmp_bytes;
     SG_CHECK(c, cub::DeviceScan::ExclusiveSum(c->cub_tmp, tb, ff, ff, m + 1, s));
     if (m > 0)
-        k_part_emit<<<nblk(m), SGIPC_BLOCK, 0, s>>>(m, c->ckey, c->cval, c->key_bits, abd_first, fa, ff, cap, abd_rows,
-                                                    abd_cols, abd_vals, fem_rows, fem_cols, fem_vals);
+        k_part_emit<<<nblk(m), SGIPC_BLOCK, 0, s>>>(m, cc.singles(), cs, abd_first, fa, ff, cap, abd_rows, abd_cols,
+                                                    abd_vals, fem_rows, fem_cols, fem_vals);
     if (npt > 0 && point_grad) k_part_grad<<<nblk(3LL * npt), SGIPC_BLOCK, 0, s>>>(npt, abd_first, c->tmp64, point_grad);
     SG_LAUNCH_CHECK(c, "contact partition");
     int cnt[2];
@@ -1702,11 +2026,10 @@ extern "C" SgipcStatus sgipc_init_kappa(SgipcCtx* c, const SgipcFemData* f, cons
     k_kinetic<<<nblk(3LL * nv), SGIPC_BLOCK, 0, s>>>(nv, f->vertexes, f->xTilta, f->masses, GE, gc);
     if ((st = launch_fem(c, f, p, s)) != SGIPC_OK) return st;
     k_gather_grad_tets<<<nblk(3LL * nv), SGIPC_BLOCK, 0, s>>>(nv, 4 * c->nt, c->vinc_ptr, c->vinc, c->egrad, GE);
-    if (c->nsoft > 0) {
-        BlockSink bs = sink(c, f);
+    if (c->nsoft > 0)
         k_soft<<<nblk(c->nsoft), SGIPC_BLOCK, 0, s>>>(c->nsoft, c->soft_idx, f->vertexes, f->targetVert,
-                                                      p->motionRate * p->softRate * p->softRate, GE, bs, 0);
-    }
+                                                      p->motionRate * p->softRate * p->softRate, GE,
+                                                      contact_store(c, ContactCounts{}), 0);
     SgipcContacts only = *k;
     only.fric_num = 0;
     only.fric_gd_num = 0;
@@ -1714,7 +2037,7 @@ extern "C" SgipcStatus sgipc_init_kappa(SgipcCtx* c, const SgipcFemData* f, cons
     p1.kappa = 1.0;
     p1.frictionRate = 0.0;
     p1.gd_frictionRate = 0.0;
-    launch_contacts(c, f, &only, &p1, gc, s);
+    launch_contacts<true>(c, f, &only, &p1, gc, s);
     SG_LAUNCH_CHECK(c, "init kappa gradients");
     if ((st = dot64(c, gc, GE, 3 * nv, c->dot_out, s)) != SGIPC_OK) return st;
     if ((st = dot64(c, gc, gc, 3 * nv, c->dot_out + 1, s)) != SGIPC_OK) return st;
@@ -1865,23 +2188,20 @@ SgipcStatus assemble_time_hook(SgipcCtx* c, const char* name, cudaStream_t s, do
         // upper value out, the full-pattern FP64 + FP32 copy, and the transposed copy off the
         // diagonal
         *bytes = (double)c->n_eblk * (72 + 4) + (double)c->nnz * (28 + 72 + 108) + (double)(c->nnz - c->n) * 108;
-    } else if (!strcmp(name, "barrier")) {
-        if (!k || k->pair_num <= 0) return SGIPC_BAD_INPUT;
-        SG_COUNT(c, 1);
-        BlockSink bs = sink(c, f);
-        k_barrier<<<nblk(k->pair_num, 128), 128, 0, s>>>(k->pair_num, (const int4*)k->pairs, f->vertexes,
-                                                          f->rest_vertexes, p->dHat, p->kappa, scratch, bs, 0);
-        // pair + 4 positions (+ 4 rest positions) in; 10 keyed FP64 blocks and 12 gradient entries out
-        *bytes = (double)k->pair_num * (16 + 4 * 24 + 4 * 24 + 10 * (72 + 8 + 4) + 12 * 8);
-    } else if (!strcmp(name, "friction")) {
-        if (!k || k->fric_num <= 0) return SGIPC_BAD_INPUT;
-        SG_COUNT(c, 1);
-        BlockSink bs = sink(c, f);
-        k_friction<<<nblk(k->fric_num, 128), 128, 0, s>>>(k->fric_num, (const int4*)k->fric_pairs, f->vertexes,
-                                                           f->o_vertexes, k->fric_lambda, k->fric_coord, k->fric_basis,
-                                                           p->frictionRate, p->fDhat * p->dt * p->dt, scratch, bs,
-                                                           10 * (k->pair_num > 0 ? k->pair_num : 0));
-        *bytes = (double)k->fric_num * (16 + 8 + 16 + 48 + 8 * 24 + 10 * (72 + 8 + 4) + 12 * 8);
+    } else if (!strcmp(name, "barrier") || !strcmp(name, "friction")) {
+        // one kind's launch (its factors and keys are rewritten with the same values)
+        if (!k) return SGIPC_BAD_INPUT;
+        const bool fric = name[0] == 'f';
+        SgipcContacts only = *k;
+        only.ground_num = only.fric_gd_num = 0;
+        if (fric) only.pair_num = 0;
+        else only.fric_num = 0;
+        const ContactCounts cc = contact_counts(&only, p);
+        if (cc.pairs() <= 0) return SGIPC_BAD_INPUT;
+        launch_contacts<false>(c, f, &only, p, scratch, s);
+        // pair, 4 positions and 4 rest (or start-of-step) positions in, the friction data; ids,
+        // incidence keys and values, and the factors out
+        *bytes = (double)cc.pairs() * (16 + 8 * 24 + (fric ? 8 + 16 + 48 : 0) + 16 + 4 * 8 + 8 * kFac);
     } else {
         return SGIPC_NOT_READY;
     }

@@ -324,15 +324,20 @@ extern "C" SgipcStatus sgipc_create(const SgipcTopology* t_in, int device, Sgipc
     long long cap = 10LL * c->max_pairs + 10LL * c->max_fric + c->max_ground + c->max_fric_gd + c->nsoft + 1;
     if (cap > (1LL << 30)) return fail(SGIPC_CAPACITY);
     c->cap_cblk = (int)cap;
-    if ((st = dalloc(c, &c->ckey, cap)) || (st = dalloc(c, &c->ckey_s, cap)) || (st = dalloc(c, &c->cidx, cap)) ||
-        (st = dalloc(c, &c->cidx_s, cap)) || (st = dalloc(c, &c->cval, cap * 9)) ||
-        (st = dalloc(c, &c->run_start, cap + 1)) ||
-        (st = dalloc(c, &c->cflag, cap + 1)) || (st = dalloc(c, &c->nuc, 4)) || (st = dalloc(c, &c->uc_row, cap)) ||
-        (st = dalloc(c, &c->uc_col, cap)) || (st = dalloc(c, &c->uc64, cap * 9)) ||
-        (st = dalloc(c, &c->uc32, cap * 9)) || (st = dalloc(c, &c->cu_ptr, n + 1)) ||
-        (st = dalloc(c, &c->cl_ptr, n + 1)) || (st = dalloc(c, &c->cl_idx, cap)) || (st = dalloc(c, &c->lcount, 2 * (size_t)n + 1)) ||
-        (st = dalloc(c, &c->cl_col, cap)) || (st = dalloc(c, &c->cl64, cap * 9)) || (st = dalloc(c, &c->cl32, cap * 9)) ||
-        (st = dalloc(c, &c->lpos, cap)) || (st = dalloc(c, &c->dflag, 4)))
+    const size_t np = (size_t)c->max_pairs + c->max_fric, ns = (size_t)c->max_ground + c->max_fric_gd + c->nsoft;
+    const size_t ninc = 4 * np + ns;
+    if ((st = dalloc(c, &c->con_ids, np)) || (st = dalloc(c, &c->con_fac, 16 * np)) ||
+        (st = dalloc(c, &c->con_fac2, 16 * (size_t)c->max_pairs)) || (st = dalloc(c, &c->con_sid, ns)) ||
+        (st = dalloc(c, &c->con_sval, 9 * ns)) || (st = dalloc(c, &c->con_key, ninc)) ||
+        (st = dalloc(c, &c->con_val, ninc)) || (st = dalloc(c, &c->con_key_s, ninc)) ||
+        (st = dalloc(c, &c->con_val_s, ninc)) || (st = dalloc(c, &c->inc_ptr, (size_t)n + 1)) ||
+        (st = dalloc(c, &c->row_list, 2 * (size_t)n)) || (st = dalloc(c, &c->row_cnt, 2)) ||
+        (st = dalloc(c, &c->ucnt, (size_t)n + 1)) || (st = dalloc(c, &c->uoff, (size_t)n + 1)) ||
+        (st = dalloc(c, &c->part_a, cap + 1)) || (st = dalloc(c, &c->part_f, cap + 1)) ||
+        (st = dalloc(c, &c->nuc, 4)) || (st = dalloc(c, &c->uc_row, cap)) || (st = dalloc(c, &c->uc_col, cap)) ||
+        (st = dalloc(c, &c->uc64, cap * 9)) || (st = dalloc(c, &c->uc32, cap * 9)) ||
+        (st = dalloc(c, &c->cu_ptr, n + 1)) || (st = dalloc(c, &c->cl_ptr, n + 1)) || (st = dalloc(c, &c->cl_col, cap)) ||
+        (st = dalloc(c, &c->cl64, cap * 9)) || (st = dalloc(c, &c->cl32, cap * 9)) || (st = dalloc(c, &c->dflag, 4)))
         return fail(st);
     SG_CHECK(c, cudaMemset(c->dflag, 0, 4 * sizeof(int)));
     // energy partial sums: one per CTA of every term's kernel at the context's capacities
@@ -352,16 +357,16 @@ extern "C" SgipcStatus sgipc_create(const SgipcTopology* t_in, int device, Sgipc
         SG_CHECK(c, cudaMemset(c->en_ticket, 0, sizeof(unsigned int)));
         SG_CHECK(c, cudaMallocHost((void**)&c->h_en, sizeof(double) * 16));
     }
-    // contact block keys are (row << bits) | col with row, col < 2^bits - 1, so that the
-    // all-ones key of an unused slot sorts after every real block
+    // incidence keys are vertices < n < 2^bits; unused incidences have the key n and sort last
     int bits = 1;
     while ((1LL << bits) < (long long)n + 2) bits++;
     c->key_bits = bits;
-    // CUB temporary storage: radix sort of cap pairs, exclusive scans of cap + 1 and n + 1 ints
+    // CUB temporary storage: radix sort of the incidences, exclusive scans of cap + 1 ints and
+    // n + 1 words
     size_t b1 = 0, b2 = 0, b3 = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, b1, c->ckey, c->ckey_s, c->cidx, c->cidx_s, (int)cap, 0, 64);
-    cub::DeviceScan::ExclusiveSum(nullptr, b2, c->cflag, c->cflag, (int)cap + 1);
-    cub::DeviceScan::ExclusiveSum(nullptr, b3, c->lcount, c->cl_ptr, n + 1);
+    cub::DeviceRadixSort::SortPairs(nullptr, b1, c->con_key, c->con_key_s, c->con_val, c->con_val_s, (int)ninc, 0, bits);
+    cub::DeviceScan::ExclusiveSum(nullptr, b2, c->part_a, c->part_a, (int)cap + 1);
+    cub::DeviceScan::ExclusiveSum(nullptr, b3, c->ucnt, c->uoff, n + 1);
     c->cub_tmp_bytes = std::max(std::max(b1, b2), b3) + 256;
     if ((st = dalloc(c, (char**)&c->cub_tmp, c->cub_tmp_bytes)) != SGIPC_OK) return fail(st);
     SG_CHECK(c, cudaMemset(c->nuc, 0, 4 * sizeof(int)));
@@ -381,10 +386,11 @@ extern "C" SgipcStatus sgipc_destroy(SgipcCtx* c) {
     mas_destroy(c);
     void* ptrs[] = {c->row_ptr, c->col, c->slot_row, c->diag_slot, c->low_ptr, c->low_slot, c->val64,
                     c->eblk, c->contrib_ptr, c->contrib, c->egrad, c->vinc_ptr, c->vinc, c->tets, c->tris,
-                    c->hinges, c->hinge_adj, c->soft_idx, c->shape_grads, c->fb, c->b, c->ckey, c->ckey_s,
-                    c->cidx, c->cidx_s, c->cval, c->cflag, c->nuc, c->uc_row, c->uc_col, c->uc64, c->uc32,
-                    c->cu_ptr, c->cl_ptr, c->cl_idx, c->lcount, c->lpos, c->cub_tmp, c->dflag,
-                    c->frow_ptr, c->fcol, c->fup, c->flo, c->fval64, c->fval32, c->cl_col, c->cl64, c->cl32, c->run_start, c->en_part, c->en_terms, c->ccd_part, c->ccd_out, c->ccd_bad, c->en_ticket, c->ccd_ticket,
+                    c->hinges, c->hinge_adj, c->soft_idx, c->shape_grads, c->fb, c->b, c->con_ids,
+                    c->con_fac, c->con_fac2, c->con_sid, c->con_sval, c->con_key, c->con_val, c->con_key_s,
+                    c->con_val_s, c->inc_ptr, c->row_list, c->row_cnt, c->ucnt, c->uoff, c->part_a, c->part_f, c->nuc, c->uc_row, c->uc_col, c->uc64, c->uc32,
+                    c->cu_ptr, c->cl_ptr, c->cub_tmp, c->dflag,
+                    c->frow_ptr, c->fcol, c->fup, c->flo, c->fval64, c->fval32, c->cl_col, c->cl64, c->cl32, c->en_part, c->en_terms, c->ccd_part, c->ccd_out, c->ccd_bad, c->en_ticket, c->ccd_ticket,
                     c->cs.ptr, c->cs.cols, c->cs.lcol, c->cs.dslot, c->cs_small.ptr, c->cs_small.cols, c->cs_small.lcol,
                     c->cs_small.dslot, c->close_gid, c->close_gval, c->close_pid,
                     c->close_pval, c->close_cnt};

@@ -172,13 +172,22 @@ struct SgipcCtx {
 
     // ---- dynamic contact blocks -------------------------------------------------------
     int cap_cblk;
-    unsigned long long* ckey;     // [cap]
-    unsigned long long* ckey_s;   // sorted
-    int* cidx;                    // [cap]
-    int* cidx_s;
-    double* cval;                 // [cap*9]
-    int* run_start;               // [cap+1] first sorted index of each unique block's run
-    int* cflag;                   // [cap+1] segment heads -> unique ids
+    int4* con_ids;                // [pairs] factors of the contact terms (ContactStore, sgipc_assemble.cu)
+    double* con_fac;              // [16 * pairs]
+    double* con_fac2;             // [16 * max_pairs] second line of the mollified pairs
+    int* con_sid;                 // [singles] ground contacts, ground friction, soft constraints
+    double* con_sval;             // [9 * singles]
+    uint32_t* con_key;            // [4 * pairs + singles] vertex of each incidence, and the incidence
+    uint32_t* con_val;
+    uint32_t* con_key_s;          // sorted by vertex
+    uint32_t* con_val_s;
+    int* inc_ptr;                 // [n+1] incidences of each vertex
+    int* row_list;                // [2n] vertices with short lists, and with long ones
+    int* row_cnt;                 // [2] their numbers
+    unsigned long long* ucnt;     // [n+1] unique blocks per row: upper ones, transposed ones << 32
+    unsigned long long* uoff;     // their exclusive scan
+    int* part_a;                  // [cap+1] flags and places of the class partition
+    int* part_f;
     int* nuc;                     // device: number of unique contact blocks
     int* uc_row;                  // [cap]
     int* uc_col;
@@ -186,12 +195,9 @@ struct SgipcCtx {
     float* uc32;
     int* cu_ptr;                  // [n+1] unique contact blocks by row (upper)
     int* cl_ptr;                  // [n+1] transposed entries by row
-    int* cl_idx;                  // [cap] unique block of each transposed slot, in placement order
     int* cl_col;                  // [cap] column of each transposed entry (= uc_row of its block)
     double* cl64;                 // [cap*9] transposed copy of the block (SpMV reads it directly)
     float* cl32;
-    int* lcount;                  // [2n+1] transposed entries per row [0, n], then fill cursors [n+1, 2n]
-    int* lpos;                    // [cap] transposed slot of each unique block (-1: diagonal)
     void* cub_tmp;
     size_t cub_tmp_bytes;
     int key_bits;

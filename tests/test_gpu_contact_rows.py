@@ -1,0 +1,78 @@
+"""Rows of the contact matrix against the oracle's assembly, at the sizes where the row kernels
+change: a warp or a CTA per row (128 incidences), windows of 80 columns, batches of 8 pairs a
+half-warp, every pair kind (mollified ones included) and
+rows of fixed vertices.
+
+The pairs are synthetic (random vertices of two small cubes, d-hat wider than the scene), so a row
+can be given any length.  Tolerance: the same products in 64 bits, summed in another order; a row
+of m terms differs by at most about m eps of its largest term, 1e-12 for the longest here, and
+the pair geometry's own rounding grows with the pair's conditioning: 1e-9 of the largest block, the
+bound of the other assembly tests.
+"""
+import dataclasses
+
+import numpy as np
+import pytest
+
+import oracle
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+if not torch.cuda.is_available():  # pragma: no cover - CPU container
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+from sgipc import scenes, system  # noqa: E402
+
+
+def _pairs(rng, nv, hub, columns, repeats, mollified):
+    """Pairs that give vertex `hub` about `columns` other columns and `repeats` more incidences,
+    and a background of random pairs of every kind."""
+    other = np.setdiff1d(rng.permutation(nv), [hub])
+    out = [(-hub - 1, w, -1, -1) for w in other[:columns]]
+    near = other[:max(3, min(columns, 12))]
+    for _ in range(repeats):
+        a, b, c = rng.choice(near, 3, replace=False)
+        out.append([(-hub - 1, a, -1, -1), (-hub - 1, a, b, -1), (-hub - 1, a, b, c), (hub, a, b, c)][rng.integers(4)])
+    for _ in range(60):
+        a, b, c, d = rng.choice(nv, 4, replace=False)
+        kinds = [(-a - 1, b, -1, -1), (-a - 1, b, c, -1), (-a - 1, b, c, d), (a, b, c, d)]
+        if mollified:
+            kinds += [(a, b, c, -d - 1), (-a - 1, -b - 1, c, -d - 1), (-a - 1, -b - 1, -c - 1, -d - 1)]
+        out.append(kinds[rng.integers(len(kinds))])
+    return np.asarray(out, np.int32)[rng.permutation(len(out))]
+
+
+@pytest.mark.parametrize("columns,repeats,mollified", [(1, 0, False), (7, 1, True), (15, 112, False), (15, 113, True),
+                                                       (15, 114, False), (79, 0, False), (80, 40, True),
+                                                       (81, 60, False), (161, 0, True), (330, 1000, True)])
+def test_rows_match_the_oracle(columns, repeats, mollified):
+    rng = np.random.default_rng(columns + repeats)
+    sc = scenes.scene_two_cubes(6, seed=4)
+    hub = int(rng.integers(sc.nv))
+    pairs = _pairs(rng, sc.nv, hub, columns, repeats, mollified)
+    fp = pairs[rng.permutation(len(pairs))[:len(pairs) // 2 + 1]]
+    lam = rng.uniform(0.5, 2.0, len(fp))
+    coord = rng.uniform(0.1, 0.4, (len(fp), 2))
+    basis = np.linalg.qr(rng.normal(size=(len(fp), 3, 2)))[0]
+    btype = sc.boundary_type.copy()
+    btype[rng.choice(sc.nv, 20, replace=False)] = 1
+    sc = dataclasses.replace(sc, pairs=pairs, fric_pairs=fp, fric_lambda=lam, fric_coord=coord, fric_basis=basis,
+                             boundary_type=btype, params=dict(sc.params, dHat=0.2, kappa=1.0),
+                             o_vertexes=sc.vertexes + rng.uniform(-1e-3, 1e-3, sc.vertexes.shape))
+    g = system.GIPC(sc)
+    g.computeGradientAndHessian()
+    rows, cols, vals = g.export_bcoo()
+    b, orow, ocol, oval, _ = oracle.assemble(sc)
+    assert np.array_equal(rows, orow) and np.array_equal(cols, ocol)
+    assert np.abs(vals - oval).max() <= 1e-9 * np.abs(oval).max()
+    assert np.abs(g.rhs().cpu().numpy() - b).max() <= 1e-9 * np.abs(b).max()
+    # the transposed lists: A times a vector against the upper blocks and their transposes
+    x = rng.normal(size=3 * sc.nv)
+    y = g.spmv(torch.tensor(x, device="cuda")).cpu().numpy()
+    ref = oracle.spmv(orow, ocol, oval, sc.nv, x)
+    assert np.abs(y - ref).max() <= 1e-9 * np.abs(ref).max()
+    # the same sums on every run
+    g.computeGradientAndHessian()
+    assert np.array_equal(g.export_bcoo()[2], vals)
+    g.close()
