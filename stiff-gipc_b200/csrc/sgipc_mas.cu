@@ -15,6 +15,8 @@
 // The B200 version keeps every level's bookkeeping on the device (no per-level host
 // copy), builds the per-level masks with one thread per vertex / per contact pair and
 // resolves a bank's components with one thread per bank.
+#include <algorithm>
+
 #include <cub/cub.cuh>
 #include <mutex>
 #include <vector>
@@ -41,66 +43,64 @@ __global__ void k_init_level0(int nv, const int* __restrict__ real_map, int L, i
     table[(size_t)v * L] = p;
 }
 
-// OR `bit` into mask[a]; lanes of a warp with the same target combine their bits first
-// (at coarse levels most edges of a warp land on the same few nodes)
-__device__ __forceinline__ void mask_or_warp(uint32_t* mask, int a, uint32_t bit) {
-    const unsigned grp = __match_any_sync(0xffffffffu, a);
-    const uint32_t bits = __reduce_or_sync(grp, bit);
-    if (a >= 0 && bits && (int)(threadIdx.x & 31) == __ffs(grp) - 1) atomicOr(mask + a, bits);
+// OR bits into mask[a] unless they are there: most connections are met many times (a contact
+// by each of its pairs, a coarse edge by each fine one), and a stale read only costs an atomic
+__device__ __forceinline__ void mask_or(uint32_t* mask, int a, uint32_t bits) {
+    if (bits & ~__ldcg(mask + a)) atomicOr(mask + a, bits);
+}
+
+// the mesh edge between nodes a and b
+__device__ __forceinline__ void mask_edge(uint32_t* mask, int a, int b) {
+    if (a != b && (a >> 4) == (b >> 4)) mask_or(mask, a, 1u << (b & 15));
 }
 
 // one thread per neighbour-list slot (row[k] is the slot's vertex)
 __global__ void k_mask_edges(int nnz, const int* __restrict__ row, const int* __restrict__ nbr,
                              const int* __restrict__ node, uint32_t* __restrict__ mask) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    int a = -1;
-    uint32_t bit = 0;
-    if (k < nnz) {
-        a = node[row[k]];
-        const int b = node[nbr[k]];
-        if (a != b && (a >> 4) == (b >> 4)) bit = 1u << (b & 15);
-    }
-    mask_or_warp(mask, bit ? a : -1, bit);
+    if (k < nnz) mask_edge(mask, node[row[k]], node[nbr[k]]);
 }
 
-// The connectivity bits of one contact pair (its decoded vertices, all ordered pairs inside
-// one bank); every lane of the warp calls it (idle lanes: e = nullptr).
-__device__ __forceinline__ void mask_pair_warp(const int4* e_ptr, int nv, const int* __restrict__ node,
-                                               uint32_t* __restrict__ mask) {
-    int v[4] = {-1, -1, -1, -1}, n = 0;
-    if (e_ptr) {
-        const int4 e = *e_ptr;
-        if (e.x >= 0) {
-            v[0] = e.x; v[1] = e.y; v[2] = e.z; v[3] = e.w < 0 ? -e.w - 1 : e.w; n = 4;
-        } else {
-            v[0] = -e.x - 1;
-            if (e.z < 0) {
-                if (e.y < 0) { v[1] = -e.y - 1; v[2] = -e.z - 1; v[3] = -e.w - 1; n = 4; }
-                else { v[1] = e.y; n = 2; }
-            } else if (e.w < 0) {
-                if (e.y < 0) { v[1] = -e.y - 1; v[2] = e.z; v[3] = -e.w - 1; n = 4; }
-                else { v[1] = e.y; v[2] = e.z; n = 3; }
-            } else { v[1] = e.y; v[2] = e.z; v[3] = e.w; n = 4; }
+// the nodes of a contact pair's vertices (-1: fewer than four, or no vertex of the mesh)
+__device__ __forceinline__ void pair_nodes(int4 e, int nv, const int* __restrict__ node, int (&a)[4]) {
+    int v[4] = {e.x, e.y, e.z, e.w};
+    if (e.x >= 0) {
+        if (e.w < 0) v[3] = -e.w - 1;
+    } else {
+        v[0] = -e.x - 1;
+        if (e.y < 0 && (e.z < 0 || e.w < 0)) {  // mollified point-point or point-edge
+            v[1] = -e.y - 1;
+            v[2] = e.z < 0 ? -e.z - 1 : e.z;
+            v[3] = e.w < 0 ? -e.w - 1 : e.w;
+        } else if (e.z < 0) {
+            v[2] = v[3] = -1;
+        } else if (e.w < 0) {
+            v[3] = -1;
         }
     }
-    int a[4] = {-1, -1, -1, -1};
-    for (int i = 0; i < n; i++) a[i] = (v[i] >= 0 && v[i] < nv) ? node[v[i]] : -1;
-    // the 12 ordered vertex pairs, each one warp-aggregated OR
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < 4; i++) a[i] = v[i] >= 0 && v[i] < nv ? node[v[i]] : -1;
+}
+
+// the connections of a contact pair: every two of its nodes inside one bank
+__device__ __forceinline__ void mask_pair(uint32_t* mask, const int (&a)[4]) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            if (i == j) continue;
-            const int x = a[i], y = a[j];
-            const bool on = x >= 0 && y >= 0 && x != y && (x >> 4) == (y >> 4);
-            mask_or_warp(mask, on ? x : -1, on ? 1u << (y & 15) : 0u);
-        }
+    for (int i = 0; i < 4; i++) {
+        uint32_t bits = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (i != j && a[j] >= 0 && a[i] != a[j] && (a[i] >> 4) == (a[j] >> 4)) bits |= 1u << (a[j] & 15);
+        if (a[i] >= 0 && bits) mask_or(mask, a[i], bits);
+    }
 }
 
 __global__ void k_mask_pairs(int np, const int4* __restrict__ pairs, int nv, const int* __restrict__ node,
                              uint32_t* __restrict__ mask) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    mask_pair_warp(p < np ? pairs + p : nullptr, nv, node, mask);
+    if (p >= np) return;
+    int a[4];
+    pair_nodes(pairs[p], nv, node, a);
+    mask_pair(mask, a);
 }
 
 // Half a warp per bank (bk; all 32 lanes call it), writing its nodes' component ranks and
@@ -323,15 +323,18 @@ __global__ void k_scatter_contact(int cap, const int* __restrict__ nuc, const in
     __shared__ double s_top[kTopLevels][2304];
     __shared__ int s_hot[kTopLevels];
     const int l_top = top_levels(L);
-    int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (blockIdx.x * blockDim.x >= nuc[0]) return;  // whole block beyond the unique blocks
-    zero_top(table, L, ur[blockIdx.x * blockDim.x], l_top, s_hot, s_top);
-    bool valid = u < cap && u < nuc[0];
-    double B[9];
+    const int n = min(cap, nuc[0]);
+    for (int u0 = blockIdx.x * blockDim.x; u0 < n; u0 += gridDim.x * blockDim.x) {  // CTA-uniform
+        const int u = u0 + threadIdx.x;
+        zero_top(table, L, ur[u0], l_top, s_hot, s_top);
+        const bool valid = u < n;
+        double B[9];
 #pragma unroll
-    for (int q = 0; q < 9; q++) B[q] = valid ? val[9 * (size_t)u + q] : 0.0;
-    scatter_block_warp(dom, table, L, valid ? ur[u] : 0, valid ? uc[u] : 0, B, valid, 0, l_top, s_hot, s_top);
-    flush_top(L - l_top, s_hot, s_top, dom);
+        for (int q = 0; q < 9; q++) B[q] = valid ? val[9 * (size_t)u + q] : 0.0;
+        scatter_block_warp(dom, table, L, valid ? ur[u] : 0, valid ? uc[u] : 0, B, valid, 0, l_top, s_hot, s_top);
+        flush_top(L - l_top, s_hot, s_top, dom);
+        __syncthreads();  // the copies are zeroed for the next blocks
+    }
 }
 
 // Gauss-Jordan inversion without pivoting, in place, one 48x48 domain per 64-thread CTA.
@@ -577,6 +580,9 @@ constexpr int kHierMaxCtas = 296;      // the largest grid the build may take (h
 // the MAS build ends at 0.41 ms with 32 CTAs, 0.36 ms with 74 and 0.41 ms with 148 (the
 // assembly's kernels then lose their SMs)
 constexpr int kHierDefaultCtas = 74;
+// ... and with this many pairs or more: a chip's worth of threads for the pairs' gathers, which
+// then take longer than the assembly beside them (one 256^2 rolled cloth: a million pairs)
+constexpr int kHierManyPairs = 200000;
 constexpr long long kHierSpinLimit = 1LL << 24;
 
 struct HierArgs {
@@ -664,20 +670,35 @@ __global__ void __launch_bounds__(kHierThreads) k_hierarchy(HierArgs h) {
         const int count = info[8 + l], start = info[l];
         const int nbank = (count + 15) >> 4;
         // (the masks of this level were zeroed by the previous phase)
-        // edge masks (one lane per neighbour slot) and contact-pair masks, warp-aggregated
-        for (int k0 = gw * 32; k0 < h.nnbr; k0 += nw * 32) {
-            const int k = k0 + lane;
-            int a = -1;
-            uint32_t bit = 0;
-            if (k < h.nnbr) {
-                a = h.node[h.nbr_row[k]];
-                const int b = h.node[h.nbr[k]];
-                if (a != b && (a >> 4) == (b >> 4)) bit = 1u << (b & 15);
+        // edge masks (one thread per neighbour slot) and contact-pair masks, the gathers of four
+        // slots, or two pairs, in flight together
+        for (int k0 = tid; k0 < h.nnbr; k0 += 4 * nth) {
+            int r[4], c[4], a[4], b[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int k = k0 + u * nth;
+                r[u] = k < h.nnbr ? __ldg(h.nbr_row + k) : -1;
+                c[u] = k < h.nnbr ? __ldg(h.nbr + k) : -1;
             }
-            mask_or_warp(h.mask, bit ? a : -1, bit);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                a[u] = r[u] >= 0 ? h.node[r[u]] : 0;
+                b[u] = r[u] >= 0 ? h.node[c[u]] : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) mask_edge(h.mask, a[u], b[u]);
         }
-        for (int p0 = gw * 32; p0 < h.npairs; p0 += nw * 32)
-            mask_pair_warp(p0 + lane < h.npairs ? h.pairs + p0 + lane : nullptr, h.nv, h.node, h.mask);
+        for (int p0 = tid; p0 < h.npairs; p0 += 2 * nth) {
+            int a[2][4];
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int p = p0 + u * nth;
+                if (p < h.npairs) pair_nodes(__ldg(h.pairs + p), h.nv, h.node, a[u]);
+                else a[u][0] = a[u][1] = a[u][2] = a[u][3] = -1;
+            }
+#pragma unroll
+            for (int u = 0; u < 2; u++) mask_pair(h.mask, a[u]);
+        }
         if (!hier_barrier(info, epoch, h.spin_limit)) return;
         // components, half a warp per bank; bank nbank gets a zero count (the scan's total)
         for (int b0 = gw * 2; b0 <= nbank; b0 += nw * 2)
@@ -860,6 +881,7 @@ SgipcStatus mas_create(SgipcCtx* c, const SgipcTopology* t) {
         const char* e = getenv("SGIPC_HIER_CTAS");
         if (e && atoi(e) > 0) want = atoi(e) < kHierMaxCtas ? atoi(e) : kHierMaxCtas;
         m.hier_grid = coop && per > 0 ? (nsm * per < want ? nsm * per : want) : 0;
+        m.hier_grid_many = e ? m.hier_grid : (nsm * per < kHierMaxCtas ? nsm * per : kHierMaxCtas);
     }
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, m.bank_cnt, m.bank_off, m.npos / 16 + 2);
@@ -920,8 +942,8 @@ static SgipcStatus mas_hierarchy(SgipcCtx* c, const SgipcContacts* con, cudaStre
         SG_CHECK(c, cudaMemsetAsync(m.info + 20, 0, 2 * sizeof(int), s));
         void* args[] = {&h};
         SG_COUNT(c, 1);
-        SG_CHECK(c, cudaLaunchCooperativeKernel((const void*)k_hierarchy, dim3(m.hier_grid), dim3(kHierThreads), args,
-                                                0, s));
+        const int grid = h.npairs >= kHierManyPairs ? m.hier_grid_many : m.hier_grid;
+        SG_CHECK(c, cudaLaunchCooperativeKernel((const void*)k_hierarchy, dim3(grid), dim3(kHierThreads), args, 0, s));
         SG_CHECK(c, cudaMemcpyAsync(m.h_info_pinned, m.info, sizeof(int) * 22, cudaMemcpyDeviceToHost, s));
         return SGIPC_OK;
     }
@@ -1040,7 +1062,9 @@ SgipcStatus mas_build(SgipcCtx* c, const SgipcContacts* con, SgipcPrecision prec
                                                               m.info, m.dom64);
     }
     SG_COUNT(c, 2);
-    k_scatter_contact<<<nblk(c->cap_cblk), SGIPC_BLOCK, 0, s>>>(c->cap_cblk, c->nuc, c->uc_row, c->uc_col, c->uc64,
+    // (the number of unique blocks is on the device: a CTA per 256 blocks up to some waves of the
+    // chip, a loop beyond; the capacity alone is 156 000 CTAs for two million pairs)
+    k_scatter_contact<<<std::min(nblk(c->cap_cblk), 148 * 32), SGIPC_BLOCK, 0, s>>>(c->cap_cblk, c->nuc, c->uc_row, c->uc_col, c->uc64,
                                                                m.table, L, m.info, m.dom64);
     const int w64 = prec == SGIPC_FP64 ? 1 : 0, w32 = prec == SGIPC_FP64 ? 0 : 1;
     k_invert<<<ndom, 64, 0, s>>>(ndom, m.dom64, m.dom32, w64, w32);
