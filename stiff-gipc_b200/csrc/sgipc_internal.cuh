@@ -265,6 +265,7 @@ struct SgipcCtx {
     unsigned int* dot_ticket;
     double* dot_out;          // [16]
     double* h_pinned;         // host pinned scalars
+    sgipc::PcgScalars* h_scalars;  // [4] pinned landing area of a solve's scalars
     cudaStream_t cap_stream;  // capture stream
     // assembly: the contact kernels and their merge run on asm_stream beside the element
     // kernels on the caller's stream (joined before the right-hand side)

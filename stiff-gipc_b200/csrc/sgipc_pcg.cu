@@ -658,6 +658,7 @@ SgipcStatus pcg_create(SgipcCtx* c) {
     SG_CHECK(c, cudaMemset(c->dot_ticket, 0, sizeof(unsigned int) * 4));
     SG_CHECK(c, cudaMalloc((void**)&c->dot_out, sizeof(double) * 16));
     SG_CHECK(c, cudaMallocHost((void**)&c->h_pinned, sizeof(double) * 64));
+    SG_CHECK(c, cudaMallocHost((void**)&c->h_scalars, sizeof(PcgScalars) * 4));
     SG_CHECK(c, cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
     // the contact merge is a chain of small dependent kernels on the assembly's critical path:
     // its stream gets the highest priority, so that its blocks go ahead of the element and MAS
@@ -676,6 +677,7 @@ void pcg_destroy(SgipcCtx* c) {
     for (void* p : ps)
         if (p) cudaFree(p);
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
+    if (c->h_scalars) cudaFreeHost(c->h_scalars);
     if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
     if (c->asm_stream) {
         cudaStreamSynchronize(c->asm_stream);
@@ -716,23 +718,52 @@ extern "C" SgipcStatus sgipc_spmv(SgipcCtx* c, const double* x, double* y, void*
     return spmv_t<double>(c, x, y, (cudaStream_t)stream);
 }
 
-// true relative residual ||b - A x|| / ||b|| (FP64)
-static SgipcStatus true_residual(SgipcCtx* c, const double* b, const double* x, double* out, cudaStream_t s) {
-    const int n3 = 3 * c->n;
-    SgipcStatus st = spmv_t<double>(c, x, c->tmp64b, s);
-    if (st != SGIPC_OK) return st;
+// ||b - A x||^2 of right-hand sides blockIdx.y = 0 .. (b, x rhs-major) in one launch: rows by groups
+// of kSpG lanes, per-CTA partials, the last CTA of a right-hand side adds them in order
+constexpr int kResidualCtas = 256;  // per right-hand side: dot_partial holds four times as many
+__global__ void __launch_bounds__(256) k_true_residual(Topo tp, MatView<double> A, const double* __restrict__ b,
+                                                       const double* __restrict__ x, double* __restrict__ partial,
+                                                       unsigned int* __restrict__ ticket, double* __restrict__ out) {
+    __shared__ double smem[32];
+    const size_t first = 3 * (size_t)tp.n * blockIdx.y;
+    Operand<double, 1> op;
+    op.a = x + first;
+    op.b = nullptr;
+    op.beta[0] = 0;
+    constexpr int rows = 256 / kSpG;
+    double v[1] = {0.0};
+    for (int i0 = blockIdx.x * rows; i0 < tp.n; i0 += gridDim.x * rows) {  // CTA-uniform
+        const int i = i0 + (int)threadIdx.x / kSpG, g = threadIdx.x % kSpG;
+        double acc[1][3];
+        row_mv<double, 1>(tp, A, op, i, g, acc);
+        if (i < tp.n && g == 0)
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const double r = b[first + 3 * (size_t)i + q] - acc[0][q];
+                v[0] += r * r;
+            }
+    }
+    double tot[1];
+    if (grid_sum<1>(v, partial + blockIdx.y * kResidualCtas, ticket + blockIdx.y, tot, smem) && threadIdx.x == 0)
+        out[blockIdx.y] = tot[0];
+}
+
+// enqueue ||b - A x||^2 of nrhs <= 4 right-hand sides, on their way to h_pinned[0 ..]
+static SgipcStatus enqueue_residuals(SgipcCtx* c, const double* b, const double* x, int nrhs, cudaStream_t s) {
     SG_COUNT(c, 1);
-    k_axpby_res<<<nblk(n3), 256, 0, s>>>(n3, b, c->tmp64b, c->tmp64b);
-    if ((st = dot64(c, c->tmp64b, c->tmp64b, n3, c->dot_out, s)) != SGIPC_OK) return st;
-    if ((st = dot64(c, b, b, n3, c->dot_out + 1, s)) != SGIPC_OK) return st;
-    SG_CHECK(c, cudaMemcpyAsync(c->h_pinned, c->dot_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
-    SG_CHECK(c, cudaStreamSynchronize(s));
-    *out = c->h_pinned[1] > 0 ? sqrt(c->h_pinned[0] / c->h_pinned[1]) : 0.0;
+    const int grid = spmv_grid(c->n) < kResidualCtas ? spmv_grid(c->n) : kResidualCtas;
+    k_true_residual<<<dim3(grid, nrhs), 256, 0, s>>>(topo_of(c), mat_view<double>(c), b, x, c->dot_partial,
+                                                     c->dot_ticket, c->dot_out);
+    SG_LAUNCH_CHECK(c, "true residual");
+    SG_CHECK(c, cudaMemcpyAsync(c->h_pinned, c->dot_out, nrhs * sizeof(double), cudaMemcpyDeviceToHost, s));
     return SGIPC_OK;
 }
 
 // pinned host word for the device input-error flag, read with a solve's final copies
 static int* input_flag(SgipcCtx* c) { return reinterpret_cast<int*>(c->h_pinned + 32); }
+
+// pinned landing area of a solve's scalars (four right-hand sides at most)
+static PcgScalars* pinned_scalars(SgipcCtx* c) { return c->h_scalars; }
 
 static SgipcStatus input_error(SgipcCtx* c, cudaStream_t s) {
     *input_flag(c) = 0;
@@ -756,8 +787,10 @@ static SgipcStatus solve_one(SgipcCtx* c, SgipcPrecision prec, SgipcCriterion cr
             st = run_pcg<double, double, 1>(c, c->pcg64, 0, b, tol, max_iter, (int)crit, s, 10);
         if (st != SGIPC_OK) return st;
         SG_CHECK(c, cudaMemcpyAsync(x, c->pcg64.x, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s));
-        PcgScalars hs;
+        // the solve's scalars, its input flag and the true residual come back together
+        PcgScalars& hs = *pinned_scalars(c);
         SG_CHECK(c, cudaMemcpyAsync(&hs, c->pcg64.sc, sizeof(hs), cudaMemcpyDeviceToHost, s));
+        if ((st = enqueue_residuals(c, b, x, 1, s)) != SGIPC_OK) return st;
         // the persistent solve copies the bad-input flag into its scalars: one read-back
         if (!c->pcg64.last_coop)
             SG_CHECK(c, cudaMemcpyAsync(input_flag(c), c->dflag, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -769,6 +802,7 @@ static SgipcStatus solve_one(SgipcCtx* c, SgipcPrecision prec, SgipcCriterion cr
         out.refinements = 0;
         out.rz0 = hs.rz0;
         out.rz = hs.rz_next;
+        out.rel_residual = hs.bnorm2 > 0.0 ? sqrt(c->h_pinned[0] / hs.bnorm2) : 0.0;
         out.status = final_status(c, hs);
     } else {
         // mixed: FP32 MAS-PCG inner solves on the FP32 matrix copy, FP64 residual refinement
@@ -792,7 +826,7 @@ static SgipcStatus solve_one(SgipcCtx* c, SgipcPrecision prec, SgipcCriterion cr
             st = run_pcg<float, float, 1>(c, c->pcg32, 1, ref == 0 ? b : r64, inner_tol, max_iter, (int)crit, s, 20,
                                           &rf);
             if (st != SGIPC_OK) return st;
-            PcgScalars hs;
+            PcgScalars& hs = *pinned_scalars(c);
             if (!rf.done) {
                 SG_COUNT(c, 2);
                 k_add_f32<<<nblk(n3), 256, 0, s>>>(n3, (const float*)c->pcg32.x, x, ref == 0 ? 1 : 0);
@@ -842,7 +876,6 @@ static SgipcStatus solve_one(SgipcCtx* c, SgipcPrecision prec, SgipcCriterion cr
         // ||b||^2 is the first inner solve's right-hand side norm
         out.rel_residual = bn2 > 0.0 ? sqrt(c->h_pinned[1] / bn2) : 0.0;
     }
-    if (prec != SGIPC_MIXED && (st = true_residual(c, b, x, &out.rel_residual, s)) != SGIPC_OK) return st;
     if (stats) *stats = out;
     return (SgipcStatus)out.status;
 }
@@ -911,8 +944,9 @@ extern "C" SgipcStatus sgipc_pcg_solve_batched(SgipcCtx* c, SgipcPrecision prec,
         k_interleave<float, double><<<nblk(4LL * n3), 256, 0, s>>>(n3, 4, (const float*)w.x, x, 0);
     else
         k_interleave<double, double><<<nblk(4LL * n3), 256, 0, s>>>(n3, 4, (const double*)w.x, x, 0);
-    PcgScalars hs[4];
-    SG_CHECK(c, cudaMemcpyAsync(hs, w.sc, sizeof(hs), cudaMemcpyDeviceToHost, s));
+    PcgScalars* hs = pinned_scalars(c);
+    SG_CHECK(c, cudaMemcpyAsync(hs, w.sc, 4 * sizeof(PcgScalars), cudaMemcpyDeviceToHost, s));
+    if (stats && (st = enqueue_residuals(c, b, x, 4, s)) != SGIPC_OK) return st;
     SG_CHECK(c, cudaStreamSynchronize(s));
     SgipcStatus worst = SGIPC_OK;
     SG_COUNT(c, 4LL * hs[0].bodies);
@@ -924,9 +958,7 @@ extern "C" SgipcStatus sgipc_pcg_solve_batched(SgipcCtx* c, SgipcPrecision prec,
             stats[r].rz0 = hs[r].rz0;
             stats[r].rz = hs[r].rz_next;
             stats[r].status = fs;
-            double rel = 0;
-            if ((st = true_residual(c, b + (size_t)r * n3, x + (size_t)r * n3, &rel, s)) != SGIPC_OK) return st;
-            stats[r].rel_residual = rel;
+            stats[r].rel_residual = hs[r].bnorm2 > 0.0 ? sqrt(c->h_pinned[r] / hs[r].bnorm2) : 0.0;
         }
         if (fs != SGIPC_OK) worst = (SgipcStatus)fs;
     }
