@@ -872,14 +872,16 @@ __global__ void k_soft(int ns, const uint32_t* __restrict__ idx, const double* _
 // of the contact matrix is made from v's list alone: every pair in it gives the blocks (v, w) of
 // its vertices w.  One warp takes a row of up to kRowLong incidences, a CTA a longer one.  The
 // distinct columns go into a small hash table in shared memory and are ranked; the blocks are
-// added up in shared memory, pair by pair in the list's order (half-warps take consecutive parts
-// of the list and their sums are added in order): the same result on every run.  A row of more columns than the
+// added up in shared memory, pair by pair in the list's order (each half-warp its share, the
+// shares' sums in order): the same result on every run.  A row of more columns than the
 // table holds is made in windows of columns.
 constexpr int kRowWarps = 4;
-constexpr int kRowLong = 128;  // incidences above which a CTA takes the row
+// incidences above which a CTA takes the row (rolled cloth, a third of whose rows are longer: the
+// Newton system takes 8 % longer with 64, 5 % with 413, where k_row_counts goes from 159 to 352 us)
+constexpr int kRowLong = 128;
 constexpr int kRowHash = 256;
-constexpr int kRowCols = 80;   // columns of a window (each of 32 * kRowWarps lanes may add one more)
-constexpr int kRowBatch = 16;  // pairs staged at a time
+constexpr int kRowCols = 40;   // columns of a window (each of 32 * kRowWarps lanes may add one more)
+constexpr int kRowCtas = 4;    // CTAs of k_row_sums per SM (128 registers, 55 KB)
 static_assert(kRowCols + 32 * kRowWarps < kRowHash, "the hash table never fills up");
 
 // row pointers of the sorted incidences, the lists of rows to make, zeroed block counts
@@ -952,6 +954,7 @@ struct RowTable {
     int hash[kRowHash];             // column, -1: free
     unsigned char rank[kRowHash];   // its place among the window's sorted columns
     unsigned short slot[kRowCols + 32 * kRowWarps];  // table slots in use, in order of arrival
+    int found[kRowCols + 32 * kRowWarps];            // and their columns
     int col[kRowCols];              // sorted columns
     int used, over;
 };
@@ -969,12 +972,21 @@ __device__ __forceinline__ bool row_columns(const RowArgs& a, RowTable& T, int i
     for (int k = t; k < kRowHash; k += nt) T.hash[k] = -1;
     if (t == 0) T.used = T.over = 0;
     row_sync<kCta>();
-    for (int i = i0 + t; i < i1; i += nt) {
-        int v[4], item, local;
-        inc_pair(a, __ldg(a.inc + i), v, item, local);
+    constexpr int kU = 4;  // pairs in flight
+    for (int k0 = i0 + t; k0 < i1; k0 += kU * nt) {
+        uint32_t inc[kU];
+        int v[kU][4];
 #pragma unroll
-        for (int b = 0; b < 4; b++) {
-            const int c = v[b];
+        for (int u = 0; u < kU; u++) inc[u] = k0 + u * nt < i1 ? __ldg(a.inc + k0 + u * nt) : ~0u;
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            int item, local;
+            if (inc[u] != ~0u) inc_pair(a, inc[u], v[u], item, local);
+            else v[u][0] = v[u][1] = v[u][2] = v[u][3] = -1;
+        }
+#pragma unroll
+        for (int e = 0; e < 4 * kU; e++) {
+            const int c = v[e / 4][e % 4];
             if (c < lo || c >= hi) continue;  // (-1 is below every window)
             unsigned h = ((unsigned)c * 2654435761u) >> 24;
             for (;;) {
@@ -988,7 +1000,9 @@ __device__ __forceinline__ bool row_columns(const RowArgs& a, RowTable& T, int i
                     const int old = atomicCAS(&T.hash[h], -1, c);
                     if (old == c) break;
                     if (old < 0) {
-                        T.slot[atomicAdd(&T.used, 1)] = (unsigned short)h;
+                        const int k = atomicAdd(&T.used, 1);
+                        T.slot[k] = (unsigned short)h;
+                        T.found[k] = c;
                         break;
                     }
                 }
@@ -1007,10 +1021,11 @@ template <bool kCta>
 __device__ __forceinline__ void row_ranks(RowTable& T, int t, int nt) {
     const int U = T.used;
     for (int k = t; k < U; k += nt) {
-        const int h = T.slot[k], c = T.hash[h];
+        const int c = T.found[k];
         int r = 0;
-        for (int j = 0; j < U; j++) r += T.hash[T.slot[j]] < c;
-        T.rank[h] = (unsigned char)r;
+#pragma unroll 4
+        for (int j = 0; j < U; j++) r += T.found[j] < c;
+        T.rank[T.slot[k]] = (unsigned char)r;
         T.col[r] = c;
     }
     row_sync<kCta>();
@@ -1051,7 +1066,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_row_counts(RowArgs a, unsign
         unsigned up = 0, low = 0;  // of this thread's share of the columns
         row_windows<decltype(cta)::value>(a, T, a.ptr[v], a.ptr[v + 1], t, nt, [&]() {
             for (int k = t; k < T.used; k += nt) {
-                if (T.hash[T.slot[k]] >= v) up++;
+                if (T.found[k] >= v) up++;
                 else low++;
             }
         });
@@ -1080,122 +1095,169 @@ struct RowOut {
     double* grad;
 };
 
-// A half-warp adds up its part of a row's list: lanes 0..11 take column q of the block of vertex b
-// (three entries each), lanes 12..14 the gradient's component q.  (With one lane per entry a pair
-// took 36 lanes, twice the instructions of a warp for each: 1557 us for the rolled cloth's eight
-// million incidences.)
+// A half-warp adds up its share of a row's list (every second pair of a warp's, every eighth of a
+// CTA's): a lane stages one pair, scaled for this row, and then lanes 0..11 take column q of the
+// block of vertex b (three entries each) and lanes 12..14 the gradient's component q, four
+// shared-memory reads and three products for a pair whatever its kind; the next pairs' lines are
+// on their way meanwhile.  1062 us for the rolled cloth's eight million incidences, 46 warp
+// instructions each; the shared-memory pipe is busy 59 % of it, mostly with the sums.  (One lane
+// per entry, each kind its own code: 1557 us; two lanes a pair staging, in place: 1516, pipelined:
+// 1187.)
+// A staged line: barrier [0..2] g_v, [3..14] g, friction [0..8] W, [9..12] c_v c, single [0..8] its
+// block, [9..12] 1; [15..17] the pair's gradient at v, [18] 1, [19] lam or 1.  Each product is the
+// same for the transposed block.
+constexpr int kLine = 21;  // odd: the two halves' lines start in different banks
 struct RowWarp {
     double acc[2][kRowCols * 9];
-    double fac[kRowBatch][kFac];
-    int meta[kRowBatch];                 // type | local vertex << 8 (-1: none)
-    int item[kRowBatch];
-    signed char col[kRowBatch][4];       // window column of each of the pair's vertices, -1: none
+    double line[32][kLine];
+    signed char col[32][4];   // window column of each of the pair's vertices, -1: none
+    signed char wide[32];     // 1: the block is c_b times nine numbers
 };
 constexpr size_t kRowShared = sizeof(RowTable) * kRowWarps + sizeof(RowWarp) * kRowWarps;
 
-// [j0, j1): this half-warp's part of the list, into its acc (zeroed) and, in the first window, g
-__device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable& T, RowWarp& W, int v, int U, int j0,
-                                               int j1, int lo, int hi, bool first, double& g) {
-    constexpr int kHalf = kRowBatch / 2;
+// half-warp hw of nh over the list [i0, i1): its acc (zeroed) and, in the first window, g
+__device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable& T, RowWarp& W, int v, int U, int i0,
+                                               int i1, int hw, int nh, int lo, int hi, bool first, double& g) {
     const int lane = threadIdx.x & 31, h = lane >> 4, hl = lane & 15;
     const bool grad = hl >= 12;
     const int b = grad ? 0 : hl / 3, q = hl % 3;
     double* acc = W.acc[h];
     for (int k = lane; k < 9 * U; k += 32) W.acc[0][k] = W.acc[1][k] = 0.0;
-    int turns = (j1 - j0 + kHalf - 1) / kHalf;
-    turns = max(turns, __shfl_xor_sync(0xffffffffu, turns, 16));
+    W.line[lane][18] = 1.0;
+    // (lane 15 of a half reads with the others and keeps nothing)
+    const int s_thin = grad ? 18 : 3 + 3 * b + q, s_wide = grad ? 18 : 9 + b;
+    const int r_thin = grad ? 15 + (hl < 15 ? q : 0) : 0, r_wide = grad ? r_thin : q;
+    const int d_thin = grad ? 0 : 1, d_wide = grad ? 0 : 3, s_lam = grad ? 18 : 19;
+    const int turns = (i1 - i0 + 16 * nh - 1) / (16 * nh);  // the same for all of the row's half-warps
+    auto incidence = [&](int t) -> uint32_t {
+        const int i = i0 + nh * (16 * t + hl) + hw;
+        return i < i1 ? __ldg(a.inc + i) : ~0u;
+    };
+    // a turn's pair is read while the sums of the turn before run
+    double2 f[8];
+    int vert[4], pair = 0, local = 0, type = -1;
+    auto fetch = [&](uint32_t inc) {
+        type = -1;
+        if (inc == ~0u) return;
+        type = inc_pair(a, inc, vert, pair, local);
+        if (type == kPairSingle || type == kPairMollified) return;
+        const double2* src = reinterpret_cast<const double2*>(a.cs.fac + kFac * (size_t)pair);
+#pragma unroll
+        for (int k = 0; k < 8; k++) f[k] = __ldg(src + k);
+    };
+    bool moll = false;
+    fetch(incidence(0));
+    uint32_t inc_next = incidence(1);
     for (int t = 0; t < turns; t++) {
-        // two lanes per pair: ids, then half of its line each and the window columns of two vertices
-        const int j = lane >> 1, half = lane & 1, i = j0 + t * kHalf + (j & (kHalf - 1));
         __syncwarp();
-        int meta = -1;
-        if (i < j1) {
-            int w[4], item, local;
-            const int type = inc_pair(a, __ldg(a.inc + i), w, item, local);
-            meta = type | (local << 8);
-            if (type == kPairSingle) {
-                if (half == 0)
+        double* L = W.line[lane];
+        int u[4] = {-1, -1, -1, -1};
+        double gr[3] = {0.0, 0.0, 0.0};
+        if (type == kPairBarrier) {
+            double w[16];
 #pragma unroll
-                    for (int k = 0; k < 9; k++) W.fac[j][k] = a.cs.sval[9 * (size_t)item + k];
-            } else {
-                const double2* src = reinterpret_cast<const double2*>(a.cs.fac + kFac * (size_t)item) + 4 * half;
-                double2 f[4];
+            for (int k = 0; k < 8; k++) w[2 * k] = f[k].x, w[2 * k + 1] = f[k].y;
+            double gv[3];
 #pragma unroll
-                for (int k = 0; k < 4; k++) f[k] = __ldg(src + k);
+            for (int p = 0; p < 3; p++)
+                gv[p] = local == 0 ? w[1 + p] : (local == 1 ? w[4 + p] : (local == 2 ? w[7 + p] : w[10 + p]));
 #pragma unroll
-                for (int k = 0; k < 4; k++) reinterpret_cast<double2*>(W.fac[j])[4 * half + k] = f[k];
+            for (int p = 0; p < 3; p++) {
+                L[p] = gv[p];
+                gr[p] = w[13] * gv[p];
             }
-            if (half == 0) W.item[j] = item;
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                if ((k >> 1) != half) continue;
-                const int c = w[k];
-                int u = -1;
-                // (a vertex named twice by a pair: its block is counted in the pair's order only)
-                if (c >= lo && c < hi && !(c == v && k < local)) {
-                    unsigned x = ((unsigned)c * 2654435761u) >> 24;
-                    while (T.hash[x] != c) x = (x + 1) & (kRowHash - 1);
-                    u = T.rank[x];
-                }
-                W.col[j][k] = (signed char)u;
-            }
+            for (int k = 0; k < 12; k++) L[3 + k] = w[1 + k];
+            L[19] = w[0];
+        } else if (type == kPairFriction) {
+            double w[16];
+#pragma unroll
+            for (int k = 0; k < 8; k++) w[2 * k] = f[k].x, w[2 * k + 1] = f[k].y;
+            const double cv = local == 0 ? w[9] : (local == 1 ? w[10] : (local == 2 ? w[11] : w[12]));
+#pragma unroll
+            for (int k = 0; k < 9; k++) L[k] = w[k];
+#pragma unroll
+            for (int k = 0; k < 4; k++) L[9 + k] = cv * w[9 + k];
+            L[19] = 1.0;
+#pragma unroll
+            for (int p = 0; p < 3; p++) gr[p] = cv * w[13 + p];
+        } else if (type == kPairSingle) {
+#pragma unroll
+            for (int k = 0; k < 9; k++) L[k] = a.cs.sval[9 * (size_t)pair + k];
+#pragma unroll
+            for (int k = 0; k < 4; k++) L[9 + k] = 1.0;
+            L[19] = 1.0;
         }
-        if (half == 0) W.meta[j] = meta;
-        __syncwarp();
-        // four pairs at a time: their products first, then the sums one pair after another
 #pragma unroll
-        for (int k0 = 0; k0 < kHalf; k0 += 4) {
-            double x[4][3];
-            int u[4];
+        for (int p = 0; p < 3; p++) L[15 + p] = first ? gr[p] : 0.0;
+        if (type == kPairMollified) moll = true;  // below
+        else if (type >= 0)
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                const int j2 = h * kHalf + k0 + k, m = W.meta[j2], type = m & 0xff, la = (m >> 8) & 3;
-                const double* f = W.fac[j2];
-                u[k] = m < 0 || hl == 15 ? -1 : (grad ? (first ? 0 : -1) : W.col[j2][b]);
-                if (type == kPairBarrier && m >= 0) {
-                    // lam (g_a g_b): the same product for the transposed block
-                    const double s = f[grad ? 13 : 1 + 3 * b + q], lam = grad ? 1.0 : f[0];
-                    const double* r = f + 1 + 3 * la + (grad ? q : 0);
-                    x[k][0] = lam * (r[0] * s);
-                    x[k][1] = lam * (r[grad ? 0 : 1] * s);
-                    x[k][2] = lam * (r[grad ? 0 : 2] * s);
-                } else if (type == kPairFriction && m >= 0) {
-                    const double s = f[9 + la] * (grad ? 1.0 : f[9 + b]);
-                    const double* r = f + (grad ? 13 + q : q);
-                    x[k][0] = s * r[0];
-                    x[k][1] = s * r[grad ? 0 : 3];
-                    x[k][2] = s * r[grad ? 0 : 6];
-                } else {
-                    x[k][0] = x[k][1] = x[k][2] = 0.0;
-                    if (m >= 0 && type == kPairSingle) {
-                        if (grad) u[k] = -1;  // the singles' gradient is added where they are made
-                        else
+                const int c = vert[k];
+                // (a vertex named twice by a pair: its block is counted in the pair's order only)
+                if (c < lo || c >= hi || (c == v && k < local)) continue;
+                unsigned x = ((unsigned)c * 2654435761u) >> 24;
+                while (T.hash[x] != c) x = (x + 1) & (kRowHash - 1);
+                u[k] = T.rank[x];
+            }
+        *reinterpret_cast<char4*>(W.col[lane]) = make_char4(u[0], u[1], u[2], u[3]);
+        W.wide[lane] = type == kPairBarrier ? 0 : 1;
+        fetch(inc_next);
+        inc_next = incidence(t + 2);
+        __syncwarp();
+        const int kmax = min(16, (i1 - i0 - 16 * nh * t + nh - 1) / nh);  // warp-uniform
+        for (int k0 = 0; k0 < kmax; k0 += 4) {
+            double x[4][3];
+            int d[4];
 #pragma unroll
-                            for (int p = 0; p < 3; p++) x[k][p] = f[3 * p + q];
-                    } else if (m >= 0) {
-                        const double* f2 = a.cs.fac2 + kFac * (size_t)W.item[j2];
-                        if (grad) x[k][0] = pair_grad(type, f, f2, la, q);
-                        else
-#pragma unroll
-                            for (int p = 0; p < 3; p++) x[k][p] = pair_entry(type, f, f2, la, b, p, q);
-                    }
-                }
+            for (int k = 0; k < 4; k++) {
+                const int j = 16 * h + k0 + k;
+                const double* m = W.line[j];
+                const bool wide = W.wide[j] != 0;
+                const double sc = m[wide ? s_wide : s_thin];
+                const double* r = m + (wide ? r_wide : r_thin);
+                const int dr = wide ? d_wide : d_thin;
+                const double lam = m[s_lam];
+                x[k][0] = lam * (sc * r[0]);
+                x[k][1] = lam * (sc * r[dr]);
+                x[k][2] = lam * (sc * r[2 * dr]);
+                d[k] = grad ? -1 : W.col[j][b];
             }
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                if (u[k] >= 0) {
-                    if (grad) {
-                        g += x[k][0];
-                    } else {
-                        double* d = acc + 9 * u[k] + q;
-                        const double d0 = d[0], d1 = d[3], d2 = d[6];
-                        d[0] = d0 + x[k][0];
-                        d[3] = d1 + x[k][1];
-                        d[6] = d2 + x[k][2];
-                    }
+                if (grad) {
+                    g += x[k][0];
+                } else if (d[k] >= 0) {
+                    double* o = acc + 9 * d[k] + q;
+                    const double o0 = o[0], o1 = o[3], o2 = o[6];
+                    o[0] = o0 + x[k][0];
+                    o[3] = o1 + x[k][1];
+                    o[6] = o2 + x[k][2];
                 }
                 __syncwarp();
             }
+        }
+    }
+    // mollified pairs (none come from the pair search), one after another
+    if (__any_sync(0xffffffffu, moll)) {
+        for (int i = i0 + hw; i - hw < i1; i += nh) {  // the same turns in both halves
+            int w[4], item, la, ty = -1;
+            if (i < i1) ty = inc_pair(a, __ldg(a.inc + i), w, item, la);
+            if (ty == kPairMollified && hl < 15) {
+                const double *m = a.cs.fac + kFac * (size_t)item, *m2 = a.cs.fac2 + kFac * (size_t)item;
+                const int c = w[b];
+                if (grad) {
+                    if (first) g += pair_grad(ty, m, m2, la, q);
+                } else if (c >= lo && c < hi && !(c == v && b < la)) {
+                    unsigned x = ((unsigned)c * 2654435761u) >> 24;
+                    while (T.hash[x] != c) x = (x + 1) & (kRowHash - 1);
+                    double* o = acc + 9 * T.rank[x] + q;
+#pragma unroll
+                    for (int p = 0; p < 3; p++) o[3 * p] += pair_entry(ty, m, m2, la, b, p, q);
+                }
+            }
+            __syncwarp();
         }
     }
     __syncwarp();
@@ -1234,7 +1296,7 @@ __device__ __forceinline__ void row_store(const RowArgs& a, const RowOut& o, con
     low += nlow;
 }
 
-__global__ void __launch_bounds__(32 * kRowWarps) k_row_sums(RowArgs a, RowOut o) {
+__global__ void __launch_bounds__(32 * kRowWarps, kRowCtas) k_row_sums(RowArgs a, RowOut o) {
     extern __shared__ __align__(16) unsigned char row_smem[];
     __shared__ double s_grad[2 * kRowWarps][3];
     RowWarp* warps = reinterpret_cast<RowWarp*>(row_smem);
@@ -1252,7 +1314,6 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_row_sums(RowArgs a, RowOut o
         [&](int v) {
             RowTable& T = tables[0];
             const int i0 = a.ptr[v], i1 = a.ptr[v + 1];
-            const int part = (i1 - i0 + 2 * kRowWarps - 1) / (2 * kRowWarps);
             unsigned up = (unsigned)(o.uoff[v] & 0xffffffffull), low = (unsigned)(o.uoff[v] >> 32);
             double g = 0.0;
             bool first = true;
@@ -1263,8 +1324,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_row_sums(RowArgs a, RowOut o
                     continue;
                 }
                 row_ranks<true>(T, threadIdx.x, 32 * kRowWarps);
-                row_accumulate(a, T, warps[w], v, T.used, min(i1, i0 + hw * part), min(i1, i0 + (hw + 1) * part), lo, hi,
-                               first, g);
+                row_accumulate(a, T, warps[w], v, T.used, i0, i1, hw, 2 * kRowWarps, lo, hi, first, g);
                 __syncthreads();
                 row_store<true>(a, o, T, warps, v, T.used, threadIdx.x, 32 * kRowWarps, up, low);
                 __syncthreads();
@@ -1295,8 +1355,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_row_sums(RowArgs a, RowOut o
                     continue;
                 }
                 row_ranks<false>(T, lane, 32);
-                const int mid = i0 + (i1 - i0 + 1) / 2;
-                row_accumulate(a, T, warps[w], v, T.used, lane < 16 ? i0 : mid, lane < 16 ? mid : i1, lo, hi, first, g);
+                row_accumulate(a, T, warps[w], v, T.used, i0, i1, lane >> 4, 2, lo, hi, first, g);
                 row_store<false>(a, o, T, warps + w, v, T.used, lane, 32, up, low);
                 __syncwarp();
                 first = false;
@@ -1710,7 +1769,7 @@ static SgipcStatus merge_contacts(SgipcCtx* c, const ContactCounts& cc, int sing
                                                 0, c->key_bits, s));
     k_inc_rows<<<nblk(n + 1), SGIPC_BLOCK, 0, s>>>(n, m, c->con_key_s, c->inc_ptr, c->row_list, c->row_cnt, c->ucnt);
     const RowArgs a{contact_store(c, cc), c->con_val_s, c->inc_ptr, c->row_list, c->row_cnt, n};
-    // (the grids cover the chip once; a CTA of k_row_sums holds 62 KB)
+    // (the grids cover the chip once)
     const int most = nblk(m, 8);  // no more CTAs than a small call has work for
     k_row_counts<<<std::min(most, 148 * 8), 32 * kRowWarps, 0, s>>>(a, c->ucnt);
     tb = c->cub_tmp_bytes;
@@ -1718,7 +1777,7 @@ static SgipcStatus merge_contacts(SgipcCtx* c, const ContactCounts& cc, int sing
     const RowOut o{c->uoff, btype, c->nuc, c->cu_ptr, c->cl_ptr, c->uc_row, c->uc_col, c->uc64, c->uc32, c->cl_col,
                    c->cl64, c->cl32, grad};
     SG_CHECK(c, cudaFuncSetAttribute(k_row_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowShared));
-    k_row_sums<<<std::min(std::max(most, 148), 148 * 3), 32 * kRowWarps, kRowShared, s>>>(a, o);
+    k_row_sums<<<std::min(std::max(most, 148), 148 * kRowCtas), 32 * kRowWarps, kRowShared, s>>>(a, o);
     SG_LAUNCH_CHECK(c, "contact rows");
     return SGIPC_OK;
 }

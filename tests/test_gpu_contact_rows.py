@@ -1,5 +1,5 @@
 """Rows of the contact matrix against the oracle's assembly, at the sizes where the row kernels
-change: a warp or a CTA per row (128 incidences), windows of 80 columns, batches of 8 pairs a
+change: a warp or a CTA per row (128 incidences), windows of 40 columns, batches of 16 pairs a
 half-warp, every pair kind (mollified ones included) and
 rows of fixed vertices.
 
@@ -44,8 +44,8 @@ def _pairs(rng, nv, hub, columns, repeats, mollified):
 
 
 @pytest.mark.parametrize("columns,repeats,mollified", [(1, 0, False), (7, 1, True), (15, 112, False), (15, 113, True),
-                                                       (15, 114, False), (79, 0, False), (80, 40, True),
-                                                       (81, 60, False), (161, 0, True), (330, 1000, True)])
+                                                       (15, 114, False), (39, 0, False), (40, 40, True),
+                                                       (41, 60, False), (81, 0, True), (330, 1000, True)])
 def test_rows_match_the_oracle(columns, repeats, mollified):
     rng = np.random.default_rng(columns + repeats)
     sc = scenes.scene_two_cubes(6, seed=4)
