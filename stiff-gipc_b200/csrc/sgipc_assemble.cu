@@ -293,12 +293,14 @@ __global__ void __launch_bounds__(128) k_tri_bw(int nf, const uint32_t* __restri
 // quadratic bending (femEnergy.cu:2623-2753; Q from the rest shape, :2492-2618): per
 // interior edge with vertices [e0, e1, opposite of triangle 1, opposite of triangle 2],
 // E = 1/2 c x^T (Q (x) I3) x, c = |rest e0 - rest e1| * bendStiff * dt^2: gradient c Q x,
-// constant Hessian c Q (x) I3.  Boundary edges (no second triangle) contribute nothing.
+// constant Hessian c Q (x) I3.  Boundary edges (no second triangle) contribute nothing.  A block
+// c Q(a,b) I3 is stored as its one number (hblk, 10 per hinge; k_gather_blocks puts it on the
+// diagonal): as 3x3 blocks the 195 000 hinges of a 256^2 cloth were 140 MB to write and read.
 // ------------------------------------------------------------------------------------------
 __global__ void k_hinge_quad(int nh, const uint32_t* __restrict__ edges, const int32_t* __restrict__ adj,
                              const double* __restrict__ x, const double* __restrict__ rest,
-                             const double* __restrict__ Qcm, double kb_dt2, int eoff, int goff,
-                             double* __restrict__ eblk, double* __restrict__ egrad) {
+                             const double* __restrict__ Qcm, double kb_dt2, int goff,
+                             double* __restrict__ hblk, double* __restrict__ egrad) {
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= nh) return;
     const int v[4] = {(int)edges[2 * h], (int)edges[2 * h + 1], adj[2 * h], adj[2 * h + 1]};
@@ -331,16 +333,16 @@ __global__ void k_hinge_quad(int nh, const uint32_t* __restrict__ edges, const i
         o[2] = g.z;
     }
     const int pa[10] = {0, 0, 0, 0, 1, 1, 1, 2, 2, 3}, pb[10] = {0, 1, 2, 3, 1, 2, 3, 2, 3, 3};
+    double d[10];
 #pragma unroll
     for (int k = 0; k < 10; k++) {
-        // block (a, b) is c Q(a,b) I3; stored as the (min, max) block, i.e. from Q(b,a) when
-        // the element's vertex order is reversed
+        // block (a, b) is that of (min, max): from Q(b,a) when the element's order is reversed
         const bool tr = v[pa[k]] > v[pb[k]];
-        const double d = c * (tr ? Q[pb[k]][pa[k]] : Q[pa[k]][pb[k]]);
-        double* o = eblk + 9 * ((size_t)eoff + 10 * (size_t)h + k);
-#pragma unroll
-        for (int q = 0; q < 9; q++) o[q] = (q % 4 == 0) ? d : 0.0;
+        d[k] = c * (tr ? Q[pb[k]][pa[k]] : Q[pa[k]][pb[k]]);
     }
+    double2* o = reinterpret_cast<double2*>(hblk + 10 * (size_t)h);
+#pragma unroll
+    for (int k = 0; k < 5; k++) o[k] = make_double2(d[2 * k], d[2 * k + 1]);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -354,9 +356,11 @@ struct StaticOut {
     float* f32;
 };
 
+// kHinges: contributions from hfirst on are hinges (without any, their test cost the tets' gather 15 %)
+template <bool kHinges>
 __global__ void k_gather_blocks(int nnz, const int* __restrict__ cptr, const int* __restrict__ contrib,
-                                const double* __restrict__ eblk, const int* __restrict__ slot_row,
-                                const int* __restrict__ col, const int32_t* __restrict__ btype,
+                                const double* __restrict__ eblk, const double* __restrict__ hblk, int hfirst,
+                                const int* __restrict__ slot_row, const int* __restrict__ col, const int32_t* __restrict__ btype,
                                 const double* __restrict__ mass, StaticOut o) {
     long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (tid >= 9LL * nnz) return;
@@ -366,6 +370,11 @@ __global__ void k_gather_blocks(int nnz, const int* __restrict__ cptr, const int
     // the contributions four at a time, their index and value loads issued together (one by
     // one, each waited out two L2 round trips), added in list order as before; the boundary
     // test is applied after the loads
+    const bool diag = q % 4 == 0;  // a hinge's block is a multiple of the identity
+    auto entry = [&](int i) -> double {
+        if (!kHinges || i < hfirst) return eblk[9 * (size_t)i + q];
+        return diag ? hblk[i - hfirst] : 0.0;
+    };
     double acc = 0.0;
     int k = k0;
     for (; k + 4 <= k1; k += 4) {
@@ -374,11 +383,11 @@ __global__ void k_gather_blocks(int nnz, const int* __restrict__ cptr, const int
         for (int u = 0; u < 4; u++) ix[u] = contrib[k + u];
         double e[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) e[u] = eblk[9 * (size_t)ix[u] + q];
+        for (int u = 0; u < 4; u++) e[u] = entry(ix[u]);
 #pragma unroll
         for (int u = 0; u < 4; u++) acc += e[u];
     }
-    for (; k < k1; k++) acc += eblk[9 * (size_t)contrib[k] + q];
+    for (; k < k1; k++) acc += entry(contrib[k]);
     if (btype[r] != 0 || btype[c] != 0) acc = 0.0;
     if (r == c && (q == 0 || q == 4 || q == 8)) acc += mass[r];
     o.v64[tid] = acc;
@@ -1799,19 +1808,24 @@ static SgipcStatus launch_fem(SgipcCtx* c, const SgipcFemData* f, const SgipcPar
     if (c->nh > 0) {
         SG_COUNT(c, 1);
         k_hinge_quad<<<nblk(c->nh), SGIPC_BLOCK, 0, s>>>(c->nh, c->hinges, c->hinge_adj, f->vertexes, f->rest_vertexes,
-                                                         f->quad_bending_Q, p->bendStiff * dt2,
-                                                         10 * c->nt + 6 * c->nf, 4 * c->nt + 3 * c->nf, c->eblk,
-                                                         c->egrad);
+                                                         f->quad_bending_Q, p->bendStiff * dt2, 4 * c->nt + 3 * c->nf,
+                                                         c->hblk, c->egrad);
     }
     SG_LAUNCH_CHECK(c, "fem element kernels");
     return SGIPC_OK;
 }
 
+static void launch_gather_blocks(SgipcCtx* c, const SgipcFemData* f, cudaStream_t s) {
+    auto* kernel = c->nh > 0 ? k_gather_blocks<true> : k_gather_blocks<false>;
+    kernel<<<nblk(9LL * c->nnz), SGIPC_BLOCK, 0, s>>>(c->nnz, c->contrib_ptr, c->contrib, c->eblk, c->hblk,
+                                                      10 * c->nt + 6 * c->nf, c->slot_row, c->col, f->BoundaryType,
+                                                      f->masses, static_out(c));
+}
+
 static SgipcStatus gather_static(SgipcCtx* c, const SgipcFemData* f, cudaStream_t s) {
     c->mas.pre_scattered = 0;  // a scatter of the previous static matrix is stale
     SG_COUNT(c, 1 + (c->n_egrad > 0));
-    k_gather_blocks<<<nblk(9LL * c->nnz), SGIPC_BLOCK, 0, s>>>(c->nnz, c->contrib_ptr, c->contrib, c->eblk, c->slot_row,
-                                                                c->col, f->BoundaryType, f->masses, static_out(c));
+    launch_gather_blocks(c, f, s);
     if (c->n_egrad > 0)
         k_gather_grad<<<nblk(3LL * c->nv), SGIPC_BLOCK, 0, s>>>(c->nv, c->vinc_ptr, c->vinc, c->egrad, c->shape_grads);
     SG_LAUNCH_CHECK(c, "static gather");
@@ -2240,13 +2254,12 @@ SgipcStatus assemble_time_hook(SgipcCtx* c, const char* name, cudaStream_t s, do
         *bytes = (double)c->nt * (4 * 24 + 72 + 8 + 16 + 16 + 10 * 72 + 12 * 8);
     } else if (!strcmp(name, "gather_blocks")) {
         SG_COUNT(c, 1);
-        k_gather_blocks<<<nblk(9LL * c->nnz), SGIPC_BLOCK, 0, s>>>(c->nnz, c->contrib_ptr, c->contrib, c->eblk,
-                                                                    c->slot_row, c->col, f->BoundaryType, f->masses,
-                                                                    static_out(c));
+        launch_gather_blocks(c, f, s);
         // element blocks and their indices in; per upper slot its indices, flags and the FP64
         // upper value out, the full-pattern FP64 + FP32 copy, and the transposed copy off the
         // diagonal
-        *bytes = (double)c->n_eblk * (72 + 4) + (double)c->nnz * (28 + 72 + 108) + (double)(c->nnz - c->n) * 108;
+        *bytes = (double)(10LL * c->nt + 6LL * c->nf) * 72 + 80.0 * c->nh + 4.0 * c->n_eblk +
+                 (double)c->nnz * (28 + 72 + 108) + (double)(c->nnz - c->n) * 108;
     } else if (!strcmp(name, "barrier") || !strcmp(name, "friction")) {
         // one kind's launch (its factors and keys are rewritten with the same values)
         if (!k) return SGIPC_BAD_INPUT;

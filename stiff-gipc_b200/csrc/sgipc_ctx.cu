@@ -214,7 +214,8 @@ static SgipcStatus build_static(SgipcCtx* c, const SgipcTopology* t) {
     SG_TRY(upload(c, &c->vinc_ptr, vptr));
     SG_TRY(upload(c, &c->vinc, vinc));
     SG_TRY(dalloc(c, &c->val64, (size_t)nnz * 9));
-    SG_TRY(dalloc(c, &c->eblk, (size_t)c->n_eblk * 9));
+    SG_TRY(dalloc(c, &c->eblk, (10 * (size_t)c->nt + 6 * (size_t)c->nf) * 9));
+    SG_TRY(dalloc(c, &c->hblk, 10 * (size_t)c->nh));
     SG_TRY(dalloc(c, &c->egrad, (size_t)c->n_egrad * 3));
     return SGIPC_OK;
 }
@@ -385,7 +386,7 @@ extern "C" SgipcStatus sgipc_destroy(SgipcCtx* c) {
     pcg_destroy(c);
     mas_destroy(c);
     void* ptrs[] = {c->row_ptr, c->col, c->slot_row, c->diag_slot, c->low_ptr, c->low_slot, c->val64,
-                    c->eblk, c->contrib_ptr, c->contrib, c->egrad, c->vinc_ptr, c->vinc, c->tets, c->tris,
+                    c->eblk, c->hblk, c->contrib_ptr, c->contrib, c->egrad, c->vinc_ptr, c->vinc, c->tets, c->tris,
                     c->hinges, c->hinge_adj, c->soft_idx, c->shape_grads, c->fb, c->b, c->con_ids,
                     c->con_fac, c->con_fac2, c->con_sid, c->con_sval, c->con_key, c->con_val, c->con_key_s,
                     c->con_val_s, c->inc_ptr, c->row_list, c->row_cnt, c->ucnt, c->uoff, c->part_a, c->part_f, c->nuc, c->uc_row, c->uc_col, c->uc64, c->uc32,

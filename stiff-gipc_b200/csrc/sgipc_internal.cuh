@@ -152,7 +152,8 @@ struct SgipcCtx {
     float* fval32;            // [nnz_full*9]
     // element blocks and their gather lists
     int n_eblk;               // 10 per tet, 6 per triangle, 10 per hinge
-    double* eblk;             // [n_eblk*9] oriented element blocks
+    double* eblk;             // [(10 nt + 6 nf) * 9] oriented element blocks of the tets and triangles
+    double* hblk;             // [10 nh] the hinges' blocks, one number each (a multiple of the identity)
     int* contrib_ptr;         // [nnz+1]
     int* contrib;             // [n_eblk] element block ids sorted by slot
     int n_egrad;              // 4 per tet, 3 per triangle, 4 per hinge
