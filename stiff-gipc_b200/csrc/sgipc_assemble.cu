@@ -2285,7 +2285,8 @@ SgipcStatus assemble_time_hook(SgipcCtx* c, const char* name, cudaStream_t s, do
 // ------------------------------------------------------------------------------------------
 // line-search energy: host side
 // ------------------------------------------------------------------------------------------
-// Launch the energy kernels and the final sum into c->en_terms on s (no synchronisation).
+// Launch the energy kernels and the final sum on s (no synchronisation); the last CTA writes the
+// terms straight into pinned host memory (c->h_en).
 // Terms: 0 kinetic, 1 tets, 2 triangles, 3 hinges, 4 soft, 5 barrier, 6 ground, 7 friction,
 // 8 ground friction; 9 the total.  *bytes: algorithmic bytes of the launch sequence.
 static SgipcStatus energy_launch(SgipcCtx* c, const SgipcFemData* f, const SgipcContacts* k, const SgipcParams* p,
@@ -2316,7 +2317,7 @@ static SgipcStatus energy_launch(SgipcCtx* c, const SgipcFemData* f, const Sgipc
     a.dt2 = dt2; a.kst = p->stretchStiff; a.ksh = p->shearStiff; a.srate = p->strainRate; a.kb_dt2 = p->bendStiff * dt2;
     a.ksoft = p->motionRate * p->softRate * p->softRate; a.dhat = p->dHat; a.kappa = p->kappa;
     a.offset = p->ground_offset; a.mu = p->frictionRate; a.mu_gd = p->gd_frictionRate; a.eps2 = eps2;
-    k_energy<<<o.off[9], SGIPC_BLOCK, 0, s>>>(a, o, c->en_part, c->en_terms, c->en_ticket);
+    k_energy<<<o.off[9], SGIPC_BLOCK, 0, s>>>(a, o, c->en_part, c->h_en, c->en_ticket);
     SG_COUNT(c, 1);
     SG_LAUNCH_CHECK(c, "energy");
     if (bytes)  // positions (and the per-element inputs) in, one partial per CTA out and back
@@ -2335,7 +2336,6 @@ extern "C" SgipcStatus sgipc_compute_energy(SgipcCtx* c, const SgipcFemData* f, 
     cudaStream_t s = (cudaStream_t)stream;
     SG_DEVICE(c);
     if ((st = energy_launch(c, f, k, p, s, nullptr)) != SGIPC_OK) return st;
-    SG_CHECK(c, cudaMemcpyAsync(c->h_en, c->en_terms, sizeof(double) * 10, cudaMemcpyDeviceToHost, s));
     SG_CHECK(c, cudaStreamSynchronize(s));
     *energy = c->h_en[9];
     if (terms)

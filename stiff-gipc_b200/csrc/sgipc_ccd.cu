@@ -95,6 +95,10 @@ __device__ double accd(bool ee, d3* X, d3* D, double eta, double thick) {
 
 // fixed-size grid of the step-size kernels (grid-stride loops over the candidates)
 constexpr int kCcdGrid = 148 * 4;
+// A candidate's advances are one long FP64 chain, so few candidates are spread over all SMs in
+// CTAs of two warps (21 628 of them in CTAs of 256 left 63 SMs idle; with the results written to
+// pinned memory a line search of two 21^3 cubes went from 166 to 138 us); many fill them anyway.
+constexpr int kCcdSmallBlock = 64;
 
 // How a step-size launch ends: the last CTA to finish (ticket) takes m = max(init, every
 // CTA's maximum), writes out[0] = 1 / m (step sizes) or m (speeds) and out[1] = the
@@ -102,7 +106,7 @@ constexpr int kCcdGrid = 148 * 4;
 struct StepFinish {
     double init;
     int invert;
-    double* out;
+    double* out;  // pinned host memory: read after the stream's synchronisation
     int* bad;
     unsigned int* ticket;
 };
@@ -209,13 +213,12 @@ __global__ void __launch_bounds__(SGIPC_BLOCK) k_cfl_speed(int ns, int nv, const
 }
 
 StepFinish step_finish(SgipcCtx* c, bool speed) {
-    return {speed ? 0.0 : 1.0, speed ? 0 : 1, c->ccd_out, c->ccd_bad, c->ccd_ticket};
+    return {speed ? 0.0 : 1.0, speed ? 0 : 1, c->h_en + 12, c->ccd_bad, c->ccd_ticket};
 }
 
 SgipcStatus read_step(SgipcCtx* c, cudaStream_t s, double* value, const char* what) {
     SG_COUNT(c, 1);
     SG_LAUNCH_CHECK(c, what);
-    SG_CHECK(c, cudaMemcpyAsync(c->h_en + 12, c->ccd_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
     SG_CHECK(c, cudaStreamSynchronize(s));
     if (c->h_en[13] != 0.0) {
         snprintf(c->err, sizeof(c->err), "%s: a candidate names a vertex outside [0, %d)", what, c->nv);
@@ -258,9 +261,10 @@ extern "C" SgipcStatus sgipc_self_step_size(SgipcCtx* c, const double* x, const 
     if (!(slackness > 0.0 && slackness <= 1.0)) return SGIPC_BAD_INPUT;
     SG_DEVICE(c);
     cudaStream_t s = (cudaStream_t)stream;
-    const int grid = std::max(1, std::min(nblk(npairs), kCcdGrid));
-    k_self_step<<<grid, SGIPC_BLOCK, 0, s>>>(npairs, c->nv, (const int4*)pairs, x, move_dir, 1.0 - slackness, toi,
-                                             c->ccd_part, step_finish(c, false));
+    const int block = npairs <= kCcdGrid * kCcdSmallBlock ? kCcdSmallBlock : SGIPC_BLOCK;
+    const int grid = std::max(1, std::min(nblk(npairs, block), kCcdGrid));
+    k_self_step<<<grid, block, 0, s>>>(npairs, c->nv, (const int4*)pairs, x, move_dir, 1.0 - slackness, toi,
+                                       c->ccd_part, step_finish(c, false));
     return read_step(c, s, alpha, "self step size");
 }
 

@@ -348,8 +348,8 @@ extern "C" SgipcStatus sgipc_create(const SgipcTopology* t_in, int device, Sgipc
         long long ecap = 1;
         for (long long v : cnt) ecap += nblk(v);
         c->en_cap = (int)ecap;
-        if ((st = dalloc(c, &c->en_part, ecap)) || (st = dalloc(c, &c->en_terms, 16)) ||
-            (st = dalloc(c, &c->ccd_part, 148 * 4)) || (st = dalloc(c, &c->ccd_out, 2)) ||
+        if ((st = dalloc(c, &c->en_part, ecap)) ||
+            (st = dalloc(c, &c->ccd_part, 148 * 4)) ||
             (st = dalloc(c, &c->ccd_bad, 1)) || (st = dalloc(c, &c->en_ticket, 1)) ||
             (st = dalloc(c, &c->ccd_ticket, 1)))
             return fail(st);
@@ -391,7 +391,7 @@ extern "C" SgipcStatus sgipc_destroy(SgipcCtx* c) {
                     c->con_fac, c->con_fac2, c->con_sid, c->con_sval, c->con_key, c->con_val, c->con_key_s,
                     c->con_val_s, c->inc_ptr, c->row_list, c->row_cnt, c->ucnt, c->uoff, c->part_a, c->part_f, c->nuc, c->uc_row, c->uc_col, c->uc64, c->uc32,
                     c->cu_ptr, c->cl_ptr, c->cub_tmp, c->dflag,
-                    c->frow_ptr, c->fcol, c->fup, c->flo, c->fval64, c->fval32, c->cl_col, c->cl64, c->cl32, c->en_part, c->en_terms, c->ccd_part, c->ccd_out, c->ccd_bad, c->en_ticket, c->ccd_ticket,
+                    c->frow_ptr, c->fcol, c->fup, c->flo, c->fval64, c->fval32, c->cl_col, c->cl64, c->cl32, c->en_part, c->ccd_part, c->ccd_bad, c->en_ticket, c->ccd_ticket,
                     c->cs.ptr, c->cs.cols, c->cs.lcol, c->cs.dslot, c->cs_small.ptr, c->cs_small.cols, c->cs_small.lcol,
                     c->cs_small.dslot, c->close_gid, c->close_gval, c->close_pid,
                     c->close_pval, c->close_cnt};

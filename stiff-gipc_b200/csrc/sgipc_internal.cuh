@@ -207,11 +207,10 @@ struct SgipcCtx {
     int* dflag;                   // device: input errors found by kernels (bit 0: pair index)
     double* en_part;              // [en_cap] per-CTA partial sums of the line-search energy terms
     int en_cap;
-    double* en_terms;             // [16] device: the nine terms and their total
     unsigned int* en_ticket;      // [1] device: CTAs of the energy launch done (0 between launches)
-    double* h_en;                 // [16] pinned landing area of en_terms ([12], [13]: step sizes)
+    double* h_en;                 // [16] pinned: the nine energy terms and their total; [12], [13] a step size
+                                  //   (or speed) and the out-of-range flag; the kernels write them
     double* ccd_part;             // [592] per-CTA maxima of the step-size kernels
-    double* ccd_out;              // [2] the step (or speed) and the out-of-range flag
     int* ccd_bad;                 // [1] a candidate with an out-of-range vertex (0 between launches)
     unsigned int* ccd_ticket;     // [1] CTAs of a step-size launch done (0 between launches)
     // last inputs (for re-timing kernels against the current state)

@@ -74,6 +74,24 @@ def test_random_candidates_match_oracle(g, scale):
     assert 0.0 < a <= 1.0 and np.all(tg > 0) and np.all(tg <= 1.0)
 
 
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 592 * 64, 592 * 64 + 1])
+def test_step_of_few_and_many_candidates(g, n):
+    """CTAs of two warps up to 592 * 64 candidates, of eight above: each candidate's bound and their
+    minimum are those of the candidates taken alone, bit for bit (the same arithmetic, an exact
+    maximum)."""
+    sc, gg = g
+    rng = np.random.default_rng(7)
+    x = sc.vertexes + 1e-3 * rng.standard_normal((sc.nv, 3))
+    d = 0.05 * rng.standard_normal((sc.nv, 3))
+    few = _candidates(sc.nv, 50, rng)
+    alone = np.array([gg.self_largestFeasibleStepSize(0.8, _dev(d), _dev(p[None], torch.int32), x=_dev(x)) for p in few])
+    pick = rng.integers(len(few), size=n)
+    toi = torch.zeros(n, dtype=torch.float64, device="cuda")
+    a = gg.self_largestFeasibleStepSize(0.8, _dev(d), _dev(few[pick], torch.int32), x=_dev(x), toi=toi)
+    assert a == alone[pick].min()
+    assert np.abs(toi.cpu().numpy() / alone[pick] - 1.0).max() <= 4e-16  # (a bound is 1 / (1 / toi))
+
+
 def test_ground_bound_matches_oracle(g):
     sc, gg = g
     rng = np.random.default_rng(3)
