@@ -50,3 +50,30 @@ def test_large_scene_persistent_and_graph_agree(big, monkeypatch):
     assert abs(sa.iterations - sb.iterations) <= 1
     if sa.iterations == sb.iterations:
         assert float((xa - xb).abs().max() / xb.abs().max()) < 1e-9
+
+
+@pytest.mark.parametrize("n", [28, 33])
+def test_banks_by_cta_and_by_half_cta_agree_with_graph(n, monkeypatch):
+    """The position pass with fewer level-1 banks than CTAs (28^3) and with more (33^3, two banks a
+    CTA at a time, the last CTA one): the graph of kernels, which sums in another order, reaches the
+    same solution.  Both stop at a true residual of 1e-10 |b|, so each is within 1e-10 cond(A) |x| of
+    the exact one, and cond(A) is below 1e4 here (the mass term)."""
+    sc = scenes.scene_cube(n, touching=True)
+    g = system.GIPC(sc)
+    g.computeGradientAndHessian()
+    mas = system.MASPreconditioner(g)
+    mas.setPreconditioner("fp64")
+    banks = (int(mas.info()[1][1]) + 15) // 16
+    assert sc.nv > 148 * 128 and (banks > 148) == (n == 33)
+    b = torch.randn(3 * sc.nv, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(n))
+    solver = system.PCGSolver(g, system.PCGSolverConfig(precision="fp64", criterion=N.CRIT_TRUE, global_tol_rate=1e-10,
+                                                        max_iter_ratio=1.0))
+    xa, sa = solver.solve(b)
+    monkeypatch.setenv("SGIPC_PCG_GRAPH", "1")
+    xb, sb = solver.solve(b)
+    monkeypatch.delenv("SGIPC_PCG_GRAPH")
+    assert sa.status == N.OK and sb.status == N.OK
+    for x in (xa, xb):
+        assert float((b - g.spmv(x)).norm() / b.norm()) < 1.1e-10
+    assert float((xa - xb).norm() / xb.norm()) < 1e-6
+    g.close()
