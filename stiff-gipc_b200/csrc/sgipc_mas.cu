@@ -425,10 +425,17 @@ __global__ void __launch_bounds__(64, 6) k_invert(int ndom, double* __restrict__
 namespace sgipc {
 
 // level 0 and level 1 of the restriction: one thread per position
-template <class T, class M>
+// what the apply's kernels look at before they do anything: the stop flag of the coupled solve, whose
+// next iteration is enqueued before the last one's outcome is known, or nothing (the flag's test alone
+// cost an apply of a small system 5 %)
+struct NoStop {};
+__device__ __forceinline__ bool stopped(NoStop) { return false; }
+__device__ __forceinline__ bool stopped(const int* stop) { return *stop != 0; }
+
+template <class T, class M, class Stop = NoStop>
 __global__ void k_restrict01(int npos, const T* __restrict__ r, const int* __restrict__ part_map,
-                             const int* __restrict__ up, M* __restrict__ R, const int* __restrict__ stop = nullptr) {
-    if (stop && *stop) return;
+                             const int* __restrict__ up, M* __restrict__ R, Stop stop = Stop()) {
+    if (stopped(stop)) return;
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     int v = p < npos ? part_map[p] : -1;
     M val[3] = {0, 0, 0};
@@ -445,19 +452,19 @@ __global__ void k_restrict01(int npos, const T* __restrict__ r, const int* __res
     bank_reduce_store<M, 1>(v >= 0 ? up[p] : -1, val, R);
 }
 
-template <class M>
+template <class M, class Stop = NoStop>
 __global__ void __launch_bounds__(1024) k_restrict_coarse(const int* __restrict__ info, const int* __restrict__ up,
                                                           int L, M* __restrict__ R,
-                                                          const int* __restrict__ stop = nullptr) {
-    if (stop && *stop) return;
+                                                          Stop stop = Stop()) {
+    if (stopped(stop)) return;
     restrict_coarse_cta<M, 1>(info, up, L, R);
 }
 
 // one level of it over many CTAs
-template <class M>
+template <class M, class Stop = NoStop>
 __global__ void k_restrict_level(const int* __restrict__ info, const int* __restrict__ up, int l, M* __restrict__ R,
-                                 const int* __restrict__ stop) {
-    if (stop && *stop) return;
+                                 Stop stop) {
+    if (stopped(stop)) return;
     const int a = blockIdx.x * blockDim.x + threadIdx.x, g = info[l] + a;
     const bool on = a < info[8 + l];
     M v[3] = {0, 0, 0};
@@ -468,12 +475,12 @@ __global__ void k_restrict_level(const int* __restrict__ info, const int* __rest
 }
 
 // Z_d = A_d^-1 R_d, four domains per 192-thread CTA
-template <class M>
+template <class M, class Stop = NoStop>
 __global__ void __launch_bounds__(192) k_domain_mv(const int* __restrict__ info, const M* __restrict__ inv,
                                                    const M* __restrict__ R, M* __restrict__ Z,
-                                                   const int* __restrict__ stop = nullptr) {
+                                                   Stop stop = Stop()) {
     __shared__ M sR[4][48];
-    if (stop && *stop) return;
+    if (stopped(stop)) return;
     const int ndom = info[16] >> 4;
     const int ld = threadIdx.x / 48, i = threadIdx.x % 48;
     const int d = blockIdx.x * 4 + ld;
@@ -504,11 +511,11 @@ __global__ void k_prolong(int nv, const int* __restrict__ table, int L, const M*
     z[3 * v + 2] = (T)w;
 }
 
-template <class T, class M>
-static void restrict_and_solve(SgipcCtx* c, const T* r, const M* inv, M* R, M* Z, const int* stop, cudaStream_t s) {
+template <class T, class M, class Stop>
+static void restrict_and_solve(SgipcCtx* c, const T* r, const M* inv, M* R, M* Z, Stop stop, cudaStream_t s) {
     MasWork& m = c->mas;
     const int L = m.levelnum, ndom = m.h_info[16] / 16;
-    k_restrict01<T, M><<<nblk(m.npos), SGIPC_BLOCK, 0, s>>>(m.npos, r, m.part_map, m.up, R, stop);
+    k_restrict01<T, M, Stop><<<nblk(m.npos), SGIPC_BLOCK, 0, s>>>(m.npos, r, m.part_map, m.up, R, stop);
     // One CTA takes 1024 nodes of a level per turn, about 1.5 us each (24 us for the 16 turns of
     // 500 boxes over a bed, 4000 of whose points no contact joins); a launch of its own costs a
     // level about 2.5 us, so it pays from two turns a level on.
@@ -517,19 +524,23 @@ static void restrict_and_solve(SgipcCtx* c, const T* r, const M* inv, M* R, M* Z
     if (turns > 2 * (L - 2)) {
         SG_COUNT(c, L);
         for (int l = 1; l + 1 < L; l++)
-            k_restrict_level<M><<<nblk(m.h_info[8 + l]), SGIPC_BLOCK, 0, s>>>(m.info, m.up, l, R, stop);
+            k_restrict_level<M, Stop><<<nblk(m.h_info[8 + l]), SGIPC_BLOCK, 0, s>>>(m.info, m.up, l, R, stop);
     } else {
         SG_COUNT(c, 3);
-        k_restrict_coarse<M><<<1, 1024, 0, s>>>(m.info, m.up, L, R, stop);
+        k_restrict_coarse<M, Stop><<<1, 1024, 0, s>>>(m.info, m.up, L, R, stop);
     }
-    k_domain_mv<M><<<(ndom + 3) / 4, 192, 0, s>>>(m.info, inv, R, Z, stop);
+    k_domain_mv<M, Stop><<<(ndom + 3) / 4, 192, 0, s>>>(m.info, inv, R, Z, stop);
 }
 
 SgipcStatus mas_domains(SgipcCtx* c, const double* r, int fp32_inv, const int* stop, cudaStream_t s) {
     MasWork& m = c->mas;
     if (!m.built) return SGIPC_NOT_READY;
-    if (fp32_inv) restrict_and_solve<double, float>(c, r, m.dom32, m.R32, m.Z32, stop, s);
-    else restrict_and_solve<double, double>(c, r, m.dom64, m.R64, m.Z64, stop, s);
+    auto solve = [&](auto flag) {
+        if (fp32_inv) restrict_and_solve(c, r, m.dom32, m.R32, m.Z32, flag, s);
+        else restrict_and_solve(c, r, m.dom64, m.R64, m.Z64, flag, s);
+    };
+    if (stop) solve(stop);
+    else solve(NoStop());
     SG_LAUNCH_CHECK(c, "mas domains");
     return SGIPC_OK;
 }
@@ -541,10 +552,10 @@ SgipcStatus mas_apply_t(SgipcCtx* c, const T* r, T* z, int fp32_inv, cudaStream_
     const int L = m.levelnum;
     SG_COUNT(c, 1);
     if (fp32_inv) {
-        restrict_and_solve<T, float>(c, r, m.dom32, m.R32, m.Z32, nullptr, s);
+        restrict_and_solve(c, r, m.dom32, m.R32, m.Z32, NoStop(), s);
         k_prolong<T, float><<<nblk(c->nv), SGIPC_BLOCK, 0, s>>>(c->nv, m.table, L, m.Z32, z);
     } else {
-        restrict_and_solve<T, double>(c, r, m.dom64, m.R64, m.Z64, nullptr, s);
+        restrict_and_solve(c, r, m.dom64, m.R64, m.Z64, NoStop(), s);
         k_prolong<T, double><<<nblk(c->nv), SGIPC_BLOCK, 0, s>>>(c->nv, m.table, L, m.Z64, z);
     }
     SG_LAUNCH_CHECK(c, "mas apply");
