@@ -653,7 +653,7 @@ SgipcStatus pcg_create(SgipcCtx* c) {
     if ((st = alloc_work(c, c->pcg32, sizeof(float), c->max_rhs)) != SGIPC_OK) return st;
     SG_CHECK(c, cudaMalloc((void**)&c->tmp64, sizeof(double) * 3 * (size_t)c->n * c->max_rhs));
     SG_CHECK(c, cudaMalloc((void**)&c->tmp64b, sizeof(double) * 3 * (size_t)c->n * c->max_rhs));
-    SG_CHECK(c, cudaMalloc((void**)&c->dot_partial, sizeof(double) * 1024));
+    SG_CHECK(c, cudaMalloc((void**)&c->dot_partial, sizeof(double) * 2048));
     SG_CHECK(c, cudaMalloc((void**)&c->dot_ticket, sizeof(unsigned int) * 4));
     SG_CHECK(c, cudaMemset(c->dot_ticket, 0, sizeof(unsigned int) * 4));
     SG_CHECK(c, cudaMalloc((void**)&c->dot_out, sizeof(double) * 16));
@@ -718,20 +718,20 @@ extern "C" SgipcStatus sgipc_spmv(SgipcCtx* c, const double* x, double* y, void*
     return spmv_t<double>(c, x, y, (cudaStream_t)stream);
 }
 
-// ||b - A x||^2 of right-hand sides blockIdx.y = 0 .. (b, x rhs-major) in one launch: rows by groups
+// ||b - A x||^2 and ||b||^2 of right-hand sides blockIdx.y = 0 .. (b, x rhs-major) in one launch: rows by groups
 // of kSpG lanes, per-CTA partials, the last CTA of a right-hand side adds them in order
-constexpr int kResidualCtas = 256;  // per right-hand side: dot_partial holds four times as many
+constexpr int kResidualCtas = 256;  // per right-hand side: dot_partial holds two sums of four
 __global__ void __launch_bounds__(256) k_true_residual(Topo tp, MatView<double> A, const double* __restrict__ b,
                                                        const double* __restrict__ x, double* __restrict__ partial,
                                                        unsigned int* __restrict__ ticket, double* __restrict__ out) {
-    __shared__ double smem[32];
+    __shared__ double smem[2 * 32];
     const size_t first = 3 * (size_t)tp.n * blockIdx.y;
     Operand<double, 1> op;
     op.a = x + first;
     op.b = nullptr;
     op.beta[0] = 0;
     constexpr int rows = 256 / kSpG;
-    double v[1] = {0.0};
+    double v[2] = {0.0, 0.0};
     for (int i0 = blockIdx.x * rows; i0 < tp.n; i0 += gridDim.x * rows) {  // CTA-uniform
         const int i = i0 + (int)threadIdx.x / kSpG, g = threadIdx.x % kSpG;
         double acc[1][3];
@@ -739,23 +739,26 @@ __global__ void __launch_bounds__(256) k_true_residual(Topo tp, MatView<double> 
         if (i < tp.n && g == 0)
 #pragma unroll
             for (int q = 0; q < 3; q++) {
-                const double r = b[first + 3 * (size_t)i + q] - acc[0][q];
+                const double bi = b[first + 3 * (size_t)i + q], r = bi - acc[0][q];
                 v[0] += r * r;
+                v[1] += bi * bi;
             }
     }
-    double tot[1];
-    if (grid_sum<1>(v, partial + blockIdx.y * kResidualCtas, ticket + blockIdx.y, tot, smem) && threadIdx.x == 0)
-        out[blockIdx.y] = tot[0];
+    double tot[2];
+    if (grid_sum<2>(v, partial + blockIdx.y * 2 * kResidualCtas, ticket + blockIdx.y, tot, smem) && threadIdx.x == 0) {
+        out[2 * blockIdx.y] = tot[0];
+        out[2 * blockIdx.y + 1] = tot[1];
+    }
 }
 
-// enqueue ||b - A x||^2 of nrhs <= 4 right-hand sides, on their way to h_pinned[0 ..]
+// enqueue ||b - A x||^2 and ||b||^2 of nrhs <= 4 right-hand sides, on their way to h_pinned[0 ..]
 static SgipcStatus enqueue_residuals(SgipcCtx* c, const double* b, const double* x, int nrhs, cudaStream_t s) {
     SG_COUNT(c, 1);
     const int grid = spmv_grid(c->n) < kResidualCtas ? spmv_grid(c->n) : kResidualCtas;
     k_true_residual<<<dim3(grid, nrhs), 256, 0, s>>>(topo_of(c), mat_view<double>(c), b, x, c->dot_partial,
                                                      c->dot_ticket, c->dot_out);
     SG_LAUNCH_CHECK(c, "true residual");
-    SG_CHECK(c, cudaMemcpyAsync(c->h_pinned, c->dot_out, nrhs * sizeof(double), cudaMemcpyDeviceToHost, s));
+    SG_CHECK(c, cudaMemcpyAsync(c->h_pinned, c->dot_out, 2 * nrhs * sizeof(double), cudaMemcpyDeviceToHost, s));
     return SGIPC_OK;
 }
 
@@ -802,7 +805,7 @@ static SgipcStatus solve_one(SgipcCtx* c, SgipcPrecision prec, SgipcCriterion cr
         out.refinements = 0;
         out.rz0 = hs.rz0;
         out.rz = hs.rz_next;
-        out.rel_residual = hs.bnorm2 > 0.0 ? sqrt(c->h_pinned[0] / hs.bnorm2) : 0.0;
+        out.rel_residual = c->h_pinned[1] > 0.0 ? sqrt(c->h_pinned[0] / c->h_pinned[1]) : 0.0;
         out.status = final_status(c, hs);
     } else {
         // mixed: FP32 MAS-PCG inner solves on the FP32 matrix copy, FP64 residual refinement
@@ -958,7 +961,7 @@ extern "C" SgipcStatus sgipc_pcg_solve_batched(SgipcCtx* c, SgipcPrecision prec,
             stats[r].rz0 = hs[r].rz0;
             stats[r].rz = hs[r].rz_next;
             stats[r].status = fs;
-            stats[r].rel_residual = hs[r].bnorm2 > 0.0 ? sqrt(c->h_pinned[r] / hs[r].bnorm2) : 0.0;
+            stats[r].rel_residual = c->h_pinned[2 * r + 1] > 0.0 ? sqrt(c->h_pinned[2 * r] / c->h_pinned[2 * r + 1]) : 0.0;
         }
         if (fs != SGIPC_OK) worst = (SgipcStatus)fs;
     }
