@@ -420,7 +420,6 @@ extern "C" SgipcStatus sgipc_global_pcg_solve(SgipcCtx* f, SgipcAbdCtx* a, Sgipc
         if ((st = grow(f, &a->g_vec, 5 * (size_t)g.N)) || (st = grow(f, &a->g_part, parts)) ||
             (st = grow(f, &a->g_dot, 32)))
             return st;
-        SG_CHECK(f, cudaMemset(a->g_dot, 0, sizeof(double) * 32));  // the ticket
         a->g_cap_vec = (size_t)g.N;
     }
     for (cudaEvent_t& e : a->g_ev)
@@ -450,6 +449,10 @@ extern "C" SgipcStatus sgipc_global_pcg_solve(SgipcCtx* f, SgipcAbdCtx* a, Sgipc
                  a->u_val};
     GState* hs = reinterpret_cast<GState*>(f->h_pinned + 40);  // [2], pinned
     static_assert(2 * sizeof(GState) <= 24 * sizeof(double) && sizeof(GState) <= 24 * sizeof(double), "state slots");
+    // state and ticket, in the caller's stream order (a plain cudaMemset runs on the default stream,
+    // which a side stream does not wait for), and for every solve: one that left early on an error
+    // leaves no ticket behind
+    SG_CHECK(f, cudaMemsetAsync(a->g_dot, 0, sizeof(double) * 32, g.s));
     SG_COUNT(f, 1);
     k_g_init<<<gb, kGThreads, 0, g.s>>>(g.N, g.st, b, x, r, g.part, g.ticket);
     if ((st = g_precond(g, r, z, true))) return st;
