@@ -454,6 +454,8 @@ __global__ void k_rhs(int nv, const double* __restrict__ fb, const double* __res
 // transpose).  Ground contacts and soft constraints ("singles") store their 3x3 block.
 constexpr int kFac = 16;
 constexpr int kMollBit = 1 << 30;  // in vertex 0 of a mollified pair's ids
+constexpr int kTwiceBit = 1 << 29;  // ... of a pair that names a vertex twice (a mesh has far fewer vertices)
+constexpr int kIdMask = ~(kMollBit | kTwiceBit);
 struct ContactStore {
     int4* ids;         // [pairs] vertices, -1 where a pair has fewer (all -1: no blocks)
     double* fac;       // [kFac * pairs]
@@ -485,7 +487,13 @@ __device__ __forceinline__ void store_ids(const ContactStore& cs, int item, int 
         id[a] = a < nvp ? v[a] : -1;
         k[a] = a < nvp ? (uint32_t)v[a] : (uint32_t)cs.n;
     }
+    bool twice = false;
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int b = a + 1; b < 4; b++) twice |= b < nvp && v[a] == v[b];
     if (moll && nvp > 0) id[0] |= kMollBit;
+    if (twice) id[0] |= kTwiceBit;
     cs.ids[item] = make_int4(id[0], id[1], id[2], id[3]);
     reinterpret_cast<uint4*>(cs.key)[item] = make_uint4(k[0], k[1], k[2], k[3]);
     const uint32_t o = 4u * (uint32_t)item;
@@ -506,7 +514,8 @@ __device__ __forceinline__ void store_single(const ContactStore& cs, int j, int 
 // Entry (p, q) of a pair's block at (row vertex a, column vertex b): the product is formed with
 // the pair's earlier vertex first, so that the blocks (a, b) and (b, a) are exact transposes.
 // f: the pair's factors, f2: the second line (mollified pairs).
-enum PairType { kPairBarrier = 0, kPairFriction = 1, kPairMollified = 2, kPairSingle = 3 };
+// kPairApart: added to the type of the rare pairs that the row sums take one after another.
+enum PairType { kPairBarrier = 0, kPairFriction = 1, kPairMollified = 2, kPairSingle = 3, kPairApart = 4 };
 __device__ __forceinline__ double pair_entry(int type, const double* f, const double* f2, int a, int b, int p, int q) {
     if (a > b) {
         const int t = a, u = p;
@@ -849,7 +858,7 @@ __global__ void __launch_bounds__(kConThreads) k_contacts(ContactLaunch L, doubl
                   : barrier_one(p, L.pairs, L.x, L.rest, L.dhat, L.kappa, cs, item0 + t, stage[t]);
     if (kGrad && on) {
         const int4 id = cs.ids[item0 + t];
-        const int v[4] = {id.x & ~kMollBit, id.y, id.z, id.w};
+        const int v[4] = {id.x & kIdMask, id.y, id.z, id.w};
         const int type = fric ? kPairFriction : ((id.x & kMollBit) ? kPairMollified : kPairBarrier);
         const double* f2 = type == kPairMollified ? cs.fac2 + kFac * (size_t)(item0 + t) : nullptr;
         for (int a = 0; a < 4; a++)
@@ -954,8 +963,9 @@ __device__ __forceinline__ int inc_pair(const RowArgs& a, uint32_t i, int (&v)[4
     item = (int)(i >> 2);
     local = (int)(i & 3u);
     const int4 id = __ldg(a.cs.ids + item);
-    v[0] = id.x & ~kMollBit, v[1] = id.y, v[2] = id.z, v[3] = id.w;
-    return item >= a.cs.barrier_pairs ? kPairFriction : ((id.x & kMollBit) ? kPairMollified : kPairBarrier);
+    v[0] = id.x & kIdMask, v[1] = id.y, v[2] = id.z, v[3] = id.w;
+    const int type = item >= a.cs.barrier_pairs ? kPairFriction : ((id.x & kMollBit) ? kPairMollified : kPairBarrier);
+    return (id.x & (kMollBit | kTwiceBit)) ? type | kPairApart : type;
 }
 
 // shared state of one row: a warp's, or (long rows) the CTA's, kept in the first warp's
@@ -1149,12 +1159,12 @@ __device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable&
         type = -1;
         if (inc == ~0u) return;
         type = inc_pair(a, inc, vert, pair, local);
-        if (type == kPairSingle || type == kPairMollified) return;
+        if (type == kPairSingle || (type & kPairApart)) return;
         const double2* src = reinterpret_cast<const double2*>(a.cs.fac + kFac * (size_t)pair);
 #pragma unroll
         for (int k = 0; k < 8; k++) f[k] = __ldg(src + k);
     };
-    bool moll = false;
+    bool apart = false;
     fetch(incidence(0));
     uint32_t inc_next = incidence(1);
     for (int t = 0; t < turns; t++) {
@@ -1199,13 +1209,12 @@ __device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable&
         }
 #pragma unroll
         for (int p = 0; p < 3; p++) L[15 + p] = first ? gr[p] : 0.0;
-        if (type == kPairMollified) moll = true;  // below
+        if (type >= 0 && (type & kPairApart)) apart = true;  // below
         else if (type >= 0)
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const int c = vert[k];
-                // (a vertex named twice by a pair: its block is counted in the pair's order only)
-                if (c < lo || c >= hi || (c == v && k < local)) continue;
+                if (c < lo || c >= hi) continue;
                 unsigned x = ((unsigned)c * 2654435761u) >> 24;
                 while (T.hash[x] != c) x = (x + 1) & (kRowHash - 1);
                 u[k] = T.rank[x];
@@ -1248,25 +1257,35 @@ __device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable&
             }
         }
     }
-    // mollified pairs (none come from the pair search), one after another
-    if (__any_sync(0xffffffffu, moll)) {
+    // Mollified pairs and pairs that name a vertex twice (none come from the pair search), one
+    // after another.  Two equal vertices of a pair have one column, so the blocks of a row are added
+    // vertex by vertex; the row of such a vertex meets the pair once for each of its places, which
+    // gives all four of the vertex's blocks.
+    if (__any_sync(0xffffffffu, apart)) {
         for (int i = i0 + hw; i - hw < i1; i += nh) {  // the same turns in both halves
-            int w[4], item, la, ty = -1;
+            int w[4], item = 0, la = 0, ty = -1, d = -1;
+            double x[3] = {0.0, 0.0, 0.0};
             if (i < i1) ty = inc_pair(a, __ldg(a.inc + i), w, item, la);
-            if (ty == kPairMollified && hl < 15) {
+            if (ty >= 0 && (ty & kPairApart) && hl < 15) {
+                const int base = ty & ~kPairApart;
                 const double *m = a.cs.fac + kFac * (size_t)item, *m2 = a.cs.fac2 + kFac * (size_t)item;
                 const int c = w[b];
                 if (grad) {
-                    if (first) g += pair_grad(ty, m, m2, la, q);
-                } else if (c >= lo && c < hi && !(c == v && b < la)) {
-                    unsigned x = ((unsigned)c * 2654435761u) >> 24;
-                    while (T.hash[x] != c) x = (x + 1) & (kRowHash - 1);
-                    double* o = acc + 9 * T.rank[x] + q;
+                    if (first) g += pair_grad(base, m, m2, la, q);
+                } else if (c >= lo && c < hi) {
+                    unsigned s = ((unsigned)c * 2654435761u) >> 24;
+                    while (T.hash[s] != c) s = (s + 1) & (kRowHash - 1);
+                    d = 9 * T.rank[s] + q;
 #pragma unroll
-                    for (int p = 0; p < 3; p++) o[3 * p] += pair_entry(ty, m, m2, la, b, p, q);
+                    for (int p = 0; p < 3; p++) x[p] = pair_entry(base, m, m2, la, b, p, q);
                 }
             }
-            __syncwarp();
+            for (int turn = 0; turn < 4; turn++) {
+                if (d >= 0 && b == turn)
+#pragma unroll
+                    for (int p = 0; p < 3; p++) acc[d + 3 * p] += x[p];
+                __syncwarp();
+            }
         }
     }
     __syncwarp();
@@ -1949,7 +1968,7 @@ __device__ __forceinline__ bool part_slot(const ContactStore& cs, int singles, i
     a = k < 4 ? 0 : (k < 7 ? 1 : (k < 9 ? 2 : 3));
     b = k < 4 ? k : (k < 7 ? k - 3 : (k < 9 ? k - 5 : 3));
     const int4 id = cs.ids[item];
-    const int v[4] = {id.x < 0 ? -1 : id.x & ~kMollBit, id.y, id.z, id.w};
+    const int v[4] = {id.x < 0 ? -1 : id.x & kIdMask, id.y, id.z, id.w};
     r = v[a], c = v[b];
     if (r < 0 || c < 0) return false;
     if (r > c) {

@@ -76,3 +76,39 @@ def test_rows_match_the_oracle(columns, repeats, mollified):
     g.computeGradientAndHessian()
     assert np.array_equal(g.export_bcoo()[2], vals)
     g.close()
+
+
+@pytest.mark.parametrize("copies", [1, 40])
+def test_pairs_that_name_a_vertex_twice(copies):
+    """Every way in which two places of a pair can hold one vertex: all of its blocks count, as in the
+    oracle (friction pairs: a barrier pair of that kind is at distance zero).  40 copies of each
+    give the rows of a CTA.  Tolerance as above."""
+    rng = np.random.default_rng(copies)
+    sc = scenes.scene_two_cubes(5, seed=4)
+    shapes = [(0, 0), (0, 1), (0, 0, 1), (0, 1, 0), (1, 0, 0), (0, 1, 1), (0, 0, 0),
+              (0, 0, 1, 2), (0, 1, 0, 2), (0, 1, 2, 0), (1, 0, 0, 2), (1, 0, 2, 0), (1, 2, 0, 0),
+              (0, 0, 1, 1), (0, 1, 0, 1), (0, 1, 1, 0), (0, 0, 0, 1), (1, 0, 0, 0), (0, 1, 2, 3)]
+    fp = []
+    for _ in range(copies):
+        v = rng.choice(12, 4, replace=False)
+        for s in shapes:
+            u = [int(v[k]) for k in s]
+            fp.append([-u[0] - 1] + u[1:] + [-1] * (4 - len(u)))
+            if len(u) == 4:
+                fp.append(u)
+    fp = np.asarray(fp, np.int32)[rng.permutation(len(fp))]
+    sc = dataclasses.replace(sc, pairs=np.zeros((0, 4), np.int32), fric_pairs=fp,
+                             fric_lambda=rng.uniform(0.5, 2.0, len(fp)), fric_coord=rng.uniform(0.1, 0.4, (len(fp), 2)),
+                             fric_basis=np.linalg.qr(rng.normal(size=(len(fp), 3, 2)))[0],
+                             o_vertexes=sc.vertexes + rng.uniform(-1e-3, 1e-3, sc.vertexes.shape))
+    g = system.GIPC(sc)
+    g.computeGradientAndHessian()
+    rows, cols, vals = g.export_bcoo()
+    b, orow, ocol, oval, _ = oracle.assemble(sc)
+    assert np.array_equal(rows, orow) and np.array_equal(cols, ocol)
+    assert np.abs(vals - oval).max() <= 1e-9 * np.abs(oval).max()
+    assert np.abs(g.rhs().cpu().numpy() - b).max() <= 1e-9 * np.abs(b).max()
+    x = rng.normal(size=3 * sc.nv)
+    ref = oracle.spmv(orow, ocol, oval, sc.nv, x)
+    assert np.abs(g.spmv(torch.tensor(x, device="cuda")).cpu().numpy() - ref).max() <= 1e-9 * np.abs(ref).max()
+    g.close()
