@@ -888,7 +888,7 @@ __global__ void k_soft(int ns, const uint32_t* __restrict__ idx, const double* _
 // ---- contact rows ---------------------------------------------------------------------------
 // After the incidences are sorted by vertex (stable: each vertex's list is in pair order), row v
 // of the contact matrix is made from v's list alone: every pair in it gives the blocks (v, w) of
-// its vertices w.  One warp takes a row of up to kRowLong incidences, a CTA a longer one.  The
+// its vertices w >= v, and the columns w < v, whose blocks are copied from row w.  One warp takes a row of up to kRowLong incidences, a CTA a longer one.  The
 // distinct columns go into a small hash table in shared memory and are ranked; the blocks are
 // added up in shared memory, pair by pair in the list's order (each half-warp its share, the
 // shares' sums in order): the same result on every run.  A row of more columns than the
@@ -1109,8 +1109,6 @@ struct RowOut {
     double* u64;
     float* u32;
     int* cl_col;
-    double* l64;
-    float* l32;
     double* grad;
 };
 
@@ -1123,8 +1121,7 @@ struct RowOut {
 // per entry, each kind its own code: 1557 us; two lanes a pair staging, in place: 1516, pipelined:
 // 1187.)
 // A staged line: barrier [0..2] g_v, [3..14] g, friction [0..8] W, [9..12] c_v c, single [0..8] its
-// block, [9..12] 1; [15..17] the pair's gradient at v, [18] 1, [19] lam or 1.  Each product is the
-// same for the transposed block.
+// block, [9..12] 1; [15..17] the pair's gradient at v, [18] 1, [19] lam or 1.
 constexpr int kLine = 21;  // odd: the two halves' lines start in different banks
 struct RowWarp {
     double acc[2][kRowCols * 9];
@@ -1214,7 +1211,7 @@ __device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable&
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const int c = vert[k];
-                if (c < lo || c >= hi) continue;
+                if (c < max(lo, v) || c >= hi) continue;  // upper blocks only
                 unsigned x = ((unsigned)c * 2654435761u) >> 24;
                 while (T.hash[x] != c) x = (x + 1) & (kRowHash - 1);
                 u[k] = T.rank[x];
@@ -1272,7 +1269,7 @@ __device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable&
                 const int c = w[b];
                 if (grad) {
                     if (first) g += pair_grad(base, m, m2, la, q);
-                } else if (c >= lo && c < hi) {
+                } else if (c >= max(lo, v) && c < hi) {
                     unsigned s = ((unsigned)c * 2654435761u) >> 24;
                     while (T.hash[s] != c) s = (s + 1) & (kRowHash - 1);
                     d = 9 * T.rank[s] + q;
@@ -1291,33 +1288,28 @@ __device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable&
     __syncwarp();
 }
 
-// stores the window's blocks (threads t of nt), acc summed over the row's warps in order
+// stores the window's upper blocks (threads t of nt), acc summed over the row's warps in order, and
+// the columns of both lists
 template <bool kCta>
 __device__ __forceinline__ void row_store(const RowArgs& a, const RowOut& o, const RowTable& T, const RowWarp* W, int v,
                                           int U, int t, int nt, unsigned& up, unsigned& low) {
     int nlow = 0;
     for (int k = 0; k < U; k++) nlow += T.col[k] < v;
+    for (int u = t; u < nlow; u += nt) o.cl_col[low + u] = T.col[u];
     const bool fixed_row = o.btype && o.btype[v] != 0;
-    for (int e = t; e < 9 * U; e += nt) {
+    for (int e = 9 * nlow + t; e < 9 * U; e += nt) {
         const int u = e / 9, q = e % 9, c = T.col[u];
         double s = W[0].acc[0][e] + W[0].acc[1][e];
         if (kCta)
 #pragma unroll
             for (int w = 1; w < kRowWarps; w++) s = s + W[w].acc[0][e] + W[w].acc[1][e];
         if (fixed_row || (o.btype && o.btype[c] != 0)) s = 0.0;
-        if (c < v) {
-            const size_t k = low + u;
-            o.l64[9 * k + q] = s;
-            o.l32[9 * k + q] = (float)s;
-            if (q == 0) o.cl_col[k] = c;
-        } else {
-            const size_t k = up + (u - nlow);
-            o.u64[9 * k + q] = s;
-            o.u32[9 * k + q] = (float)s;
-            if (q == 0) {
-                o.uc_row[k] = v;
-                o.uc_col[k] = c;
-            }
+        const size_t k = up + (u - nlow);
+        o.u64[9 * k + q] = s;
+        o.u32[9 * k + q] = (float)s;
+        if (q == 0) {
+            o.uc_row[k] = v;
+            o.uc_col[k] = c;
         }
     }
     up += U - nlow;
@@ -1393,6 +1385,46 @@ __global__ void __launch_bounds__(32 * kRowWarps, kRowCtas) k_row_sums(RowArgs a
             g += __shfl_down_sync(0xffffffffu, g, 16);  // the halves in list order
             if (lane >= 12 && lane < 15) o.grad[3 * (size_t)v + lane - 12] += g;
         });
+}
+
+// The transposed copies: block u = (r, c), r < c, goes to the place of column r in c's list.  A copy,
+// not a second sum over c's list, whose pairs are shared out differently: the matrix stays exactly
+// symmetric (the solve's p.Ap recurrence takes it so), in FP64 and in FP32.  A warp finds the places
+// of 32 blocks, one a lane, and then moves their 288 entries with whole lines on the reading side.
+__global__ void __launch_bounds__(SGIPC_BLOCK) k_row_transposes(const int* __restrict__ nuc,
+                                                                const int* __restrict__ uc_row,
+                                                                const int* __restrict__ uc_col,
+                                                                const double* __restrict__ u64,
+                                                                const float* __restrict__ u32,
+                                                                const int* __restrict__ cl_ptr,
+                                                                const int* __restrict__ cl_col,
+                                                                double* __restrict__ l64, float* __restrict__ l32) {
+    const int nu = nuc[0], lane = threadIdx.x & 31;
+    const int step = (gridDim.x * blockDim.x) & ~31;
+    for (int u0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; u0 < nu; u0 += step) {  // warp-uniform
+        int k = -1;
+        if (u0 + lane < nu) {
+            const int r = uc_row[u0 + lane], c = uc_col[u0 + lane];
+            if (r < c) {
+                k = cl_ptr[c];
+                int hi = cl_ptr[c + 1];
+                while (k < hi) {  // first place whose column is not below r: r is in the list
+                    const int mid = (k + hi) >> 1;
+                    if (__ldg(cl_col + mid) < r) k = mid + 1;
+                    else hi = mid;
+                }
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 9; t++) {
+            const int e = 32 * t + lane, q = e % 9;
+            const int at = __shfl_sync(0xffffffffu, k, e / 9);
+            if (at < 0) continue;
+            const size_t to = 9 * (size_t)at + 3 * (q % 3) + q / 3;
+            l64[to] = u64[9 * (size_t)u0 + e];
+            l32[to] = u32[9 * (size_t)u0 + e];
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1790,7 +1822,7 @@ static SgipcStatus merge_contacts(SgipcCtx* c, const ContactCounts& cc, int sing
         SG_CHECK(c, cudaMemsetAsync(c->cl_ptr, 0, sizeof(int) * (n + 1), s));
         return SGIPC_OK;
     }
-    SG_COUNT(c, 3);
+    SG_COUNT(c, 4);
     SG_CHECK(c, cudaMemsetAsync(c->row_cnt, 0, 2 * sizeof(int), s));
     size_t tb = c->cub_tmp_bytes;
     SG_CHECK(c, cub::DeviceRadixSort::SortPairs(c->cub_tmp, tb, c->con_key, c->con_key_s, c->con_val, c->con_val_s, m,
@@ -1803,9 +1835,12 @@ static SgipcStatus merge_contacts(SgipcCtx* c, const ContactCounts& cc, int sing
     tb = c->cub_tmp_bytes;
     SG_CHECK(c, cub::DeviceScan::ExclusiveSum(c->cub_tmp, tb, c->ucnt, c->uoff, n + 1, s));
     const RowOut o{c->uoff, btype, c->nuc, c->cu_ptr, c->cl_ptr, c->uc_row, c->uc_col, c->uc64, c->uc32, c->cl_col,
-                   c->cl64, c->cl32, grad};
+                   grad};
     SG_CHECK(c, cudaFuncSetAttribute(k_row_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowShared));
     k_row_sums<<<std::min(std::max(most, 148), 148 * kRowCtas), 32 * kRowWarps, kRowShared, s>>>(a, o);
+    // (no pair has more than six blocks off the diagonal)
+    k_row_transposes<<<std::min(nblk(6LL * cc.pairs() + 1), 148 * 8), SGIPC_BLOCK, 0, s>>>(
+        c->nuc, c->uc_row, c->uc_col, c->uc64, c->uc32, c->cl_ptr, c->cl_col, c->cl64, c->cl32);
     SG_LAUNCH_CHECK(c, "contact rows");
     return SGIPC_OK;
 }

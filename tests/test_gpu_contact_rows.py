@@ -112,3 +112,26 @@ def test_pairs_that_name_a_vertex_twice(copies):
     ref = oracle.spmv(orow, ocol, oval, sc.nv, x)
     assert np.abs(g.spmv(torch.tensor(x, device="cuda")).cpu().numpy() - ref).max() <= 1e-9 * np.abs(ref).max()
     g.close()
+
+
+def test_transposed_blocks_are_exact_copies():
+    """Off the diagonal A e_j read at row i equals A e_i read at row j to the last bit, for rows of warps
+    and of CTAs (a product with a unit vector adds one static and one contact entry to zeros)."""
+    rng = np.random.default_rng(5)
+    sc = scenes.scene_two_cubes(6, seed=4)
+    hub = int(rng.integers(sc.nv))
+    pairs = _pairs(rng, sc.nv, hub, 60, 150, True)
+    fp = pairs[rng.permutation(len(pairs))[:len(pairs) // 2]]
+    sc = dataclasses.replace(sc, pairs=pairs, fric_pairs=fp, fric_lambda=rng.uniform(0.5, 2.0, len(fp)),
+                             fric_coord=rng.uniform(0.1, 0.4, (len(fp), 2)),
+                             fric_basis=np.linalg.qr(rng.normal(size=(len(fp), 3, 2)))[0],
+                             params=dict(sc.params, dHat=0.2, kappa=1.0),
+                             o_vertexes=sc.vertexes + rng.uniform(-1e-3, 1e-3, sc.vertexes.shape))
+    g = system.GIPC(sc)
+    g.computeGradientAndHessian()
+    e = torch.eye(3 * sc.nv, dtype=torch.float64, device="cuda")
+    A = torch.stack([g.spmv(e[k]) for k in range(3 * sc.nv)])
+    block = torch.arange(3 * sc.nv, device="cuda") // 3
+    off = block[:, None] != block
+    assert torch.equal(A[off], A.T[off])
+    g.close()
