@@ -888,11 +888,13 @@ __global__ void k_soft(int ns, const uint32_t* __restrict__ idx, const double* _
 // ---- contact rows ---------------------------------------------------------------------------
 // After the incidences are sorted by vertex (stable: each vertex's list is in pair order), row v
 // of the contact matrix is made from v's list alone: every pair in it gives the blocks (v, w) of
-// its vertices w >= v, and the columns w < v, whose blocks are copied from row w.  One warp takes a row of up to kRowLong incidences, a CTA a longer one.  The
-// distinct columns go into a small hash table in shared memory and are ranked; the blocks are
-// added up in shared memory, pair by pair in the list's order (each half-warp its share, the
-// shares' sums in order): the same result on every run.  A row of more columns than the
-// table holds is made in windows of columns.
+// its vertices w >= v, and the columns w < v, whose blocks are copied from row w.  One warp takes a
+// row of up to kRowLong incidences, a CTA a longer one.  The distinct columns go into a small hash
+// table in shared memory and are ranked; the blocks are added up in shared memory, pair by pair in
+// the list's order (each half-warp its share, the shares' sums in order): the same result on every
+// run.  A row of more columns than the table holds (a corner of a large triangle under a fine
+// cloth) is split into windows of kRowCols columns, each with the list of the pairs that have one
+// there, and the windows are summed as rows are: the work stays in proportion to the list.
 constexpr int kRowWarps = 4;
 // incidences above which a CTA takes the row (rolled cloth, a third of whose rows are longer: the
 // Newton system takes 8 % longer with 64, 5 % with 413, where k_row_counts goes from 159 to 352 us)
@@ -942,13 +944,30 @@ __global__ void k_inc_rows(int n, int m, const uint32_t* __restrict__ ks, int* _
     }
 }
 
+// numbers of: rows with short and with long lists, rows to split; places of the split's scratch in
+// use; windows with short and with long lists; next short list to be summed
+enum RowCount { kRowsShort = 0, kRowsLong = 1, kRowsSplit = 2, kSplitCols = 3, kSplitList = 4, kWinShort = 5,
+                kWinLong = 6, kRowNext = 7, kRowCounts = 8 };
+
+// a window of a split row: kRowCols columns of it from the diagonal on, and their pairs
+struct RowWindow {
+    int v;
+    int i0, len;    // list: of the whole row (first = 0) or in RowArgs::wlist
+    int c0, cols;   // columns, in RowArgs::wcol
+    int first;      // their first one's place among the row's upper blocks
+};
+
 struct RowArgs {
     ContactStore cs;
     const uint32_t* inc;   // sorted incidences
     const int* ptr;
-    const int* list;
-    const int* cnt;
+    int* list;             // [3n] rows with short lists, with long ones (~v: split), rows to split
+    int* cnt;              // [kRowCounts]
     int n;
+    int* wcol;             // [4 * incidences] sorted columns of the split rows
+    uint32_t* wlist;       // [3 * incidences] lists of their windows
+    RowWindow* win;        // [win_cap] windows: short lists from the front, long ones from the back
+    int win_cap;
 };
 
 // the vertices of incidence i's pair (a single's vertex alone); returns its type
@@ -984,15 +1003,15 @@ __device__ __forceinline__ void row_sync() {
     else __syncwarp();
 }
 
-// The distinct columns of the row in [lo, hi) into the table; false: more than kRowCols of them.
+// The distinct columns of the row into the table; false: more than kRowCols of them.
 // t: this thread's index among the nt of its row.
 template <bool kCta>
-__device__ __forceinline__ bool row_columns(const RowArgs& a, RowTable& T, int i0, int i1, int lo, int hi, int t, int nt) {
+__device__ __forceinline__ bool row_columns(const RowArgs& a, RowTable& T, int i0, int i1, int t, int nt) {
     for (int k = t; k < kRowHash; k += nt) T.hash[k] = -1;
     if (t == 0) T.used = T.over = 0;
     row_sync<kCta>();
     constexpr int kU = 4;  // pairs in flight
-    for (int k0 = i0 + t; k0 < i1; k0 += kU * nt) {
+    for (int k0 = i0 + t; k0 < i1 && !*(volatile int*)&T.over; k0 += kU * nt) {
         uint32_t inc[kU];
         int v[kU][4];
 #pragma unroll
@@ -1006,13 +1025,13 @@ __device__ __forceinline__ bool row_columns(const RowArgs& a, RowTable& T, int i
 #pragma unroll
         for (int e = 0; e < 4 * kU; e++) {
             const int c = v[e / 4][e % 4];
-            if (c < lo || c >= hi) continue;  // (-1 is below every window)
+            if (c < 0) continue;
             unsigned h = ((unsigned)c * 2654435761u) >> 24;
             for (;;) {
                 const int seen = *(volatile int*)&T.hash[h];
                 if (seen == c) break;
                 if (seen < 0) {
-                    if (*(volatile int*)&T.used > kRowCols) {  // full: the caller takes a smaller window
+                    if (*(volatile int*)&T.used > kRowCols) {  // full
                         T.over = 1;
                         break;
                     }
@@ -1050,52 +1069,224 @@ __device__ __forceinline__ void row_ranks(RowTable& T, int t, int nt) {
     row_sync<kCta>();
 }
 
-// calls fn() with each window's columns in the table, windows in column order
-template <bool kCta, class Fn>
-__device__ __forceinline__ void row_windows(const RowArgs& a, RowTable& T, int i0, int i1, int t, int nt, Fn fn) {
-    int lo = 0, hi = a.n;
-    while (lo < a.n) {  // uniform over the row's threads
-        if (!row_columns<kCta>(a, T, i0, i1, lo, hi, t, nt)) {
-            hi = lo + (hi - lo + 1) / 2;  // a window of one column always fits
-            continue;
-        }
-        fn();
-        row_sync<kCta>();
-        lo = hi;
-        hi = a.n;
+// the table of a window: its columns are known and sorted
+template <bool kCta>
+__device__ __forceinline__ void window_table(const RowArgs& a, RowTable& T, int c0, int cols, int t, int nt) {
+    for (int k = t; k < kRowHash; k += nt) T.hash[k] = -1;
+    if (t == 0) T.used = cols;
+    row_sync<kCta>();
+    for (int k = t; k < cols; k += nt) {
+        const int c = a.wcol[c0 + k];
+        unsigned h = ((unsigned)c * 2654435761u) >> 24;
+        while (atomicCAS(&T.hash[h], -1, c) != -1) h = (h + 1) & (kRowHash - 1);
+        T.rank[h] = (unsigned char)k;
+        T.col[k] = c;
     }
+    row_sync<kCta>();
 }
 
-// rows of the grid's share: long ones by CTA, short ones by warp; fn(v, t, nt, table, cta flag)
-template <class Long, class Short>
-__device__ __forceinline__ void for_rows(const RowArgs& a, Long f_long, Short f_short) {
-    const int n_short = a.cnt[0], n_long = a.cnt[1];
-    for (int k = blockIdx.x; k < n_long; k += gridDim.x) f_long(a.list[(size_t)a.n + k]);
-    __syncthreads();
-    const int nw = gridDim.x * kRowWarps;
-    // (counted from the last CTA: the first ones may have taken a long row more)
-    for (int k = (gridDim.x - 1 - blockIdx.x) * kRowWarps + (threadIdx.x >> 5); k < n_short; k += nw)
-        f_short(a.list[k]);
-}
-
-// unique blocks of every row: upper ones (column >= row) and transposed ones (<< 32)
+// unique blocks of every row: upper ones (column >= row) and transposed ones (<< 32); rows that the
+// table does not hold are listed for k_row_split
 __global__ void __launch_bounds__(32 * kRowWarps) k_row_counts(RowArgs a, unsigned long long* __restrict__ ucnt) {
     __shared__ RowTable tables[kRowWarps];
-    auto count = [&](auto cta, int v, RowTable& T, int t, int nt) {
-        unsigned up = 0, low = 0;  // of this thread's share of the columns
-        row_windows<decltype(cta)::value>(a, T, a.ptr[v], a.ptr[v + 1], t, nt, [&]() {
-            for (int k = t; k < T.used; k += nt) {
-                if (T.found[k] >= v) up++;
-                else low++;
+    auto count = [&](auto cta, int* entry, RowTable& T, int t, int nt) {
+        const int v = *entry;
+        if (!row_columns<decltype(cta)::value>(a, T, a.ptr[v], a.ptr[v + 1], t, nt)) {
+            if (t == 0) {
+                *entry = ~v;
+                a.list[2 * (size_t)a.n + atomicAdd(a.cnt + kRowsSplit, 1)] = v;
             }
-        });
+            return;
+        }
+        unsigned up = 0, low = 0;  // of this thread's share of the columns
+        for (int k = t; k < T.used; k += nt) {
+            if (T.found[k] >= v) up++;
+            else low++;
+        }
         up = __reduce_add_sync(0xffffffffu, up);
         low = __reduce_add_sync(0xffffffffu, low);
         if ((threadIdx.x & 31) == 0 && (up | low)) atomicAdd(ucnt + v, (unsigned long long)up | ((unsigned long long)low << 32));
+        row_sync<decltype(cta)::value>();
     };
-    for_rows(
-        a, [&](int v) { count(std::true_type{}, v, tables[0], threadIdx.x, 32 * kRowWarps); },
-        [&](int v) { count(std::false_type{}, v, tables[threadIdx.x >> 5], threadIdx.x & 31, 32); });
+    const int n_short = a.cnt[kRowsShort], n_long = a.cnt[kRowsLong];
+    for (int k = blockIdx.x; k < n_long; k += gridDim.x)
+        count(std::true_type{}, a.list + (size_t)a.n + k, tables[0], threadIdx.x, 32 * kRowWarps);
+    __syncthreads();
+    // (counted from the last CTA: the first ones may have taken a long row more)
+    for (int k = (gridDim.x - 1 - blockIdx.x) * kRowWarps + (threadIdx.x >> 5); k < n_short; k += gridDim.x * kRowWarps)
+        count(std::false_type{}, a.list + k, tables[threadIdx.x >> 5], threadIdx.x & 31, 32);
+}
+
+// Rows of more than kRowCols columns, a CTA each: their sorted distinct columns by a bitmap of the
+// vertices, their block counts, and windows of kRowCols upper columns with the lists of the pairs that
+// have a column there.  The first window starts at the diagonal, which every pair has: its list is the
+// row's.  The others' lists are a stable split of it: each warp counts, and then places, its own part
+// of the list in order.  Three passes over the list whatever its columns, bound by the latency of its
+// gathers: 24 us for a row of 1000 pairs and columns, 110 us for 5000, 340 us for 20 000, with 45, 147
+// and 470 us of k_row_sums; the whole assembly of a 31^3 cube with such a row 270, 495 and 1087 us, and
+// 317, 506 and 1139 us when the pairs' blocks were sorted.  (Windows found by halving from all columns, each
+// attempt and each sum reading the whole list, made it 3.0, 136 and 3491 ms.)
+constexpr int kSplitWarps = 8;
+constexpr int kSplitSpan = 1 << 18;  // columns of the bitmap (32 KB); a larger mesh takes several
+constexpr int kSplitWin = 896;       // windows listed at a time: kSplitWarps counts each and their first columns
+static_assert((kSplitWarps + 1) * kSplitWin <= kSplitSpan / 32 && kSplitWin <= 4 * 32 * kSplitWarps, "shared memory");
+
+__global__ void __launch_bounds__(32 * kSplitWarps) k_row_split(RowArgs a, unsigned long long* __restrict__ ucnt) {
+    __shared__ unsigned s_mem[kSplitSpan / 32];  // bitmap, then the windows' first columns and counts
+    __shared__ int s_sum[kSplitWarps];
+    __shared__ int s_base, s_low, s_list;
+    const int t = threadIdx.x, nt = 32 * kSplitWarps, w = t >> 5, lane = t & 31;
+    // exclusive sum over the CTA in thread order, and the total
+    auto scan = [&](int x, int& total) -> int {
+        int in = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, in, o);
+            if (lane >= o) in += y;
+        }
+        __syncthreads();  // s_sum is free
+        if (lane == 31) s_sum[w] = in;
+        __syncthreads();
+        int before = 0;
+        total = 0;
+#pragma unroll
+        for (int k = 0; k < kSplitWarps; k++) {
+            if (k < w) before += s_sum[k];
+            total += s_sum[k];
+        }
+        return before + in - x;
+    };
+    auto put = [&](const RowWindow& x) {
+        if (x.len > kRowLong) a.win[a.win_cap - 1 - atomicAdd(a.cnt + kWinLong, 1)] = x;
+        else a.win[atomicAdd(a.cnt + kWinShort, 1)] = x;
+    };
+    const int rows = a.cnt[kRowsSplit];
+    for (int row = blockIdx.x; row < rows; row += gridDim.x) {  // CTA-uniform
+        const int v = a.list[2 * (size_t)a.n + row], i0 = a.ptr[v], i1 = a.ptr[v + 1], len = i1 - i0;
+        if (t == 0) s_base = atomicAdd(a.cnt + kSplitCols, 3 * len + 1);  // a pair has three other vertices
+        int cols = 0;
+        for (int s0 = 0; s0 < a.n; s0 += kSplitSpan) {
+            const int span = min(kSplitSpan, a.n - s0), words = (span + 31) >> 5;
+            __syncthreads();
+            for (int k = t; k < words; k += nt) s_mem[k] = 0u;
+            __syncthreads();
+            for (int k0 = i0 + t; k0 < i1; k0 += 4 * nt) {
+                uint32_t inc[4];
+                int id[4][4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) inc[u] = k0 + u * nt < i1 ? __ldg(a.inc + k0 + u * nt) : ~0u;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    int item, local;
+                    if (inc[u] != ~0u) inc_pair(a, inc[u], id[u], item, local);
+                    else id[u][0] = id[u][1] = id[u][2] = id[u][3] = -1;
+                }
+#pragma unroll
+                for (int e = 0; e < 16; e++) {
+                    const int c = id[e / 4][e % 4] - s0;
+                    if (c < 0 || c >= span) continue;  // (-1 too)
+                    const unsigned bit = 1u << (c & 31);
+                    if (!(*(volatile unsigned*)&s_mem[c >> 5] & bit)) atomicOr(&s_mem[c >> 5], bit);
+                }
+            }
+            __syncthreads();
+            for (int k0 = 0; k0 < words; k0 += nt) {  // CTA-uniform
+                unsigned m = k0 + t < words ? s_mem[k0 + t] : 0u;
+                int total, at = cols + scan(__popc(m), total);
+                for (; m; m &= m - 1, at++) {
+                    const int c = s0 + 32 * (k0 + t) + __ffs(m) - 1;
+                    a.wcol[s_base + at] = c;
+                    if (c == v) s_low = at;
+                }
+                cols += total;
+            }
+        }
+        __syncthreads();
+        const int low = s_low, up = cols - low, c0 = s_base + low, nwin = (up + kRowCols - 1) / kRowCols;
+        if (t == 0) {
+            ucnt[v] = (unsigned long long)(unsigned)up | ((unsigned long long)(unsigned)low << 32);
+            put({v, i0, len, c0, min(kRowCols, up), 0});
+        }
+        int* first = reinterpret_cast<int*>(s_mem);  // a window's first column
+        int* count = first + kSplitWin;              // [kSplitWarps][kSplitWin]
+        const int part = ((len + kSplitWarps - 1) / kSplitWarps + 31) & ~31;
+        const int b0 = i0 + w * part, b1 = min(i1, b0 + part);
+        for (int w0 = 1; w0 < nwin; w0 += kSplitWin) {  // CTA-uniform
+            const int nw = min(kSplitWin, nwin - w0);
+            __syncthreads();
+            for (int k = t; k < nw; k += nt) first[k] = a.wcol[c0 + kRowCols * (w0 + k)];
+            for (int k = t; k < kSplitWarps * kSplitWin; k += nt) count[k] = 0;
+            const int end = w0 + nw < nwin ? a.wcol[c0 + kRowCols * (w0 + nw)] : a.n;
+            __syncthreads();
+            // the windows (of these nw) of incidence i's pair, each once, -1: none
+            auto windows = [&](uint32_t i, int (&id)[4]) {
+                int item, local;
+                if (i != ~0u) inc_pair(a, i, id, item, local);
+                else id[0] = id[1] = id[2] = id[3] = -1;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int c = id[k];
+                    int lo = -1;
+                    if (c >= first[0] && c < end) {
+                        lo = 0;  // last window whose first column is not above c
+                        for (int hi = nw; hi - lo > 1;) {
+                            const int mid = (lo + hi) >> 1;
+                            if (first[mid] <= c) lo = mid;
+                            else hi = mid;
+                        }
+                    }
+                    id[k] = lo;
+                }
+#pragma unroll
+                for (int k = 1; k < 4; k++)
+#pragma unroll
+                    for (int j = 0; j < k; j++)
+                        if (id[k] == id[j]) id[k] = -1;
+            };
+            for (int i = b0 + lane; i < b1; i += 32) {
+                int id[4];
+                windows(__ldg(a.inc + i), id);
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (id[k] >= 0) atomicAdd(count + w * kSplitWin + id[k], 1);
+            }
+            __syncthreads();
+            // places: window by window, warp by warp; a thread's four windows are neighbours
+            int sum = 0, total;
+            for (int k = 4 * t; k < min(4 * t + 4, nw); k++)
+                for (int j = 0; j < kSplitWarps; j++) sum += count[j * kSplitWin + k];
+            int at = scan(sum, total);
+            if (t == 0) s_list = atomicAdd(a.cnt + kSplitList, total);
+            __syncthreads();
+            for (int k = 4 * t; k < min(4 * t + 4, nw); k++) {
+                const int start = at;
+                for (int j = 0; j < kSplitWarps; j++) {
+                    const int c = count[j * kSplitWin + k];
+                    count[j * kSplitWin + k] = at;
+                    at += c;
+                }
+                const int f = kRowCols * (w0 + k);
+                put({v, s_list + start, at - start, c0 + f, min(kRowCols, up - f), f});
+            }
+            __syncthreads();
+            uint32_t* out = a.wlist + s_list;
+            for (int i = b0; i < b1; i += 32) {  // warp-uniform
+                const uint32_t inc = i + lane < b1 ? __ldg(a.inc + i + lane) : ~0u;
+                int id[4];
+                windows(inc, id);
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const unsigned same = __match_any_sync(0xffffffffu, id[k]);
+                    int* c = count + w * kSplitWin + id[k];
+                    if (id[k] >= 0) out[*c + __popc(same & ((1u << lane) - 1u))] = inc;
+                    __syncwarp();
+                    if (id[k] >= 0 && lane == __ffs(same) - 1) *c += __popc(same);
+                    __syncwarp();
+                }
+            }
+        }
+        __syncthreads();
+    }
 }
 
 struct RowOut {
@@ -1131,9 +1322,11 @@ struct RowWarp {
 };
 constexpr size_t kRowShared = sizeof(RowTable) * kRowWarps + sizeof(RowWarp) * kRowWarps;
 
-// half-warp hw of nh over the list [i0, i1): its acc (zeroed) and, in the first window, g
-__device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable& T, RowWarp& W, int v, int U, int i0,
-                                               int i1, int hw, int nh, int lo, int hi, bool first, double& g) {
+// half-warp hw of nh over list[i0, i1): its acc (zeroed) of the columns in [lo, hi), and g, the gradient
+// (first: in the window of the diagonal, whose list is the whole row's)
+__device__ __forceinline__ void row_accumulate(const RowArgs& a, const uint32_t* __restrict__ list, const RowTable& T,
+                                               RowWarp& W, int v, int U, int i0, int i1, int hw, int nh, int lo,
+                                               int hi, bool first, double& g) {
     const int lane = threadIdx.x & 31, h = lane >> 4, hl = lane & 15;
     const bool grad = hl >= 12;
     const int b = grad ? 0 : hl / 3, q = hl % 3;
@@ -1147,7 +1340,7 @@ __device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable&
     const int turns = (i1 - i0 + 16 * nh - 1) / (16 * nh);  // the same for all of the row's half-warps
     auto incidence = [&](int t) -> uint32_t {
         const int i = i0 + nh * (16 * t + hl) + hw;
-        return i < i1 ? __ldg(a.inc + i) : ~0u;
+        return i < i1 ? __ldg(list + i) : ~0u;
     };
     // a turn's pair is read while the sums of the turn before run
     double2 f[8];
@@ -1211,7 +1404,7 @@ __device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable&
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const int c = vert[k];
-                if (c < max(lo, v) || c >= hi) continue;  // upper blocks only
+                if (c < lo || c >= hi) continue;
                 unsigned x = ((unsigned)c * 2654435761u) >> 24;
                 while (T.hash[x] != c) x = (x + 1) & (kRowHash - 1);
                 u[k] = T.rank[x];
@@ -1262,14 +1455,14 @@ __device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable&
         for (int i = i0 + hw; i - hw < i1; i += nh) {  // the same turns in both halves
             int w[4], item = 0, la = 0, ty = -1, d = -1;
             double x[3] = {0.0, 0.0, 0.0};
-            if (i < i1) ty = inc_pair(a, __ldg(a.inc + i), w, item, la);
+            if (i < i1) ty = inc_pair(a, __ldg(list + i), w, item, la);
             if (ty >= 0 && (ty & kPairApart) && hl < 15) {
                 const int base = ty & ~kPairApart;
                 const double *m = a.cs.fac + kFac * (size_t)item, *m2 = a.cs.fac2 + kFac * (size_t)item;
                 const int c = w[b];
                 if (grad) {
                     if (first) g += pair_grad(base, m, m2, la, q);
-                } else if (c >= max(lo, v) && c < hi) {
+                } else if (c >= lo && c < hi) {
                     unsigned s = ((unsigned)c * 2654435761u) >> 24;
                     while (T.hash[s] != c) s = (s + 1) & (kRowHash - 1);
                     d = 9 * T.rank[s] + q;
@@ -1288,14 +1481,11 @@ __device__ __forceinline__ void row_accumulate(const RowArgs& a, const RowTable&
     __syncwarp();
 }
 
-// stores the window's upper blocks (threads t of nt), acc summed over the row's warps in order, and
-// the columns of both lists
+// stores the upper blocks of the table's columns nlow .. U - 1 (threads t of nt) from place `up` on, acc
+// summed over the row's warps in order
 template <bool kCta>
-__device__ __forceinline__ void row_store(const RowArgs& a, const RowOut& o, const RowTable& T, const RowWarp* W, int v,
-                                          int U, int t, int nt, unsigned& up, unsigned& low) {
-    int nlow = 0;
-    for (int k = 0; k < U; k++) nlow += T.col[k] < v;
-    for (int u = t; u < nlow; u += nt) o.cl_col[low + u] = T.col[u];
+__device__ __forceinline__ void row_store(const RowOut& o, const RowTable& T, const RowWarp* W, int v, int nlow, int U,
+                                          int t, int nt, size_t up) {
     const bool fixed_row = o.btype && o.btype[v] != 0;
     for (int e = 9 * nlow + t; e < 9 * U; e += nt) {
         const int u = e / 9, q = e % 9, c = T.col[u];
@@ -1312,8 +1502,6 @@ __device__ __forceinline__ void row_store(const RowArgs& a, const RowOut& o, con
             o.uc_col[k] = c;
         }
     }
-    up += U - nlow;
-    low += nlow;
 }
 
 __global__ void __launch_bounds__(32 * kRowWarps, kRowCtas) k_row_sums(RowArgs a, RowOut o) {
@@ -1329,62 +1517,77 @@ __global__ void __launch_bounds__(32 * kRowWarps, kRowCtas) k_row_sums(RowArgs a
         o.cl_ptr[i] = (int)(f >> 32);
         if (i == a.n) o.nuc[0] = (int)(f & 0xffffffffull);
     }
-    for_rows(
-        a,
-        [&](int v) {
-            RowTable& T = tables[0];
-            const int i0 = a.ptr[v], i1 = a.ptr[v + 1];
-            unsigned up = (unsigned)(o.uoff[v] & 0xffffffffull), low = (unsigned)(o.uoff[v] >> 32);
-            double g = 0.0;
-            bool first = true;
-            int lo = 0, hi = a.n;
-            while (lo < a.n) {
-                if (!row_columns<true>(a, T, i0, i1, lo, hi, threadIdx.x, 32 * kRowWarps)) {
-                    hi = lo + (hi - lo + 1) / 2;
-                    continue;
-                }
-                row_ranks<true>(T, threadIdx.x, 32 * kRowWarps);
-                row_accumulate(a, T, warps[w], v, T.used, i0, i1, hw, 2 * kRowWarps, lo, hi, first, g);
-                __syncthreads();
-                row_store<true>(a, o, T, warps, v, T.used, threadIdx.x, 32 * kRowWarps, up, low);
-                __syncthreads();
-                first = false;
-                lo = hi;
-                hi = a.n;
+    // a row, or a window of a split one (win), by nt threads: its blocks, the columns of its transposed
+    // list and its gradient
+    auto make = [&](auto cta, RowTable& T, RowWarp* W, int t, int nt, int v, const RowWindow* win) {
+        constexpr bool kCta = decltype(cta)::value;
+        int i0, i1, lo, hi, nlow = 0;
+        size_t up = (size_t)(o.uoff[v] & 0xffffffffull);
+        const int low = (int)(o.uoff[v] >> 32);
+        const uint32_t* list = a.inc;
+        bool first = true;
+        if (win) {
+            first = win->first == 0;
+            if (!first) list = a.wlist;
+            i0 = win->i0;
+            i1 = i0 + win->len;
+            window_table<kCta>(a, T, win->c0, win->cols, t, nt);
+            lo = T.col[0];
+            hi = T.col[T.used - 1] + 1;
+            up += win->first;
+            if (first) {
+                const int n = (int)(o.uoff[v + 1] >> 32) - low;
+                for (int k = t; k < n; k += nt) o.cl_col[low + k] = a.wcol[win->c0 - n + k];
             }
+        } else {
+            i0 = a.ptr[v];
+            i1 = a.ptr[v + 1];
+            row_columns<kCta>(a, T, i0, i1, t, nt);
+            row_ranks<kCta>(T, t, nt);
+            lo = v;  // upper blocks only
+            hi = a.n;
+            nlow = (int)(o.uoff[v + 1] >> 32) - low;
+            for (int k = t; k < nlow; k += nt) o.cl_col[low + k] = T.col[k];
+        }
+        double g = 0.0;
+        row_accumulate(a, list, T, W[kCta ? w : 0], v, T.used, i0, i1, kCta ? hw : (hw & 1), kCta ? 2 * kRowWarps : 2, lo,
+                       hi, first, g);
+        row_sync<kCta>();
+        row_store<kCta>(o, T, W, v, nlow, T.used, t, nt, up);
+        if (kCta) {
             if (hl >= 12 && hl < 15) s_grad[hw][hl - 12] = g;
             __syncthreads();
-            if (threadIdx.x < 3) {
+            if (first && threadIdx.x < 3) {
                 double s = s_grad[0][lane];
 #pragma unroll
                 for (int k = 1; k < 2 * kRowWarps; k++) s += s_grad[k][lane];
                 o.grad[3 * (size_t)v + lane] += s;
             }
-            __syncthreads();
-        },
-        [&](int v) {
-            RowTable& T = tables[w];
-            const int i0 = a.ptr[v], i1 = a.ptr[v + 1];
-            unsigned up = (unsigned)(o.uoff[v] & 0xffffffffull), low = (unsigned)(o.uoff[v] >> 32);
-            double g = 0.0;
-            bool first = true;
-            int lo = 0, hi = a.n;
-            while (lo < a.n) {
-                if (!row_columns<false>(a, T, i0, i1, lo, hi, lane, 32)) {
-                    hi = lo + (hi - lo + 1) / 2;
-                    continue;
-                }
-                row_ranks<false>(T, lane, 32);
-                row_accumulate(a, T, warps[w], v, T.used, i0, i1, lane >> 4, 2, lo, hi, first, g);
-                row_store<false>(a, o, T, warps + w, v, T.used, lane, 32, up, low);
-                __syncwarp();
-                first = false;
-                lo = hi;
-                hi = a.n;
-            }
+        } else {
             g += __shfl_down_sync(0xffffffffu, g, 16);  // the halves in list order
-            if (lane >= 12 && lane < 15) o.grad[3 * (size_t)v + lane - 12] += g;
-        });
+            if (first && lane >= 12 && lane < 15) o.grad[3 * (size_t)v + lane - 12] += g;
+        }
+        row_sync<kCta>();
+    };
+    const int n_short = a.cnt[kRowsShort], n_long = a.cnt[kRowsLong];
+    const int w_short = a.cnt[kWinShort], w_long = a.cnt[kWinLong];
+    for (int k = blockIdx.x; k < w_long + n_long; k += gridDim.x) {
+        const RowWindow* win = k < w_long ? a.win + (a.win_cap - 1 - k) : nullptr;
+        const int v = win ? win->v : a.list[(size_t)a.n + k - w_long];
+        if (v >= 0) make(std::true_type{}, tables[0], warps, threadIdx.x, 32 * kRowWarps, v, win);
+    }
+    __syncthreads();
+    // Short lists go to whichever warp is free, the next one fetched ahead: the kernel runs beside the static
+    // scatter, and CTAs that find their place late had held up a fixed share of the rows (rolled
+    // cloth: from 950 to 1500 us).
+    auto next = [&]() { return lane == 0 ? atomicAdd(a.cnt + kRowNext, 1) : 0; };
+    for (int k = __shfl_sync(0xffffffffu, next(), 0); k < n_short + w_short;) {
+        const int ahead = next();
+        const RowWindow* win = k < n_short ? nullptr : a.win + (k - n_short);
+        const int v = win ? win->v : a.list[k];
+        if (v >= 0) make(std::false_type{}, tables[w], warps + w, lane, 32, v, win);
+        k = __shfl_sync(0xffffffffu, ahead, 0);
+    }
 }
 
 // The transposed copies: block u = (r, c), r < c, goes to the place of column r in c's list.  A copy,
@@ -1822,16 +2025,25 @@ static SgipcStatus merge_contacts(SgipcCtx* c, const ContactCounts& cc, int sing
         SG_CHECK(c, cudaMemsetAsync(c->cl_ptr, 0, sizeof(int) * (n + 1), s));
         return SGIPC_OK;
     }
-    SG_COUNT(c, 4);
-    SG_CHECK(c, cudaMemsetAsync(c->row_cnt, 0, 2 * sizeof(int), s));
+    SG_COUNT(c, 5);
+    SG_CHECK(c, cudaMemsetAsync(c->row_cnt, 0, kRowCounts * sizeof(int), s));
     size_t tb = c->cub_tmp_bytes;
     SG_CHECK(c, cub::DeviceRadixSort::SortPairs(c->cub_tmp, tb, c->con_key, c->con_key_s, c->con_val, c->con_val_s, m,
                                                 0, c->key_bits, s));
     k_inc_rows<<<nblk(n + 1), SGIPC_BLOCK, 0, s>>>(n, m, c->con_key_s, c->inc_ptr, c->row_list, c->row_cnt, c->ucnt);
-    const RowArgs a{contact_store(c, cc), c->con_val_s, c->inc_ptr, c->row_list, c->row_cnt, n};
+    // The split's scratch lies in the transposed blocks' values, which are written last: 72 bytes for each
+    // of a pair's ten block slots, against 32 for each of its four incidences.  (A split row has at least
+    // 14 incidences and no more than 3 len / 40 + 1 windows: a sixth of its incidences bounds them.)
+    int* wcol = reinterpret_cast<int*>(c->cl64);
+    uint32_t* wlist = reinterpret_cast<uint32_t*>(wcol + 4 * (size_t)m);
+    RowWindow* win = reinterpret_cast<RowWindow*>(wlist + 3 * (size_t)m);
+    static_assert(sizeof(RowWindow) == 24 && 7 * 4 + 24 / 6 <= 32, "the scratch fits");
+    const RowArgs a{contact_store(c, cc), c->con_val_s, c->inc_ptr, c->row_list, c->row_cnt, n, wcol, wlist, win,
+                    m / 6 + 1};
     // (the grids cover the chip once)
     const int most = nblk(m, 8);  // no more CTAs than a small call has work for
     k_row_counts<<<std::min(most, 148 * 8), 32 * kRowWarps, 0, s>>>(a, c->ucnt);
+    k_row_split<<<std::min(most, 148 * 4), 32 * kSplitWarps, 0, s>>>(a, c->ucnt);
     tb = c->cub_tmp_bytes;
     SG_CHECK(c, cub::DeviceScan::ExclusiveSum(c->cub_tmp, tb, c->ucnt, c->uoff, n + 1, s));
     const RowOut o{c->uoff, btype, c->nuc, c->cu_ptr, c->cl_ptr, c->uc_row, c->uc_col, c->uc64, c->uc32, c->cl_col,

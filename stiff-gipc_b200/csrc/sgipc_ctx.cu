@@ -332,7 +332,7 @@ extern "C" SgipcStatus sgipc_create(const SgipcTopology* t_in, int device, Sgipc
         (st = dalloc(c, &c->con_sval, 9 * ns)) || (st = dalloc(c, &c->con_key, ninc)) ||
         (st = dalloc(c, &c->con_val, ninc)) || (st = dalloc(c, &c->con_key_s, ninc)) ||
         (st = dalloc(c, &c->con_val_s, ninc)) || (st = dalloc(c, &c->inc_ptr, (size_t)n + 1)) ||
-        (st = dalloc(c, &c->row_list, 2 * (size_t)n)) || (st = dalloc(c, &c->row_cnt, 2)) ||
+        (st = dalloc(c, &c->row_list, 3 * (size_t)n)) || (st = dalloc(c, &c->row_cnt, 8)) ||
         (st = dalloc(c, &c->ucnt, (size_t)n + 1)) || (st = dalloc(c, &c->uoff, (size_t)n + 1)) ||
         (st = dalloc(c, &c->part_a, cap + 1)) || (st = dalloc(c, &c->part_f, cap + 1)) ||
         (st = dalloc(c, &c->nuc, 4)) || (st = dalloc(c, &c->uc_row, cap)) || (st = dalloc(c, &c->uc_col, cap)) ||

@@ -184,8 +184,8 @@ struct SgipcCtx {
     uint32_t* con_key_s;          // sorted by vertex
     uint32_t* con_val_s;
     int* inc_ptr;                 // [n+1] incidences of each vertex
-    int* row_list;                // [2n] vertices with short lists, and with long ones
-    int* row_cnt;                 // [2] their numbers
+    int* row_list;                // [3n] vertices with short lists, with long ones, and rows to split
+    int* row_cnt;                 // [8] their numbers, and those of the split rows' windows (RowCount)
     unsigned long long* ucnt;     // [n+1] unique blocks per row: upper ones, transposed ones << 32
     unsigned long long* uoff;     // their exclusive scan
     int* part_a;                  // [cap+1] flags and places of the class partition

@@ -1,7 +1,7 @@
 """Rows of the contact matrix against the oracle's assembly, at the sizes where the row kernels
 change: a warp or a CTA per row (128 incidences), windows of 40 columns, batches of 16 pairs a
 half-warp, every pair kind (mollified ones included) and
-rows of fixed vertices.
+rows of fixed vertices; and rows of thousands of columns, which are split.
 
 The pairs are synthetic (random vertices of two small cubes, d-hat wider than the scene), so a row
 can be given any length.  Tolerance: the same products in 64 bits, summed in another order; a row
@@ -135,3 +135,82 @@ def test_transposed_blocks_are_exact_copies():
     off = block[:, None] != block
     assert torch.equal(A[off], A.T[off])
     g.close()
+
+
+def _wide(rng, nv, hub, columns, fan):
+    """Pairs that give `hub` about `columns` other columns: `fan` of them three or four at a time with
+    the same two neighbours (a corner of a large triangle), the rest alone; and some of each twice."""
+    other = np.setdiff1d(rng.permutation(nv), [hub])
+    rng.shuffle(other)
+    a, b = other[:2]
+    far = other[2:columns]
+    out = [(-w - 1, hub, a, b) for w in far[:fan]] + [(-hub - 1, w, -1, -1) for w in far[fan:]]
+    out += [(-w - 1, hub, a, -1) for w in far[::7]] + [(hub, a, b, w) for w in far[::11]] + [(-a - 1, b, -1, -1)]
+    return np.asarray(out, np.int32)[rng.permutation(len(out))]
+
+
+@pytest.mark.parametrize("n,columns,fan,hub", [(10, 44, 20, 0.5), (10, 90, 0, 0.0), (10, 999, 600, 1.0),
+                                               (18, 5000, 2500, 0.3), (18, 5830, 0, 0.0), (34, 39300, 3000, 0.0),
+                                               (34, 39300, 0, 0.05)])
+def test_split_rows_match_the_oracle(n, columns, fan, hub):
+    """Rows of up to 39 300 columns (983 windows: more than are listed at a time), the hub's columns
+    above it, below it or both; same blocks, gradient and product as the oracle's."""
+    rng = np.random.default_rng(columns + fan)
+    sc = scenes.scene_cube(n, seed=4)
+    pairs = _wide(rng, sc.nv, int(hub * (sc.nv - 1)), columns, fan)
+    btype = sc.boundary_type.copy()
+    btype[rng.choice(sc.nv, 20, replace=False)] = 1
+    sc = dataclasses.replace(sc, pairs=pairs, boundary_type=btype, params=dict(sc.params, dHat=0.2, kappa=1.0))
+    g = system.GIPC(sc, max_rhs=1)
+    g.computeGradientAndHessian()
+    rows, cols, vals = g.export_bcoo()
+    b, orow, ocol, oval, _ = oracle.assemble(sc)
+    assert np.array_equal(rows, orow) and np.array_equal(cols, ocol)
+    assert np.abs(vals - oval).max() <= 1e-9 * np.abs(oval).max()
+    assert np.abs(g.rhs().cpu().numpy() - b).max() <= 1e-9 * np.abs(b).max()
+    x = rng.normal(size=3 * sc.nv)
+    ref = oracle.spmv(orow, ocol, oval, sc.nv, x)
+    assert np.abs(g.spmv(torch.tensor(x, device="cuda")).cpu().numpy() - ref).max() <= 1e-9 * np.abs(ref).max()
+    g.computeGradientAndHessian()
+    assert np.array_equal(g.export_bcoo()[2], vals)
+    g.close()
+
+
+def test_split_rows_of_a_mesh_beyond_the_bitmap():
+    """More vertices than the bitmap of a split has columns (2^18): a hub whose columns lie on both sides
+    of that line, windows across it."""
+    sc = scenes.scene_cloth_on_sphere(520, 300, contacts=False)
+    assert sc.nv > 1 << 18
+    rng = np.random.default_rng(1)
+    hub = sc.nv - 3000
+    w = np.sort(np.concatenate([rng.choice((1 << 18) - 1, 2000, replace=False),
+                                rng.choice(np.arange(1 << 18, hub), 700, replace=False), np.arange(hub + 1, sc.nv, 2)]))
+    pairs = np.stack([-hub - 1 + 0 * w, w, -1 + 0 * w, -1 + 0 * w], 1).astype(np.int32)[rng.permutation(len(w))]
+    sc = dataclasses.replace(sc, pairs=pairs, ground_pairs=sc.ground_pairs[:0], params=dict(sc.params, dHat=4.0, kappa=1.0))
+    assert ((sc.vertexes[w] - sc.vertexes[hub]) ** 2).sum(1).max() < 4.0
+    g = system.GIPC(sc, max_rhs=1)
+    g.computeGradientAndHessian()
+    base = dataclasses.replace(sc, pairs=pairs[:0])
+    g0 = system.GIPC(base, max_rhs=1)
+    g0.computeGradientAndHessian()
+    grad = (g.rhs() - g0.rhs()).cpu().numpy().reshape(-1, 3)
+    e = torch.zeros(3 * sc.nv, dtype=torch.float64, device="cuda")
+    X, R = sc.vertexes.reshape(-1), sc.rest_vertexes.reshape(-1)
+    want = np.zeros((sc.nv, 3, 3))  # the hub's rows of the contact matrix, by column vertex
+    gw = np.zeros((sc.nv, 3))
+    for p in pairs:
+        vid, _, gr, H = oracle.barrier_pair(p, X, R, 4.0, 1.0)
+        for a, va in enumerate(vid):
+            gw[va] += gr[3 * a:3 * a + 3]
+        k = list(vid).index(hub)
+        for a, va in enumerate(vid):
+            want[va] += H[3 * k:3 * k + 3, 3 * a:3 * a + 3]
+    for q in range(3):
+        e.zero_()
+        e[3 * hub + q] = 1.0
+        col = (g.spmv(e) - g0.spmv(e)).cpu().numpy().reshape(-1, 3)  # A e: entry (vertex, p) of column (hub, q)
+        assert np.abs(col - want[:, q, :]).max() <= 1e-9 * np.abs(want).max()
+    free = sc.boundary_type == 0
+    assert np.abs(np.abs(grad[free]) - np.abs(gw[free])).max() <= 1e-9 * np.abs(gw).max()
+    g.close()
+    g0.close()
