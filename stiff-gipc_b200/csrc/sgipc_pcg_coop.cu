@@ -2158,11 +2158,15 @@ SgipcStatus run_pcg_coop(SgipcCtx* c, PcgWork& w, int fp32_mas, const double* b,
     const char* fz = getenv("SGIPC_PCG_FUSED");
     SgipcCtx::CoopCfg& fcfg = c->fused_cfg[inst];
     bool fused = false;
-    // (FP64 vectors with four right-hand sides measured slower fused: kept four-phase)
+    // FP64 vectors with four right-hand sides take the four-phase iteration (the fused grid form measured
+    // slower) but for the smallest cluster form, 16 rows a CTA: 128 and 250 rows 1668 and 1848 us against
+    // 1867 and 2069, with 32 rows a CTA (432) 2388 against 2312, with 128 (1458, 2000)
+    // 3223 and 3775 against 2462 and 2898.  The others are 1.02 to 1.44 times faster on the cluster.
+    const bool wide = sizeof(T) == 8 && sizeof(M) == 8 && NR == 4;
     // (a caller's wait limit needs barriers that can run out: not the cluster form's)
     SgipcCtx::CoopCfg& scfg = c->small_cfg[inst];
     bool cluster = false;
-    if (L >= 3 && !(fz && fz[0] == '0')) {
+    if (L >= 3 && !(fz && fz[0] == '0') && (!wide || c->n <= kClusterCtas * kClusterMinRows)) {
         if (!scfg.valid) {
             SgipcStatus st = fused_configure<T, M, NR, true>(c, scfg);
             if (st != SGIPC_OK) return st;
@@ -2170,7 +2174,7 @@ SgipcStatus run_pcg_coop(SgipcCtx* c, PcgWork& w, int fp32_mas, const double* b,
         cluster = scfg.usable && c->wait_limit == 0;
         fused = cluster;
     }
-    if (!cluster && L >= 3 && !(fz && fz[0] == '0') && !(sizeof(T) == 8 && sizeof(M) == 8 && NR == 4)) {
+    if (!cluster && L >= 3 && !(fz && fz[0] == '0') && !wide) {
         if (!fcfg.valid) {
             SgipcStatus st = fused_configure<T, M, NR, false>(c, fcfg);
             if (st != SGIPC_OK) return st;
