@@ -934,12 +934,14 @@ extern "C" SgipcStatus sgipc_build_cp(SgipcCtx* c, const double* x, const double
             k_boxes<<<tri_nodes + edge_nodes, kNodeLeaves, 0, s>>>(x, surf->faces, nf, surf->edges, ne, tri_nodes,
                                                                    w.val_s, gap, w.d_counts, w.leaf, w.group, w.node);
         }
-        SG_COUNT(c, 2);
         const int tri_chunks = nblk(tri_nodes, 32);
         const long long warps = (long long)edge_groups * nblk(edge_nodes, 32) +
                                 (long long)point_groups * (tri_chunks > 1 ? tri_chunks : 1);
-        k_items<<<nblk(warps, kQueryWarps), 32 * kQueryWarps, 0, s>>>(qa);
-        k_query<<<148 * kQueryCtas, 32 * kQueryWarps, 0, s>>>(qa);
+        if (warps > 0) {  // (none with triangles alone: no points, no edges, nothing to search with)
+            SG_COUNT(c, 2);
+            k_items<<<nblk(warps, kQueryWarps), 32 * kQueryWarps, 0, s>>>(qa);
+            k_query<<<148 * kQueryCtas, 32 * kQueryWarps, 0, s>>>(qa);
+        }
     }
     SG_CHECK(c, cudaMemcpyAsync(w.h_counts, w.d_counts, sizeof(unsigned) * kCntNum, cudaMemcpyDeviceToHost, s));
     SG_CHECK(c, cudaStreamSynchronize(s));

@@ -225,3 +225,39 @@ def test_pairs_of_loose_triangles(kind, n):
         with pytest.raises(Exception, match="capacity"):
             g.buildCP(update=False, capacity=len(p) - 1)
     g.close()
+
+
+@pytest.mark.parametrize("points,tris,edges", [(0, 1, 1), (1, 0, 1), (1, 1, 0), (1, 0, 0), (0, 1, 0), (0, 0, 1), (0, 0, 0)])
+def test_surfaces_with_empty_lists(points, tris, edges):
+    """Each list of the surface empty or not: the pairs that the rest gives, as the host generator finds
+    them; without surface points the scene has no bounds, which is an input error (not a launch of
+    no CTAs) and leaves the context usable."""
+    from sgipc import _native as N
+
+    sc = scenes.scene_two_cubes(7, seed=5)
+    few = scenes.Scene(**{**sc.__dict__})
+    if not points:
+        few.surf_verts = sc.surf_verts[:0]
+    if not tris:
+        few.surf_tris = sc.surf_tris[:0]
+    if not edges:
+        few.surf_edges = sc.surf_edges[:0]
+    g = system.GIPC(sc, pair_capacity=4 * len(sc.pairs))
+    g.scene = few
+    if points:
+        out = g.buildCP(update=False)
+        pairs, ccd = contacts.find_pairs(few.vertexes, few.rest_vertexes, few.surf_tris, few.surf_edges, few.surf_verts,
+                                         few.params["dHat"], few.body_of_vertex, with_ccd=True)
+        assert len(out["pairs"]) == len(pairs) and (len(pairs) > 0) == bool(tris or edges)
+        if len(pairs):
+            assert np.array_equal(_rows_sorted(out["pairs"].cpu().numpy(), out["ccd_pairs"].cpu().numpy()),
+                                  _rows_sorted(pairs, ccd))
+        ground = contacts.ground_pairs(few.vertexes, few.surf_verts, few.params["dHat"], few.params["ground_offset"])
+        assert np.array_equal(out["ground_pairs"].cpu().numpy(), ground)
+    else:
+        with pytest.raises(N.SgipcError) as e:
+            g.buildCP(update=False)
+        assert e.value.status == N.BAD_INPUT
+    g.scene, g._surf = sc, None
+    assert g.buildCP(update=False)["cp_num"][0] == len(sc.pairs)
+    g.close()
