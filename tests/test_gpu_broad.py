@@ -261,3 +261,40 @@ def test_surfaces_with_empty_lists(points, tris, edges):
     g.scene, g._surf = sc, None
     assert g.buildCP(update=False)["cp_num"][0] == len(sc.pairs)
     g.close()
+
+
+@pytest.mark.parametrize("which", ["edges", "points"])
+def test_more_group_pairs_than_the_list_holds(which):
+    """The search lists 64 meeting pairs of groups per query group and 1024 more, and searches what finds no
+    room on the spot.  Here nearly every two groups meet: segments (or triangles) that run from one
+    octant into the opposite one, 150 groups of edges (11 325 pairs for 10 624 places), or 32 groups of
+    points against 110 of triangles (3520 for 3072)."""
+    rng = np.random.default_rng(3)
+    n = 2400  # vertices in each octant
+    a, b = rng.uniform(0.01, 0.03, (n, 3)), rng.uniform(-0.03, -0.01, (n, 3))
+    tris = np.stack([rng.integers(n, size=3520), n + rng.integers(n, size=3520), n + rng.integers(n, size=3520)], 1)
+    tris = tris[tris[:, 1] != tris[:, 2]]
+    v, t = scenes.lattice_tets(2, 0.01, (0.5, scenes.GROUND_OFFSET + 0.5, 0.5))
+    verts = np.concatenate([a, b]) + np.array([0.0, scenes.GROUND_OFFSET + 0.1, 0.0])
+    sc = scenes.build_tet_scene("crossing", [dict(verts=v, tets=t, E=1e5), dict(verts=verts, tris=tris, affine=True)],
+                                dt=0.01, dhat_abs=1e-5, density=1000.0, nu=0.4, mu_friction=0.0, seed=1, perturb=0.0)
+    few = scenes.Scene(**{**sc.__dict__})
+    first = len(v)
+    if which == "edges":
+        few.surf_tris, few.surf_verts = sc.surf_tris[:0], first + np.arange(32)
+        e = np.unique(np.stack([rng.integers(n, size=4900), n + rng.integers(n, size=4900)], 1), axis=0)[:4800]
+        few.surf_edges = first + rng.permutation(e)
+    else:
+        few.surf_tris, few.surf_edges = first + tris, sc.surf_edges[:0]
+        few.surf_verts = first + rng.permutation(2 * n)[:1024]
+    pairs, ccd = contacts.find_pairs(few.vertexes, few.rest_vertexes, few.surf_tris, few.surf_edges, few.surf_verts,
+                                     few.params["dHat"], few.body_of_vertex, with_ccd=True)
+    assert len(pairs) > 100
+    g = system.GIPC(sc, pair_capacity=len(pairs))
+    g.scene = few
+    out = g.buildCP(update=False)
+    assert np.array_equal(_rows_sorted(out["pairs"].cpu().numpy(), out["ccd_pairs"].cpu().numpy()),
+                          _rows_sorted(pairs, ccd))
+    again = g.buildCP(update=False)
+    assert torch.equal(again["pairs"], out["pairs"]) and torch.equal(again["mat_index"], out["mat_index"])
+    g.close()
