@@ -117,7 +117,6 @@ struct MasWork {
     int* h_info_pinned;      // [32] pinned landing area of the level counts (and [21]: abort)
     int* hier_part;          // [32] chunk totals of the fused hierarchy kernel's scan
     int hier_grid;           // CTAs of the fused hierarchy kernel (0: per-level kernels), -1 unset
-    int hier_grid_many;      // ... with many contact pairs
     int hier_pending;
     const void* hier_pairs;
     int hier_pair_num;

@@ -589,11 +589,10 @@ constexpr int kHierThreads = 256;
 constexpr int kHierMaxCtas = 296;      // the largest grid the build may take (hier_part size)
 // its grid beside the assembly (SGIPC_HIER_CTAS overrides): measured on the two-cube bench step,
 // the MAS build ends at 0.41 ms with 32 CTAs, 0.36 ms with 74 and 0.41 ms with 148 (the
-// assembly's kernels then lose their SMs)
+// assembly's kernels then lose their SMs).  Rolled cloths of 51 000 to 978 000 pairs the same: assembly
+// and MAS build 280, 412, 620, 894, 1211 and 2136 us with 74 CTAs (51, 132, 244, 385, 548 and 978
+// thousand pairs), 338, 483, 692, 977, 1283 and 2224 with 296, between them with 148.
 constexpr int kHierDefaultCtas = 74;
-// ... and with this many pairs or more: a chip's worth of threads for the pairs' gathers, which
-// then take longer than the assembly beside them (one 256^2 rolled cloth: a million pairs)
-constexpr int kHierManyPairs = 200000;
 constexpr long long kHierSpinLimit = 1LL << 24;
 
 struct HierArgs {
@@ -892,7 +891,6 @@ SgipcStatus mas_create(SgipcCtx* c, const SgipcTopology* t) {
         const char* e = getenv("SGIPC_HIER_CTAS");
         if (e && atoi(e) > 0) want = atoi(e) < kHierMaxCtas ? atoi(e) : kHierMaxCtas;
         m.hier_grid = coop && per > 0 ? (nsm * per < want ? nsm * per : want) : 0;
-        m.hier_grid_many = e ? m.hier_grid : (nsm * per < kHierMaxCtas ? nsm * per : kHierMaxCtas);
     }
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, m.bank_cnt, m.bank_off, m.npos / 16 + 2);
@@ -953,8 +951,8 @@ static SgipcStatus mas_hierarchy(SgipcCtx* c, const SgipcContacts* con, cudaStre
         SG_CHECK(c, cudaMemsetAsync(m.info + 20, 0, 2 * sizeof(int), s));
         void* args[] = {&h};
         SG_COUNT(c, 1);
-        const int grid = h.npairs >= kHierManyPairs ? m.hier_grid_many : m.hier_grid;
-        SG_CHECK(c, cudaLaunchCooperativeKernel((const void*)k_hierarchy, dim3(grid), dim3(kHierThreads), args, 0, s));
+        SG_CHECK(c, cudaLaunchCooperativeKernel((const void*)k_hierarchy, dim3(m.hier_grid), dim3(kHierThreads), args,
+                                                0, s));
         SG_CHECK(c, cudaMemcpyAsync(m.h_info_pinned, m.info, sizeof(int) * 22, cudaMemcpyDeviceToHost, s));
         return SGIPC_OK;
     }
