@@ -156,7 +156,8 @@ const char* sgipc_last_error(const SgipcCtx* ctx);
  * out raises the kernel's abort word, every CTA leaves, and the call returns
  * SGIPC_CUDA_ERROR with a message, the context staying usable.  A watchdog for hosts that
  * must bound a call's time; 1 makes nearly every wait run out.  (Without a limit, solves of up
- * to 2048 rows run on one thread-block cluster, whose hardware barrier needs none.) */
+ * to 2048 rows, 256 for a batch in FP64, run on one thread-block cluster, whose hardware
+ * barrier needs none.) */
 SgipcStatus sgipc_set_wait_limit(SgipcCtx* ctx, int64_t polls);
 
 /* ---- assembly (GIPC::computeGradientAndHessian, StiffGIPC/GIPC.cu:10110-10344) -------- */

@@ -896,8 +896,10 @@ __global__ void k_soft(int ns, const uint32_t* __restrict__ idx, const double* _
 // cloth) is split into windows of kRowCols columns, each with the list of the pairs that have one
 // there, and the windows are summed as rows are: the work stays in proportion to the list.
 constexpr int kRowWarps = 4;
-// incidences above which a CTA takes the row (rolled cloth, a third of whose rows are longer: the
-// Newton system takes 8 % longer with 64, 5 % with 413, where k_row_counts goes from 159 to 352 us)
+// incidences above which a CTA takes the row.  Newton step of rolled cloths with 244, 548 and 978 thousand
+// pairs: 1125, 2304 and 3294 us with 64, 1073, 2190 and 3075 with 128, 1064, 2142 and 2961 with 256,
+// 1070, 2137 and 2946 with 512; two 21^3 cubes, whose longest rows are these: k_row_counts 7.0, 7.6, 11.5
+// and 11.4 us, k_row_sums 36.6, 41.4, 42.1 and 44.6.
 constexpr int kRowLong = 128;
 constexpr int kRowHash = 256;
 constexpr int kRowCols = 40;   // columns of a window (each of 32 * kRowWarps lanes may add one more)
@@ -2527,7 +2529,8 @@ SgipcStatus assemble_time_hook(SgipcCtx* c, const char* name, cudaStream_t s, do
         *bytes = (double)(10LL * c->nt + 6LL * c->nf) * 72 + 80.0 * c->nh + 4.0 * c->n_eblk +
                  (double)c->nnz * (28 + 72 + 108) + (double)(c->nnz - c->n) * 108;
     } else if (!strcmp(name, "barrier") || !strcmp(name, "friction")) {
-        // one kind's launch (its factors and keys are rewritten with the same values)
+        // one kind's launch, into the places of the first pairs (the factors and keys are scratch: every
+        // assembly writes them anew before it reads them)
         if (!k) return SGIPC_BAD_INPUT;
         const bool fric = name[0] == 'f';
         SgipcContacts only = *k;

@@ -70,7 +70,7 @@ using namespace sgipc;
 
 namespace {
 
-constexpr int kCellBits = 21;
+constexpr int kSpanBits = 21;  // a scene's extent over its largest primitive's, at most
 constexpr int kGroupBits = 21;  // packed rank fields: three 21-bit counters in one 64-bit word
 constexpr int kQueryWarps = 4;
 constexpr int kQueryCtas = 4;  // per SM (128 registers a thread)
@@ -150,7 +150,7 @@ __device__ int scene_error(const unsigned long long* bounds, double gap) {
 #pragma unroll
     for (int q = 0; q < 3; q++) {
         const double lo = unord(bounds[q]), hi = unord(bounds[3 + q]);
-        if (!(hi >= lo) || (hi - (lo - gap - h)) / h + 2.0 >= (double)(1 << kCellBits)) bad = 1;
+        if (!(hi >= lo) || (hi - (lo - gap - h)) / h + 2.0 >= (double)(1 << kSpanBits)) bad = 1;
     }
     return bounds[7] ? 2 : bad;
 }
@@ -955,8 +955,9 @@ extern "C" SgipcStatus sgipc_build_cp(SgipcCtx* c, const double* x, const double
         return SGIPC_BAD_INPUT;
     }
     if (h[kCntBad]) {
-        snprintf(c->err, sizeof(c->err), "build_cp: the scene spans more than 2^%d grid cells along an axis",
-                 kCellBits);
+        snprintf(c->err, sizeof(c->err),
+                 "build_cp: the surface points' bounds are empty, not finite or more than 2^%d times the largest primitive",
+                 kSpanBits);
         return SGIPC_BAD_INPUT;
     }
     if (total > cap || ng > ground_cap) {

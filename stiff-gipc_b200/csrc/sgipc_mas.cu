@@ -424,7 +424,6 @@ __global__ void __launch_bounds__(64, 6) k_invert(int ndom, double* __restrict__
 // ------------------------------------------------------------------------------------------
 namespace sgipc {
 
-// level 0 and level 1 of the restriction: one thread per position
 // what the apply's kernels look at before they do anything: the stop flag of the coupled solve, whose
 // next iteration is enqueued before the last one's outcome is known, or nothing (the flag's test alone
 // cost an apply of a small system 5 %)
@@ -432,6 +431,7 @@ struct NoStop {};
 __device__ __forceinline__ bool stopped(NoStop) { return false; }
 __device__ __forceinline__ bool stopped(const int* stop) { return *stop != 0; }
 
+// level 0 and level 1 of the restriction: one thread per position
 template <class T, class M, class Stop = NoStop>
 __global__ void k_restrict01(int npos, const T* __restrict__ r, const int* __restrict__ part_map,
                              const int* __restrict__ up, M* __restrict__ R, Stop stop = Stop()) {
